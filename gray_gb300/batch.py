@@ -6,7 +6,7 @@ graph, with the kernel variant and persistent-grid size picked by an autotuner.
 
 Per pixel the result is bit-identical to rendering the same view alone with forward_pass_display
 (same ray arithmetic, same traversal and selection); the batch only changes how work is scheduled:
-one launch whose warps pull 32-ray packets of every view from a global counter.  The first render of
+one launch whose blocks pull groups of 2x2 32-ray packets of every view from a global counter.  The first render of
 a batch signature (the scenes and resolutions of its views) autotunes and captures a CUDA graph;
 later renders with the same signature update the camera poses in pinned host memory and replay.
 """

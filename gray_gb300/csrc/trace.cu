@@ -1,22 +1,24 @@
 // trace.cu -- forward and backward ray tracing of the Gaussians on the LBVH.
 //
 // Forward (replaces the OptiX launch of cuda/shaders.cu:69-106 with cuda/forward_pass.cu):
-//   A block renders an 8x16-pixel tile, each warp a 4x8 (or 8x4) pixel packet of camera rays that
-//   share one origin.  A per-tile kernel first walks the top of the BVH with the tile's frustum and
+//   A block renders an 8x16-pixel tile of camera rays that share one origin, each warp a 4x8 (or 8x4)
+//   pixel packet of it.  A per-tile kernel first walks the top of the BVH with the tile's frustum and
 //   records the tile's frontier (the nodes of at most 64 leaves it reaches, sorted front to back);
-//   every packet traversal starts there.  The packet traverses as a frustum: each step pops up to
-//   32 nodes (one per lane) from a per-warp shared-memory stack, tests both child boxes against the
-//   frustum, pushes the nearer child last and queues leaves; queued leaves are culled by an exact
-//   ellipsoid-frustum test, cached in shared memory, tested by every lane against its own ray with a
-//   division-free conservative pretest, and the lanes then walk their masks of possible hits through
-//   the intersection program of cuda/shaders.cu:10-67, which decides each hit.  The first traversal accumulates, over ALL hits, the full transmittance
+//   the block's traversal starts there.  The block traverses as one frustum: each step pops up to
+//   128 nodes (one per thread) from a shared-memory stack, tests both child boxes against the
+//   frustum, pushes the nearer child last and queues leaves.  Queued leaves are taken in batches of
+//   128: culled by an exact ellipsoid-frustum test and cached in shared memory with the conic their
+//   support sphere projects to on the tile's pixels; every ray evaluates the conics at its pixel (a
+//   conservative pretest of five FMAs) and the lanes then walk their masks of possible hits through
+//   the intersection program of cuda/shaders.cu:10-67, which decides each hit.  The first traversal
+//   accumulates, over ALL hits, the full transmittance
 //   (an order-independent fixed-point sum of log(1 - alpha)) and the alpha-weighted colour sums of
 //   the reference's truncated-tail estimate, and every traversal keeps the KB nearest hits above a
 //   resume key in a per-lane shared-memory buffer of 64-bit keys (fp16 distance | gaussian id |
 //   fp16 alpha).  The buffer is consumed by a state machine that reproduces the reference's
 //   32-slot multi-pass selection exactly (pass boundaries, the strict `distance > tmin` drop of
 //   equal distances, the 99-pass cap, zfar, t_threshold).  Composited ids are appended to the
-//   backward hit list in warp-aggregated segments.  Rays from Python, jittered rays and packets
+//   backward hit list in warp-aggregated segments.  Rays from Python, jittered rays and tiles
 //   whose traversal overflows the shared stack take a per-ray slab traversal instead.
 // Backward (cuda/backward_pass.cu:2-142): one thread per pixel walks its segments back to front,
 //   recomputes alpha in fp32 and reduces the 16 per-hit gradient values into the per-Gaussian
@@ -37,9 +39,10 @@ constexpr int kPassSlots = 32;               // BUFFER_SIZE, cuda/forward_pass.c
 constexpr int kMaxPasses = 99;               // MAX_ITERATIONS, cuda/forward_pass.cu:3
 constexpr int kMaxTraversals = 4 * kMaxPasses * 2;  // bound on re-traversals of one ray
 constexpr unsigned kFull = 0xffffffffu;
-constexpr int kWideStack = 256;  // per-warp shared stack of the frustum traversal
-constexpr int kCand = 32;        // leaves processed per flush (one per lane)
-constexpr int kQueue = 3 * kCand; // per-warp queue of leaves: < kCand before a step, + up to 64 per step
+constexpr int kBatch = 128;       // leaves fetched and tested together by a block (one per thread)
+constexpr int kTileStack = 448;   // per-block traversal stack
+constexpr int kTileQueue = kBatch + 2 * kFwdThreads;  // queued leaves: < kBatch before a step, + up to 2 per thread
+static_assert(kBatch == kFwdThreads, "one leaf per thread");
 constexpr int kSchedHeader = 64;  // schedule words before the per-tile estimates
 // Header words [kSchedZeroWords, kSchedHeader) outlive a forward: the automatic kernel choice (see
 // plan_forward) keeps there the packet counts of the last scheduled forward and the choice the scan
@@ -56,8 +59,7 @@ constexpr uint32_t kChoiceNarrow = 1u, kChoiceWide = 2u;
 constexpr uint32_t kWideSixteenths = 2u;
 // Per pixel tile, the BVH frontier its frustum reaches (kFrontierWords words: count, then up to
 // kFrontierMax node or leaf entries); a count of kFrontierNone means "start at the root".  A frontier
-// goes onto the traversal stack, so it leaves room there for the traversal's own pushes (up to 64
-// per step; the stack above a frontier peaks near 70 entries on the benchmark scene).
+// goes onto the traversal stack, so it leaves room there for the traversal's own pushes.
 constexpr int kFrontierWords = GRAY_FRONTIER_WORDS;
 constexpr int kFrontierMax = kFrontierWords - 1;
 constexpr int kFrontierSort = 256;  // sort buffer of the frontier walk (a power of two > kFrontierMax)
@@ -236,14 +238,6 @@ __device__ __forceinline__ void on_leaf(const TraceScene &sc, uint32_t gid, bool
                      rd, k, st, kbuf);
 }
 
-// Per-warp shared-memory copy of the queued leaves' records, filled once per flush by the lanes
-// (one candidate each, all loads in flight together) and read by every lane afterwards.
-struct CandCache {
-    float4 g[kCand][3];  // snapshot rows with the packet's object-space origin: (M | M (o - mu))
-    int4 c[kCand];       // colour in 2^-24 fixed point (x, y, z), live opacity bits (w)
-    float sf[kCand];     // live scaling factor
-};
-
 __device__ __forceinline__ void stack_push(uint32_t &stk0, uint32_t &stk1, int &sp, uint32_t v, int lane,
                                            int32_t *status) {
     if (sp < kStackMax) {
@@ -356,207 +350,337 @@ __device__ __forceinline__ bool frustum_ellipsoid(const Frustum &fr, const float
     return true;
 }
 
-// Processes the packet's queued leaves (cand[0, nc), at most kCand = 32; every lane of the warp calls
-// this together).  (1) Lane j takes candidate j: it tests the candidate's ellipsoid against the
-// packet frustum and fetches its snapshot rows, live values and colour; the survivors are
-// compacted into the warp's shared-memory cache, each with its object-space ray origin (the
-// packet's rays share the origin, so it is computed once per candidate, not once per lane).  (2) Every lane runs the hit test of its own ray
-// against every cached candidate and keeps a 32-bit mask of its possible hits (may_hit: division-free
-// and conservative, a superset of the hits).  (3) The lanes walk their masks together, one candidate
-// per lane per step, through the intersection program, which decides the hit, and the selection.
-// The order in which a lane sees its hits does not matter: the all-hit sums are order-independent
-// and the selection is by key.  The cache keeps each candidate's object-space ray origin in place of
-// its mean (computed once by the fetching lane with local_origin, the arithmetic of local_ray).
-template <int KB>
-__device__ __forceinline__ void flush_candidates(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, bool want,
-                                                 bool first, LaneState &st, unsigned long long (*kbuf)[kFwdThreads],
-                                                 const Frustum &fr, uint32_t *cand, CandCache &cc, int nc) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t lanemask_lt = (1u << lane) - 1u;
-    uint32_t gid = 0;
-    bool keep = false;
-    float4 g0, g1, g2;
-    int4 cv;
-    float sfv = 0.0f;
-    if (lane < nc) {
-        gid = cand[lane];
-        g0 = sc.geom[3 * (size_t)gid];
-        g1 = sc.geom[3 * (size_t)gid + 1];
-        g2 = sc.geom[3 * (size_t)gid + 2];
-        const float2 lv = sc.live[gid];
-        const float *cp = sc.channels + 3 * (size_t)gid;
-        cv = make_int4(colour_fixed(cp[0]), colour_fixed(cp[1]), colour_fixed(cp[2]), __float_as_int(lv.x));
-        sfv = lv.y;
-        keep = sc.l2w ? frustum_ellipsoid(fr, sc.l2w + 3 * (size_t)gid) : true;
-        const f3 lo = local_origin(g0, g1, g2, ro);
-        g0.w = lo.x;
-        g1.w = lo.y;
-        g2.w = lo.z;
-    }
-    const uint32_t bal = __ballot_sync(kFull, keep);
-    __syncwarp();  // every read of cand[] precedes the compacting writes
-    if (keep) {
-        const int slot = __popc(bal & lanemask_lt);
-        cand[slot] = gid;
-        cc.g[slot][0] = g0;
-        cc.g[slot][1] = g1;
-        cc.g[slot][2] = g2;
-        cc.c[slot] = cv;
-        cc.sf[slot] = sfv;
-    }
-    nc = __popc(bal);
-    __syncwarp();
-    uint32_t mask = 0u;
-    if (want) {
-        for (int j = 0; j < nc; j++) {
-            if (may_hit_lo(cc.g[j][0], cc.g[j][1], cc.g[j][2], __int_as_float(cc.c[j].w), rd, k.athr))
-                mask |= 1u << j;
-        }
-    }
-    while (__any_sync(kFull, mask != 0u)) {
-        if (mask != 0u) {
-            const int j = __ffs(mask) - 1;
-            mask &= mask - 1u;
-            const int4 c = cc.c[j];
-            on_leaf_data<KB, true>(cand[j], cc.g[j][0], cc.g[j][1], cc.g[j][2],
-                                   make_float2(__int_as_float(c.w), cc.sf[j]), c.x, c.y, c.z, first, ro, rd, k, st,
-                                   kbuf);
-        }
-    }
-    __syncwarp();
+// Division-free pretest of a block's candidates as conics in the tile's pixel plane.
+//
+// A tile's rays share the origin o and have (unnormalised) directions v(x, y) = v0 + x du + y dv, with
+// (x, y) the pixel's offset from the tile's centre.  With lo = M (o - mu) and l = M v, a ray's line
+// passes a Gaussian's unit sphere within its radius iff |lo x l|^2 <= |l|^2, and both sides are
+// quadratic in (x, y).  The thread that fetches a candidate computes the six coefficients of
+// h(x, y) = |l|^2 - |lo x l|^2 + margin once; every ray then evaluates h at its own (x, y) with five
+// FMAs instead of transforming its direction into the candidate's frame (about 45 instructions).
+// The coefficients are centred on the tile, so they carry no cancellation beyond the tile's own extent.
+//
+// Margin (u = 2^-24; norms are Euclidean): the ray direction the intersection program uses and v(x, y)
+// differ by at most 32u V, V the sum of the magnitudes of the terms that make up a direction (camera_ray's
+// and the basis' own roundings); M times either adds 3u |M|_F V on each side and the cross product 3u of
+// its terms, so |lo x l| is known within eta = 64u (|lo| + 1) |M|_F V (48u + 6u of it from the terms above).
+// A hit of the intersection program puts the line within 1 + 8u of the unit sphere (its max-density
+// point lo + t ld is a point of the line up to one rounding), so |c| <= (1 + 8u) |l| + eta, and
+// |c|^2 <= |l|^2 + 2.1 |l| eta + eta^2 + 17u |l|^2.  Coefficients and evaluation round by at most
+// 24u (|l|^2 + |c|^2) of their largest values Lm, Cm over the tile; 48u is taken.  Outside the range in
+// which every square stays a normal number the candidate is kept (h = +inf), and so it is on a NaN:
+// rays read the sign bit of h, which is clear for +inf and for the NaN the arithmetic generates.
+// The intersection program still decides every hit.
+struct ConicBasis {
+    float v0[3], du[3], dv[3];
+    float hx, hy;  // largest |x| and |y| of the tile
+    float mag;     // V
+};
+
+// (a.x * b.x + c.x, a.y * b.y + c.y), each rounded once: one issue slot for two FMAs.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+        "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
 }
 
-// One full traversal of the packet (camera rays with a common origin) with the node work spread
-// over the lanes: each step pops up to 32 nodes, one per lane, tests their child boxes against the
-// packet frustum, pushes surviving internal children and queues surviving leaves; queued leaves
-// are then intersected by every lane with its own ray (on_leaf).  With a tile frontier (at
-// front_base + front_off: count, entries; a count of kFrontierNone or a null base: none; base and
-// offset are kept apart so that a kernel-parameter base needs no register) the traversal starts there instead
-// of at the root: the frontier goes onto the stack with its first entry on top, and a frontier leaf
-// is queued when it is popped.  Returns false if the shared stack overflowed (the caller then
-// repeats the traversal per ray).
+__device__ __forceinline__ float sqrt_approx(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float norm_approx(f3 a) { return sqrt_approx(fdot3(a, a)); }
+
+__device__ __forceinline__ f3 cross3(f3 a, f3 b) {
+    return mk3(fmaf(a.y, b.z, -(a.z * b.y)), fmaf(a.z, b.x, -(a.x * b.z)), fmaf(a.x, b.y, -(a.y * b.x)));
+}
+
+// Coefficients (F, D, E, A, B, C) of h(x, y) = F + x (D + x A + y B) + y (E + y C) for the candidate
+// with snapshot rows g0..g2 (columns M) and object-space origin lo.
+__device__ __forceinline__ void conic_coefficients(const ConicBasis &cb, const float4 g0, const float4 g1,
+                                                   const float4 g2, f3 lo, float q[6]) {
+    const f3 v0 = mk3(cb.v0[0], cb.v0[1], cb.v0[2]), du = mk3(cb.du[0], cb.du[1], cb.du[2]),
+             dv = mk3(cb.dv[0], cb.dv[1], cb.dv[2]);
+    const f3 l0 = mk3(fdot3(g0, v0), fdot3(g1, v0), fdot3(g2, v0));
+    const f3 lu = mk3(fdot3(g0, du), fdot3(g1, du), fdot3(g2, du));
+    const f3 lv = mk3(fdot3(g0, dv), fdot3(g1, dv), fdot3(g2, dv));
+    const f3 c0 = cross3(lo, l0), cu = cross3(lo, lu), cv = cross3(lo, lv);
+    const float ll0 = fdot3(l0, l0), lluu = fdot3(lu, lu), llvv = fdot3(lv, lv);
+    const float cc0 = fdot3(c0, c0), ccuu = fdot3(cu, cu), ccvv = fdot3(cv, cv);
+    const float lm = fmaf(cb.hy, sqrt_approx(llvv), fmaf(cb.hx, sqrt_approx(lluu), sqrt_approx(ll0)));
+    const float cm = fmaf(cb.hy, sqrt_approx(ccvv), fmaf(cb.hx, sqrt_approx(ccuu), sqrt_approx(cc0)));
+    const float mf = sqrt_approx(g0.x * g0.x + g0.y * g0.y + g0.z * g0.z + g1.x * g1.x + g1.y * g1.y + g1.z * g1.z +
+                                 g2.x * g2.x + g2.y * g2.y + g2.z * g2.z);
+    const float nl = norm_approx(lo);
+    const float eta = 0x1.0p-18f * (nl + 1.0f) * mf * cb.mag;
+    const float margin = fmaf(eta, fmaf(2.1f, lm, eta), 0x1.8p-19f * fmaf(lm, lm, cm * cm));
+    const bool ok = lm >= 0x1.0p-50f && lm <= 0x1.0p50f && cm <= 0x1.0p50f && nl <= 0x1.0p40f && eta <= 0x1.0p50f;
+    q[0] = ok ? (ll0 - cc0) + margin : __int_as_float(0x7f800000);
+    q[1] = ok ? 2.0f * (fdot3(l0, lu) - fdot3(c0, cu)) : 0.0f;
+    q[2] = ok ? 2.0f * (fdot3(l0, lv) - fdot3(c0, cv)) : 0.0f;
+    q[3] = ok ? lluu - ccuu : 0.0f;
+    q[4] = ok ? 2.0f * (fdot3(lu, lv) - fdot3(cu, cv)) : 0.0f;
+    q[5] = ok ? llvv - ccvv : 0.0f;
+}
+
+// Shared memory of a block that traces one pixel tile (one ray per thread).
 template <int KB>
-__device__ __forceinline__ bool traverse_frustum(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, bool want,
-                                                 bool first, LaneState &st, unsigned long long (*kbuf)[kFwdThreads],
-                                                 const Frustum &fr, uint32_t *stk, uint32_t *cand,
-                                                 CandCache &cc, const uint32_t *front_base, uint32_t front_off,
-                                                 int32_t *status) {
-    const int lane = threadIdx.x & 31;
+struct TileShared {
+    unsigned long long kbuf[KB][kFwdThreads];
+    // the batch's candidates, filled once per batch by the block (one candidate per thread):
+    float4 g[kBatch][3];       // snapshot rows with the tile's object-space origin: (M | M (o - mu))
+    int4 c[kBatch];            // colour in 2^-24 fixed point (x, y, z), live opacity bits (w)
+    float4 conic[kBatch / 2][3];  // coefficients of candidates 2i, 2i+1: (F F' D D') (E E' A A') (B B' C C')
+    float sf[kBatch];          // live scaling factor
+    uint32_t gid[kBatch];
+    uint32_t stk[kTileStack];
+    uint32_t queue[kTileQueue];
+    Frustum fr;
+    ConicBasis cb;
+    uint32_t cnt[kWarps];      // per-warp counts of a step
+};
+
+// A batch: the block's queued leaves queue[0, take) (take <= kBatch, every thread calls this together;
+// leaves beyond them move to the front of the queue).  (1) Thread j takes leaf j: it tests the leaf's
+// ellipsoid against the tile's frustum, fetches its snapshot rows, live values and colour, computes
+// its object-space ray origin (with local_origin, the arithmetic of local_ray) and its conic, and the
+// survivors are compacted into the shared cache.  A tile's four warps share the fetched records and
+// the batch spans up to 128 candidates, where packets of their own batches fetched every record up to
+// four times and tested 21 survivors at a time.  (2) Every ray evaluates the conics at its pixel, two
+// candidates per step, into a bit mask of its possible hits.  (3) The lanes of a warp walk their masks
+// together, one candidate per lane per step, through the intersection program, which decides the hit,
+// and the selection.  The order in which a ray sees its hits does not matter: the all-hit sums are
+// order-independent and the selection is by key.
+template <int KB>
+__device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px,
+                                                   float py, bool want, bool first, LaneState &st,
+                                                   TileShared<KB> &sh, int take, int nc) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t lanemask_lt = (1u << lane) - 1u;
+    {
+        uint32_t gid = 0;
+        bool keep = false;
+        float4 g0, g1, g2;
+        int4 cv;
+        float sfv = 0.0f;
+        float q[6];
+        if (t < take) {
+            gid = sh.queue[t];
+            g0 = sc.geom[3 * (size_t)gid];
+            g1 = sc.geom[3 * (size_t)gid + 1];
+            g2 = sc.geom[3 * (size_t)gid + 2];
+            const float2 lv = sc.live[gid];
+            const float *cp = sc.channels + 3 * (size_t)gid;
+            const float c0 = cp[0], c1 = cp[1], c2 = cp[2];
+            // no ray hits a Gaussian at or below the alpha threshold (intersect_lo's first test)
+            keep = !(lv.x <= k.athr) && (sc.l2w ? frustum_ellipsoid(sh.fr, sc.l2w + 3 * (size_t)gid) : true);
+            cv = make_int4(colour_fixed(c0), colour_fixed(c1), colour_fixed(c2), __float_as_int(lv.x));
+            sfv = lv.y;
+            const f3 lo = local_origin(g0, g1, g2, ro);
+            conic_coefficients(sh.cb, g0, g1, g2, lo, q);
+            g0.w = lo.x;
+            g1.w = lo.y;
+            g2.w = lo.z;
+        }
+        const int rest = nc - take;
+        const uint32_t r0 = t < rest ? sh.queue[take + t] : 0u;
+        const uint32_t r1 = t + kFwdThreads < rest ? sh.queue[take + kFwdThreads + t] : 0u;
+        const uint32_t bal = __ballot_sync(kFull, keep);
+        if (lane == 0) sh.cnt[warp] = __popc(bal);
+        __syncthreads();  // the counts; every read of the queue and of the previous batch's cache is done
+        if (t < rest) sh.queue[t] = r0;
+        if (t + kFwdThreads < rest) sh.queue[kFwdThreads + t] = r1;
+        if (keep) {
+            int slot = __popc(bal & lanemask_lt);
+            for (int w = 0; w < warp; w++) slot += (int)sh.cnt[w];
+            sh.g[slot][0] = g0;
+            sh.g[slot][1] = g1;
+            sh.g[slot][2] = g2;
+            sh.c[slot] = cv;
+            sh.sf[slot] = sfv;
+            sh.gid[slot] = gid;
+            float *cq = reinterpret_cast<float *>(sh.conic[slot >> 1]) + (slot & 1);
+#pragma unroll
+            for (int e = 0; e < 6; e++) cq[2 * e] = q[e];
+        }
+    }
+    int kept = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) kept += (int)sh.cnt[w];
+    __syncthreads();  // the cache is complete
+    if (!__any_sync(kFull, want)) return;
+    uint32_t m[kBatch / 32];
+    const float2 x2 = make_float2(px, px), y2 = make_float2(py, py);
+#pragma unroll
+    for (int w = 0; w < kBatch / 32; w++) {
+        m[w] = 0u;
+        if (32 * w < kept) {
+            uint32_t miss = 0u;  // candidate 32 w + i ends up in bit 31 - i
+#pragma unroll 4
+            for (int i = 0; i < 16; i++) {
+                const float4 qa = sh.conic[16 * w + i][0], qb = sh.conic[16 * w + i][1], qc = sh.conic[16 * w + i][2];
+                float2 h = fma2(x2, make_float2(qb.z, qb.w), make_float2(qa.z, qa.w));
+                h = fma2(y2, make_float2(qc.x, qc.y), h);
+                h = fma2(x2, h, make_float2(qa.x, qa.y));
+                h = fma2(y2, fma2(y2, make_float2(qc.z, qc.w), make_float2(qb.x, qb.y)), h);
+                miss = __funnelshift_l(__float_as_uint(h.x), miss, 1);
+                miss = __funnelshift_l(__float_as_uint(h.y), miss, 1);
+            }
+            const int left = kept - 32 * w;  // candidates of this word (the rest of its slots are stale)
+            const uint32_t valid = left >= 32 ? 0xffffffffu : ~(0xffffffffu >> left);
+            m[w] = want ? ~miss & valid : 0u;
+        }
+    }
+    int base = 0;
+    for (;;) {
+        if (m[0] == 0u) {
+            base += 32;
+#pragma unroll
+            for (int w = 0; w + 1 < kBatch / 32; w++) m[w] = m[w + 1];
+            m[kBatch / 32 - 1] = 0u;
+        }
+        uint32_t any = m[0];
+#pragma unroll
+        for (int w = 1; w < kBatch / 32; w++) any |= m[w];
+        if (!__any_sync(kFull, any != 0u)) break;
+        if (m[0] != 0u) {
+            const int b = __clz((int)m[0]);
+            m[0] &= ~(0x80000000u >> b);
+            const int j = base + b;
+            const int4 c = sh.c[j];
+            on_leaf_data<KB, true>(sh.gid[j], sh.g[j][0], sh.g[j][1], sh.g[j][2],
+                                   make_float2(__int_as_float(c.w), sh.sf[j]), c.x, c.y, c.z, first, ro, rd, k, st,
+                                   sh.kbuf);
+        }
+    }
+}
+
+// One full traversal of the tile (rays with a common origin inside sh.fr) by the whole block, all of
+// whose threads call this together: each step pops up to 128 nodes, one per thread, tests their child
+// boxes against the tile's frustum, pushes surviving internal children and queues surviving leaves;
+// every 128 queued leaves become a batch (trace_batch_leaves).  Four packets that walked the tree each
+// for itself popped and fetched mostly the same nodes (per tile 270-690 pops and 90-260 queued leaves
+// instead of 4 x 970 and 4 x 268 at 3M Gaussians; with the conics, the forward of 3M / 1080p went from
+// 3.11 to 2.75 ms, 500k / 640x480 from 0.83 to 0.58 ms, 6M / 4K from 18.3 to 15.6 ms, the image and its
+// colours included; the kernel is bound by instruction issue and the latency of each ray's own
+// hit chain, at six or four blocks per SM).  With a frontier (count, entries; a count above
+// kFrontierMax or a null pointer: none) the traversal starts there instead of at the root: the frontier
+// goes onto the stack with its first entry on top, and a frontier leaf is queued when it is popped.
+// px, py: the ray's offset from the tile's centre in the conics' basis.  Returns false if the stack
+// filled up (the caller then repeats the traversal per ray).
+template <int KB>
+__device__ __forceinline__ bool traverse_tile(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px,
+                                              float py, bool want, bool first, LaneState &st, TileShared<KB> &sh,
+                                              const uint32_t *front, int32_t *status) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
     const int n = sc.n;
     const float *rb = sc.root_box;
     const float rmin[3] = {rb[0], rb[1], rb[2]}, rmax[3] = {rb[4], rb[5], rb[6]};
-    if (n <= 0 || !frustum_box(fr, rmin, rmax)) return true;
+    if (n <= 0 || !frustum_box(sh.fr, rmin, rmax)) return true;
     if (n == 1) {
-        on_leaf<KB>(sc, 0u, want, first, ro, rd, k, st, kbuf);
+        on_leaf<KB>(sc, 0u, want, first, ro, rd, k, st, sh.kbuf);
         return true;
     }
-    const uint32_t *front = front_base ? front_base + front_off : nullptr;
-    int sp = front ? (int)front[0] : -1, nc = 0;
-    if (sp >= 0 && sp <= kFrontierMax) {
-        for (int i = lane; i < sp; i += 32) stk[sp - 1 - i] = front[1 + i];
-    } else {
-        if (lane == 0) stk[0] = 0u;
-        sp = 1;
+    const uint32_t fcount = front ? front[0] : kFrontierNone;
+    int sp = 1, nc = 0;
+    if (fcount <= (uint32_t)kFrontierMax) {
+        sp = (int)fcount;
+        for (int i = t; i < sp; i += kFwdThreads) sh.stk[sp - 1 - i] = front[1 + i];
+    } else if (t == 0) {
+        sh.stk[0] = 0u;
     }
-    __syncwarp();
-    bool ok = true, draining = false;
-    long long budget = (long long)n;  // a valid tree pushes each internal node at most once per traversal
+    __syncthreads();
+    int budget = n;  // a valid tree pushes each internal node at most once per traversal
     for (;;) {
-        if (!draining) {
-            if (sp == 0) {
-                draining = true;
-            } else if (--budget < 0) {
+        while (sp > 0 && nc < kBatch) {
+            if (--budget < 0) {
                 raise_status(status, GRAY_STATUS_STACK_OVERFLOW);
-                draining = true;
-            } else {
-                const int take = sp < 32 ? sp : 32;
-                uint32_t node = GRAY_NULL;
-                if (lane < take) node = stk[sp - 1 - lane];
-                __syncwarp();
-                sp -= take;
-                // children as (a, b) = (nearer, farther) along the packet's mean direction
-                bool pa = false, pb = false;
-                uint32_t ca = 0, cb = 0;
-                if (node != GRAY_NULL) {
-                    if (node & GRAY_LEAF_BIT) {
-                        ca = node;  // a leaf of the tile's frontier: queued below
-                        pa = true;
-                    } else if (node >= (uint32_t)(n - 1)) {
-                        raise_status(status, GRAY_STATUS_STACK_OVERFLOW);
-                    } else {
-                        const float4 q0 = sc.nodes[4 * node], q1 = sc.nodes[4 * node + 1],
-                                     q2 = sc.nodes[4 * node + 2], q3 = sc.nodes[4 * node + 3];
-                        const float b0min[3] = {q0.x, q0.y, q0.z}, b0max[3] = {q0.w, q1.x, q1.y};
-                        const float b1min[3] = {q1.z, q1.w, q2.x}, b1max[3] = {q2.y, q2.z, q2.w};
-                        const uint32_t c0 = __float_as_uint(q3.x), c1 = __float_as_uint(q3.y);
-                        const bool p0 = frustum_box(fr, b0min, b0max), p1 = frustum_box(fr, b1min, b1max);
-                        // box centres (times 2) projected on the mean direction; the origin is common
-                        const float4 c = fr.pn[4];
-                        const float s0 = fmaf(q0.z + q1.y, c.z, fmaf(q0.y + q1.x, c.y, (q0.x + q0.w) * c.x));
-                        const float s1 = fmaf(q2.x + q2.w, c.z, fmaf(q1.w + q2.z, c.y, (q1.z + q2.y) * c.x));
-                        const bool sw = s1 < s0;
-                        ca = sw ? c1 : c0;
-                        cb = sw ? c0 : c1;
-                        pa = sw ? p1 : p0;
-                        pb = sw ? p0 : p1;
-                    }
-                }
-                const bool ia = pa && !(ca & GRAY_LEAF_BIT), ib = pb && !(cb & GRAY_LEAF_BIT);
-                const bool la = pa && (ca & GRAY_LEAF_BIT) && (ca & ~GRAY_LEAF_BIT) < (uint32_t)n;
-                const bool lb = pb && (cb & GRAY_LEAF_BIT) && (cb & ~GRAY_LEAF_BIT) < (uint32_t)n;
-                // The popped nodes are in visit order (lane 0 took the top).  Their internal children
-                // go back so that the next pops see lane 0's nearer child first, then its farther
-                // one, then lane 1's, ...; the leaves are queued in the same order.
-                const uint32_t ma = __ballot_sync(kFull, ia), mb = __ballot_sync(kFull, ib);
-                const int ni = __popc(ma) + __popc(mb);
-                if (sp + ni > kWideStack) {
-                    ok = false;  // frontier too wide for the shared stack
-                    break;
-                }
-                const int above = __popc(ma & lanemask_lt) + __popc(mb & lanemask_lt);
-                if (ia) stk[sp + ni - 1 - above] = ca;
-                if (ib) stk[sp + ni - 1 - above - (ia ? 1 : 0)] = cb;
-                sp += ni;
-                // queue the leaves found (nc < kCand before the step, at most 64 added)
-                const uint32_t qa = __ballot_sync(kFull, la), qb = __ballot_sync(kFull, lb);
-                const int before = nc + __popc(qa & lanemask_lt) + __popc(qb & lanemask_lt);
-                if (la) cand[before] = ca & ~GRAY_LEAF_BIT;
-                if (lb) cand[before + (la ? 1 : 0)] = cb & ~GRAY_LEAF_BIT;
-                nc += __popc(qa) + __popc(qb);
-                __syncwarp();
+                sp = 0;
+                break;
             }
+            // a popped node frees its entry and pushes at most two
+            const int take = min(min(sp, kFwdThreads), kTileStack - sp);
+            if (take <= 0) return false;
+            const uint32_t node = t < take ? sh.stk[sp - 1 - t] : GRAY_NULL;
+            // children as (a, b) = (nearer, farther) along the tile's mean direction
+            bool pa = false, pb = false;
+            uint32_t ca = 0, cb = 0;
+            if (node != GRAY_NULL) {
+                if (node & GRAY_LEAF_BIT) {
+                    ca = node;  // a leaf of the tile's frontier: queued below
+                    pa = true;
+                } else if (node >= (uint32_t)(n - 1)) {
+                    raise_status(status, GRAY_STATUS_STACK_OVERFLOW);
+                } else {
+                    const float4 q0 = sc.nodes[4 * (size_t)node], q1 = sc.nodes[4 * (size_t)node + 1],
+                                 q2 = sc.nodes[4 * (size_t)node + 2], q3 = sc.nodes[4 * (size_t)node + 3];
+                    const float b0min[3] = {q0.x, q0.y, q0.z}, b0max[3] = {q0.w, q1.x, q1.y};
+                    const float b1min[3] = {q1.z, q1.w, q2.x}, b1max[3] = {q2.y, q2.z, q2.w};
+                    const uint32_t c0 = __float_as_uint(q3.x), c1 = __float_as_uint(q3.y);
+                    const bool p0 = frustum_box(sh.fr, b0min, b0max), p1 = frustum_box(sh.fr, b1min, b1max);
+                    // box centres (times 2) projected on the mean direction; the origin is common
+                    const float4 c = sh.fr.pn[4];
+                    const float s0 = fmaf(q0.z + q1.y, c.z, fmaf(q0.y + q1.x, c.y, (q0.x + q0.w) * c.x));
+                    const float s1 = fmaf(q2.x + q2.w, c.z, fmaf(q1.w + q2.z, c.y, (q1.z + q2.y) * c.x));
+                    const bool sw = s1 < s0;
+                    ca = sw ? c1 : c0;
+                    cb = sw ? c0 : c1;
+                    pa = sw ? p1 : p0;
+                    pb = sw ? p0 : p1;
+                }
+            }
+            const bool ia = pa && !(ca & GRAY_LEAF_BIT), ib = pb && !(cb & GRAY_LEAF_BIT);
+            const bool la = pa && (ca & GRAY_LEAF_BIT) && (ca & ~GRAY_LEAF_BIT) < (uint32_t)n;
+            const bool lb = pb && (cb & GRAY_LEAF_BIT) && (cb & ~GRAY_LEAF_BIT) < (uint32_t)n;
+            // The popped nodes are in visit order (thread 0 took the top).  Their internal children go
+            // back so that the next pops see thread 0's nearer child first, then its farther one, then
+            // thread 1's, ...; the leaves are queued in the same order.
+            const uint32_t ma = __ballot_sync(kFull, ia), mb = __ballot_sync(kFull, ib);
+            const uint32_t qa = __ballot_sync(kFull, la), qb = __ballot_sync(kFull, lb);
+            if (lane == 0) sh.cnt[warp] = (uint32_t)(__popc(ma) + __popc(mb)) | (uint32_t)(__popc(qa) + __popc(qb)) << 16;
+            __syncthreads();  // the counts; every pop has been read
+            uint32_t before = 0u, total = 0u;  // (internal, leaves << 16) of the warps before this one, of all
+#pragma unroll
+            for (int w = 0; w < kWarps; w++) {
+                const uint32_t c = sh.cnt[w];
+                if (w < warp) before += c;
+                total += c;
+            }
+            const int ni = (int)(total & 0xffffu);
+            sp -= take;
+            const int above = (int)(before & 0xffffu) + __popc(ma & lanemask_lt) + __popc(mb & lanemask_lt);
+            if (ia) sh.stk[sp + ni - 1 - above] = ca;
+            if (ib) sh.stk[sp + ni - 1 - above - (ia ? 1 : 0)] = cb;
+            sp += ni;
+            const int at = nc + (int)(before >> 16) + __popc(qa & lanemask_lt) + __popc(qb & lanemask_lt);
+            if (la) sh.queue[at] = ca & ~GRAY_LEAF_BIT;
+            if (lb) sh.queue[at + (la ? 1 : 0)] = cb & ~GRAY_LEAF_BIT;
+            nc += (int)(total >> 16);
+            __syncthreads();  // the pushes; the counts are free again
         }
-        // keep the queue below kCand before the next step (a step adds at most 64 < kQueue - kCand)
-        while (nc >= kCand || (draining && nc > 0)) {
-            // process the first kCand queued leaves, then move the rest to the front
-            const int take = nc < kCand ? nc : kCand;
-            flush_candidates<KB>(sc, k, ro, rd, want, first, st, kbuf, fr, cand, cc, take);
-            const int rest = nc - take;
-            const uint32_t r0 = lane < rest ? cand[kCand + lane] : 0u;
-            const uint32_t r1 = lane + 32 < rest ? cand[kCand + 32 + lane] : 0u;
-            __syncwarp();
-            if (lane < rest) cand[lane] = r0;
-            if (lane + 32 < rest) cand[32 + lane] = r1;
-            __syncwarp();
-            nc = rest;
-        }
-        if (draining) break;
+        if (nc == 0) break;
+        const int take = min(nc, kBatch);
+        trace_batch_leaves<KB>(sc, k, ro, rd, px, py, want, first, st, sh, take, nc);
+        nc -= take;
     }
-    __syncwarp();
-    return ok;
+    return true;
 }
 
-// Trace the warp's 32 rays (one per lane; `alive` lanes only) through the scene: traversal,
-// selection, compositing (cuda/forward_pass.cu:6-151 minus the write-out).  Every lane of the
-// warp must call this together.
+// Trace a block's rays (one per thread; `alive` threads only) through the scene: traversal, selection,
+// compositing (cuda/forward_pass.cu:6-151 minus the write-out).  tile: the block's rays share one origin
+// and lie inside sh.fr, and are traversed together from the frontier `front` (see traverse_tile, px,
+// py); else every warp traverses its own rays.  Every thread of the block calls this together.
 template <int KB>
-__device__ __forceinline__ void trace_ray(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, bool alive,
-                                          bool grads, const HitSink &hs, int32_t *status,
-                                          unsigned long long (*kbuf)[kFwdThreads], RayResult &res,
-                                          const Frustum *fr = nullptr, uint32_t *wstk = nullptr,
-                                          uint32_t *wcand = nullptr, CandCache *wcc = nullptr,
-                                          const uint32_t *front_base = nullptr, uint32_t front_off = 0) {
+__device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px, float py,
+                                           bool alive, bool tile, bool grads, const HitSink &hs, int32_t *status,
+                                           TileShared<KB> &sh, const uint32_t *front, RayResult &res) {
+    unsigned long long(*kbuf)[kFwdThreads] = sh.kbuf;
     const int lane = threadIdx.x & 31;
     LaneState &st = res.st;
     st.lfx = 0;
@@ -579,16 +703,14 @@ __device__ __forceinline__ void trace_ray(const TraceScene &sc, const TraceKnobs
     // on past the 16 nearest keys of its first traversal (the same 16 the narrow kernel holds)
     bool deep = false;
     const int n = sc.n;
-    while (__any_sync(kFull, !done)) {
+    while (tile ? __syncthreads_or(!done) : __any_sync(kFull, !done)) {
         const bool want = !done;
         st.kcount = 0;
         st.ncand = 0;
         // ---------------- traversal ----------------
-        bool per_ray = fr == nullptr;
-        if (!per_ray &&
-            !traverse_frustum<KB>(sc, k, ro, rd, want, first, st, kbuf, *fr, wstk, wcand, *wcc, front_base, front_off,
-                                      status)) {
-            // the frustum traversal gave up (stack overflow): discard what it gathered, trace per ray
+        bool per_ray = !tile;
+        if (tile && !traverse_tile<KB>(sc, k, ro, rd, px, py, want, first, st, sh, front, status)) {
+            // the tile's stack filled up: discard what was gathered, trace per ray
             st.kcount = 0;
             st.ncand = 0;
             if (first) {
@@ -828,27 +950,37 @@ __device__ __forceinline__ float3 camera_ray3(const float *w, float fov, int px,
     return make_float3(r.x, r.y, r.z);
 }
 
-// Shared memory of a forward block.
-template <int KB>
-struct FwdShared {
-    unsigned long long kbuf[KB][kFwdThreads];
-    Frustum sfr[kWarps];
-    uint32_t sstk[kWarps][kWideStack];
-    uint32_t scand[kWarps][kQueue];
-    CandCache scc[kWarps];
-    uint32_t front[kFrontierWords];  // the tile's BVH frontier (count, entries)
-};
+// The tile's ray basis for the conics: directions v(x, y) = v0 + x du + y dv of the pinhole camera's
+// pixels at the offset (x, y) from pixel position (cx, cy), as camera_ray forms them.  One thread.
+__device__ __forceinline__ void make_conic_basis(ConicBasis &cb, const float *w, float fov, float cx, float cy,
+                                                 float hx, float hy, uint32_t width, uint32_t height) {
+    const float vs = tanf(fov / 2.0f), ax = (float)width / (float)height * vs;
+    const float x0 = ax * (2.0f * (cx + 0.5f) / (float)width - 1.0f), y0 = vs * (1.0f - 2.0f * (cy + 0.5f) / (float)height);
+    const float dx = 2.0f * ax / (float)width, dy = -2.0f * vs / (float)height;
+    float n0 = 0.0f, n1 = 0.0f, n2 = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        cb.v0[e] = w[e] * x0 + w[3 + e] * y0 - w[6 + e];
+        cb.du[e] = w[e] * dx;
+        cb.dv[e] = w[3 + e] * dy;
+        n0 += w[e] * w[e];
+        n1 += w[3 + e] * w[3 + e];
+        n2 += w[6 + e] * w[6 + e];
+    }
+    cb.hx = hx;
+    cb.hy = hy;
+    // |x0 + x dx| <= ax over the image's pixels, and twice that over a tile that reaches past it
+    cb.mag = 2.0f * (sqrtf(n0) * fabsf(ax) + sqrtf(n1) * fabsf(vs)) + sqrtf(n2);
+}
 
-// Packet (wx, wy) of pixel tile (bx, by) (a tile is 2x2 packets of tile_w x tile_h pixels), traced
-// by the calling warp; front_base + front_off: the tile's BVH frontier (count, entries), or a null base.
+// The block's pixel tile (bx, by): 2x2 packets of tile_w x tile_h pixels, one packet per warp.  Returns
+// whether the calling warp's packet needs more than one traversal with 16 hit slots (RayResult::retraced).
 template <int KB>
-__device__ __forceinline__ bool forward_packet(const FwdArgs &a, int bx, int by, int wx, int wy,
-                                               const uint32_t *front_base, uint32_t front_off, FwdShared<KB> &sh) {
-    unsigned long long(*kbuf)[kFwdThreads] = sh.kbuf;
-    Frustum *sfr = sh.sfr;
+__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, TileShared<KB> &sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int px = bx * (a.tile_w * kBlockWarpsX) + wx * a.tile_w + (lane % a.tile_w);
-    const int py = by * (a.tile_h * kBlockWarpsY) + wy * a.tile_h + (lane / a.tile_w);
+    const int tx0 = bx * (a.tile_w * kBlockWarpsX), ty0 = by * (a.tile_h * kBlockWarpsY);
+    const int px = tx0 + (warp % kBlockWarpsX) * a.tile_w + (lane % a.tile_w);
+    const int py = ty0 + (warp / kBlockWarpsX) * a.tile_h + (lane / a.tile_w);
     const bool inside = px < (int)a.render_w && py < (int)a.render_h;
     const uint32_t pixel = (uint32_t)py * a.alloc_w + (uint32_t)px;
 
@@ -866,8 +998,8 @@ __device__ __forceinline__ bool forward_packet(const FwdArgs &a, int bx, int by,
     // ---- ray generation (cuda/shaders.cu:76-88) ----
     f3 ro = mk3(0.0f, 0.0f, 0.0f), rd = mk3(0.0f, 0.0f, 0.0f);
     bool alive = false;
-    // every lane holds the camera origin, inactive ones too (a packet's candidates get their
-    // object-space origin from whichever lane fetches them)
+    // every thread holds the camera origin, inactive ones too (a tile's candidates get their
+    // object-space origin from whichever thread fetches them)
     if (!*a.rays_from_python) ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
     if (inside) {
         if (*a.rays_from_python) {
@@ -886,18 +1018,23 @@ __device__ __forceinline__ bool forward_packet(const FwdArgs &a, int bx, int by,
         alive = !(sqrtf(dot3(rd, rd)) == 0.0f);
     }
 
-    // camera rays of the packet share the origin: trace with the frustum traversal
-    const bool frustum = !*a.rays_from_python && !*a.jitter;
-    if (frustum) {
-        const int x0 = px - lane % a.tile_w, y0 = py - lane / a.tile_w;
-        const int x1 = x0 + a.tile_w - 1, y1 = y0 + a.tile_h - 1;
-        make_frustum_warp(sfr[warp], mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, x0, y0, x1,
-                          y1, a.render_w, a.render_h, a.root_box);
+    // camera rays share the origin: the block traverses its tile together
+    const bool tile = !*a.rays_from_python && !*a.jitter;
+    const float hx = (float)(a.tile_w * kBlockWarpsX - 1) * 0.5f, hy = (float)(a.tile_h * kBlockWarpsY - 1) * 0.5f;
+    const uint32_t *front = nullptr;
+    if (tile) {
+        // (the loop of trace_rays starts with a block barrier)
+        if (warp == 0)
+            make_frustum_warp(sh.fr, mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, tx0, ty0,
+                              tx0 + a.tile_w * kBlockWarpsX - 1, ty0 + a.tile_h * kBlockWarpsY - 1, a.render_w,
+                              a.render_h, a.root_box);
+        if (threadIdx.x == kFwdThreads - 1)
+            make_conic_basis(sh.cb, a.w2c, *a.fov, (float)tx0 + hx, (float)ty0 + hy, hx, hy, a.render_w, a.render_h);
+        if (a.frontier) front = a.frontier + (size_t)(by * a.tiles_x + bx) * kFrontierWords;
     }
     RayResult r;
-    trace_ray<KB>(sc, k, ro, rd, alive, grads, hs, a.status, kbuf, r, frustum ? &sfr[warp] : nullptr, sh.sstk[warp],
-                  sh.scand[warp], &sh.scc[warp], frustum ? front_base : nullptr, front_off);
-
+    trace_rays<KB>(sc, k, ro, rd, (float)(px - tx0) - hx, (float)(py - ty0) - hy, alive, tile, grads, hs, a.status, sh,
+                   front, r);
     if (!inside) return r.retraced;
     if (!alive) {
         a.head[pixel] = GRAY_NULL;  // inactive pixel: empty list, nothing else written
@@ -937,28 +1074,10 @@ __device__ __forceinline__ bool forward_packet(const FwdArgs &a, int bx, int by,
     return r.retraced;
 }
 
-// One block's pixel tile (bx, by): its four packets, one per warp; the tile's frontier is copied
-// into shared memory once by the block.  Returns whether the calling warp's packet needs more than
-// one traversal with 16 hit slots (RayResult::retraced).
-template <int KB>
-__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, FwdShared<KB> &sh) {
-    const int warp = threadIdx.x >> 5;
-    {   // every thread of the block gets here together
-        const uint32_t *src = a.frontier ? a.frontier + (size_t)(by * a.tiles_x + bx) * kFrontierWords : nullptr;
-        const uint32_t cnt = src ? src[0] : kFrontierNone;
-        const bool use = cnt <= (uint32_t)kFrontierMax;
-        if (use)
-            for (uint32_t i = threadIdx.x; i < cnt; i += kFwdThreads) sh.front[1 + i] = src[1 + i];
-        if (threadIdx.x == 0) sh.front[0] = use ? cnt : kFrontierNone;
-        __syncthreads();
-    }
-    return forward_packet<KB>(a, bx, by, warp % kBlockWarpsX, warp / kBlockWarpsX, sh.front, 0u, sh);
-}
-
 // Grid launch: block (x, y) renders tile (x, y).
 template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_kernel(const FwdArgs a) {
-    __shared__ FwdShared<KB> sh;
+    __shared__ TileShared<KB> sh;
     if (*a.render_ellipsoids) return;  // the ellipsoid view (ellipsoid_kernel) renders this frame
     forward_tile<KB>(a, blockIdx.x, blockIdx.y, sh);
 }
@@ -970,7 +1089,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_kernel(const 
 // reads them).
 template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(const FwdArgs a) {
-    __shared__ FwdShared<KB> sh;
+    __shared__ TileShared<KB> sh;
     __shared__ uint32_t s_next, s_packets, s_retraced;
     if (*a.render_ellipsoids) return;
     // automatic choice: both kernels are launched, the one the scan kernel did not choose leaves
@@ -996,27 +1115,6 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
     if (threadIdx.x == 0 && s_packets > 0u) {
         atomicAdd(&a.schedule[kStatPackets], s_packets);
         atomicAdd(&a.schedule[kStatRetraced], s_retraced);
-    }
-}
-
-// Persistent launch with packets taken per warp: every warp claims the next packet (a quarter of a
-// pixel tile, tiles in the schedule's densest-first order) from the global counter on its own, so no
-// warp waits at a block barrier for a tile's slowest packet; a tile's four packets usually land on
-// different SMs, though, so they no longer share an L1.  Packets read their tile's frontier from
-// the schedule buffer (L2).
-template <int KB, int MINB>
-__global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_claim_kernel(const FwdArgs a) {
-    __shared__ FwdShared<KB> sh;
-    if (*a.render_ellipsoids) return;
-    for (;;) {
-        uint32_t q = 0u;
-        if ((threadIdx.x & 31) == 0) q = atomicAdd(a.schedule, 1u);
-        q = __shfl_sync(kFull, q, 0);
-        if (q >= (uint32_t)kWarps * (uint32_t)a.ntiles) break;
-        const uint32_t tile = a.schedule[kSchedHeader + a.ntiles + q / kWarps], sub = q % kWarps;
-        forward_packet<KB>(a, (int)(tile % (uint32_t)a.tiles_x), (int)(tile / (uint32_t)a.tiles_x),
-                                       (int)(sub % kBlockWarpsX), (int)(sub / kBlockWarpsX), a.frontier,
-                                       tile * (uint32_t)kFrontierWords, sh);
     }
 }
 
@@ -1591,18 +1689,11 @@ __global__ void __launch_bounds__(kEllTileX * kEllTileY) ellipsoid_kernel(const 
 
 // ---------------------------------------------------------------------------------------------
 // Batched render: many views (of one or several resident scenes) in one persistent launch.
-// Warps pull 32-ray packets from a global counter; packet -> (view, tile) through the views'
-// packet offsets.  Forward only (no gradients, no hit lists); per view the output is RGB.
-// A view's packets form groups of 2x2 (group_offset numbers them across views); with a frontier
-// buffer, batch_frontier_kernel first writes each group's BVH frontier and the packets of the group
-// start their traversals there, as the plain forward's blocks do.
+// Blocks pull groups of 2x2 packets from a global counter, the groups of all views counted in order of
+// the views, and trace them as the plain forward's blocks trace a tile.  Forward only (no gradients, no
+// hit lists); per view the output is RGB.  With a frontier buffer (group_offset numbers the groups
+// in it), batch_frontier_kernel first writes each group's BVH frontier, and the traversals start there.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ int batch_view_of(const gray_batch_view *views, int nviews, uint32_t packet) {
-    int v = 0;
-    while (v + 1 < nviews && views[v + 1].packet_offset <= packet) v++;
-    return v;
-}
-
 __global__ void __launch_bounds__(32) batch_frontier_kernel(const gray_batch_scene *__restrict__ scenes,
                                                             const gray_batch_view *__restrict__ views, int nviews,
                                                             uint32_t *__restrict__ frontier, int tile_w,
@@ -1635,70 +1726,73 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
                        int nviews, uint32_t total_packets, float *__restrict__ out, uint32_t *__restrict__ counter,
                        int tile_w, const uint32_t *__restrict__ frontier, uint32_t total_groups,
                        int32_t *status) {
-    __shared__ unsigned long long kbuf[KB][kFwdThreads];
-    __shared__ Frustum sfr[kWarps];
-    __shared__ uint32_t sstk[kWarps][kWideStack];
-    __shared__ uint32_t scand[kWarps][kQueue];
-    __shared__ CandCache scc[kWarps];
-    // the packet's scene and view parameters live in shared memory (read where used), which keeps
+    __shared__ TileShared<KB> sh;
+    // the group's scene and view parameters live in shared memory (read where used), which keeps
     // them out of the registers the traversal needs
-    __shared__ TraceScene s_sc[kWarps];
-    __shared__ TraceKnobs s_k[kWarps];
+    __shared__ TraceScene s_sc;
+    __shared__ TraceKnobs s_k;
+    __shared__ uint32_t s_view, s_local;  // view of the block's group, group inside the view
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tile_h = 32 / tile_w;
+    const float hx = (float)(tile_w * kBlockWarpsX - 1) * 0.5f, hy = (float)(tile_h * kBlockWarpsY - 1) * 0.5f;
     for (;;) {
-        __syncwarp();
-        uint32_t packet = 0;
-        if (lane == 0) packet = atomicAdd(counter, 1u);
-        packet = __shfl_sync(kFull, packet, 0);
-        if (packet >= total_packets) break;
-        const gray_batch_view &vw = views[batch_view_of(views, nviews, packet)];
-        const gray_batch_scene &bs = scenes[vw.scene];
-        const uint32_t local = packet - vw.packet_offset;
-        const uint32_t tiles_x = (vw.width + tile_w - 1) / tile_w;
-        const int px = (int)((local % tiles_x) * tile_w) + lane % tile_w;
-        const int py = (int)((local / tiles_x) * tile_h) + lane / tile_w;
-        const bool inside = px < (int)vw.width && py < (int)vw.height;
-        if (lane == 0) {
-            TraceKnobs &k = s_k[warp];
-            k.znear = vw.znear;
-            k.zfar = vw.zfar;
-            k.athr = bs.alpha_threshold;
-            k.pw = bs.exp_power;
-            k.tthr = bs.t_threshold;
-            k.render_depth = false;
-            s_sc[warp] = TraceScene{reinterpret_cast<const float4 *>(bs.geom), reinterpret_cast<const float4 *>(bs.l2w),
-                                    reinterpret_cast<const float2 *>(bs.live), vw.channels,
-                                    reinterpret_cast<const float4 *>(bs.nodes), bs.root_box, bs.n};
-        }
-        __syncwarp();
-        const TraceScene &sc = s_sc[warp];
-        const TraceKnobs &k = s_k[warp];
-        const HitSink hs{nullptr, nullptr, 0};
-        f3 ro = mk3(vw.origin[0], vw.origin[1], vw.origin[2]);
-        f3 rd = mk3(0.0f, 0.0f, 0.0f);
-        if (inside) rd = camera_ray(vw.w2c, vw.fov_y, px, py, vw.width, vw.height, 0.0f, 0.0f);
-        {
-            const int x0 = (int)((local % tiles_x) * tile_w), y0 = (int)((local / tiles_x) * tile_h);
-            make_frustum_warp(sfr[warp], ro, vw.w2c, vw.fov_y, x0, y0, x0 + tile_w - 1, y0 + tile_h - 1, vw.width,
-                              vw.height, s_sc[warp].root_box);
-        }
-        const uint32_t *front = nullptr;
-        uint32_t front_off = 0u;
-        if (frontier) {
-            const uint32_t tx = local % tiles_x, ty = local / tiles_x;
-            const uint32_t grp = vw.group_offset + (ty / 2) * ((tiles_x + 1) / 2) + tx / 2;
-            if (grp < total_groups) {  // else: from the root
-                front = frontier;
-                front_off = grp * (uint32_t)kFrontierWords;
+        __syncthreads();  // every thread is done with the previous group
+        if (threadIdx.x == 0) {
+            uint32_t g = atomicAdd(counter, 1u);
+            int v = 0;
+            for (; v < nviews; v++) {
+                const uint32_t tx = (views[v].width + tile_w - 1) / tile_w, ty = (views[v].height + tile_h - 1) / tile_h;
+                const uint32_t groups = ((tx + 1) / 2) * ((ty + 1) / 2);
+                if (g < groups) break;
+                g -= groups;
+            }
+            s_view = (uint32_t)v;
+            s_local = g;
+            if (v < nviews) {
+                const gray_batch_view &vw = views[v];
+                const gray_batch_scene &bs = scenes[vw.scene];
+                s_k.znear = vw.znear;
+                s_k.zfar = vw.zfar;
+                s_k.athr = bs.alpha_threshold;
+                s_k.pw = bs.exp_power;
+                s_k.tthr = bs.t_threshold;
+                s_k.render_depth = false;
+                s_sc = TraceScene{reinterpret_cast<const float4 *>(bs.geom), reinterpret_cast<const float4 *>(bs.l2w),
+                                  reinterpret_cast<const float2 *>(bs.live), vw.channels,
+                                  reinterpret_cast<const float4 *>(bs.nodes), bs.root_box, bs.n};
             }
         }
+        __syncthreads();
+        if (s_view >= (uint32_t)nviews) break;
+        const gray_batch_view &vw = views[s_view];
+        const TraceScene &sc = s_sc;
+        const TraceKnobs &k = s_k;
+        const uint32_t tiles_x = (vw.width + tile_w - 1) / tile_w, gxn = (tiles_x + 1) / 2;
+        const uint32_t gx = s_local % gxn, gy = s_local / gxn;
+        const uint32_t wx = 2 * gx + warp % kBlockWarpsX, wy = 2 * gy + warp / kBlockWarpsX;
+        const int x0 = (int)(gx * 2 * tile_w), y0 = (int)(gy * 2 * tile_h);
+        const int px = (int)(wx * tile_w) + lane % tile_w, py = (int)(wy * tile_h) + lane / tile_w;
+        // (packets past the launch's total, and past the view's edges, render nothing)
+        const bool inside = px < (int)vw.width && py < (int)vw.height &&
+                            vw.packet_offset + wy * tiles_x + wx < total_packets;
+        const f3 ro = mk3(vw.origin[0], vw.origin[1], vw.origin[2]);
+        f3 rd = mk3(0.0f, 0.0f, 0.0f);
+        if (inside) rd = camera_ray(vw.w2c, vw.fov_y, px, py, vw.width, vw.height, 0.0f, 0.0f);
+        // (the loop of trace_rays starts with a block barrier)
+        if (warp == 0)
+            make_frustum_warp(sh.fr, ro, vw.w2c, vw.fov_y, x0, y0, x0 + 2 * tile_w - 1, y0 + 2 * tile_h - 1, vw.width,
+                              vw.height, s_sc.root_box);
+        if (threadIdx.x == kFwdThreads - 1)
+            make_conic_basis(sh.cb, vw.w2c, vw.fov_y, (float)x0 + hx, (float)y0 + hy, hx, hy, vw.width, vw.height);
+        // the group's frontier (a group beyond the launch's total starts at the root)
+        const uint32_t grp = vw.group_offset + s_local;
+        const uint32_t *front = frontier && grp < total_groups ? frontier + (size_t)grp * kFrontierWords : nullptr;
         RayResult r;
-        trace_ray<KB>(sc, k, ro, rd, inside, false, hs, status, kbuf, r, &sfr[warp], sstk[warp], scand[warp],
-                      &scc[warp], front, front_off);
+        trace_rays<KB>(sc, k, ro, rd, (float)(px - x0) - hx, (float)(py - y0) - hy, inside, true, false,
+                       HitSink{nullptr, nullptr, 0}, status, sh, front, r);
         if (!inside) continue;
         float r0, r1, r2;
-        finish_ray(r, bs.bg, 1e-12f, false, r0, r1, r2);
+        finish_ray(r, scenes[vw.scene].bg, 1e-12f, false, r0, r1, r2);
         float *o = out + vw.out_offset + 3 * ((size_t)py * vw.width + px);
         o[0] = r.C0;
         o[1] = r.C1;
@@ -1794,8 +1888,7 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     FwdArgs &a = q.a;
     a = forward_args(p, display);
     // variant: bits 0-1 select (buffer size, register cap), bit 2 the packet shape, bits 3-4 the
-    // tile frontier's cut (64 leaves, 32, 128, no frontier), bit 5 packets claimed per warp
-    // (trace_forward_claim_kernel) instead of tiles per block
+    // tile frontier's cut (64 leaves, 32, 128, no frontier); bit 5 is accepted and has no effect
     // variant 0 (the default) chooses between the narrow and the wide kernel of kDefaultTraceVariant's
     // packet shape and cut from the last scheduled forward's re-traversals: the 16-slot hit buffer with
     // six blocks per SM is faster where few rays composite more than 16 hits, the 32-slot one with
@@ -1803,7 +1896,6 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     const bool automatic = p.trace_variant <= 0;
     const int v = p.trace_variant > 0 ? p.trace_variant : kDefaultTraceVariant;
     const int fcut = (v >> 3) & 3;
-    const bool claim = (v & 32) != 0;
     q.kern_wide = nullptr;
     a.tile_w = (v & 4) ? 4 : 8;
     a.tile_h = 32 / a.tile_w;
@@ -1817,7 +1909,6 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     q.sched = p.hitlist.schedule && a.ntiles > 0 && (size_t)a.ntiles <= (words - kSchedHeader) / 2;
 #define GRAY_FWD_KERNEL(KB, MINB)                                                                   \
     (!q.sched ? reinterpret_cast<const void *>(&trace_forward_kernel<KB, MINB>)                     \
-     : claim  ? reinterpret_cast<const void *>(&trace_forward_claim_kernel<KB, MINB>)               \
               : reinterpret_cast<const void *>(&trace_forward_sched_kernel<KB, MINB>))
     switch (v & 3) {
         case 0: q.kern = GRAY_FWD_KERNEL(32, 1); break;

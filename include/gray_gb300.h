@@ -172,8 +172,8 @@ typedef struct gray_params {
     int32_t *status; /* device int32, GRAY_STATUS_* bits */
     /* forward-trace kernel variant: bits 0-1 = physical hit buffer of 32 or 16 keys and register
      * cap, bit 2 = 8x4 or 4x8 pixel packets, bits 3-4 = where a pixel tile's traversals start (BVH
-     * nodes of at most 64, 32 or 128 leaves that the tile's frustum reaches, or the root), bit 5 =
-     * how the scheduled launch hands out work (one pixel tile per block, or one packet per warp).
+     * nodes of at most 64, 32 or 128 leaves that the tile's frustum reaches, or the root), bit 5 is
+     * accepted and has no effect.
      * 0 (default): 4x8 packets from 64-leaf frontiers, with the 16-key buffer (six blocks per SM)
      * or the 32-key one (four blocks per SM) chosen on the device from the previous scheduled
      * forward of the same schedule buffer (the 32-key one when more than 1/8 of its packets
@@ -186,7 +186,7 @@ typedef struct gray_params {
  * No reference counterpart: the reference renders one view per OptiX launch
  * (cuda/raytracer.h:104-114 forward_pass_display).  A batch renders any number of views of one or
  * several resident scenes, each at its own resolution, forward only (inference), in one launch
- * whose warps pull 32-ray packets from a global counter.  Per pixel the result is bit-identical to
+ * whose blocks pull groups of 2x2 32-ray packets from a global counter.  Per pixel the result is bit-identical to
  * gray_forward_pass_display of the same view. */
 typedef struct gray_batch_scene {
     const float *geom, *live, *nodes, *root_box; /* a scene's gray_scene buffers after rebuild/update */

@@ -705,9 +705,9 @@ static int hit_local(const float lo[3], const float ld[3]) {
     return !(fdot3(u, u) > 1.0f);
 }
 
-/* Restatement of the CUDA path's division-free pretest (may_hit_local): 0 means "certainly no
- * hit".  Not part of the reference's algorithm: the kernels use it to skip pairs before the
- * intersection program, so it must never reject a pair that hit_local() accepts. */
+/* A division-free pretest of one pair by its cross product: 0 means "certainly no hit".  Not part of
+ * the reference's algorithm, and no longer on the CUDA path (its tiles test candidates as conics);
+ * it must never reject a pair that hit_local() accepts. */
 static int may_hit_local(const float lo[3], const float ld[3]) {
     const float b = fdot3(lo, ld);
     if (b > 0.0f) return 0;
