@@ -21,8 +21,15 @@ namespace gray {
 // and the degree-7 Taylor polynomial of e^r in Horner form; 2^k applied through the exponent
 // field (two steps for results in the subnormal range).
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ float exp_poly(float x, int &ki) {
-    float k = rintf(x * 0x1.715476p+0f);
+// k = the integer nearest to x log2(e) (ties to even): adding 1.5 2^23 rounds to it and leaves its low
+// bits in the sum's significand, so no float-integer conversion is needed (|x log2(e)| < 2^22).  The
+// hit loop is a chain of dependent operations, and conversions go through a unit of a quarter of the
+// rate: without them here, in the log and in the fixed-point sum, the forward of 3M / 1080p went from
+// 2.60 to 2.52 ms (16-key kernel 3.65 to 3.53 ms).
+__device__ __forceinline__ float exp_poly(float x, int &kbits) {
+    const float t = x * 0x1.715476p+0f + 0x1.8p23f;
+    kbits = __float_as_int(t);
+    const float k = t - 0x1.8p23f;
     float r = fmaf(-k, 0x1.62ep-1f, x);
     r = fmaf(-k, 0x1.0bfbe8p-15f, r);
     float p = 0x1.a01a02p-13f;
@@ -33,7 +40,6 @@ __device__ __forceinline__ float exp_poly(float x, int &ki) {
     p = fmaf(p, r, 0x1.0p-1f);
     p = fmaf(p, r, 1.0f);
     p = fmaf(p, r, 1.0f);
-    ki = (int)k;
     return p;
 }
 
@@ -42,12 +48,13 @@ __device__ __forceinline__ float gexp(float x) {
     // |x| <= 87: k in [-126, 126], 2^k a normal float (the hit loop's case: one test)
     if (fabsf(x) <= 87.0f) {
         float p = exp_poly(x, ki);
-        return p * __int_as_float((ki + 127) << 23);
+        return p * __int_as_float((ki << 23) + 0x3f800000);  // the shift leaves k alone in the exponent
     }
     if (x != x) return x;
     if (x > 89.0f) return __int_as_float(0x7f800000);
     if (x < -104.0f) return 0.0f;
     float p = exp_poly(x, ki);
+    ki -= 0x4b400000;
     if (ki > 127) {
         p = p * 2.0f;
         ki -= 1;
@@ -60,11 +67,11 @@ __device__ __forceinline__ float gexp(float x) {
 }
 
 // log: x = m 2^e, m in [sqrt(1/2), sqrt(2)]; log m = 2 atanh(s), s = (m-1)/(m+1), series to s^11.
-__device__ __forceinline__ float log_poly(float m, int e) {
-    if (m > 0x1.6a09e6p+0f) {
-        m = m * 0.5f;
-        e += 1;
-    }
+// For a positive normal x with bits u, subtracting the bits of sqrt(1/2) (rounded up) leaves e in the
+// exponent field; e becomes a float by the same addition trick as in exp.
+__device__ __forceinline__ float log_normal(uint32_t u, int de) {
+    const int e = (int)(u - 0x3f3504f4u) >> 23;
+    float m = __uint_as_float(u - ((uint32_t)e << 23));
     float f = m - 1.0f;
     float s = f / (2.0f + f);
     float z = s * s;
@@ -75,22 +82,19 @@ __device__ __forceinline__ float log_poly(float m, int e) {
     q = fmaf(q, z, 0x1.555556p-2f);
     float two_s = 2.0f * s;
     float lm = fmaf(two_s * z, q, two_s);
-    float ef = (float)e;
+    float ef = __int_as_float(0x4b400000 + e + de) - 0x1.8p23f;
     return fmaf(ef, 0x1.62ep-1f, fmaf(ef, 0x1.0bfbe8p-15f, lm));
 }
 
 __device__ __forceinline__ float glog(float x) {
     uint32_t u = __float_as_uint(x);
     // positive normal x (the hit loop's case: one test)
-    if (u - 0x00800000u < 0x7f000000u)
-        return log_poly(__uint_as_float((u & 0x007fffffu) | 0x3f800000u), (int)(u >> 23) - 127);
+    if (u - 0x00800000u < 0x7f000000u) return log_normal(u, 0);
     if (x != x) return x;
     if (x < 0.0f) return __int_as_float(0x7fc00000);
     if (x == 0.0f) return __int_as_float(0xff800000);
     if (x == __int_as_float(0x7f800000)) return x;
-    x = x * 0x1.0p23f;  // positive subnormal
-    u = __float_as_uint(x);
-    return log_poly(__uint_as_float((u & 0x007fffffu) | 0x3f800000u), (int)(u >> 23) - 127 - 23);
+    return log_normal(__float_as_uint(x * 0x1.0p23f), -23);  // positive subnormal
 }
 
 __device__ __forceinline__ float gpow(float a, float b) { return gexp(b * glog(a)); }
@@ -241,7 +245,19 @@ __device__ __forceinline__ bool intersect(const float4 g0, const float4 g1, cons
 // number of hits.
 constexpr long long kLogFixFloor = -105LL * (1LL << 40);
 __device__ __forceinline__ void add_log_transmittance(long long &s, float alpha) {
-    if (s > kLogFixFloor) s += to_fixed(glog(1.0f - alpha), 0x1.0p40f);
+    if (!(s > kLogFixFloor)) return;
+    const float v = -glog(1.0f - alpha);
+    if (v >= 0.0f && v < 16.0f) {
+        // v >= 0 split exactly as i 2^-19 + r, r < 2^-19: adding 2^23 with rounding toward zero leaves
+        // floor(v 2^19), then floor(r 2^40), in the significand (to_fixed's truncation in 8 instead of
+        // about 25 instructions)
+        const float i = __fmaf_rz(v, 0x1.0p19f, 0x1.0p23f);
+        const float r = fmaf(-(i - 0x1.0p23f), 0x1.0p-19f, v);
+        const float j = __fmaf_rz(r, 0x1.0p40f, 0x1.0p23f);
+        s -= ((long long)(__float_as_int(i) - 0x4b000000) << 21) + (long long)(__float_as_int(j) - 0x4b000000);
+    } else {
+        s -= to_fixed(v, 0x1.0p40f);
+    }
 }
 __device__ __forceinline__ float full_transmittance(long long s) { return gexp(__ll2float_rn(s) * 0x1.0p-40f); }
 
