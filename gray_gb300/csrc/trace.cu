@@ -402,8 +402,8 @@ __device__ __forceinline__ f3 cross3(f3 a, f3 b) {
 
 // Coefficients (F, D, E, A, B, C) of h(x, y) = F + x (D + x A + y B) + y (E + y C) for the candidate
 // with snapshot rows g0..g2 (columns M) and object-space origin lo.
-__device__ __forceinline__ void conic_coefficients(const ConicBasis &cb, const float4 g0, const float4 g1,
-                                                   const float4 g2, f3 lo, float q[6]) {
+__device__ __forceinline__ float conic_coefficients(const ConicBasis &cb, const float4 g0, const float4 g1,
+                                                    const float4 g2, f3 lo, float q[6]) {
     const f3 v0 = mk3(cb.v0[0], cb.v0[1], cb.v0[2]), du = mk3(cb.du[0], cb.du[1], cb.du[2]),
              dv = mk3(cb.dv[0], cb.dv[1], cb.dv[2]);
     const f3 l0 = mk3(fdot3(g0, v0), fdot3(g1, v0), fdot3(g2, v0));
@@ -426,6 +426,7 @@ __device__ __forceinline__ void conic_coefficients(const ConicBasis &cb, const f
     q[3] = ok ? lluu - ccuu : 0.0f;
     q[4] = ok ? 2.0f * (fdot3(lu, lv) - fdot3(cu, cv)) : 0.0f;
     q[5] = ok ? llvv - ccvv : 0.0f;
+    return -__fdividef(fdot3(lo, l0), ll0);
 }
 
 // Shared memory of a block that traces one pixel tile (one ray per thread).
@@ -439,7 +440,7 @@ struct TileShared {
     float sf[kBatch];          // live scaling factor
     uint32_t gid[kBatch];
     uint32_t stk[kTileStack];
-    uint32_t queue[kTileQueue];
+    alignas(16) uint32_t queue[kTileQueue];
     Frustum fr;
     ConicBasis cb;
     uint32_t cnt[kWarps];      // per-warp counts of a step
@@ -449,7 +450,11 @@ struct TileShared {
 // leaves beyond them move to the front of the queue).  (1) Thread j takes leaf j: it tests the leaf's
 // ellipsoid against the tile's frustum, fetches its snapshot rows, live values and colour, computes
 // its object-space ray origin (with local_origin, the arithmetic of local_ray) and its conic, and the
-// survivors are compacted into the shared cache.  A tile's four warps share the fetched records and
+// survivors go to the shared cache in order of their max-density points along the tile's central ray
+// (each thread ranks its key among the batch's 128: 32 16-byte loads), so that a ray finds its hits
+// nearly front to back and its sorted buffer mostly appends: unsorted batches cost 2.60 instead of
+// 2.38 ms at 3M / 1080p and 2.27 instead of 2.20 ms in a train step at 1M / 1600x1040; a scene of few
+// hits per ray pays the ranking (500k / 640x480 0.671 to 0.686 ms).  A tile's four warps share the fetched records and
 // the batch spans up to 128 candidates, where packets of their own batches fetched every record up to
 // four times and tested 21 survivors at a time.  (2) Every ray evaluates the conics at its pixel, two
 // candidates per step, into a bit mask of its possible hits.  (3) The lanes of a warp walk their masks
@@ -461,7 +466,6 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
                                                    float py, bool want, bool first, LaneState &st,
                                                    TileShared<KB> &sh, int take, int nc) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t lanemask_lt = (1u << lane) - 1u;
     {
         uint32_t gid = 0;
         bool keep = false;
@@ -469,6 +473,7 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
         int4 cv;
         float sfv = 0.0f;
         float q[6];
+        uint32_t key = 0xffffffffu;  // order along the tile's central ray; dropped leaves sort last
         if (t < take) {
             gid = sh.queue[t];
             g0 = sc.geom[3 * (size_t)gid];
@@ -482,7 +487,8 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
             cv = make_int4(colour_fixed(c0), colour_fixed(c1), colour_fixed(c2), __float_as_int(lv.x));
             sfv = lv.y;
             const f3 lo = local_origin(g0, g1, g2, ro);
-            conic_coefficients(sh.cb, g0, g1, g2, lo, q);
+            const float at = conic_coefficients(sh.cb, g0, g1, g2, lo, q);
+            if (keep) key = (__float_as_uint(fmaxf(at, 0.0f)) & ~(uint32_t)(kBatch - 1)) | (uint32_t)t;
             g0.w = lo.x;
             g1.w = lo.y;
             g2.w = lo.z;
@@ -495,9 +501,16 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
         __syncthreads();  // the counts; every read of the queue and of the previous batch's cache is done
         if (t < rest) sh.queue[t] = r0;
         if (t + kFwdThreads < rest) sh.queue[kFwdThreads + t] = r1;
+        uint32_t *keys = sh.queue + kTileQueue - kBatch;  // (free: fewer than kTileQueue - kBatch leaves are left)
+        keys[t] = key;
+        __syncthreads();
         if (keep) {
-            int slot = __popc(bal & lanemask_lt);
-            for (int w = 0; w < warp; w++) slot += (int)sh.cnt[w];
+            int slot = 0;
+#pragma unroll 4
+            for (int i = 0; i < kBatch / 4; i++) {
+                const uint4 o = reinterpret_cast<const uint4 *>(keys)[i];
+                slot += (o.x < key) + (o.y < key) + (o.z < key) + (o.w < key);
+            }
             sh.g[slot][0] = g0;
             sh.g[slot][1] = g1;
             sh.g[slot][2] = g2;
