@@ -810,11 +810,28 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
         if (want) {
             const int t = threadIdx.x;
             const unsigned long long last_key = st.kcount > 0 ? kbuf[st.kcount - 1][t] : 0ull;
+            // the next entry and its colour are fetched while this one is composited
+            unsigned long long next = st.kcount > 0 ? kbuf[0][t] : 0ull;
+            const float *nc0 = sc.channels + 3 * (size_t)(uint32_t)(next >> 16);
+            float nx = 0.0f, ny = 0.0f, nz = 0.0f;
+            if (st.kcount > 0) {
+                nx = nc0[0];
+                ny = nc0[1];
+                nz = nc0[2];
+            }
             for (int i = 0; i < st.kcount; i++) {
                 if constexpr (KB > 16) {
                     if (i == 16 && first) deep = true;
                 }
-                const unsigned long long key = kbuf[i][t];
+                const unsigned long long key = next;
+                const float cx = nx, cy = ny, cz = nz;
+                if (i + 1 < st.kcount) {
+                    next = kbuf[i + 1][t];
+                    const float *c = sc.channels + 3 * (size_t)(uint32_t)(next >> 16);
+                    nx = c[0];
+                    ny = c[1];
+                    nz = c[2];
+                }
                 const float d = h2f_bits((uint16_t)(key >> 48));
                 if (!(d > tmin_sel)) continue;
                 if (slots == kPassSlots) {
@@ -839,8 +856,6 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
                 }
                 const uint32_t gid = (uint32_t)(key >> 16);
                 const float al = h2f_bits((uint16_t)(key & 0xFFFFu));
-                const float *c = sc.channels + 3 * (size_t)gid;
-                const float cx = c[0], cy = c[1], cz = c[2];
                 const long long a = alpha16_fixed((uint16_t)(key & 0xFFFFu));
                 st.afx -= a;
                 st.cfx0 -= mul_fixed(a, colour_fixed(cx));
