@@ -44,10 +44,15 @@ constexpr int kTileStack = 448;   // per-block traversal stack
 constexpr int kTileQueue = kBatch + 2 * kFwdThreads;  // queued leaves: < kBatch before a step, + up to 2 per thread
 static_assert(kBatch == kFwdThreads, "one leaf per thread");
 constexpr int kSchedHeader = 64;  // schedule words before the per-tile estimates
-// Header words [kSchedZeroWords, kSchedHeader) outlive a forward: the automatic kernel choice (see
-// plan_forward) keeps there the packet counts of the last scheduled forward and the choice the scan
-// kernel made from them; only the words before them are cleared at the start of a schedule.
-constexpr int kSchedZeroWords = 48;
+constexpr int kSchedItems = 1;       // header word: tiles of the work order
+constexpr int kSchedSplitNext = 2;   // work counter of the split tiles' packets
+constexpr int kSchedSplitItems = 3;  // packets of split tiles
+constexpr int kItemShift = 29;       // a split tile's packet: its tile, and the packet from this bit on
+constexpr uint32_t kItemTile = (1u << kItemShift) - 1u;
+constexpr int kOrderPerTile = 5;     // words of the work order per tile: itself, or its four packets
+// Header words [kStatPackets, kStatChoice] outlive a forward: the automatic kernel choice (see
+// plan_forward) keeps there the packet counts of the last scheduled forward and the choice the order
+// kernel made from them.
 constexpr int kStatPackets = 48;   // packets traced by the last scheduled forward
 constexpr int kStatRetraced = 49;  // of them, packets that need more than one traversal with 16 slots
 constexpr int kStatChoice = 50;    // kernel of the automatic choice: kChoiceNarrow or kChoiceWide
@@ -79,6 +84,7 @@ struct FwdArgs {
     int auto_role;  // 0, or kChoiceNarrow / kChoiceWide: the launch of the automatic choice this is
     uint32_t *schedule;  // work order of the pixel tiles (null: tiles in launch order)
     int tiles_x, ntiles;
+    int slots_narrow, slots_wide;  // blocks resident at once in the narrow and in the wide kernel
     uint32_t *frontier;  // per-tile BVH frontiers (null: packets start at the root)
     uint32_t frontier_cut;
     uint32_t *super_frontier;  // per super-tile coarse frontiers seeding the tile walks (null: root)
@@ -461,7 +467,7 @@ struct TileShared {
 // together, one candidate per lane per step, through the intersection program, which decides the hit,
 // and the selection.  The order in which a ray sees its hits does not matter: the all-hit sums are
 // order-independent and the selection is by key.
-template <int KB>
+template <int KB, bool SPLIT>
 __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px,
                                                    float py, bool want, bool first, LaneState &st,
                                                    TileShared<KB> &sh, int take, int nc) {
@@ -511,6 +517,8 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
                 const uint4 o = reinterpret_cast<const uint4 *>(keys)[i];
                 slot += (o.x < key) + (o.y < key) + (o.z < key) + (o.w < key);
             }
+            // split: pairs of ranks go round the four warps' words (see merge_split)
+            if constexpr (SPLIT) slot = 32 * ((slot >> 1) & 3) + 2 * (slot >> 3) + (slot & 1);
             sh.g[slot][0] = g0;
             sh.g[slot][1] = g1;
             sh.g[slot][2] = g2;
@@ -532,7 +540,13 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
 #pragma unroll
     for (int w = 0; w < kBatch / 32; w++) {
         m[w] = 0u;
-        if (32 * w < kept) {
+        // candidates of this word (the rest of its slots are stale); split: of this warp's word alone
+        int left = kept - 32 * w;
+        if constexpr (SPLIT) {
+            const int mine = kept - 2 * warp;  // ranks from 2 warp on, two of every eight
+            left = w == warp ? 2 * (mine >> 3) + min(mine & 7, 2) : 0;
+        }
+        if (left > 0) {
             uint32_t miss = 0u;  // candidate 32 w + i ends up in bit 31 - i
 #pragma unroll 4
             for (int i = 0; i < 16; i++) {
@@ -544,7 +558,6 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
                 miss = __funnelshift_l(__float_as_uint(h.x), miss, 1);
                 miss = __funnelshift_l(__float_as_uint(h.y), miss, 1);
             }
-            const int left = kept - 32 * w;  // candidates of this word (the rest of its slots are stale)
             const uint32_t valid = left >= 32 ? 0xffffffffu : ~(0xffffffffu >> left);
             m[w] = want ? ~miss & valid : 0u;
         }
@@ -586,10 +599,10 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
 // goes onto the stack with its first entry on top, and a frontier leaf is queued when it is popped.
 // px, py: the ray's offset from the tile's centre in the conics' basis.  Returns false if the stack
 // filled up (the caller then repeats the traversal per ray).
-template <int KB>
+template <int KB, bool SPLIT>
 __device__ __forceinline__ bool traverse_tile(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px,
-                                              float py, bool want, bool first, LaneState &st, TileShared<KB> &sh,
-                                              const uint32_t *front, int32_t *status) {
+                                              float py, bool want, bool first, LaneState &st,
+                                              TileShared<KB> &sh, const uint32_t *front, int32_t *status) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
     const int n = sc.n;
@@ -679,20 +692,110 @@ __device__ __forceinline__ bool traverse_tile(const TraceScene &sc, const TraceK
         }
         if (nc == 0) break;
         const int take = min(nc, kBatch);
-        trace_batch_leaves<KB>(sc, k, ro, rd, px, py, want, first, st, sh, take, nc);
+        trace_batch_leaves<KB, SPLIT>(sc, k, ro, rd, px, py, want, first, st, sh, take, nc);
         nc -= take;
     }
     return true;
 }
 
+// A split tile's block traces one packet: its four warps hold the same 32 rays and each took a quarter of
+// the candidates.  After a traversal every thread calls this together, and every warp then holds the
+// rays' whole state: the all-hit sums added up (integers, so the order does not matter; a sum that
+// stopped at its floor stays at or below it), and the order of the four warps' keys: entry (w, i) of
+// rank r is named by src[32 r + lane] = 32 w + i.  The ranks are complete up to the last key of a
+// buffer that was full and dropped keys; at most kSplitKeys of them are kept.  The cache's memory
+// carries all of it, and the composited ids (see trace_rays).
+constexpr int kSplitKeys = 64;
+
+template <int KB>
+struct SplitView {
+    uint32_t *gids;  // [kSplitKeys][32]
+    uint8_t *src;    // [kSplitKeys][32]
+    int *bound;      // [kWarps][32]
+    __device__ __forceinline__ explicit SplitView(TileShared<KB> &sh)
+        : gids(reinterpret_cast<uint32_t *>(sh.g)), src(reinterpret_cast<uint8_t *>(sh.conic)),
+          bound(reinterpret_cast<int *>(sh.sf)) {}
+};
+
+template <int KB>
+__device__ __forceinline__ void merge_split(LaneState &st, TileShared<KB> &sh, bool first) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    long long *sums = reinterpret_cast<long long *>(sh.g);          // [5][128]
+    int *counts = reinterpret_cast<int *>(sums + 5 * kFwdThreads);  // [3][128]
+    const SplitView<KB> v(sh);
+    static_assert((5 * 8 + 3 * 4) * kFwdThreads <= sizeof(sh.g) + sizeof(sh.c), "sums do not fit");
+    static_assert(kSplitKeys * 32 * 4 <= sizeof(sh.g) + sizeof(sh.c) && kSplitKeys * 32 <= sizeof(sh.conic) &&
+                      KB <= 32 && kWarps * 32 * 4 <= sizeof(sh.sf),
+                  "a split packet's keys do not fit");
+    __syncthreads();  // every warp is done with the cache
+    if (first) {
+        sums[t] = st.lfx;
+        sums[kFwdThreads + t] = st.afx;
+        sums[2 * kFwdThreads + t] = st.cfx0;
+        sums[3 * kFwdThreads + t] = st.cfx1;
+        sums[4 * kFwdThreads + t] = st.cfx2;
+        counts[t] = st.nhit;
+    }
+    counts[kFwdThreads + t] = st.ncand;
+    counts[2 * kFwdThreads + t] = st.kcount;
+    __syncthreads();
+    const int own = st.kcount;
+    const bool full = st.ncand > st.kcount;  // this warp's buffer dropped keys
+    int total = 0, kc[kWarps], at[kWarps];
+    st.ncand = 0;
+    if (first) {
+        st.lfx = st.afx = st.cfx0 = st.cfx1 = st.cfx2 = 0;
+        st.nhit = 0;
+    }
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        const int o = 32 * w + lane;
+        if (first) {
+            st.lfx += sums[o];
+            st.afx += sums[kFwdThreads + o];
+            st.cfx0 += sums[2 * kFwdThreads + o];
+            st.cfx1 += sums[3 * kFwdThreads + o];
+            st.cfx2 += sums[4 * kFwdThreads + o];
+            st.nhit += counts[o];
+        }
+        st.ncand += counts[kFwdThreads + o];
+        kc[w] = counts[2 * kFwdThreads + o];
+        total += kc[w];
+        at[w] = 0;
+    }
+    int bound = kSplitKeys;
+    for (int i = 0; i < own; i++) {
+        const unsigned long long key = sh.kbuf[i][t];
+        int rank = i;
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) {
+            if (w != warp) {
+                while (at[w] < kc[w] && sh.kbuf[at[w]][32 * w + lane] < key) at[w]++;
+                rank += at[w];
+            }
+        }
+        if (rank >= kSplitKeys) break;
+        v.src[32 * rank + lane] = (uint8_t)(32 * warp + i);
+        if (full && i == own - 1) bound = rank + 1;
+    }
+    v.bound[t] = bound;
+    __syncthreads();  // the ranks; the sums have been read
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) total = min(total, v.bound[32 * w + lane]);
+    st.kcount = total;
+}
+
 // Trace a block's rays (one per thread; `alive` threads only) through the scene: traversal, selection,
 // compositing (cuda/forward_pass.cu:6-151 minus the write-out).  tile: the block's rays share one origin
 // and lie inside sh.fr, and are traversed together from the frontier `front` (see traverse_tile, px,
-// py); else every warp traverses its own rays.  Every thread of the block calls this together.
-template <int KB>
+// py); else every warp traverses its own rays.  SPLIT: the four warps hold the same 32 rays and share
+// their candidates (see merge_split); each ends with the same result, and warp 0 alone writes hit
+// lists.  Every thread of the block calls this together.
+template <int KB, bool SPLIT>
 __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px, float py,
-                                           bool alive, bool tile, bool grads, const HitSink &hs, int32_t *status,
-                                           TileShared<KB> &sh, const uint32_t *front, RayResult &res) {
+                                           bool alive, bool tile, bool grads, const HitSink &hs,
+                                           int32_t *status, TileShared<KB> &sh, const uint32_t *front,
+                                           RayResult &res) {
     unsigned long long(*kbuf)[kFwdThreads] = sh.kbuf;
     const int lane = threadIdx.x & 31;
     LaneState &st = res.st;
@@ -722,7 +825,13 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
         st.ncand = 0;
         // ---------------- traversal ----------------
         bool per_ray = !tile;
-        if (tile && !traverse_tile<KB>(sc, k, ro, rd, px, py, want, first, st, sh, front, status)) {
+        bool ranked = false;  // the keys are those of the four warps, in merge_split's order
+        if (tile && traverse_tile<KB, SPLIT>(sc, k, ro, rd, px, py, want, first, st, sh, front, status)) {
+            if constexpr (SPLIT) {
+                merge_split<KB>(st, sh, first);
+                ranked = true;
+            }
+        } else if (tile) {
             // the tile's stack filled up: discard what was gathered, trace per ray
             st.kcount = 0;
             st.ncand = 0;
@@ -807,11 +916,27 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
         }
         // ---------------- consume (cuda/forward_pass.cu:46-125) ----------------
         int nc = 0;
+        const auto key_at = [&](int i) -> unsigned long long {
+            if constexpr (SPLIT) {
+                if (ranked) {
+                    const uint32_t s = SplitView<KB>(sh).src[32 * i + lane];
+                    return kbuf[s & 31u][(s & ~31u) + lane];
+                }
+            }
+            return kbuf[i][threadIdx.x];
+        };
+        // composited ids replace the keys already looked at (split: the keys are shared by the warps,
+        // so every warp writes the same ids beside them)
+        const auto gid_at = [&](int i) -> uint32_t & {
+            if constexpr (SPLIT) {
+                if (ranked) return SplitView<KB>(sh).gids[32 * i + lane];
+            }
+            return *reinterpret_cast<uint32_t *>(&kbuf[i][threadIdx.x]);
+        };
         if (want) {
-            const int t = threadIdx.x;
-            const unsigned long long last_key = st.kcount > 0 ? kbuf[st.kcount - 1][t] : 0ull;
+            const unsigned long long last_key = st.kcount > 0 ? key_at(st.kcount - 1) : 0ull;
             // the next entry and its colour are fetched while this one is composited
-            unsigned long long next = st.kcount > 0 ? kbuf[0][t] : 0ull;
+            unsigned long long next = st.kcount > 0 ? key_at(0) : 0ull;
             const float *nc0 = sc.channels + 3 * (size_t)(uint32_t)(next >> 16);
             float nx = 0.0f, ny = 0.0f, nz = 0.0f;
             if (st.kcount > 0) {
@@ -820,13 +945,13 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
                 nz = nc0[2];
             }
             for (int i = 0; i < st.kcount; i++) {
-                if constexpr (KB > 16) {
+                if constexpr (KB > 16 || SPLIT) {
                     if (i == 16 && first) deep = true;
                 }
                 const unsigned long long key = next;
                 const float cx = nx, cy = ny, cz = nz;
                 if (i + 1 < st.kcount) {
-                    next = kbuf[i + 1][t];
+                    next = key_at(i + 1);
                     const float *c = sc.channels + 3 * (size_t)(uint32_t)(next >> 16);
                     nx = c[0];
                     ny = c[1];
@@ -867,7 +992,7 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
                 C2 = C2 + cz * w;
                 if (k.render_depth) depth = depth + d * w;
                 T = T * (1.0f - al);
-                kbuf[nc][t] = gid;
+                gid_at(nc) = gid;
                 nc++;
                 nacc++;
                 if (T < k.tthr) {
@@ -899,7 +1024,7 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
         }
         // ---------------- backward hit list segment (warp aggregated) ----------------
         if (grads) {
-            const uint32_t need = nc > 0 ? (uint32_t)nc + 2u : 0u;
+            const uint32_t need = nc > 0 && (!SPLIT || threadIdx.x < 32) ? (uint32_t)nc + 2u : 0u;
             uint32_t incl = need;
 #pragma unroll
             for (int off = 1; off < 32; off <<= 1) {
@@ -918,7 +1043,7 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
                 if (fits) {
                     hs.pool[off] = head;
                     hs.pool[off + 1] = (uint32_t)nc;
-                    for (int j = 0; j < nc; j++) hs.pool[off + 2 + j] = (uint32_t)kbuf[j][threadIdx.x];
+                    for (int j = 0; j < nc; j++) hs.pool[off + 2 + j] = gid_at(j);
                     head = off;
                 } else {
                     raise_status(status, GRAY_STATUS_HITLIST_OVERFLOW);
@@ -1001,14 +1126,19 @@ __device__ __forceinline__ void make_conic_basis(ConicBasis &cb, const float *w,
     cb.mag = 2.0f * (sqrtf(n0) * fabsf(ax) + sqrtf(n1) * fabsf(vs)) + sqrtf(n2);
 }
 
-// The block's pixel tile (bx, by): 2x2 packets of tile_w x tile_h pixels, one packet per warp.  Returns
-// whether the calling warp's packet needs more than one traversal with 16 hit slots (RayResult::retraced).
-template <int KB>
-__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, TileShared<KB> &sh) {
+// The block's pixel tile (bx, by): 2x2 packets of tile_w x tile_h pixels, one packet per warp; or, SPLIT:
+// packet sub of it alone, its candidates shared by the four warps.  Returns whether the calling
+// warp's packet needs more than one traversal with 16 hit slots (RayResult::retraced).
+template <int KB, bool SPLIT>
+__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, int sub, TileShared<KB> &sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int tx0 = bx * (a.tile_w * kBlockWarpsX), ty0 = by * (a.tile_h * kBlockWarpsY);
-    const int px = tx0 + (warp % kBlockWarpsX) * a.tile_w + (lane % a.tile_w);
-    const int py = ty0 + (warp / kBlockWarpsX) * a.tile_h + (lane / a.tile_w);
+    const int rw = SPLIT ? a.tile_w : a.tile_w * kBlockWarpsX, rh = SPLIT ? a.tile_h : a.tile_h * kBlockWarpsY;
+    const int pk = SPLIT ? sub : warp;  // the warp's packet
+    const int px0 = bx * (a.tile_w * kBlockWarpsX) + (pk % kBlockWarpsX) * a.tile_w;
+    const int py0 = by * (a.tile_h * kBlockWarpsY) + (pk / kBlockWarpsX) * a.tile_h;
+    // the pixels the block traces start at (tx0, ty0)
+    const int tx0 = SPLIT ? px0 : bx * (a.tile_w * kBlockWarpsX), ty0 = SPLIT ? py0 : by * (a.tile_h * kBlockWarpsY);
+    const int px = px0 + (lane % a.tile_w), py = py0 + (lane / a.tile_w);
     const bool inside = px < (int)a.render_w && py < (int)a.render_h;
     const uint32_t pixel = (uint32_t)py * a.alloc_w + (uint32_t)px;
 
@@ -1048,21 +1178,21 @@ __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, T
 
     // camera rays share the origin: the block traverses its tile together
     const bool tile = !*a.rays_from_python && !*a.jitter;
-    const float hx = (float)(a.tile_w * kBlockWarpsX - 1) * 0.5f, hy = (float)(a.tile_h * kBlockWarpsY - 1) * 0.5f;
+    const float hx = (float)(rw - 1) * 0.5f, hy = (float)(rh - 1) * 0.5f;
     const uint32_t *front = nullptr;
     if (tile) {
         // (the loop of trace_rays starts with a block barrier)
         if (warp == 0)
             make_frustum_warp(sh.fr, mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, tx0, ty0,
-                              tx0 + a.tile_w * kBlockWarpsX - 1, ty0 + a.tile_h * kBlockWarpsY - 1, a.render_w,
-                              a.render_h, a.root_box);
+                              tx0 + rw - 1, ty0 + rh - 1, a.render_w, a.render_h, a.root_box);
         if (threadIdx.x == kFwdThreads - 1)
             make_conic_basis(sh.cb, a.w2c, *a.fov, (float)tx0 + hx, (float)ty0 + hy, hx, hy, a.render_w, a.render_h);
         if (a.frontier) front = a.frontier + (size_t)(by * a.tiles_x + bx) * kFrontierWords;
     }
     RayResult r;
-    trace_rays<KB>(sc, k, ro, rd, (float)(px - tx0) - hx, (float)(py - ty0) - hy, alive, tile, grads, hs, a.status, sh,
-                   front, r);
+    trace_rays<KB, SPLIT>(sc, k, ro, rd, (float)(px - tx0) - hx, (float)(py - ty0) - hy, alive, tile, grads, hs,
+                          a.status, sh, front, r);
+    if (SPLIT && warp != 0) return false;
     if (!inside) return r.retraced;
     if (!alive) {
         a.head[pixel] = GRAY_NULL;  // inactive pixel: empty list, nothing else written
@@ -1102,12 +1232,21 @@ __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, T
     return r.retraced;
 }
 
+// Programmatic launches (see launch_trace_forward): a kernel of the chain lets the next one start once
+// all of its blocks have (griddepcontrol.launch_dependents), and block 0 of each waits at its end for
+// the launch before it to complete (griddepcontrol.wait; nothing to wait for in an ordinary launch), so
+// that the last one's completion is the chain's.  The other blocks leave their SM to the next kernel.
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait_before() {
+    if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Grid launch: block (x, y) renders tile (x, y).
 template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_kernel(const FwdArgs a) {
     __shared__ TileShared<KB> sh;
     if (*a.render_ellipsoids) return;  // the ellipsoid view (ellipsoid_kernel) renders this frame
-    forward_tile<KB>(a, blockIdx.x, blockIdx.y, sh);
+    forward_tile<KB, false>(a, blockIdx.x, blockIdx.y, 0, sh);
 }
 
 // Persistent launch: the blocks take tiles from the schedule's order, densest first, until none is
@@ -1119,25 +1258,66 @@ template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(const FwdArgs a) {
     __shared__ TileShared<KB> sh;
     __shared__ uint32_t s_next, s_packets, s_retraced;
-    if (*a.render_ellipsoids) return;
-    // automatic choice: both kernels are launched, the one the scan kernel did not choose leaves
-    if (a.auto_role != 0 && a.schedule[kStatChoice] != (uint32_t)a.auto_role) return;
+    grid_launch_next();
+    // automatic choice: both kernels are launched, the one the order kernel did not choose leaves
+    if (*a.render_ellipsoids || (a.auto_role != 0 && a.schedule[kStatChoice] != (uint32_t)a.auto_role)) {
+        grid_wait_before();
+        return;
+    }
     if (threadIdx.x == 0) {
         s_packets = 0u;
         s_retraced = 0u;
     }
+    const uint32_t items = a.schedule[kSchedItems];
     for (;;) {
         __syncthreads();  // every thread is done with the previous tile (s_next, the frontier, counts)
         if (threadIdx.x == 0) s_next = atomicAdd(a.schedule, 1u);
         __syncthreads();
         const uint32_t t = s_next;
-        if (t >= (uint32_t)a.ntiles) break;
+        if (t >= items) break;
         const uint32_t tile = a.schedule[kSchedHeader + a.ntiles + t];
         const bool again =
-            forward_tile<KB>(a, (int)(tile % (uint32_t)a.tiles_x), (int)(tile / (uint32_t)a.tiles_x), sh);
+            forward_tile<KB, false>(a, (int)(tile % (uint32_t)a.tiles_x), (int)(tile / (uint32_t)a.tiles_x), 0, sh);
         if ((threadIdx.x & 31) == 0) {
             atomicAdd(&s_packets, 1u);
             if (again) atomicAdd(&s_retraced, 1u);
+        }
+    }
+    if (threadIdx.x == 0 && s_packets > 0u) {
+        atomicAdd(&a.schedule[kStatPackets], s_packets);
+        atomicAdd(&a.schedule[kStatRetraced], s_retraced);
+    }
+    grid_wait_before();
+}
+
+// The split tiles' packets (see sched_order_kernel), launched before the kernel of the whole tiles, which
+// starts as soon as this one's blocks have and fills what they leave free.  A kernel of its own: with
+// both bodies in one, the whole tiles' loop lost registers (3M / 1080p 2.28 to 2.33 ms with a run-time
+// switch, 2.44 ms with two inlined bodies, 2.40 ms with a call).
+template <int KB, int MINB>
+__global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(const FwdArgs a) {
+    __shared__ TileShared<KB> sh;
+    __shared__ uint32_t s_next, s_packets, s_retraced;
+    grid_launch_next();
+    if (*a.render_ellipsoids) return;
+    const uint32_t items = a.schedule[kSchedSplitItems];
+    if (items == 0u) return;
+    if (threadIdx.x == 0) {
+        s_packets = 0u;
+        s_retraced = 0u;
+    }
+    for (;;) {
+        __syncthreads();  // every thread is done with the previous packet
+        if (threadIdx.x == 0) s_next = atomicAdd(a.schedule + kSchedSplitNext, 1u);
+        __syncthreads();
+        const uint32_t t = s_next;
+        if (t >= items) break;
+        const uint32_t item = a.schedule[kSchedHeader + 2 * a.ntiles + t], tile = item & kItemTile;
+        const bool again = forward_tile<KB, true>(a, (int)(tile % (uint32_t)a.tiles_x),
+                                                  (int)(tile / (uint32_t)a.tiles_x), (int)(item >> kItemShift), sh);
+        if (threadIdx.x == 0) {
+            s_packets++;
+            if (again) s_retraced++;
         }
     }
     if (threadIdx.x == 0 && s_packets > 0u) {
@@ -1161,8 +1341,8 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
 // super-tile's entries, testing each entry's own box against the tile's frustum, instead of from the
 // root.  Every leaf a ray of the tile can hit lies under an entry of the super-tile (its ancestors
 // meet the tile's frustum, hence the super-tile's), so the tile still reaches it.  Schedule words:
-// [0] work counter, [1..33] bucket counts/cursors, [kSchedHeader, +ntiles) estimates, [kSchedHeader +
-// ntiles, +ntiles) order, then (when frontiers are on) kFrontierWords words per tile, then
+// [0..3] work counters and lengths, [kSchedHeader, +ntiles) estimates, [kSchedHeader + ntiles, +ntiles)
+// order of the whole tiles, [kSchedHeader + 2 ntiles, +4 ntiles) of the split tiles' packets, then (when frontiers are on) kFrontierWords words per tile, then
 // kSuperWords words per super-tile.
 // ---------------------------------------------------------------------------------------------
 constexpr int kCostCut = 512;
@@ -1499,41 +1679,108 @@ __global__ void __launch_bounds__(32) tile_cost_kernel(const FwdArgs a, int bw, 
     } else if (out && lane == 0) {
         out[0] = kFrontierNone;
     }
-    if (lane == 0) {
-        a.schedule[kSchedHeader + tile] = est;
-        const uint32_t key = est ? (uint32_t)__clz(est) : 32u;  // larger estimate -> smaller key
-        atomicAdd(&a.schedule[1 + key], 1u);
-    }
+    if (lane == 0) a.schedule[kSchedHeader + tile] = est;
 }
 
-// Bucket offsets of the densest-first order; and the automatic kernel choice for this forward from
-// the last scheduled forward's packet counts (the narrow kernel when there are none yet).
-__global__ void sched_scan_kernel(uint32_t *sched) {
-    if (threadIdx.x != 0) return;
-    uint32_t acc = 0;
-    for (int k = 0; k <= 32; k++) {
-        const uint32_t c = sched[1 + k];
-        sched[1 + k] = acc;
-        acc += c;
-    }
-    const uint32_t packets = sched[kStatPackets], retraced = sched[kStatRetraced];
-    uint32_t choice = sched[kStatChoice];
-    if (choice != kChoiceNarrow && choice != kChoiceWide) choice = kChoiceNarrow;
-    if (packets > 0u && retraced <= packets)
-        choice = (unsigned long long)retraced * 16ull > (unsigned long long)packets * kWideSixteenths ? kChoiceWide
-                                                                                                     : kChoiceNarrow;
-    sched[kStatChoice] = choice;
-    sched[kStatPackets] = 0u;
-    sched[kStatRetraced] = 0u;
-}
+// The work order, one block: the tiles counting-sorted by log2 of their estimates, densest first, so that
+// the launch does not end with a dense tile started late; and the automatic kernel choice for this
+// forward from the last scheduled forward's packet counts (the narrow kernel when there are none yet).
+//
+// Dense tiles are split.  A tile whose estimate exceeds kSplitEighths / 8 of what the resident blocks
+// have to do on average (the sum of the estimates over the blocks resident at once) would still run when
+// the others are done: it is entered as its four packets, each traced by a block whose four warps share
+// its candidates (merge_split).  Below kSplitLeast leaves a tile is too short for that to pay.
+// Measured (render 500k / 640x480 and train step 301k / 799x533, us; unsplit 662 and 842, the longest
+// tile taking 2.7 times what the blocks had to do on average): 2/8 512 and 903, 3/8 490 and 840, 5/8 497
+// and 818, 8/8 560 and 818.  Split, a tile costs more (all of them split: 3M / 1080p 2.27 -> 5.09 ms), so
+// large frames, whose average is far above any tile, split none.
+constexpr int kOrderThreads = 1024;
+constexpr int kOrderAhead = 8;
+constexpr int kOrderBuckets = 33;  // leading zeros of an estimate
+constexpr unsigned long long kSplitEighths = 5;
+constexpr uint32_t kSplitLeast = 96;
+constexpr int kSplitBlocks = 4;  // blocks per SM of the split kernel
 
-__global__ void sched_scatter_kernel(uint32_t *sched, int ntiles) {
-    const int tile = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tile >= ntiles) return;
-    const uint32_t est = sched[kSchedHeader + tile];
-    const uint32_t key = est ? (uint32_t)__clz(est) : 32u;
-    const uint32_t pos = atomicAdd(&sched[1 + key], 1u);
-    if (pos < (uint32_t)ntiles) sched[kSchedHeader + ntiles + pos] = (uint32_t)tile;
+__global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sched, int ntiles, int slots_narrow,
+                                                                    int slots_wide) {
+    __shared__ unsigned long long s_sum[32];
+    __shared__ uint32_t s_bucket[2 * kOrderBuckets];  // whole tiles, then split ones
+    __shared__ uint32_t s_split;
+    const int t = threadIdx.x, lane = t & 31;
+    const uint32_t *est = sched + kSchedHeader;
+    unsigned long long sum = 0ull;
+#pragma unroll 8
+    for (int i = t; i < ntiles; i += kOrderThreads) sum += est[i];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
+    if (lane == 0) s_sum[t >> 5] = sum;
+    if (t < 2 * kOrderBuckets) s_bucket[t] = 0u;
+    __syncthreads();
+    if (t == 0) {
+        const uint32_t packets = sched[kStatPackets], retraced = sched[kStatRetraced];
+        uint32_t choice = sched[kStatChoice];
+        if (choice != kChoiceNarrow && choice != kChoiceWide) choice = kChoiceNarrow;
+        if (packets > 0u && retraced <= packets)
+            choice = (unsigned long long)retraced * 16ull > (unsigned long long)packets * kWideSixteenths
+                         ? kChoiceWide
+                         : kChoiceNarrow;
+        sched[kStatChoice] = choice;
+        sched[kStatPackets] = 0u;
+        sched[kStatRetraced] = 0u;
+        sched[0] = 0u;
+        sched[kSchedSplitNext] = 0u;
+        unsigned long long total = 0ull;
+        for (int w = 0; w < kOrderThreads / 32; w++) total += s_sum[w];
+        const unsigned long long slots = (unsigned long long)(choice == kChoiceWide ? slots_wide : slots_narrow);
+        const unsigned long long thr = total * kSplitEighths / (8ull * (slots > 0ull ? slots : 1ull));
+        s_split = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
+    }
+    __syncthreads();
+    const uint32_t split = s_split;
+    for (int pass = 0; pass < 2; pass++) {
+        // pass 0 counts the buckets' tiles, pass 1 writes them; the lanes of a warp that fall in one
+        // bucket share an atomic
+        uint32_t ahead[kOrderAhead];  // estimates of the next rounds, loaded together
+        for (int i0 = 0, r = 0; i0 < ntiles; i0 += kOrderThreads, r = (r + 1) % kOrderAhead) {
+            const int i = i0 + t;
+            if (r == 0) {
+#pragma unroll
+                for (int j = 0; j < kOrderAhead; j++)
+                    ahead[j] = i + j * kOrderThreads < ntiles ? est[i + j * kOrderThreads] : 0u;
+            }
+            const uint32_t e = ahead[0];
+#pragma unroll
+            for (int j = 0; j + 1 < kOrderAhead; j++) ahead[j] = ahead[j + 1];
+            const bool four = e > split;
+            const uint32_t key = i < ntiles ? (uint32_t)__clz((int)e) + (four ? (uint32_t)kOrderBuckets : 0u)
+                                            : 2u * kOrderBuckets;  // dense first
+            const uint32_t peers = __match_any_sync(kFull, key);
+            const int lead = __ffs((int)peers) - 1;
+            uint32_t base = 0u;
+            if (lane == lead && i < ntiles) base = atomicAdd(&s_bucket[key], (uint32_t)__popc(peers));
+            base = __shfl_sync(kFull, base, lead) + __popc(peers & ((1u << lane) - 1u));
+            if (pass == 1 && i < ntiles) {
+                uint32_t *out = sched + kSchedHeader + ntiles;
+                if (four) {
+                    out += ntiles + 4u * base;
+                    for (uint32_t s = 0; s < 4u; s++) out[s] = (uint32_t)i | s << kItemShift;
+                } else {
+                    out[base] = (uint32_t)i;
+                }
+            }
+        }
+        __syncthreads();
+        if (pass == 0 && t < 2) {
+            uint32_t acc = 0u;
+            for (int k = 0; k < kOrderBuckets; k++) {
+                const uint32_t c = s_bucket[t * kOrderBuckets + k];
+                s_bucket[t * kOrderBuckets + k] = acc;
+                acc += c;
+            }
+            sched[t == 0 ? kSchedItems : kSchedSplitItems] = t == 0 ? acc : 4u * acc;
+        }
+        __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1816,8 +2063,8 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
         const uint32_t grp = vw.group_offset + s_local;
         const uint32_t *front = frontier && grp < total_groups ? frontier + (size_t)grp * kFrontierWords : nullptr;
         RayResult r;
-        trace_rays<KB>(sc, k, ro, rd, (float)(px - x0) - hx, (float)(py - y0) - hy, inside, true, false,
-                       HitSink{nullptr, nullptr, 0}, status, sh, front, r);
+        trace_rays<KB, false>(sc, k, ro, rd, (float)(px - x0) - hx, (float)(py - y0) - hy, inside, true, false,
+                              HitSink{nullptr, nullptr, 0}, status, sh, front, r);
         if (!inside) continue;
         float r0, r1, r2;
         finish_ray(r, scenes[vw.scene].bg, 1e-12f, false, r0, r1, r2);
@@ -1874,6 +2121,7 @@ static FwdArgs forward_args(const gray_params &p, bool display) {
     a.status = p.status;
     a.render_ellipsoids = p.config.render_ellipsoids;
     a.ellipsoid_min_opacity = p.config.ellipsoid_min_opacity;
+    a.slots_narrow = a.slots_wide = 1;
     a.tile_w = 8;
     a.tile_h = 4;
     a.schedule = nullptr;
@@ -1934,7 +2182,8 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     a.ntiles = (int)(q.grid.x * q.grid.y);
     a.schedule = nullptr;
     const size_t words = gray_schedule_words_for(p.image_width, p.image_height);
-    q.sched = p.hitlist.schedule && a.ntiles > 0 && (size_t)a.ntiles <= (words - kSchedHeader) / 2;
+    q.sched = p.hitlist.schedule && a.ntiles > 0 &&
+              (size_t)a.ntiles <= (words - kSchedHeader) / (1 + kOrderPerTile);
 #define GRAY_FWD_KERNEL(KB, MINB)                                                                   \
     (!q.sched ? reinterpret_cast<const void *>(&trace_forward_kernel<KB, MINB>)                     \
               : reinterpret_cast<const void *>(&trace_forward_sched_kernel<KB, MINB>))
@@ -1952,13 +2201,14 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
             q.kern_wide = reinterpret_cast<const void *>(&trace_forward_sched_kernel<32, 4>);
         }
         a.frontier_cut = fcut == 0 ? kFrontierCutDefault : fcut == 1 ? 32u : fcut == 2 ? 128u : 0u;
-        if (a.frontier_cut > 0 && (size_t)a.ntiles <= (words - kSchedHeader) / (2 + kFrontierWords))
-            a.frontier = a.schedule + kSchedHeader + 2 * (size_t)a.ntiles;
+        if (a.frontier_cut > 0 && (size_t)a.ntiles <= (words - kSchedHeader) / (1 + kOrderPerTile + kFrontierWords))
+            a.frontier = a.schedule + kSchedHeader + (1 + kOrderPerTile) * (size_t)a.ntiles;
         if (a.frontier) {
             // super-tiles after the tiles' frontiers, when the buffer holds them
             const int sx = (a.tiles_x + kSuperTiles - 1) / kSuperTiles;
             const int sy = ((int)q.grid.y + kSuperTiles - 1) / kSuperTiles;
-            const size_t used = (size_t)kSchedHeader + (2 + (size_t)kFrontierWords) * (size_t)a.ntiles;
+            const size_t used =
+                (size_t)kSchedHeader + (size_t)(1 + kOrderPerTile + kFrontierWords) * (size_t)a.ntiles;
             if (used + (size_t)sx * (size_t)sy * kSuperWords <= words) {
                 a.super_frontier = a.frontier + (size_t)a.ntiles * kFrontierWords;
                 a.super_x = sx;
@@ -1974,13 +2224,25 @@ bool trace_forward_has_schedule(const gray_params &p) { return plan_forward(p, f
 cudaError_t launch_trace_schedule(const gray_params &p, bool display, cudaStream_t s) {
     const FwdPlan q = plan_forward(p, display);
     if (!q.sched) return cudaSuccess;
-    // densest tiles first: per-tile estimate and frontier, bucket by log2 of the estimate, order
+    // densest tiles first: per-tile estimate and frontier, then the work order
+    FwdArgs a = q.a;
+    int dev = 0, sms = 0;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(q.a.schedule, 0, sizeof(uint32_t) * kSchedZeroWords, s)) != cudaSuccess) return e;
-    if (q.nsuper > 0) super_cost_kernel<<<q.nsuper, 32, 0, s>>>(q.a, q.bw, q.bh, q.nsuper);
-    tile_cost_kernel<<<q.a.ntiles, 32, 0, s>>>(q.a, q.bw, q.bh);
-    sched_scan_kernel<<<1, 32, 0, s>>>(q.a.schedule);
-    sched_scatter_kernel<<<(q.a.ntiles + 255) / 256, 256, 0, s>>>(q.a.schedule, q.a.ntiles);
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    const void *kerns[2] = {q.kern, q.kern_wide ? q.kern_wide : q.kern};
+    int slots[2] = {0, 0};
+    for (int i = 0; i < 2; i++) {
+        int per_sm = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[i], kFwdThreads, 0)) != cudaSuccess)
+            return e;
+        slots[i] = sms * (per_sm > 0 ? per_sm : 1);
+    }
+    a.slots_narrow = slots[0];
+    a.slots_wide = slots[1];
+    if (q.nsuper > 0) super_cost_kernel<<<q.nsuper, 32, 0, s>>>(a, q.bw, q.bh, q.nsuper);
+    tile_cost_kernel<<<a.ntiles, 32, 0, s>>>(a, q.bw, q.bh);
+    sched_order_kernel<<<1, kOrderThreads, 0, s>>>(a.schedule, a.ntiles, a.slots_narrow, a.slots_wide);
     return cudaGetLastError();
 }
 
@@ -1996,20 +2258,31 @@ cudaError_t launch_trace_forward(const gray_params &p, bool display, bool schedu
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    // persistent grids that take the tiles in the schedule's order; with the automatic choice both
-    // kernels are launched and the one not chosen returns at once
-    const void *kerns[2] = {q.kern, q.kern_wide};
-    const int roles[2] = {q.kern_wide ? (int)kChoiceNarrow : 0, (int)kChoiceWide};
-    for (int i = 0; i < 2 && kerns[i]; i++) {
+    // persistent grids that take the split tiles' packets and the whole tiles in the schedule's order; with
+    // the automatic choice both kernels of the whole tiles are launched and the one not chosen returns
+    // at once.  The chain's second and third launch are programmatic: they run beside the one before.
+    const void *kerns[3] = {reinterpret_cast<const void *>(&trace_forward_split_kernel<16, kSplitBlocks>), q.kern,
+                            q.kern_wide};
+    const int roles[3] = {0, q.kern_wide ? (int)kChoiceNarrow : 0, (int)kChoiceWide};
+    for (int i = 0; i < 3 && kerns[i]; i++) {
         int per_sm = 0;
         if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[i], kFwdThreads, 0)) != cudaSuccess)
             return e;
         const unsigned int want = (unsigned int)(sms * (per_sm > 0 ? per_sm : 1));
-        const dim3 grid(want < (unsigned int)q.a.ntiles ? want : (unsigned int)q.a.ntiles, 1, 1);
+        const unsigned int items = (i == 0 ? 4u : 1u) * (unsigned int)q.a.ntiles;  // at most
         FwdArgs a = q.a;
         a.auto_role = roles[i];
         void *args[] = {&a};
-        if ((e = cudaLaunchKernel(kerns[i], grid, dim3(kFwdThreads), args, 0, s)) != cudaSuccess) return e;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(want < items ? want : items, 1, 1);
+        cfg.blockDim = dim3(kFwdThreads);
+        cfg.stream = s;
+        cfg.attrs = &attr;
+        cfg.numAttrs = i > 0 ? 1 : 0;
+        if ((e = cudaLaunchKernelExC(&cfg, kerns[i], args)) != cudaSuccess) return e;
     }
     return cudaGetLastError();
 }
@@ -2024,7 +2297,8 @@ size_t gray_schedule_words_for(uint32_t width, uint32_t height) {
     const size_t k = kSuperTiles;
     const size_t sa = (((width + 7) / 8 + k - 1) / k) * (((height + 15) / 16 + k - 1) / k);
     const size_t sb = (((width + 15) / 16 + k - 1) / k) * (((height + 7) / 8 + k - 1) / k);
-    return (size_t)kSchedHeader + 2 * t8 + (ta > tb ? ta : tb) * kFrontierWords + (sa > sb ? sa : sb) * kSuperWords;
+    return (size_t)kSchedHeader + 2 * t8 + (ta > tb ? ta : tb) * (kOrderPerTile - 1 + kFrontierWords) +
+           (sa > sb ? sa : sb) * kSuperWords;
 }
 
 cudaError_t launch_trace_batch(const gray_batch_scene *scenes, const gray_batch_view *views, int nviews,
