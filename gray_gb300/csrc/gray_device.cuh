@@ -127,8 +127,8 @@ __device__ __forceinline__ float scaling_factor(float opacity, float alpha_thres
 
 // Gaussian response at squared local radius d (reference: cuda/utils/kernel.cu:24-38).
 __device__ __forceinline__ float eval_gaussian(float d, float exp_power) {
+    if (exp_power == 2.0f) return gexp(-0.25f * d * d);  // the default
     if (exp_power == 1.0f) return gexp(-0.5f * d);
-    if (exp_power == 2.0f) return gexp(-0.25f * d * d);
     if (exp_power == 3.0f) return gexp(-(d * d * d) / 6.0f);
     float k = 2.0f * exp_power;
     return gexp(-gpow(d, exp_power) / k);
@@ -245,7 +245,7 @@ __device__ __forceinline__ bool intersect(const float4 g0, const float4 g1, cons
 // number of hits.
 constexpr long long kLogFixFloor = -105LL * (1LL << 40);
 __device__ __forceinline__ void add_log_transmittance(long long &s, float alpha) {
-    if (!(s > kLogFixFloor)) return;
+    if ((int)(s >> 32) < (int)(kLogFixFloor >> 32)) return;  // (at the floor itself the result is 0 either way)
     const float v = -glog(1.0f - alpha);
     if (v >= 0.0f && v < 16.0f) {
         // v >= 0 split exactly as i 2^-19 + r, r < 2^-19: adding 2^23 with rounding toward zero leaves
@@ -275,11 +275,11 @@ __device__ __forceinline__ void local_ray_lo(const float4 m0, const float4 m1, c
     h.b = fdot3(h.lo, h.ld);
 }
 
-// intersect() for rows (M | lo) from local_origin: the same arithmetic, so the same answer.
+// intersect() for rows (M | lo) from local_origin: the same arithmetic, so the same answer.  The caller has
+// dropped Gaussians at or below the alpha threshold.
 __device__ __forceinline__ bool intersect_lo(const float4 m0, const float4 m1, const float4 m2, float o, float sf,
-                                             f3 rd, float alpha_threshold, float exp_power, float znear, float zfar,
+                                             f3 rd, float exp_power, float znear, float zfar,
                                              float &dist, float &alpha) {
-    if (o <= alpha_threshold) return false;
     LocalHit h;
     local_ray_lo(m0, m1, m2, rd, h);
     if (h.b > 0.0f) return false;

@@ -149,6 +149,8 @@ struct LaneState {
     // selection buffer of the current traversal
     int kcount, ncand;
     unsigned long long kmax;
+    float dfar;  // +inf, or once the buffer is full the fp16 distance after its last key's: a hit beyond it
+                 // rounds to a larger distance than every kept key's
     // resume key for the next traversal
     unsigned long long resume;
     bool has_resume;
@@ -194,11 +196,11 @@ __device__ __forceinline__ void on_leaf_data(uint32_t gid, const float4 g0, cons
                                              unsigned long long (*kbuf)[kFwdThreads]) {
     float dist, alpha;
     if constexpr (LO) {
-        if (!intersect_lo(g0, g1, g2, lv.x, lv.y, rd, k.athr, k.pw, k.znear, k.zfar, dist, alpha)) return;
+        if (!intersect_lo(g0, g1, g2, lv.x, lv.y, rd, k.pw, k.znear, k.zfar, dist, alpha)) return;
     } else {
         if (!intersect(g0, g1, g2, lv.x, lv.y, ro, rd, k.athr, k.pw, k.znear, k.zfar, dist, alpha)) return;
     }
-    const uint16_t a16 = f2h_bits(alpha), d16 = f2h_bits(dist);
+    const uint16_t a16 = f2h_bits(alpha);
     if (first) {
         add_log_transmittance(st.lfx, alpha);
         const long long a = alpha16_fixed(a16);
@@ -208,6 +210,11 @@ __device__ __forceinline__ void on_leaf_data(uint32_t gid, const float4 g0, cons
         st.cfx2 += mul_fixed(a, cf2);
         st.nhit++;
     }
+    if (dist > st.dfar) {  // beyond every key of a full buffer
+        st.ncand++;
+        return;
+    }
+    const uint16_t d16 = f2h_bits(dist);
     if (!(h2f_bits(d16) > k.znear)) return;
     const unsigned long long key =
         ((unsigned long long)d16 << 48) | ((unsigned long long)gid << 16) | (unsigned long long)a16;
@@ -229,7 +236,10 @@ __device__ __forceinline__ void on_leaf_data(uint32_t gid, const float4 g0, cons
         pos--;
     }
     kbuf[pos][t] = key;
-    if (st.kcount == KB) st.kmax = kbuf[KB - 1][t];
+    if (st.kcount == KB) {
+        st.kmax = kbuf[KB - 1][t];
+        st.dfar = h2f_bits((uint16_t)(st.kmax >> 48) + 1u);
+    }
 }
 
 template <int KB>
@@ -823,6 +833,7 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
         const bool want = !done;
         st.kcount = 0;
         st.ncand = 0;
+        st.dfar = __int_as_float(0x7f800000);
         // ---------------- traversal ----------------
         bool per_ray = !tile;
         bool ranked = false;  // the keys are those of the four warps, in merge_split's order
@@ -835,6 +846,7 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
             // the tile's stack filled up: discard what was gathered, trace per ray
             st.kcount = 0;
             st.ncand = 0;
+            st.dfar = __int_as_float(0x7f800000);
             if (first) {
                 st.lfx = 0;
                 st.afx = st.cfx0 = st.cfx1 = st.cfx2 = 0;
