@@ -57,11 +57,17 @@ constexpr int kStatPackets = 48;   // packets traced by the last scheduled forwa
 constexpr int kStatRetraced = 49;  // of them, packets that need more than one traversal with 16 slots
 constexpr int kStatChoice = 50;    // kernel of the automatic choice: kChoiceNarrow or kChoiceWide
 constexpr uint32_t kChoiceNarrow = 1u, kChoiceWide = 2u;
-// the wide kernel (32 hit slots, four blocks per SM) is chosen when more than kWideSixteenths / 16
-// of the last forward's packets need more than one traversal with 16 slots (counted the same way by
-// both kernels, so the choice does not depend on which one ran), the narrow one (16 slots, six blocks
-// per SM) otherwise
-constexpr uint32_t kWideSixteenths = 2u;
+// The wide kernel (32 hit slots, four blocks per SM) is chosen when more than kWideLarge / 128 of the last
+// forward's packets need more than one traversal with 16 slots (counted the same way by both kernels,
+// so the choice does not depend on which one ran), the narrow one (16 slots, six blocks per SM)
+// otherwise; with at most kWideTiles tiles per resident block, more than kWideSmall / 128.  A second
+// traversal is repeated by the packet's whole tile, and in a small frame it is the launch's tail.  Measured,
+// narrow against wide: 3M / 1080p with 4% of the packets 2.88 and 3.12 ms, with 31-38% 2.7-3.7 and 2.0-2.4;
+// 1M / 1600x1040, 17-20%, 1.15-1.25 and 0.98-1.07; 500k / 1280x720 (7 tiles per block), 5.5-8.5%, 0.52-0.76
+// and 0.46-0.53; 300k / 800x600, 1.5-3%, 0.36-0.50 and 0.28-0.32; equal within 3% where none or almost
+// none do (100k / 320x240, 64 Gaussians / 256x256).
+constexpr uint32_t kWideLarge = 6u, kWideSmall = 1u;
+constexpr int kWideTiles = 8;
 // Per pixel tile, the BVH frontier its frustum reaches (kFrontierWords words: count, then up to
 // kFrontierMax node or leaf entries); a count of kFrontierNone means "start at the root".  A frontier
 // goes onto the traversal stack, so it leaves room there for the traversal's own pushes.
@@ -1732,10 +1738,11 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
         const uint32_t packets = sched[kStatPackets], retraced = sched[kStatRetraced];
         uint32_t choice = sched[kStatChoice];
         if (choice != kChoiceNarrow && choice != kChoiceWide) choice = kChoiceNarrow;
-        if (packets > 0u && retraced <= packets)
-            choice = (unsigned long long)retraced * 16ull > (unsigned long long)packets * kWideSixteenths
-                         ? kChoiceWide
-                         : kChoiceNarrow;
+        if (packets > 0u && retraced <= packets) {
+            const uint32_t most = ntiles <= kWideTiles * slots_narrow ? kWideSmall : kWideLarge;
+            choice = (unsigned long long)retraced * 128ull > (unsigned long long)packets * most ? kChoiceWide
+                                                                                                 : kChoiceNarrow;
+        }
         sched[kStatChoice] = choice;
         sched[kStatPackets] = 0u;
         sched[kStatRetraced] = 0u;
