@@ -1,7 +1,7 @@
 // trace.cu -- forward and backward ray tracing of the Gaussians on the LBVH.
 //
 // Forward (replaces the OptiX launch of cuda/shaders.cu:69-106 with cuda/forward_pass.cu):
-//   A block renders an 8x16-pixel tile of camera rays that share one origin, each warp a 4x8 (or 8x4)
+//   A block renders an 8x16-pixel tile of rays that share one origin, each warp a 4x8 (or 8x4)
 //   pixel packet of it.  A per-tile kernel first walks the top of the BVH with the tile's frustum and
 //   records the tile's frontier (the nodes of at most 64 leaves it reaches, sorted front to back);
 //   the block's traversal starts there.  The block traverses as one frustum: each step pops up to
@@ -18,8 +18,9 @@
 //   fp16 alpha).  The buffer is consumed by a state machine that reproduces the reference's
 //   32-slot multi-pass selection exactly (pass boundaries, the strict `distance > tmin` drop of
 //   equal distances, the 99-pass cap, zfar, t_threshold).  Composited ids are appended to the
-//   backward hit list in warp-aggregated segments.  Rays from Python, jittered rays and tiles
-//   whose traversal overflows the shared stack take a per-ray slab traversal instead.
+//   backward hit list in warp-aggregated segments.  Jittered rays, and rays from the caller that share
+//   their tile's origin within a cone (ray_cone_warp), go the same way; other rays from the caller, and
+//   tiles whose traversal overflows the shared stack, take a per-ray slab traversal instead.
 // Backward (cuda/backward_pass.cu:2-142): one thread per pixel walks its segments back to front,
 //   recomputes alpha in fp32 and reduces the 16 per-hit gradient values into the per-Gaussian
 //   accumulator: lanes holding the same Gaussian combine in a tree, and the lowest issues four
@@ -289,14 +290,14 @@ struct Frustum {
 // and a few roundings of 2^-24 each; the thresholds leave 1e-5 of that (about 170 roundings).
 // Boxes with an infinite or NaN coordinate (beyond M) give an infinite or NaN sum and always pass.
 __device__ __forceinline__ float3 camera_ray3(const float *w, float fov, int px, int py, uint32_t width,
-                                              uint32_t height);
+                                              uint32_t height, float jx, float jy);
 
 // Plane e of the frustum (e < 4: the side through corner rays e and e+1; e = 4: the near plane
 // orthogonal to the corners' sum).
 __device__ __forceinline__ void frustum_plane(int e, f3 o, const f3 d[4], const float *root_box, float4 &pn,
                                               float4 &pa) {
-    const f3 c = mk3(d[0].x + d[1].x + d[2].x + d[3].x, d[0].y + d[1].y + d[2].y + d[3].y,
-                     d[0].z + d[1].z + d[2].z + d[3].z);
+    const f3 sum = mk3(d[0].x + d[1].x + d[2].x + d[3].x, d[0].y + d[1].y + d[2].y + d[3].y,
+                       d[0].z + d[1].z + d[2].z + d[3].z);
     float m = 0.0f;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
@@ -304,11 +305,13 @@ __device__ __forceinline__ void frustum_plane(int e, f3 o, const f3 d[4], const 
         if (i != 3 && i != 7 && v <= 0x1.fffffep127f) m = fmaxf(m, v);
     }
     const float o1 = fabsf(o.x) + fabsf(o.y) + fabsf(o.z);
-    f3 nn = c;
+    f3 nn = sum;
     if (e < 4) {
-        const f3 a = d[e], b = d[(e + 1) & 3];
+        // a x b as a x (b - a): exact differences of neighbouring rays, so that the normal's rounding is
+        // relative to its own length and the plane holds both rays however narrow the cone is
+        const f3 a = d[e], c = d[(e + 1) & 3], b = mk3(c.x - a.x, c.y - a.y, c.z - a.z);
         nn = mk3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-        if (dot3(nn, c) < 0.0f) nn = mk3(-nn.x, -nn.y, -nn.z);
+        if (dot3(nn, sum) < 0.0f) nn = mk3(-nn.x, -nn.y, -nn.z);
     }
     const float n1 = fabsf(nn.x) + fabsf(nn.y) + fabsf(nn.z);
     const float no = fdot3(nn, o);
@@ -319,13 +322,17 @@ __device__ __forceinline__ void frustum_plane(int e, f3 o, const f3 d[4], const 
 }
 
 // The frustum built by a whole warp (every lane calls this): lanes 0-3 trace one corner ray each,
-// lanes 0-4 write one plane each.
+// lanes 0-4 write one plane each.  wide: the rays pass up to this many pixels beyond the pixels' centres.
 __device__ __forceinline__ void make_frustum_warp(Frustum &fr, f3 o, const float *w2c, float fov, int x0, int y0,
                                                   int x1, int y1, uint32_t width, uint32_t height,
-                                                  const float *root_box) {
+                                                  const float *root_box, float wide = 0.0f) {
     const int lane = threadIdx.x & 31;
     float3 dl = make_float3(0.0f, 0.0f, 0.0f);
-    if (lane < 4) dl = camera_ray3(w2c, fov, (lane == 1 || lane == 2) ? x1 : x0, lane >= 2 ? y1 : y0, width, height);
+    if (lane < 4) {
+        const bool right = lane == 1 || lane == 2, low = lane >= 2;
+        dl = camera_ray3(w2c, fov, right ? x1 : x0, low ? y1 : y0, width, height, right ? wide : -wide,
+                         low ? wide : -wide);
+    }
     f3 d[4];
 #pragma unroll
     for (int e = 0; e < 4; e++)
@@ -397,6 +404,9 @@ struct ConicBasis {
     float v0[3], du[3], dv[3];
     float hx, hy;  // largest |x| and |y| of the tile
     float mag;     // V
+    // rays from the caller (ray_cone_warp): their common origin, and the axis and centre of their cone
+    float origin[3], axis[3], ca, cb;
+    int cone;
 };
 
 // (a.x * b.x + c.x, a.y * b.y + c.y), each rounded once: one issue slot for two FMAs.
@@ -1116,8 +1126,8 @@ __device__ __forceinline__ f3 camera_ray(const float *w, float fov, int px, int 
 }
 
 __device__ __forceinline__ float3 camera_ray3(const float *w, float fov, int px, int py, uint32_t width,
-                                              uint32_t height) {
-    const f3 r = camera_ray(w, fov, px, py, width, height, 0.0f, 0.0f);
+                                              uint32_t height, float jx, float jy) {
+    const f3 r = camera_ray(w, fov, px, py, width, height, jx, jy);
     return make_float3(r.x, r.y, r.z);
 }
 
@@ -1144,10 +1154,117 @@ __device__ __forceinline__ void make_conic_basis(ConicBasis &cb, const float *w,
     cb.mag = 2.0f * (sqrtf(n0) * fabsf(ax) + sqrtf(n1) * fabsf(vs)) + sqrtf(n2);
 }
 
+// Rays that the caller supplied for the pixels [x0, x1] x [y0, y1]: when those that are alive share
+// their origin and lie within about 53 degrees of their mean direction, a warp builds their frustum and the
+// conics' basis (may be null) and returns true (on every lane; the warp calls this together).  With the
+// axis m and unit vectors u, v across it, a ray is the direction m + a u + b v up to its length; the
+// frustum spans the rectangle of the rays' (a, b), widened by 4e-6 (some 60 roundings of what they are
+// computed from), and the conics' plane is that of (a, b) about its centre.  Lengths outside [2^-10, 2^10]
+// (whose object-space squares could leave the normal range) and NaNs are left to the per-ray traversal,
+// in which a warp pops one node at a time for all of its rays: 401x301 rays over 100k Gaussians took
+// 0.66 ms that way and take 0.25 ms as tiles (the latency of their own hit chains; 950 tiles).
+// Not inlined: its registers would cost the camera rays' kernels 2%.
+__device__ __noinline__ bool ray_cone_warp(const float *__restrict__ ray_o, const float *__restrict__ ray_d,
+                                           uint32_t alloc_w, const float *__restrict__ root_box, int x0, int y0,
+                                           int x1, int y1, Frustum &fr, ConicBasis *cb) {
+    const int lane = threadIdx.x & 31;
+    const int w = x1 - x0 + 1, count = w * (y1 - y0 + 1);
+    if (w <= 0 || y1 < y0) return false;  // a split tile's packet beyond the image
+    bool have = false, bad = false;
+    f3 o = mk3(0.0f, 0.0f, 0.0f), m = mk3(0.0f, 0.0f, 0.0f);
+    for (int i = lane; i < count; i += 32) {
+        const size_t px = 3 * ((size_t)(y0 + i / w) * alloc_w + (size_t)(x0 + i % w));
+        const f3 d = mk3(ray_d[px], ray_d[px + 1], ray_d[px + 2]);
+        const float len2 = dot3(d, d);
+        if (sqrtf(len2) == 0.0f) continue;
+        if (!(len2 >= 0x1.0p-20f && len2 <= 0x1.0p20f)) bad = true;
+        const f3 ro = mk3(ray_o[px], ray_o[px + 1], ray_o[px + 2]);
+        if (!have) o = ro;
+        have = true;
+        if (!(ro.x == o.x && ro.y == o.y && ro.z == o.z)) bad = true;
+        const float inv = 1.0f / sqrtf(len2);
+        m = mk3(fmaf(d.x, inv, m.x), fmaf(d.y, inv, m.y), fmaf(d.z, inv, m.z));
+    }
+    const uint32_t who = __ballot_sync(kFull, have);
+    if (who == 0u) return false;
+    const int lead = __ffs((int)who) - 1;
+    const f3 ref = mk3(__shfl_sync(kFull, o.x, lead), __shfl_sync(kFull, o.y, lead), __shfl_sync(kFull, o.z, lead));
+    if (have && !(o.x == ref.x && o.y == ref.y && o.z == ref.z)) bad = true;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+        m = mk3(m.x + __shfl_xor_sync(kFull, m.x, off), m.y + __shfl_xor_sync(kFull, m.y, off),
+                m.z + __shfl_xor_sync(kFull, m.z, off));
+    const float inv = 1.0f / sqrtf(dot3(m, m));
+    m = mk3(m.x * inv, m.y * inv, m.z * inv);
+    if (!(dot3(m, m) > 0.99f)) bad = true;  // (directions that cancel, NaN)
+    f3 u = fabsf(m.x) < 0.7f ? mk3(0.0f, m.z, -m.y) : mk3(-m.z, 0.0f, m.x);
+    const float ul = 1.0f / sqrtf(dot3(u, u));
+    u = mk3(u.x * ul, u.y * ul, u.z * ul);
+    const f3 v = cross3(m, u);
+    const float big = __int_as_float(0x7f800000);
+    float a0 = big, a1 = -big, b0 = big, b1 = -big;
+    for (int i = lane; i < count; i += 32) {
+        const size_t px = 3 * ((size_t)(y0 + i / w) * alloc_w + (size_t)(x0 + i % w));
+        const f3 d = mk3(ray_d[px], ray_d[px + 1], ray_d[px + 2]);
+        const float len = sqrtf(dot3(d, d));
+        if (len == 0.0f) continue;
+        const float c = fdot3(d, m);
+        if (!(c >= 0.6f * len)) bad = true;
+        const float ra = fdot3(d, u) / c, rb = fdot3(d, v) / c;
+        a0 = fminf(a0, ra);
+        a1 = fmaxf(a1, ra);
+        b0 = fminf(b0, rb);
+        b1 = fmaxf(b1, rb);
+    }
+    if (__any_sync(kFull, bad)) return false;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        a0 = fminf(a0, __shfl_xor_sync(kFull, a0, off));
+        a1 = fmaxf(a1, __shfl_xor_sync(kFull, a1, off));
+        b0 = fminf(b0, __shfl_xor_sync(kFull, b0, off));
+        b1 = fmaxf(b1, __shfl_xor_sync(kFull, b1, off));
+    }
+    const float wide = 4e-6f * (1.0f + fmaxf(fabsf(a0), fabsf(a1)) + fmaxf(fabsf(b0), fabsf(b1)));
+    a0 -= wide;
+    a1 += wide;
+    b0 -= wide;
+    b1 += wide;
+    f3 d[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const float ea = e == 1 || e == 2 ? a1 : a0, eb = e >= 2 ? b1 : b0;
+        d[e] = mk3(fmaf(eb, v.x, fmaf(ea, u.x, m.x)), fmaf(eb, v.y, fmaf(ea, u.y, m.y)),
+                   fmaf(eb, v.z, fmaf(ea, u.z, m.z)));
+    }
+    if (lane < 5) frustum_plane(lane, ref, d, root_box, fr.pn[lane], fr.pa[lane]);
+    if (cb && lane == 0) {
+        const float ca = 0.5f * (a0 + a1), cc = 0.5f * (b0 + b1);
+        const float mm[3] = {m.x, m.y, m.z}, uu[3] = {u.x, u.y, u.z}, vv[3] = {v.x, v.y, v.z};
+        const float oo[3] = {ref.x, ref.y, ref.z};
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            cb->v0[e] = fmaf(cc, vv[e], fmaf(ca, uu[e], mm[e]));
+            cb->du[e] = uu[e];
+            cb->dv[e] = vv[e];
+            cb->origin[e] = oo[e];
+            cb->axis[e] = mm[e];
+        }
+        cb->ca = ca;
+        cb->cb = cc;
+        cb->hx = 0.5f * (a1 - a0);
+        cb->hy = 0.5f * (b1 - b0);
+        cb->mag = 2.0f * (1.0f + fmaxf(fabsf(a0), fabsf(a1)) + fmaxf(fabsf(b0), fabsf(b1)));
+    }
+    __syncwarp();
+    return true;
+}
+
 // The block's pixel tile (bx, by): 2x2 packets of tile_w x tile_h pixels, one packet per warp; or, SPLIT:
 // packet sub of it alone, its candidates shared by the four warps.  Returns whether the calling
 // warp's packet needs more than one traversal with 16 hit slots (RayResult::retraced).
-template <int KB, bool SPLIT>
+// ANY: rays from the caller too (they cost the camera rays' kernels registers: 1.8% of the forward); else
+// rays_from_python is off.
+template <int KB, bool SPLIT, bool ANY>
 __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, int sub, TileShared<KB> &sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rw = SPLIT ? a.tile_w : a.tile_w * kBlockWarpsX, rh = SPLIT ? a.tile_h : a.tile_h * kBlockWarpsY;
@@ -1173,17 +1290,18 @@ __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, i
 
     // ---- ray generation (cuda/shaders.cu:76-88) ----
     f3 ro = mk3(0.0f, 0.0f, 0.0f), rd = mk3(0.0f, 0.0f, 0.0f);
+    float jx = 0.0f, jy = 0.0f;
     bool alive = false;
     // every thread holds the camera origin, inactive ones too (a tile's candidates get their
     // object-space origin from whichever thread fetches them)
-    if (!*a.rays_from_python) ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
+    const bool given = ANY && *a.rays_from_python;
+    if (!given) ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
     if (inside) {
-        if (*a.rays_from_python) {
+        if (given) {
             ro = mk3(a.ray_o[3 * pixel], a.ray_o[3 * pixel + 1], a.ray_o[3 * pixel + 2]);
             rd = mk3(a.ray_d[3 * pixel], a.ray_d[3 * pixel + 1], a.ray_d[3 * pixel + 2]);
         } else {
             ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
-            float jx = 0.0f, jy = 0.0f;
             if (*a.jitter) {
                 uint32_t h = pcg_hash(pixel ^ pcg_hash(*a.total_num_calls));
                 jx = (float)(h & 0xFFFFu) * 0x1.0p-16f - 0.5f;
@@ -1194,22 +1312,41 @@ __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, i
         alive = !(sqrtf(dot3(rd, rd)) == 0.0f);
     }
 
-    // camera rays share the origin: the block traverses its tile together
-    const bool tile = !*a.rays_from_python && !*a.jitter;
-    const float hx = (float)(rw - 1) * 0.5f, hy = (float)(rh - 1) * 0.5f;
-    const uint32_t *front = nullptr;
-    if (tile) {
+    // rays that share their origin: the block traverses its tile together
+    bool tile = true;
+    float x, y;  // the ray's place in the conics' plane
+    if (given) {
+        if (warp == 0) {
+            const bool cone = ray_cone_warp(a.ray_o, a.ray_d, a.alloc_w, a.root_box, tx0, ty0,
+                                            min(tx0 + rw, (int)a.render_w) - 1, min(ty0 + rh, (int)a.render_h) - 1,
+                                            sh.fr, &sh.cb);
+            if (lane == 0) sh.cb.cone = cone ? 1 : 0;
+        }
+        __syncthreads();
+        tile = sh.cb.cone != 0;
+        const f3 m = mk3(sh.cb.axis[0], sh.cb.axis[1], sh.cb.axis[2]);
+        const float c = fdot3(rd, m);
+        x = fdot3(rd, mk3(sh.cb.du[0], sh.cb.du[1], sh.cb.du[2])) / c - sh.cb.ca;
+        y = fdot3(rd, mk3(sh.cb.dv[0], sh.cb.dv[1], sh.cb.dv[2])) / c - sh.cb.cb;
+        if (tile && !alive) ro = mk3(sh.cb.origin[0], sh.cb.origin[1], sh.cb.origin[2]);
+    } else {
+        const float wide = *a.jitter ? 0.5f : 0.0f;
+        const float hx = (float)(rw - 1) * 0.5f, hy = (float)(rh - 1) * 0.5f;
         // (the loop of trace_rays starts with a block barrier)
         if (warp == 0)
-            make_frustum_warp(sh.fr, mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, tx0, ty0,
-                              tx0 + rw - 1, ty0 + rh - 1, a.render_w, a.render_h, a.root_box);
+            make_frustum_warp(sh.fr, ro, a.w2c, *a.fov, tx0, ty0, tx0 + rw - 1, ty0 + rh - 1, a.render_w, a.render_h,
+                              a.root_box, wide);
         if (threadIdx.x == kFwdThreads - 1)
-            make_conic_basis(sh.cb, a.w2c, *a.fov, (float)tx0 + hx, (float)ty0 + hy, hx, hy, a.render_w, a.render_h);
-        if (a.frontier) front = a.frontier + (size_t)(by * a.tiles_x + bx) * kFrontierWords;
+            make_conic_basis(sh.cb, a.w2c, *a.fov, (float)tx0 + hx, (float)ty0 + hy, hx + wide, hy + wide, a.render_w,
+                             a.render_h);
+        // (pixel plus jitter as camera_ray rounds it; the differences are exact)
+        x = ((float)px + jx) - ((float)tx0 + hx);
+        y = ((float)py + jy) - ((float)ty0 + hy);
     }
+    const uint32_t *front =
+        tile && a.frontier ? a.frontier + (size_t)(by * a.tiles_x + bx) * kFrontierWords : nullptr;
     RayResult r;
-    trace_rays<KB, SPLIT>(sc, k, ro, rd, (float)(px - tx0) - hx, (float)(py - ty0) - hy, alive, tile, grads, hs,
-                          a.status, sh, front, r);
+    trace_rays<KB, SPLIT>(sc, k, ro, rd, x, y, alive, tile, grads, hs, a.status, sh, front, r);
     if (SPLIT && warp != 0) return false;
     if (!inside) return r.retraced;
     if (!alive) {
@@ -1264,7 +1401,7 @@ template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_kernel(const FwdArgs a) {
     __shared__ TileShared<KB> sh;
     if (*a.render_ellipsoids) return;  // the ellipsoid view (ellipsoid_kernel) renders this frame
-    forward_tile<KB, false>(a, blockIdx.x, blockIdx.y, 0, sh);
+    forward_tile<KB, false, true>(a, blockIdx.x, blockIdx.y, 0, sh);
 }
 
 // Persistent launch: the blocks take tiles from the schedule's order, densest first, until none is
@@ -1278,7 +1415,9 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
     __shared__ uint32_t s_next, s_packets, s_retraced;
     grid_launch_next();
     // automatic choice: both kernels are launched, the one the order kernel did not choose leaves
-    if (*a.render_ellipsoids || (a.auto_role != 0 && a.schedule[kStatChoice] != (uint32_t)a.auto_role)) {
+    // (rays from the caller are the split packets' kernel's)
+    if (*a.render_ellipsoids || *a.rays_from_python ||
+        (a.auto_role != 0 && a.schedule[kStatChoice] != (uint32_t)a.auto_role)) {
         grid_wait_before();
         return;
     }
@@ -1295,7 +1434,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
         if (t >= items) break;
         const uint32_t tile = a.schedule[kSchedHeader + a.ntiles + t];
         const bool again =
-            forward_tile<KB, false>(a, (int)(tile % (uint32_t)a.tiles_x), (int)(tile / (uint32_t)a.tiles_x), 0, sh);
+            forward_tile<KB, false, false>(a, (int)(tile % (uint32_t)a.tiles_x), (int)(tile / (uint32_t)a.tiles_x), 0, sh);
         if ((threadIdx.x & 31) == 0) {
             atomicAdd(&s_packets, 1u);
             if (again) atomicAdd(&s_retraced, 1u);
@@ -1308,7 +1447,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
     grid_wait_before();
 }
 
-// The split tiles' packets (see sched_order_kernel), launched before the kernel of the whole tiles, which
+// The split tiles' packets (see sched_order_kernel), and every tile of a forward on the caller's rays; launched before the kernel of the whole tiles, which
 // starts as soon as this one's blocks have and fills what they leave free.  A kernel of its own: with
 // both bodies in one, the whole tiles' loop lost registers (3M / 1080p 2.28 to 2.33 ms with a run-time
 // switch, 2.44 ms with two inlined bodies, 2.40 ms with a call).
@@ -1318,8 +1457,8 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(
     __shared__ uint32_t s_next, s_packets, s_retraced;
     grid_launch_next();
     if (*a.render_ellipsoids) return;
-    const uint32_t items = a.schedule[kSchedSplitItems];
-    if (items == 0u) return;
+    const uint32_t items = a.schedule[kSchedSplitItems], whole = *a.rays_from_python ? a.schedule[kSchedItems] : 0u;
+    if (items + whole == 0u) return;
     if (threadIdx.x == 0) {
         s_packets = 0u;
         s_retraced = 0u;
@@ -1329,15 +1468,23 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(
         if (threadIdx.x == 0) s_next = atomicAdd(a.schedule + kSchedSplitNext, 1u);
         __syncthreads();
         const uint32_t t = s_next;
-        if (t >= items) break;
-        const uint32_t item = a.schedule[kSchedHeader + 2 * a.ntiles + t], tile = item & kItemTile;
-        const bool again = forward_tile<KB, true>(a, (int)(tile % (uint32_t)a.tiles_x),
-                                                  (int)(tile / (uint32_t)a.tiles_x), (int)(item >> kItemShift), sh);
-        if (threadIdx.x == 0) {
-            s_packets++;
-            if (again) s_retraced++;
+        if (t >= items + whole) break;
+        bool again;
+        if (t < items) {
+            const uint32_t item = a.schedule[kSchedHeader + 2 * a.ntiles + t], tile = item & kItemTile;
+            again = forward_tile<KB, true, true>(a, (int)(tile % (uint32_t)a.tiles_x),
+                                                 (int)(tile / (uint32_t)a.tiles_x), (int)(item >> kItemShift), sh);
+        } else {
+            const uint32_t tile = a.schedule[kSchedHeader + a.ntiles + t - items];
+            again = forward_tile<KB, false, true>(a, (int)(tile % (uint32_t)a.tiles_x),
+                                                  (int)(tile / (uint32_t)a.tiles_x), 0, sh);
+        }
+        if ((threadIdx.x & 31) == 0 && (threadIdx.x == 0 || t >= items)) {
+            atomicAdd(&s_packets, 1u);
+            if (again) atomicAdd(&s_retraced, 1u);
         }
     }
+    __syncthreads();
     if (threadIdx.x == 0 && s_packets > 0u) {
         atomicAdd(&a.schedule[kStatPackets], s_packets);
         atomicAdd(&a.schedule[kStatRetraced], s_retraced);
@@ -1656,6 +1803,16 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
     return est;
 }
 
+// The frustum of this forward's rays through a pixel rectangle (a warp together); false for rays from the
+// caller that do not share an origin and a cone.
+__device__ __forceinline__ bool make_tile_frustum(const FwdArgs &a, int x0, int y0, int x1, int y1, Frustum &fr) {
+    if (*a.rays_from_python) 
+        return ray_cone_warp(a.ray_o, a.ray_d, a.alloc_w, a.root_box, x0, y0, x1, y1, fr, nullptr);
+    make_frustum_warp(fr, mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, x0, y0, x1, y1,
+                      a.render_w, a.render_h, a.root_box, *a.jitter ? 0.5f : 0.0f);
+    return true;
+}
+
 // Coarse frontiers of the super-tiles (kSuperTiles x kSuperTiles block tiles each), one warp each.
 __global__ void __launch_bounds__(32) super_cost_kernel(const FwdArgs a, int bw, int bh, int nsuper) {
     __shared__ FrontierScratch fs;
@@ -1664,16 +1821,15 @@ __global__ void __launch_bounds__(32) super_cost_kernel(const FwdArgs a, int bw,
     if (st >= nsuper) return;
     uint32_t *out = a.super_frontier + (size_t)st * kSuperWords;
     const int n = a.n;
-    if (!*a.rays_from_python && !*a.jitter && !*a.render_ellipsoids && n > 1) {
+    bool walk = !*a.render_ellipsoids && n > 1;
+    if (walk) {
         const int x0 = (st % a.super_x) * kSuperTiles * bw, y0 = (st / a.super_x) * kSuperTiles * bh;
         const int x1 = min(x0 + kSuperTiles * bw, (int)a.render_w) - 1;
         const int y1 = min(y0 + kSuperTiles * bh, (int)a.render_h) - 1;
-        make_frustum_warp(fs.fr, mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, x0, y0, x1, y1,
-                          a.render_w, a.render_h, a.root_box);
-        frontier_walk<true>(a.nodes, n, kSuperCut, fs, &ss, out, nullptr);
-    } else if (lane == 0) {
-        out[0] = kFrontierNone;
+        walk = make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
+        if (walk) frontier_walk<true>(a.nodes, n, kSuperCut, fs, &ss, out, nullptr);
     }
+    if (!walk && lane == 0) out[0] = kFrontierNone;
 }
 
 __global__ void __launch_bounds__(32) tile_cost_kernel(const FwdArgs a, int bw, int bh) {
@@ -1682,21 +1838,21 @@ __global__ void __launch_bounds__(32) tile_cost_kernel(const FwdArgs a, int bw, 
     uint32_t *out = a.frontier ? a.frontier + (size_t)tile * kFrontierWords : nullptr;
     uint32_t est = 0;
     const int n = a.n;
-    if (!*a.rays_from_python && !*a.jitter && !*a.render_ellipsoids && n > 1) {
+    bool walk = !*a.render_ellipsoids && n > 1;
+    if (walk) {
         const int x0 = (tile % a.tiles_x) * bw, y0 = (tile / a.tiles_x) * bh;
         const int x1 = min(x0 + bw, (int)a.render_w) - 1, y1 = min(y0 + bh, (int)a.render_h) - 1;
-        make_frustum_warp(fs.fr, mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, x0, y0, x1, y1,
-                          a.render_w, a.render_h, a.root_box);
+        walk = make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
         const uint32_t *seed = nullptr;
         if (a.super_frontier) {
             const int sx = (tile % a.tiles_x) / kSuperTiles, sy = (tile / a.tiles_x) / kSuperTiles;
             seed = a.super_frontier + (size_t)(sy * a.super_x + sx) * kSuperWords;
         }
-        est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut, fs, nullptr,
-                                   out, seed);
-    } else if (out && lane == 0) {
-        out[0] = kFrontierNone;
+        if (walk)
+            est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut, fs,
+                                       nullptr, out, seed);
     }
+    if (!walk && out && lane == 0) out[0] = kFrontierNone;
     if (lane == 0) a.schedule[kSchedHeader + tile] = est;
 }
 

@@ -38,3 +38,71 @@ def test_tiles_match_the_oracle(oracle, variant, size, n):
         rt.check_status()
         fwd = oracle.trace_forward(ro, rd, geom, live, chan, vis, oracle.TraceConfig(t_threshold=1e-4))
         _compare_forward(rt, fwd)
+
+
+def _supplied_rays(kind, W, H, rng):
+    """Rays of a lens the pinhole camera does not have: [W*H, 3] origins and directions."""
+    i, j = np.meshgrid(np.arange(W), np.arange(H))
+    o = np.tile(np.array([0.1, -3.5, 0.2], np.float32), (W * H, 1))
+    if kind == "panorama":  # the whole sphere: tiles near the poles are too wide for a cone
+        az, el = 2 * np.pi * (i + 0.5) / W, np.pi * ((j + 0.5) / H - 0.5)
+        d = np.stack([np.cos(el) * np.sin(az), np.cos(el) * np.cos(az), np.sin(el)], -1)
+    else:
+        x, y = 0.9 * (2 * (i + 0.5) / W - 1), 0.9 * (2 * (j + 0.5) / H - 1)
+        bend = 1.0 + 0.3 * (x * x + y * y)
+        d = np.stack([x * bend * 0.3, np.ones_like(x), -y * bend * 0.3], -1)
+    d = (d / np.linalg.norm(d, axis=-1, keepdims=True)).reshape(-1, 3)
+    if kind == "lengths":
+        d *= 2.0 ** rng.uniform(-3, 3, (W * H, 1))
+    elif kind == "extreme lengths":
+        d *= 2.0 ** rng.choice([-14.0, 0.0, 14.0], (W * H, 1))
+    elif kind == "holes":
+        d[rng.random(W * H) < 0.4] = 0.0
+        d[: 8 * W] = 0.0
+    elif kind == "origins":  # one row of tiles with an origin per ray, the others with one each
+        o = o + np.repeat(0.02 * (np.arange(H) // 16).astype(np.float32), W)[:, None]
+        o[: 16 * W] += 0.05 * rng.standard_normal((16 * W, 3))
+    elif kind == "parallel":
+        d[:] = np.array([0.02, 1.0, -0.03]) / np.linalg.norm([0.02, 1.0, -0.03])
+    elif kind == "shuffled":  # neighbouring pixels' rays all over the image
+        d = d[rng.permutation(W * H)]
+    return o.astype(np.float32), d.astype(np.float32)
+
+
+@pytest.mark.parametrize("kind", ["lens", "panorama", "lengths", "extreme lengths", "holes", "origins", "parallel",
+                                  "shuffled"])
+def test_rays_from_the_caller_match_the_oracle(oracle, kind):
+    """Supplied rays are traversed tile by tile where a tile's rays share their origin and a cone, and one
+    by one elsewhere: images, hit lists and counts are the oracle's either way."""
+    W, H, n = 45, 39, 1500
+    rng = np.random.default_rng(5)
+    sc = synthetic.small_scene(seed=n, n=n)
+    grow = np.float32(0.4)
+    chan = np.random.default_rng(n).uniform(0, 1, (n, 3)).astype(np.float32)
+    rt = G.make_tracer(W, H, sc.mean, sc.rotation, sc.scale + grow, sc.opacity, channels=chan)
+    geom, l2w, aabb, vis, live = _oracle_scene(oracle, sc.mean, sc.rotation, sc.scale + grow, sc.opacity)
+    ro, rd = _supplied_rays(kind, W, H, rng)
+    for _ in range(2):
+        rt.get_stats().reset()
+        G.trace_rays(rt, ro, rd)
+        fwd = oracle.trace_forward(ro, rd, geom, live, chan, vis, oracle.TraceConfig(t_threshold=0.03))
+        assert fwd["nhit"].max() > 3
+        _compare_forward(rt, fwd)
+
+
+@pytest.mark.parametrize("size", [(9, 17), (64, 48), (130, 70)])
+def test_jittered_tiles_match_the_oracle(oracle, size):
+    """Jittered camera rays are traversed tile by tile, up to half a pixel beyond the pixels' centres."""
+    W, H = size
+    n = 3000
+    sc = synthetic.small_scene(seed=n, n=n)
+    chan = np.random.default_rng(n).uniform(0, 1, (n, 3)).astype(np.float32)
+    rt = G.make_tracer(W, H, sc.mean, sc.rotation, sc.scale, sc.opacity, channels=chan, t_threshold=1e-3)
+    rt.get_config().jitter_primary_rays.fill_(True)
+    cam = synthetic.look_at((0.0, -3.0, 0.4), (0, 0, 0), (0, 0, 1), 0.6, W, H)
+    geom, l2w, aabb, vis, live = _oracle_scene(oracle, sc.mean, sc.rotation, sc.scale, sc.opacity)
+    for _ in range(2):
+        rt.get_stats().reset()
+        ro, rd = _camera_rays_gpu(rt, cam)
+        fwd = oracle.trace_forward(ro, rd, geom, live, chan, vis, oracle.TraceConfig(t_threshold=1e-3))
+        _compare_forward(rt, fwd)
