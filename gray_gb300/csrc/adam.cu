@@ -50,23 +50,33 @@ __device__ __forceinline__ void adam_one(float &p, float &m, float &v, float &g,
     if (zero) g = gg * 0.0f;
 }
 
+__device__ __forceinline__ bool same_bits(float4 a, float4 b) {
+    return ((__float_as_uint(a.x) ^ __float_as_uint(b.x)) | (__float_as_uint(a.y) ^ __float_as_uint(b.y)) |
+            (__float_as_uint(a.z) ^ __float_as_uint(b.z)) | (__float_as_uint(a.w) ^ __float_as_uint(b.w))) == 0u;
+}
+
+// What a step leaves as it was is not written: the zeroed gradients of Gaussians that no ray composited in
+// this view, and the whole state of those that none has yet (and of the SH bands above the current
+// degree), whose moments are zero.  The update is bound by its eight streams, half of which are writes: with
+// 11% of the Gaussians seen 3M took 888 and take 743 us, with 28% of 1M 296 and 268 (all seen: 255 either way).
 // One float4 of one group (or the scalar tail of a group whose length is not a multiple of 4).
 __device__ __forceinline__ void adam_vec(const AdamGroup &G, long long e0, bool do_adam, float lr, float b1, float b2,
                                          float bc1, float bc2, float eps, bool zero, bool vec, float4 p, float4 m,
                                          float4 v, float4 g) {
     if (vec) {
+        const float4 p0 = p, m0 = m, v0 = v, g0 = g;
         if (do_adam) {
             adam_one(p.x, m.x, v.x, g.x, lr, b1, b2, bc1, bc2, eps, zero);
             adam_one(p.y, m.y, v.y, g.y, lr, b1, b2, bc1, bc2, eps, zero);
             adam_one(p.z, m.z, v.z, g.z, lr, b1, b2, bc1, bc2, eps, zero);
             adam_one(p.w, m.w, v.w, g.w, lr, b1, b2, bc1, bc2, eps, zero);
-            *reinterpret_cast<float4 *>(G.p + e0) = p;
-            *reinterpret_cast<float4 *>(G.m + e0) = m;
-            *reinterpret_cast<float4 *>(G.v + e0) = v;
+            if (!same_bits(p, p0)) *reinterpret_cast<float4 *>(G.p + e0) = p;
+            if (!same_bits(m, m0)) *reinterpret_cast<float4 *>(G.m + e0) = m;
+            if (!same_bits(v, v0)) *reinterpret_cast<float4 *>(G.v + e0) = v;
         } else {
             g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-        if (zero) *reinterpret_cast<float4 *>(G.g + e0) = g;
+        if (zero && !same_bits(g, g0)) *reinterpret_cast<float4 *>(G.g + e0) = g;
     } else {
         for (long long e = e0; e < G.count && e < e0 + 4; e++) {
             if (do_adam) {
