@@ -100,6 +100,11 @@ def load(path: str | None = None):
         f = getattr(L, name)
         f.restype = ctypes.c_int
         f.argtypes = [ctypes.POINTER(ParamsC), ctypes.c_void_p]
+    L.gray_forward_pass_mode.restype = ctypes.c_int
+    L.gray_forward_pass_mode.argtypes = [ctypes.POINTER(ParamsC), ctypes.c_int32, ctypes.c_void_p]
+    L.gray_set_view.restype = ctypes.c_int
+    L.gray_set_view.argtypes = [ctypes.POINTER(ParamsC), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_float,
+                                ctypes.c_float, ctypes.c_float, ctypes.c_int32, ctypes.c_void_p]
     L.gray_sort_tmp_words.restype = ctypes.c_size_t
     L.gray_sort_tmp_words.argtypes = [ctypes.c_int32]
     L.gray_schedule_words.restype = ctypes.c_size_t
@@ -114,9 +119,10 @@ def load(path: str | None = None):
     return L
 
 
-def call(name: str, params: ParamsC, stream: int):
+def call(name: str, params: ParamsC, stream: int, *args):
+    """Entry point `name` on params and, before the stream, its further arguments."""
     L = load()
-    rc = getattr(L, name)(ctypes.byref(params), ctypes.c_void_p(stream))
+    rc = getattr(L, name)(ctypes.byref(params), *args, ctypes.c_void_p(stream))
     if rc != 0:
         raise GrayError(f"{name}: {L.gray_last_error().decode()} (code {rc})")
 

@@ -45,23 +45,21 @@ _CAM_STATE = ("origin", "vertical_fov_radians", "rotation_c2w", "rotation_w2c", 
 
 
 def _set_camera(tracer, camera: CameraInfo, znear=0.0, zfar=99999.9):
-    c = tracer.get_camera()
-    c.znear.fill_(znear)
-    c.zfar.fill_(zfar)
-    c.vertical_fov_radians.fill_(float(camera.fov_y))
-    c.set_pose(camera.origin_cuda(), camera.rotation_c2w_blender_cuda())
-    tracer.get_config().rays_from_python.fill_(False)
+    tracer.set_view(camera.origin_cuda(), camera.rotation_c2w_blender_cuda(), float(camera.fov_y), znear, zfar)
 
 
 def _load(tracer, names, tensors):
     g = tracer.get_gaussians()
-    with torch.no_grad():
-        for name, t in zip(names, tensors):
-            if t is None:
-                continue
-            dst = getattr(g, name)
-            if t.data_ptr() != dst.data_ptr():
-                dst.copy_(t.detach().reshape(dst.shape))
+    into, values = [], []
+    for name, t in zip(names, tensors):
+        if t is None:
+            continue
+        dst = getattr(g, name)
+        if t.data_ptr() != dst.data_ptr():
+            into.append(dst.detach())
+            values.append(t.detach().reshape(dst.shape))
+    if into:
+        torch._foreach_copy_(into, values)
 
 
 def free_device_bytes(device) -> int:
@@ -201,18 +199,18 @@ class RayTraceFunction(torch.autograd.Function):
         tracer = st.tracer
         g = tracer.get_gaussians()
         with torch.no_grad():
-            for name in ("grad_mean", "grad_rotation", "grad_scale", "grad_opacity", "grad_channels",
-                         "grad_sh_coeffs_dc", "grad_sh_coeffs_rest"):
-                getattr(g, name).zero_()
+            torch._foreach_zero_([g.grad_mean, g.grad_rotation, g.grad_scale, g.grad_opacity, g.grad_channels,
+                                  g.grad_sh_coeffs_dc, g.grad_sh_coeffs_rest])
             h, w = tracer.height, tracer.width
             tracer.get_framebuffer().grad_output_channels[:h, :w].copy_(grad_out.moveaxis(0, -1))
         tracer.backward_pass()
         st.consumed = True
         grads = [g.grad_mean, g.grad_rotation, g.grad_scale, g.grad_opacity, g.grad_channels, g.grad_sh_coeffs_dc,
                  g.grad_sh_coeffs_rest]
-        out = []
-        for gr, shape in zip(grads, ctx.shapes):
-            out.append(None if shape is None else gr.clone().reshape(shape))
+        grads = [None if shape is None else gr for gr, shape in zip(grads, ctx.shapes)]
+        out = [None if gr is None else torch.empty_like(gr) for gr in grads]
+        torch._foreach_copy_([o for o in out if o is not None], [gr for gr in grads if gr is not None])
+        out = [None if o is None else o.reshape(shape) for o, shape in zip(out, ctx.shapes)]
         return (None, None, None, *out)
 
 

@@ -374,19 +374,18 @@ class Raytracer:
         p.trace_variant = int(self.trace_variant)
         return p
 
-    def _call(self, name: str):
+    def _call(self, name: str, *args):
         if self._params is None:
             self._params = self._build_params()
-        _lib.call(name, self._params, torch.cuda.current_stream(self.device).cuda_stream)
+        _lib.call(name, self._params, torch.cuda.current_stream(self.device).cuda_stream, *args)
 
     def _invalidate(self):
         self._params = None
 
     # ---- reference methods ----
     def forward_pass(self):
-        self.meta_data.grads_enabled.fill_(torch.is_grad_enabled())
         self.generation += 1
-        self._call("gray_forward_pass")
+        self._call("gray_forward_pass_mode", int(torch.is_grad_enabled()))
 
     def forward_pass_display(self):
         self.generation += 1
@@ -430,6 +429,22 @@ class Raytracer:
         self.width = int(new_width)
         self.height = int(new_height)
         self._invalidate()
+
+    def set_view(self, c2w_origin: torch.Tensor, c2w_rotation: torch.Tensor, vertical_fov_radians: float,
+                 znear: float, zfar: float):
+        """A camera for the next forwards: what filling vertical_fov_radians, znear, zfar and
+        rays_from_python (False) and camera_data.set_pose do, in one launch."""
+        c = self.camera_data
+        for t, shape in ((c2w_origin, (3,)), (c2w_rotation, (3, 3))):
+            if tuple(t.shape) != shape or t.dtype != torch.float32 or t.device != self.device or not t.is_contiguous():
+                c.vertical_fov_radians.fill_(vertical_fov_radians)
+                c.znear.fill_(znear)
+                c.zfar.fill_(zfar)
+                self.config_data.rays_from_python.fill_(False)
+                c.set_pose(c2w_origin, c2w_rotation)
+                return
+        self._call("gray_set_view", c2w_origin.data_ptr(), c2w_rotation.data_ptr(), float(vertical_fov_radians),
+                   float(znear), float(zfar), 0)
 
     def get_camera(self):
         return self.camera_data

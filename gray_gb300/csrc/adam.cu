@@ -178,13 +178,11 @@ cudaError_t launch_adam(const gray_params &p, cudaStream_t s) {
     a.update_channels = p.config.update_channels;
     a.enable_sh = p.config.enable_sh;
     a.laziness = g.sh_update_laziness;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaError_t e;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adam_kernel, kAdamThreads, 0)) != cudaSuccess)
-        return e;
-    const long long want = (long long)sms * (per_sm > 0 ? per_sm : 1);
+    int sms = 0, per_sm = 0;
+    const cudaError_t e =
+        resident_blocks(reinterpret_cast<const void *>(&adam_kernel), kAdamThreads, 0, &sms, &per_sm);
+    if (e != cudaSuccess) return e;
+    const long long want = (long long)sms * per_sm;
     adam_kernel<<<(unsigned int)(blocks < want ? blocks : want), kAdamThreads, 0, s>>>(a);
     return cudaGetLastError();
 }

@@ -6,6 +6,7 @@
 // entry points make one side stream and two events per host thread and context on first use).
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -70,6 +71,31 @@ int cuda_fail(cudaError_t e, const char *where) {
 }
 
 int check_common(const gray_params *p) { return check_common_impl(p); }
+
+cudaError_t resident_blocks(const void *kernel, int threads, size_t smem, int *sms, int *per_sm) {
+    struct Known {
+        const void *kernel;
+        size_t smem;
+        int threads, dev, sms, per_sm;
+    };
+    static std::mutex lock;
+    static std::vector<Known> known;  // one entry per kernel of the library, shared-memory size and device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> hold(lock);
+    for (const Known &k : known)
+        if (k.kernel == kernel && k.threads == threads && k.smem == smem && k.dev == dev) {
+            *sms = k.sms;
+            *per_sm = k.per_sm;
+            return cudaSuccess;
+        }
+    if ((e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, kernel, threads, smem)) != cudaSuccess) return e;
+    if (*per_sm < 1) *per_sm = 1;
+    known.push_back(Known{kernel, smem, threads, dev, *sms, *per_sm});
+    return cudaSuccess;
+}
 
 ProfScope::ProfScope(const char *name, cudaStream_t s) : ev_(-1), s_(s) {
     if (!g_prof_on) return;
@@ -142,7 +168,7 @@ bool side_stream(SideStream *out) {
 // forward_prep (live values, colours) and the tile schedule (per-tile BVH frontier and work order,
 // from the BVH and the camera only) read and write disjoint state: the schedule runs on the side
 // stream between a fork and a join event while forward_prep runs on s, and the trace follows both.
-int forward(const gray_params *p, bool display, cudaStream_t s) {
+int forward(const gray_params *p, bool display, int grads, cudaStream_t s) {
     SideStream side;
     const bool overlap = gray::trace_forward_has_schedule(*p) && side_stream(&side);
     if (overlap) {
@@ -152,7 +178,7 @@ int forward(const gray_params *p, bool display, cudaStream_t s) {
         GRAY_LAUNCH_ON("tile_schedule", side.s, gray::launch_trace_schedule(*p, display, side.s));
         if ((e = cudaEventRecord(side.join, side.s)) != cudaSuccess) return cuda_fail(e, "join");
     }
-    GRAY_LAUNCH("forward_prep", gray::launch_forward_prep(*p, !display, s));
+    GRAY_LAUNCH("forward_prep", gray::launch_forward_prep(*p, !display, grads, s));
     if (overlap) {
         cudaError_t e = cudaStreamWaitEvent(s, side.join, 0);
         if (e != cudaSuccess) return cuda_fail(e, "join");
@@ -221,13 +247,31 @@ size_t gray_schedule_words(uint32_t width, uint32_t height) { return gray::gray_
 int gray_forward_pass(const gray_params *p, void *stream) {
     int e = check_trace(p);
     if (e) return e;
-    return forward(p, false, (cudaStream_t)stream);
+    return forward(p, false, -1, (cudaStream_t)stream);
+}
+
+int gray_forward_pass_mode(const gray_params *p, int32_t grads_enabled, void *stream) {
+    int e = check_trace(p);
+    if (e) return e;
+    if (!p->metadata.grads_enabled) return fail(GRAY_ERR_INVALID_ARGUMENT, "missing metadata buffers");
+    return forward(p, false, grads_enabled != 0 ? 1 : 0, (cudaStream_t)stream);
+}
+
+int gray_set_view(const gray_params *p, const float *origin, const float *c2w, float vertical_fov_radians,
+                  float znear, float zfar, int32_t rays_from_python, void *stream) {
+    if (!p || !origin || !c2w || !p->camera.origin || !p->camera.rotation_c2w || !p->camera.rotation_w2c ||
+        !p->camera.vertical_fov_radians || !p->camera.znear || !p->camera.zfar || !p->config.rays_from_python)
+        return fail(GRAY_ERR_INVALID_ARGUMENT, "set_view: missing camera buffers");
+    cudaStream_t s = (cudaStream_t)stream;
+    GRAY_LAUNCH("set_view", gray::launch_set_view(*p, origin, c2w, vertical_fov_radians, znear, zfar,
+                                                  rays_from_python != 0, s));
+    return GRAY_OK;
 }
 
 int gray_forward_pass_display(const gray_params *p, void *stream) {
     int e = check_trace(p);
     if (e) return e;
-    return forward(p, true, (cudaStream_t)stream);
+    return forward(p, true, -1, (cudaStream_t)stream);
 }
 
 int gray_backward_pass(const gray_params *p, void *stream) {

@@ -14,8 +14,12 @@ constexpr int kDefaultTraceVariant = 7;
 
 // scene.cu
 cudaError_t launch_snapshot(const gray_params &p, cudaStream_t s);
-// reset_frame: zero was_visible, count the call and empty the backward hit list (forward_pass)
-cudaError_t launch_forward_prep(const gray_params &p, bool reset_frame, cudaStream_t s);
+// reset_frame: zero was_visible, count the call and empty the backward hit list (forward_pass); grads: value
+// stored in metadata.grads_enabled with them (-1: left as it is)
+cudaError_t launch_forward_prep(const gray_params &p, bool reset_frame, int grads, cudaStream_t s);
+// the camera's and rays_from_python's device values
+cudaError_t launch_set_view(const gray_params &p, const float *origin, const float *c2w, float fov, float znear,
+                            float zfar, int rays_from_python, cudaStream_t s);
 cudaError_t launch_fold_and_sh_backward(const gray_params &p, cudaStream_t s);
 // a wait on an mbarrier phase that never completes, which must give up and report
 cudaError_t launch_copy_wait_selftest(int32_t *status, uint64_t limit_ns, cudaStream_t s);
@@ -55,6 +59,9 @@ cudaError_t launch_trace_batch(const gray_batch_scene *scenes, const gray_batch_
 // adam.cu
 cudaError_t launch_adam(const gray_params &p, cudaStream_t s);
 
+// capi.cu: multiprocessors of the current device, and the blocks of a kernel resident on one of them (asked
+// of the runtime once per kernel, block size, shared memory and device; any thread)
+cudaError_t resident_blocks(const void *kernel, int threads, size_t smem, int *sms, int *per_sm);
 // capi.cu: message returned by gray_last_error() on this thread
 void set_last_error(const char *what);
 // capi.cu: sets the message and returns GRAY_ERR_CUDA

@@ -292,14 +292,10 @@ cudaError_t launch_snapshot(const gray_params &p, cudaStream_t s) {
                       aligned16(p.scene.visible);
     const int tiles = bulk ? n / kSnapTile : 0;
     if (tiles > 0) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaError_t e;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, snapshot_bulk_kernel, kSnapTile, 0)) !=
-            cudaSuccess)
-            return e;
-        const int want = sms * (per_sm > 0 ? per_sm : 1);
+        int sms = 0, per_sm = 0;
+        cudaError_t e = resident_blocks(reinterpret_cast<const void *>(&snapshot_bulk_kernel), kSnapTile, 0, &sms, &per_sm);
+        if (e != cudaSuccess) return e;
+        const int want = sms * per_sm;
         snapshot_bulk_kernel<<<tiles < want ? tiles : want, kSnapTile, 0, s>>>(
             tiles, g.mean, rot, g.scale, g.opacity, p.config.alpha_threshold, p.config.exp_power,
             p.config.global_scale_factor, geom, l2w, aabb, p.scene.visible, p.status);
@@ -385,7 +381,7 @@ __global__ void __launch_bounds__(kPrepThreads) forward_prep_kernel(
     const float *__restrict__ mean, const float *__restrict__ cam_origin, const SHT *__restrict__ sh_dc,
     const SHT *__restrict__ sh_rest, float *__restrict__ channels, float2 *__restrict__ live,
     uint8_t *__restrict__ was_visible, uint32_t *__restrict__ total_num_calls, uint32_t *__restrict__ hit_counter,
-    int reset_frame, int count_call) {
+    uint8_t *__restrict__ grads_enabled, int grads, int reset_frame, int count_call) {
     extern __shared__ __align__(16) unsigned char prep_smem[];
     SHT *stage = reinterpret_cast<SHT *>(prep_smem);  // kPrepThreads * num_rest * 3 coefficients
     const int i0 = first + blockIdx.x * kPrepThreads;
@@ -393,6 +389,7 @@ __global__ void __launch_bounds__(kPrepThreads) forward_prep_kernel(
     if (count_call && blockIdx.x == 0 && threadIdx.x == 0) {
         *total_num_calls += 1u;
         *hit_counter = 0u;
+        if (grads >= 0) *grads_enabled = (uint8_t)grads;
     }
     const bool enable_sh = *cfg_enable_sh != 0;
     int degree = *current_sh_degree;
@@ -462,7 +459,7 @@ __global__ void __launch_bounds__(kPrepTile) forward_prep_bulk_kernel(
     const float *__restrict__ mean, const float *__restrict__ cam_origin, const SHT *__restrict__ sh_dc,
     const SHT *__restrict__ sh_rest, float *__restrict__ channels, float2 *__restrict__ live,
     uint8_t *__restrict__ was_visible, uint32_t *__restrict__ total_num_calls, uint32_t *__restrict__ hit_counter,
-    int reset_frame, int32_t *__restrict__ status) {
+    uint8_t *__restrict__ grads_enabled, int grads, int reset_frame, int32_t *__restrict__ status) {
     constexpr uint32_t T = kPrepTile, sb = sizeof(SHT);
     extern __shared__ __align__(16) unsigned char prep_smem[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(prep_smem);
@@ -477,6 +474,7 @@ __global__ void __launch_bounds__(kPrepTile) forward_prep_bulk_kernel(
     if (reset_frame && blockIdx.x == 0 && t == 0) {
         *total_num_calls += 1u;
         *hit_counter = 0u;
+        if (grads >= 0) *grads_enabled = (uint8_t)grads;
     }
     const bool enable_sh = *cfg_enable_sh != 0;
     int degree = *current_sh_degree;
@@ -549,7 +547,7 @@ __global__ void __launch_bounds__(kPrepTile) forward_prep_bulk_kernel(
 }
 
 template <typename SHT>
-static cudaError_t forward_prep_typed(const gray_params &p, bool reset_frame, cudaStream_t s) {
+static cudaError_t forward_prep_typed(const gray_params &p, bool reset_frame, int grads, cudaStream_t s) {
     const gray_gaussians &g = p.gaussians;
     const int n = g.count, num_rest = g.num_sh_coeffs;
     const SHT *dc = reinterpret_cast<const SHT *>(g.sh_coeffs_dc);
@@ -562,19 +560,18 @@ static cudaError_t forward_prep_typed(const gray_params &p, bool reset_frame, cu
     const int tiles = bulk ? n / kPrepTile : 0;
     cudaError_t e;
     if (tiles > 0) {
-        int dev = 0, sms = 0, per_sm = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, forward_prep_bulk_kernel<SHT>, kPrepTile,
-                                                               smem)) != cudaSuccess)
+        int sms = 0, per_sm = 0;
+        if ((e = resident_blocks(reinterpret_cast<const void *>(&forward_prep_bulk_kernel<SHT>), kPrepTile, smem, &sms,
+                                 &per_sm)) != cudaSuccess)
             return e;
         // at most kPrepBlocksPerSm blocks per SM: the forward's tile schedule runs beside this kernel
         // on another stream, and its blocks need shared memory too
-        const int want = sms * min(per_sm > 0 ? per_sm : 1, kPrepBlocksPerSm);
+        const int want = sms * min(per_sm, kPrepBlocksPerSm);
         forward_prep_bulk_kernel<SHT><<<tiles < want ? tiles : want, kPrepTile, smem, s>>>(
             tiles, num_rest, g.opacity, p.scene.visible, p.config.alpha_threshold, p.config.exp_power,
             p.config.enable_sh, g.current_sh_degree, g.max_sh_degree, g.mean, p.camera.origin, dc, rest, g.channels,
-            live, g.was_visible, p.metadata.total_num_calls, p.hitlist.total_words, reset_frame ? 1 : 0, p.status);
+            live, g.was_visible, p.metadata.total_num_calls, p.hitlist.total_words, p.metadata.grads_enabled, grads,
+            reset_frame ? 1 : 0, p.status);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     const int first = tiles * kPrepTile;
@@ -583,21 +580,47 @@ static cudaError_t forward_prep_typed(const gray_params &p, bool reset_frame, cu
         forward_prep_kernel<SHT><<<blocks_for(n - first, kPrepThreads), kPrepThreads, tail_smem, s>>>(
             first, n, num_rest, g.opacity, p.scene.visible, p.config.alpha_threshold, p.config.exp_power,
             p.config.enable_sh, g.current_sh_degree, g.max_sh_degree, g.mean, p.camera.origin, dc, rest, g.channels,
-            live, g.was_visible, p.metadata.total_num_calls, p.hitlist.total_words, reset_frame ? 1 : 0,
-            reset_frame && tiles == 0 ? 1 : 0);
+            live, g.was_visible, p.metadata.total_num_calls, p.hitlist.total_words, p.metadata.grads_enabled, grads,
+            reset_frame ? 1 : 0, reset_frame && tiles == 0 ? 1 : 0);
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_forward_prep(const gray_params &p, bool reset_frame, cudaStream_t s) {
+cudaError_t launch_forward_prep(const gray_params &p, bool reset_frame, int grads, cudaStream_t s) {
     const gray_gaussians &g = p.gaussians;
     if (reset_frame && g.count <= 0) {
         // still count the call and empty the hit list
         cudaError_t e = cudaMemsetAsync(p.hitlist.total_words, 0, sizeof(uint32_t), s);
+        if (e == cudaSuccess && grads >= 0) e = cudaMemsetAsync(p.metadata.grads_enabled, grads, 1, s);
         return e;
     }
     if (g.count <= 0) return cudaSuccess;
-    return g.sh_is_fp16 ? forward_prep_typed<__half>(p, reset_frame, s) : forward_prep_typed<float>(p, reset_frame, s);
+    return g.sh_is_fp16 ? forward_prep_typed<__half>(p, reset_frame, grads, s)
+                        : forward_prep_typed<float>(p, reset_frame, grads, s);
+}
+
+__global__ void set_view_kernel(gray_camera cam, uint8_t *rays_from_python, const float *origin, const float *c2w,
+                                float fov, float znear, float zfar, int rays) {
+    const int t = threadIdx.x;
+    if (t < 3) cam.origin[t] = origin[t];
+    if (t < 9) {
+        const float r = c2w[t];
+        cam.rotation_c2w[t] = r;
+        cam.rotation_w2c[3 * (t % 3) + t / 3] = r;
+    }
+    if (t == 0) {
+        *cam.vertical_fov_radians = fov;
+        *cam.znear = znear;
+        *cam.zfar = zfar;
+        *rays_from_python = (uint8_t)rays;
+    }
+}
+
+cudaError_t launch_set_view(const gray_params &p, const float *origin, const float *c2w, float fov, float znear,
+                            float zfar, int rays_from_python, cudaStream_t s) {
+    set_view_kernel<<<1, 32, 0, s>>>(p.camera, p.config.rays_from_python, origin, c2w, fov, znear, zfar,
+                                     rays_from_python);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -2401,17 +2401,13 @@ cudaError_t launch_trace_schedule(const gray_params &p, bool display, cudaStream
     if (!q.sched) return cudaSuccess;
     // densest tiles first: per-tile estimate and frontier, then the work order
     FwdArgs a = q.a;
-    int dev = 0, sms = 0;
-    cudaError_t e;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const void *kerns[2] = {q.kern, q.kern_wide ? q.kern_wide : q.kern};
     int slots[2] = {0, 0};
     for (int i = 0; i < 2; i++) {
-        int per_sm = 0;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[i], kFwdThreads, 0)) != cudaSuccess)
-            return e;
-        slots[i] = sms * (per_sm > 0 ? per_sm : 1);
+        int sms = 0, per_sm = 0;
+        const cudaError_t e = resident_blocks(kerns[i], kFwdThreads, 0, &sms, &per_sm);
+        if (e != cudaSuccess) return e;
+        slots[i] = sms * per_sm;
     }
     a.slots_narrow = slots[0];
     a.slots_wide = slots[1];
@@ -2430,9 +2426,6 @@ cudaError_t launch_trace_forward(const gray_params &p, bool display, bool schedu
         return cudaGetLastError();
     }
     if (!schedule_ready && (e = launch_trace_schedule(p, display, s)) != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     // persistent grids that take the split tiles' packets and the whole tiles in the schedule's order; with
     // the automatic choice both kernels of the whole tiles are launched and the one not chosen returns
     // at once.  The chain's second and third launch are programmatic: they run beside the one before.
@@ -2440,10 +2433,9 @@ cudaError_t launch_trace_forward(const gray_params &p, bool display, bool schedu
                             q.kern_wide};
     const int roles[3] = {0, q.kern_wide ? (int)kChoiceNarrow : 0, (int)kChoiceWide};
     for (int i = 0; i < 3 && kerns[i]; i++) {
-        int per_sm = 0;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[i], kFwdThreads, 0)) != cudaSuccess)
-            return e;
-        const unsigned int want = (unsigned int)(sms * (per_sm > 0 ? per_sm : 1));
+        int sms = 0, per_sm = 0;
+        if ((e = resident_blocks(kerns[i], kFwdThreads, 0, &sms, &per_sm)) != cudaSuccess) return e;
+        const unsigned int want = (unsigned int)(sms * per_sm);
         const unsigned int items = (i == 0 ? 4u : 1u) * (unsigned int)q.a.ntiles;  // at most
         FwdArgs a = q.a;
         a.auto_role = roles[i];

@@ -66,13 +66,8 @@ class Raytracer(torch.nn.Module):
         self.output_channels = None
 
     def __call__(self, cam_info: CameraInfo, znear=0.0, zfar=99999.9, skip_copy=False):
-        camera = self.cuda_module.get_camera()
-        camera.znear.fill_(znear)
-        camera.zfar.fill_(zfar)
-        config = self.cuda_module.get_config()
-        config.rays_from_python.fill_(False)
-        camera.vertical_fov_radians.fill_(cam_info.fov_y)
-        camera.set_pose(cam_info.origin_cuda(), cam_info.rotation_c2w_blender_cuda())
+        self.cuda_module.set_view(cam_info.origin_cuda(), cam_info.rotation_c2w_blender_cuda(), cam_info.fov_y, znear,
+                                  zfar)
         framebuffer = self.cuda_module.get_framebuffer()
         grad_enabled = torch.is_grad_enabled()
         assert not (skip_copy and grad_enabled), "skip_copy=True is not supported with gradients enabled"

@@ -148,8 +148,8 @@ typedef struct gray_scene {
     uint32_t *order;      /* [N] sorted leaf position -> gaussian id */
     uint32_t *codes;      /* [N] Morton codes in sorted order */
     uint32_t *refit_flags;/* [max(N-1,1)] */
-    uint32_t *sort_tmp;   /* [sort_tmp_words] radix-sort scratch of a rebuild; a refit keeps the
-                             nodes at its phases' boundaries in it (may be NULL for gray_update_bvh: the
+    uint32_t *sort_tmp;   /* [sort_tmp_words] radix-sort scratch of a rebuild; a refit queues the
+                             upper tree's first nodes in it (may be NULL for gray_update_bvh: the
                              refit then climbs the whole tree with global counters, slower) */
     float *root_box;      /* [8] */
     uint32_t *bounds;     /* [8] order-preserving encoded scene bounds (scratch) */
@@ -246,6 +246,16 @@ size_t gray_schedule_words(uint32_t width, uint32_t height);
  * hit list and was_visible, evaluates SH colours (if enable_sh) and traces the render
  * rectangle.  grads_enabled must have been set by the caller (MetaDataHolder::update). */
 int gray_forward_pass(const gray_params *p, void *stream);
+
+/* gray_forward_pass after storing grads_enabled (0 or 1) in metadata.grads_enabled, what
+ * MetaDataHolder::update does before it: one launch less. */
+int gray_forward_pass_mode(const gray_params *p, int32_t grads_enabled, void *stream);
+
+/* Camera of the next forwards in one launch: stores origin (device [3]), c2w (device [3,3], also as its
+ * transpose in rotation_w2c; CameraDataHolder::set_pose, cuda/core/camera.h:62-68), the vertical field of
+ * view, znear and zfar in p->camera and rays_from_python in p->config. */
+int gray_set_view(const gray_params *p, const float *origin, const float *c2w, float vertical_fov_radians,
+                  float znear, float zfar, int32_t rays_from_python, void *stream);
 
 /* Raytracer::forward_pass_display (cuda/raytracer.h:104-114): SH + trace, no resets. */
 int gray_forward_pass_display(const gray_params *p, void *stream);
