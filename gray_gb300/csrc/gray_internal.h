@@ -29,14 +29,19 @@ cudaError_t launch_batch_prep(const gray_params &p, const float *origins, int nv
 // lbvh.cu
 cudaError_t launch_lbvh_build(const gray_params &p, cudaStream_t s);
 cudaError_t launch_lbvh_refit(const gray_params &p, cudaStream_t s);
-// radix sort: a block sorts a tile of kSortThreads x kSortItems keys
+// radix sort: a block sorts a tile of kSortThreads x kSortItems keys, in four passes of 8-bit digits
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;
+constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;
-// sort scratch of a rebuild of n Gaussians: second key and value buffers, then 256 digit counts
-// per tile, then the 256 digit totals
+constexpr int kSortPasses = 4;
+constexpr int kSortGroup = 16;  // tiles whose digit counts are added up together
+// digit states of a pass, in rows of 256: one row per tile, then one per group of tiles
+constexpr size_t sort_state_rows(int tiles) { return (size_t)tiles + (size_t)((tiles + kSortGroup - 1) / kSortGroup); }
+// sort scratch of a rebuild of n Gaussians: second key and value buffers, then two sets of digit states (a
+// pass clears the next one's), then per pass the 256 digit totals, and the tile counters
 constexpr size_t sort_tmp_words(int n) {
-    return 2 * (size_t)n + 256 * (size_t)(n > 0 ? (n + kSortTile - 1) / kSortTile : 1) + 256;
+    return 2 * (size_t)n + 2 * 256 * sort_state_rows(n > 0 ? (n + kSortTile - 1) / kSortTile : 1) +
+           256 * kSortPasses + kSortPasses;
 }
 
 // trace.cu

@@ -1,8 +1,8 @@
 // lbvh.cu -- linear BVH over the Gaussians' leaf boxes (replaces the OptiX instance
 // acceleration structure built in cuda/optix/bvh_wrapper.h:89-115 and refit in :25-39).
 //
-// Build: scene bounds of the leaf-box centroids -> 30-bit Morton codes -> stable LSD radix
-// sort of (code, gaussian id) with 8-bit digits (4 passes, no CUB) -> Karras (2012)
+// Build: scene bounds of the leaf-box centroids -> 30-bit Morton codes and their digit histograms ->
+// stable LSD radix sort of (code, gaussian id) with 8-bit digits (4 passes of one kernel each, no CUB) -> Karras (2012)
 // hierarchy, one thread per internal node -> bottom-up boxes.
 // Refit: bottom-up boxes only; each internal node is finished by the second of its two
 // children to arrive (one visit counter per node, no spinning): first inside blocks of 256 sorted
@@ -27,10 +27,15 @@ __device__ __forceinline__ float ord2f(uint32_t u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-__global__ void bounds_init_kernel(uint32_t *bounds) {
-    int t = threadIdx.x;
-    if (t < 3) bounds[t] = 0xFFFFFFFFu;
-    else if (t < 6) bounds[t] = 0u;
+// Starting values of a build: the bounds, the digit totals and tile counters, and the first pass's states.
+__global__ void __launch_bounds__(kSortThreads) build_init_kernel(uint32_t *__restrict__ bounds,
+                                                                 uint32_t *__restrict__ totals,
+                                                                 uint32_t *__restrict__ states, int rows) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 3) bounds[i] = 0xFFFFFFFFu;
+    else if (i < 6) bounds[i] = 0u;
+    if (i < (256 + 1) * kSortPasses) totals[i] = 0u;
+    if (i < 256 * rows) states[i] = 0u;
 }
 
 // Scene bounds of the leaf-box centroids (finite ones only).  A grid-stride loop keeps each thread's
@@ -101,150 +106,206 @@ __device__ __forceinline__ uint32_t expand10(uint32_t v) {
     return v;
 }
 
-__global__ void morton_kernel(int n, const float4 *__restrict__ aabb, const uint32_t *__restrict__ bounds,
-                              uint32_t *__restrict__ codes, uint32_t *__restrict__ ids) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float4 a = aabb[2 * i], b = aabb[2 * i + 1];
-    float c[3] = {(a.x + b.x) * 0.5f, (a.y + b.y) * 0.5f, (a.z + b.z) * 0.5f};
-    bool fin = true;
-    uint32_t q[3];
+// Morton codes, and how many codes hold each value of each of the sort's digits (a block counts in shared
+// memory and adds its counts to totals[pass][digit]).
+__global__ void __launch_bounds__(kBoundsThreads) morton_kernel(int n, const float4 *__restrict__ aabb,
+                                                                const uint32_t *__restrict__ bounds,
+                                                                uint32_t *__restrict__ codes,
+                                                                uint32_t *__restrict__ totals) {
+    __shared__ uint32_t h[kSortPasses][256];
+    static_assert(kBoundsThreads == 256, "one digit per thread");
+#pragma unroll
+    for (int p = 0; p < kSortPasses; p++) h[p][threadIdx.x] = 0u;
+    __syncthreads();
+    float lo[3], ext[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        fin = fin && isfinite(c[k]);
-        float lo = ord2f(bounds[k]), hi = ord2f(bounds[3 + k]);
-        float ext = hi - lo;
-        float t = ext > 0.0f ? (c[k] - lo) / ext : 0.0f;
-        float s = fminf(fmaxf(t * 1024.0f, 0.0f), 1023.0f);
-        q[k] = fin ? (uint32_t)s : 0u;
+        lo[k] = ord2f(bounds[k]);
+        ext[k] = ord2f(bounds[3 + k]) - lo[k];
     }
-    codes[i] = fin ? ((expand10(q[0]) << 2) | (expand10(q[1]) << 1) | expand10(q[2])) : 0x40000000u;
-    ids[i] = (uint32_t)i;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 a = aabb[2 * (size_t)i], b = aabb[2 * (size_t)i + 1];
+        const float c[3] = {(a.x + b.x) * 0.5f, (a.y + b.y) * 0.5f, (a.z + b.z) * 0.5f};
+        bool fin = true;
+        uint32_t q[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            fin = fin && isfinite(c[k]);
+            const float t = ext[k] > 0.0f ? (c[k] - lo[k]) / ext[k] : 0.0f;
+            const float s = fminf(fmaxf(t * 1024.0f, 0.0f), 1023.0f);
+            q[k] = fin ? (uint32_t)s : 0u;
+        }
+        const uint32_t code =
+            fin ? ((expand10(q[0]) << 2) | (expand10(q[1]) << 1) | expand10(q[2])) : 0x40000000u;
+        codes[i] = code;
+#pragma unroll
+        for (int p = 0; p < kSortPasses; p++) atomicAdd(&h[p][(code >> 8 * p) & 0xFFu], 1u);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < kSortPasses; p++) {
+        const uint32_t v = h[p][threadIdx.x];
+        if (v) atomicAdd(&totals[256 * p + threadIdx.x], v);
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
-// Stable LSD radix sort, 8-bit digits.  A tile is kSortThreads x kSortItems keys processed in
-// kSortItems rounds of kSortThreads consecutive keys, so tile order == round-major order.
+// Stable LSD radix sort, 8-bit digits, one kernel per pass (decoupled look-back; Merrill & Garland 2016,
+// Adinets & Merrill 2022).  A block takes the next tile of kSortTile keys, ranks them (each warp its own
+// consecutive 512 keys, 32 at a time: __match_any_sync groups the lanes with one digit, the warp's
+// running counts give the rank), publishes its digit counts and adds up the counts of the tiles before
+// it: those of its group of kSortGroup tiles one by one, and the groups' before, which each group's last
+// tile publishes, back to one that knows its sum.  (Tile by tile, the 489 tiles of 2M keys, all running at
+// once, took 30 round trips to see back to the first.)  The keys are put in order in shared memory, so that
+// each digit's run is written by consecutive lanes.  Tiles are taken in order, so every tile before one
+// that waits is running or done; a wait is bounded all the same.
+// A pass is bound by the latency of one block's steps (the matches 11 of 29 us at 2M, the look-back 6), four
+// blocks per SM.  Three kernels a pass (histogram, row scan, scatter) took 32 us there, and eight launches
+// more: a build of 2000 Gaussians 136 -> 110 us, 30k 171 -> 148, 300k 213 -> 205, 2M 481 -> 475, 6M 1135 -> 1096.
 // ---------------------------------------------------------------------------------------------
-// (kSortThreads, kSortItems, kSortTile and sort_tmp_words are in gray_internal.h)
+// (kSortThreads, kSortItems, kSortTile, kSortPasses and sort_tmp_words are in gray_internal.h)
 constexpr int kSortWarps = kSortThreads / 32;
+constexpr uint32_t kTileCount = 1u << 30, kTileSum = 2u << 30;  // state: a tile's or group's count, or the sum up to it
+constexpr uint32_t kTileValue = (1u << 30) - 1u;               // (2^30 Gaussians at most)
+constexpr int kSortSpins = 1 << 22;
 
-__global__ void __launch_bounds__(kSortThreads) radix_hist_kernel(int n, int shift, const uint32_t *__restrict__ keys,
-                                                                 uint32_t *__restrict__ counts, int tiles) {
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
-    __syncthreads();
-    const int base = blockIdx.x * kSortTile;
-#pragma unroll
-    for (int r = 0; r < kSortItems; r++) {
-        int idx = base + r * kSortThreads + threadIdx.x;
-        if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 0xFFu], 1u);
-    }
-    __syncthreads();
-    counts[threadIdx.x * tiles + blockIdx.x] = h[threadIdx.x];
+__device__ __forceinline__ uint32_t load_state(const uint32_t *p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void store_state(uint32_t *p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Exclusive scan of each digit's row of tile counts (counts is digit-major: counts[d * tiles + tile]),
-// one block per digit, coalesced; the row's total goes to totals[d].  The scatter kernel adds each
-// digit's base (the exclusive scan of the 256 totals) itself.
-constexpr int kScanThreads = 512;
-
-__global__ void __launch_bounds__(kScanThreads) radix_row_scan_kernel(uint32_t *__restrict__ counts, int tiles,
-                                                                      uint32_t *__restrict__ totals) {
-    __shared__ uint32_t wsum[kScanThreads / 32];
-    __shared__ uint32_t carry;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    uint32_t *row = counts + (size_t)blockIdx.x * tiles;
-    if (t == 0) carry = 0u;
-    __syncthreads();
-    for (int c0 = 0; c0 < tiles; c0 += kScanThreads) {
-        const int i = c0 + t;
-        const uint32_t v = i < tiles ? row[i] : 0u;
-        uint32_t x = v;
+// Sum of the counts in `count` (< kSortGroup) consecutive rows, once all of them are set.
+__device__ __forceinline__ uint32_t sum_states(const uint32_t *row, int count, int &spins) {
+    for (;; spins--) {
+        uint32_t sum = 0u;
+        bool all = true;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
+        for (int j = 0; j < kSortGroup - 1; j++) {
+            const uint32_t v = j < count ? load_state(row + 256 * j) : kTileCount;
+            all = all && (v & kTileCount);
+            sum += v & kTileValue;
         }
-        if (lane == 31) wsum[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t w = lane < kScanThreads / 32 ? wsum[lane] : 0u;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, w, off);
-                if (lane >= off) w += y;
-            }
-            if (lane < kScanThreads / 32) wsum[lane] = w;  // inclusive over warps
-        }
-        __syncthreads();
-        const uint32_t before = carry + (warp > 0 ? wsum[warp - 1] : 0u);
-        if (i < tiles) row[i] = before + x - v;
-        __syncthreads();
-        if (t == 0) carry += wsum[kScanThreads / 32 - 1];
-        __syncthreads();
+        if (all || spins < 0) return sum;
     }
-    if (t == 0) totals[blockIdx.x] = carry;
 }
 
-__global__ void __launch_bounds__(kSortThreads) radix_scatter_kernel(int n, int shift,
-                                                                    const uint32_t *__restrict__ keys_in,
-                                                                    const uint32_t *__restrict__ vals_in,
-                                                                    uint32_t *__restrict__ keys_out,
-                                                                    uint32_t *__restrict__ vals_out,
-                                                                    const uint32_t *__restrict__ offsets, int tiles,
-                                                                    const uint32_t *__restrict__ totals) {
-    __shared__ uint32_t warp_cnt[kSortWarps][256];
-    __shared__ uint32_t digit_run[256];
-    __shared__ uint32_t digit_off[256];
-    __shared__ uint32_t wsum[kSortWarps];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    digit_run[t] = 0;
-    {   // digit t's base: exclusive scan of the 256 digit totals (one per thread)
-        const uint32_t v = totals[t];
-        uint32_t x = v;
+// Exclusive scan of one value per thread over the block's 256 threads (wsum: kSortWarps words).
+__device__ __forceinline__ uint32_t scan256(uint32_t v, uint32_t *wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        if (lane == 31) wsum[warp] = x;
-        __syncthreads();
-        uint32_t before = 0u;
-        for (int w = 0; w < warp; w++) before += wsum[w];
-        digit_off[t] = before + x - v + offsets[t * tiles + blockIdx.x];
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
     }
-    const uint32_t lanemask_lt = (1u << lane) - 1u;
-    const int base = blockIdx.x * kSortTile;
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    uint32_t before = 0u;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; w++)
+        if (w < warp) before += wsum[w];
+    __syncthreads();
+    return before + x - v;
+}
+
+__global__ void __launch_bounds__(kSortThreads, 4) radix_pass_kernel(
+    int n, int tiles, int shift, const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ vals_in,
+    uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, const uint32_t *__restrict__ totals,
+    uint32_t *__restrict__ states, uint32_t *__restrict__ states_next, uint32_t *__restrict__ taken,
+    int32_t *__restrict__ status) {
+    __shared__ uint32_t s_keys[kSortTile], s_vals[kSortTile];
+    __shared__ uint32_t s_cnt[kSortWarps][256];
+    __shared__ uint32_t s_local[256], s_global[256], s_wsum[kSortWarps], s_tile;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (t == 0) s_tile = atomicAdd(taken, 1u);
+#pragma unroll
+    for (int w = 0; w < kSortWarps; w++) s_cnt[w][t] = 0u;
+    __syncthreads();
+    const int tile = (int)s_tile, base = tile * kSortTile;
+    const int count = min(kSortTile, n - base);
+    states_next[256 * (size_t)tile + t] = 0u;
+    if (tile % kSortGroup == 0) states_next[256 * (size_t)(tiles + tile / kSortGroup) + t] = 0u;
+    uint32_t key[kSortItems], rank[kSortItems];
+    const int first = base + warp * 32 * kSortItems + lane;
+#pragma unroll
+    for (int r = 0; r < kSortItems; r++) key[r] = first + 32 * r < n ? keys_in[first + 32 * r] : 0u;
+#pragma unroll
     for (int r = 0; r < kSortItems; r++) {
+        const bool valid = first + 32 * r < n;
+        const uint32_t digit = (key[r] >> shift) & 0xFFu;
+        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? digit : 256u);
+        const uint32_t before = peers & ((1u << lane) - 1u);
+        uint32_t had = 0u;
+        if (valid && before == 0u) {
+            had = s_cnt[warp][digit];
+            s_cnt[warp][digit] = had + __popc(peers);
+        }
+        rank[r] = __shfl_sync(0xffffffffu, had, __ffs((int)peers) - 1) + __popc(before);
+        __syncwarp();
+    }
+    __syncthreads();
+    // thread t: digit t.  Its count before each warp, in the tile, and in the tiles before this one
+    uint32_t sum = 0u;
 #pragma unroll
-        for (int w = 0; w < kSortWarps; w++) warp_cnt[w][t] = 0;
-        __syncthreads();
-        const int idx = base + r * kSortThreads + t;
-        const bool valid = idx < n;
-        uint32_t key = valid ? keys_in[idx] : 0u, val = valid ? vals_in[idx] : 0u;
-        uint32_t digit = valid ? (key >> shift) & 0xFFu : 256u + (uint32_t)lane;  // invalid lanes never match
-        uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        uint32_t rank = __popc(peers & lanemask_lt);
-        if (valid && rank == 0) warp_cnt[warp][digit] = __popc(peers);
-        __syncthreads();
-        {   // per digit: exclusive prefix over warps, continuing the tile's running count
-            uint32_t run = digit_run[t];
+    for (int w = 0; w < kSortWarps; w++) {
+        const uint32_t c = s_cnt[w][t];
+        s_cnt[w][t] = sum;
+        sum += c;
+    }
+    uint32_t *const state = states + t, *const group = states + 256 * (size_t)tiles + t;
+    const int g = tile / kSortGroup, in_group = tile % kSortGroup;
+    store_state(state + 256 * (size_t)tile, kTileCount | sum);
+    const uint32_t local = scan256(sum, s_wsum), start = scan256(totals[t], s_wsum);
+    int spins = kSortSpins;
+    uint32_t earlier = sum_states(state + 256 * (size_t)(tile - in_group), in_group, spins);
+    if (in_group == kSortGroup - 1)
+        store_state(group + 256 * (size_t)g, (g == 0 ? kTileSum : kTileCount) | (earlier + sum));
+    uint32_t groups = 0u;
+    for (int p = g - 1; p >= 0 && spins >= 0; spins--) {
+        uint32_t v[kSortGroup];
 #pragma unroll
-            for (int w = 0; w < kSortWarps; w++) {
-                uint32_t c = warp_cnt[w][t];
-                warp_cnt[w][t] = run;
-                run += c;
+        for (int j = 0; j < kSortGroup; j++) v[j] = p - j >= 0 ? load_state(group + 256 * (size_t)(p - j)) : kTileSum;
+        bool known = true;  // every state up to here was set, and none was a sum
+#pragma unroll
+        for (int j = 0; j < kSortGroup; j++) {
+            if (known && (v[j] & (kTileCount | kTileSum))) {
+                groups += v[j] & kTileValue;
+                known = (v[j] & kTileSum) == 0u;
+                p = known ? p - 1 : -1;
+            } else {
+                known = false;
             }
-            digit_run[t] = run;
         }
-        __syncthreads();
-        if (valid) {
-            uint32_t pos = digit_off[digit] + warp_cnt[warp][digit] + rank;
-            keys_out[pos] = key;
-            vals_out[pos] = val;
+    }
+    if (in_group == kSortGroup - 1 && g > 0) store_state(group + 256 * (size_t)g, kTileSum | (groups + earlier + sum));
+    earlier += groups;
+    if (spins < 0 && status) atomicOr(status, GRAY_STATUS_REFIT_TIMEOUT);
+    s_local[t] = local;
+    s_global[t] = start + earlier - local;  // of the digit's first key, less its place in the tile
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSortItems; r++) {
+        const int i = first + 32 * r;
+        if (i < n) {
+            const uint32_t digit = (key[r] >> shift) & 0xFFu;
+            const uint32_t at = s_local[digit] + s_cnt[warp][digit] + rank[r];
+            s_keys[at] = key[r];
+            s_vals[at] = vals_in ? vals_in[i] : (uint32_t)i;
         }
-        __syncthreads();
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int i = t; i < count; i += kSortThreads) {
+        const uint32_t k = s_keys[i];
+        const uint32_t pos = s_global[(k >> shift) & 0xFFu] + (uint32_t)i;
+        if (pos < (uint32_t)n) {  // (always, unless a wait ran out)
+            keys_out[pos] = k;
+            vals_out[pos] = s_vals[i];
+        }
     }
 }
 
@@ -555,25 +616,31 @@ cudaError_t launch_lbvh_build(const gray_params &p, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const gray_scene &sc = p.scene;
     cudaError_t e;
-    bounds_init_kernel<<<1, 32, 0, s>>>(sc.bounds);
-    bounds_kernel<<<min(blocks_for(n, kBoundsThreads), (unsigned)kBoundsMaxBlocks), kBoundsThreads, 0, s>>>(
-        n, reinterpret_cast<const float4 *>(sc.aabb), sc.bounds);
-    morton_kernel<<<blocks_for(n), kThreads, 0, s>>>(n, reinterpret_cast<const float4 *>(sc.aabb), sc.bounds, sc.codes,
-                                                    sc.order);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const int tiles = (n + kSortTile - 1) / kSortTile;
-    uint32_t *keys_alt = sc.sort_tmp, *vals_alt = sc.sort_tmp + n, *counts = sc.sort_tmp + 2 * (size_t)n;
-    uint32_t *totals = counts + 256 * (size_t)tiles;
-    uint32_t *kin = sc.codes, *vin = sc.order, *kout = keys_alt, *vout = vals_alt;
-    for (int shift = 0; shift < 32; shift += 8) {
-        radix_hist_kernel<<<tiles, kSortThreads, 0, s>>>(n, shift, kin, counts, tiles);
-        radix_row_scan_kernel<<<256, kScanThreads, 0, s>>>(counts, tiles, totals);
-        radix_scatter_kernel<<<tiles, kSortThreads, 0, s>>>(n, shift, kin, vin, kout, vout, counts, tiles, totals);
-        uint32_t *tk = kin, *tv = vin;
+    uint32_t *keys_alt = sc.sort_tmp, *vals_alt = sc.sort_tmp + n, *states = sc.sort_tmp + 2 * (size_t)n;
+    uint32_t *states_alt = states + 256 * sort_state_rows(tiles);
+    uint32_t *totals = states_alt + 256 * sort_state_rows(tiles);
+    uint32_t *taken = totals + 256 * kSortPasses;
+    const int rows = (int)sort_state_rows(tiles);
+    build_init_kernel<<<rows > kSortPasses ? rows : kSortPasses + 1, kSortThreads, 0, s>>>(sc.bounds, totals, states,
+                                                                                          rows);
+    const unsigned wide = min(blocks_for(n, kBoundsThreads), (unsigned)kBoundsMaxBlocks);
+    bounds_kernel<<<wide, kBoundsThreads, 0, s>>>(n, reinterpret_cast<const float4 *>(sc.aabb), sc.bounds);
+    morton_kernel<<<wide, kBoundsThreads, 0, s>>>(n, reinterpret_cast<const float4 *>(sc.aabb), sc.bounds, sc.codes,
+                                                  totals);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    uint32_t *kin = sc.codes, *vin = nullptr, *kout = keys_alt, *vout = vals_alt;  // (first pass: ids in order)
+    for (int pass = 0; pass < kSortPasses; pass++) {
+        radix_pass_kernel<<<tiles, kSortThreads, 0, s>>>(n, tiles, 8 * pass, kin, vin, kout, vout,
+                                                         totals + 256 * pass, states, states_alt, taken + pass,
+                                                         p.status);
         kin = kout;
         vin = vout;
-        kout = tk;
-        vout = tv;
+        kout = pass & 1 ? keys_alt : sc.codes;
+        vout = pass & 1 ? vals_alt : sc.order;
+        uint32_t *const st = states;
+        states = states_alt;
+        states_alt = st;
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // four passes: the sorted keys/ids are back in codes/order
