@@ -148,19 +148,16 @@ __device__ __forceinline__ void snapshot_one(const float mu_in[3], float4 q, con
     out.vis = vis;
 }
 
-// One thread per Gaussian of [first, n): the short tail of the bulk-pipelined kernel, and the
-// whole snapshot when a pointer is not 16-byte aligned.
-__global__ void snapshot_kernel(int first, int n, const float *__restrict__ mean, const float4 *__restrict__ rotation,
-                                const float *__restrict__ scale, const float *__restrict__ opacity,
-                                const float *__restrict__ cfg_alpha_threshold, const float *__restrict__ cfg_exp_power,
-                                const float *__restrict__ cfg_gsf, float4 *__restrict__ geom, float4 *__restrict__ l2w,
-                                float4 *__restrict__ aabb, uint8_t *__restrict__ visible) {
-    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// Gaussian i's snapshot, straight from and to memory.
+__device__ __forceinline__ void snapshot_row(int i, const float *__restrict__ mean,
+                                             const float4 *__restrict__ rotation, const float *__restrict__ scale,
+                                             const float *__restrict__ opacity, float athr, float pw, float gsf,
+                                             float4 *__restrict__ geom, float4 *__restrict__ l2w,
+                                             float4 *__restrict__ aabb, uint8_t *__restrict__ visible) {
     const float mu[3] = {mean[3 * i], mean[3 * i + 1], mean[3 * i + 2]};
     const float ls[3] = {scale[3 * i], scale[3 * i + 1], scale[3 * i + 2]};
     SnapRecord r;
-    snapshot_one(mu, rotation[i], ls, opacity[i], *cfg_alpha_threshold, *cfg_exp_power, *cfg_gsf, r);
+    snapshot_one(mu, rotation[i], ls, opacity[i], athr, pw, gsf, r);
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         geom[3 * i + k] = r.g[k];
@@ -171,6 +168,19 @@ __global__ void snapshot_kernel(int first, int n, const float *__restrict__ mean
     visible[i] = r.vis ? 1 : 0;
 }
 
+// One thread per Gaussian: the whole snapshot when there are fewer than a tile or a pointer is not
+// 16-byte aligned.
+__global__ void snapshot_kernel(int n, const float *__restrict__ mean, const float4 *__restrict__ rotation,
+                                const float *__restrict__ scale, const float *__restrict__ opacity,
+                                const float *__restrict__ cfg_alpha_threshold, const float *__restrict__ cfg_exp_power,
+                                const float *__restrict__ cfg_gsf, float4 *__restrict__ geom, float4 *__restrict__ l2w,
+                                float4 *__restrict__ aabb, uint8_t *__restrict__ visible) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n)
+        snapshot_row(i, mean, rotation, scale, opacity, *cfg_alpha_threshold, *cfg_exp_power, *cfg_gsf, geom, l2w,
+                     aabb, visible);
+}
+
 // Bulk-pipelined snapshot: a persistent block takes tiles of kSnapTile consecutive Gaussians.  One
 // thread loads a tile's parameter rows (mean, rotation, scale, opacity: 44 B per Gaussian, four
 // contiguous ranges) into shared memory with bulk copies completing on an mbarrier, double-buffered
@@ -179,7 +189,8 @@ __global__ void snapshot_kernel(int first, int n, const float *__restrict__ mean
 // thread then stores with four bulk copies (geom, l2w, aabb, visible: 129 B per Gaussian) while the
 // block goes on.  Every copy starts on a 16-byte boundary and spans a multiple of 16 bytes (the
 // launcher checks the pointers; the tile is a multiple of 16 Gaussians).  Gaussians past the last
-// full tile go to snapshot_kernel.
+// full tile are the last block's, a thread each, while its first tile loads (in a launch of their own
+// they held up the stream for 4 us).
 constexpr int kSnapTile = 128;
 static_assert(kSnapTile % 16 == 0, "every per-tile range must span a multiple of 16 bytes");
 
@@ -208,7 +219,7 @@ __device__ __forceinline__ void snap_issue_loads(SnapIn &in, uint64_t *bar, int 
 }
 
 __global__ void __launch_bounds__(kSnapTile) snapshot_bulk_kernel(
-    int tiles, const float *__restrict__ mean, const float4 *__restrict__ rotation, const float *__restrict__ scale,
+    int n, int tiles, const float *__restrict__ mean, const float4 *__restrict__ rotation, const float *__restrict__ scale,
     const float *__restrict__ opacity, const float *__restrict__ cfg_alpha_threshold,
     const float *__restrict__ cfg_exp_power, const float *__restrict__ cfg_gsf, float4 *__restrict__ geom,
     float4 *__restrict__ l2w, float4 *__restrict__ aabb, uint8_t *__restrict__ visible, int32_t *__restrict__ status) {
@@ -225,6 +236,8 @@ __global__ void __launch_bounds__(kSnapTile) snapshot_bulk_kernel(
     const float athr = *cfg_alpha_threshold, pw = *cfg_exp_power, gsf = *cfg_gsf;
     int tile = blockIdx.x;
     if (t == 0 && tile < tiles) snap_issue_loads(in[0], &bar[0], tile, mean, rotation, scale, opacity);
+    if (blockIdx.x == gridDim.x - 1 && tiles * kSnapTile + t < n)
+        snapshot_row(tiles * kSnapTile + t, mean, rotation, scale, opacity, athr, pw, gsf, geom, l2w, aabb, visible);
     int it = 0;
     bool timed_out = false;
     for (; tile < tiles; it++, tile += gridDim.x) {
@@ -297,15 +310,13 @@ cudaError_t launch_snapshot(const gray_params &p, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         const int want = sms * per_sm;
         snapshot_bulk_kernel<<<tiles < want ? tiles : want, kSnapTile, 0, s>>>(
-            tiles, g.mean, rot, g.scale, g.opacity, p.config.alpha_threshold, p.config.exp_power,
+            n, tiles, g.mean, rot, g.scale, g.opacity, p.config.alpha_threshold, p.config.exp_power,
             p.config.global_scale_factor, geom, l2w, aabb, p.scene.visible, p.status);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        return cudaGetLastError();
     }
-    const int first = tiles * kSnapTile;
-    if (first < n)
-        snapshot_kernel<<<blocks_for(n - first), kThreads, 0, s>>>(
-            first, n, g.mean, rot, g.scale, g.opacity, p.config.alpha_threshold, p.config.exp_power,
-            p.config.global_scale_factor, geom, l2w, aabb, p.scene.visible);
+    snapshot_kernel<<<blocks_for(n), kThreads, 0, s>>>(n, g.mean, rot, g.scale, g.opacity, p.config.alpha_threshold,
+                                                       p.config.exp_power, p.config.global_scale_factor, geom, l2w,
+                                                       aabb, p.scene.visible);
     return cudaGetLastError();
 }
 
@@ -370,23 +381,23 @@ __device__ __forceinline__ void sh_colour(const float mu[3], const float *cam, c
     }
 }
 
-// One thread per Gaussian of [first, n), SH rows staged through shared memory with coalesced loads:
-// the tail of the bulk-pipelined kernel, and the whole pass when a pointer is not 16-byte aligned.
-// count_call: this launch counts the forward call and empties the backward hit list.
+// One thread per Gaussian, SH rows staged through shared memory with coalesced loads: the whole pass when
+// there are fewer than a tile or a pointer is not 16-byte aligned.
+// reset_frame: this launch counts the forward call and empties the backward hit list too.
 template <typename SHT>
 __global__ void __launch_bounds__(kPrepThreads) forward_prep_kernel(
-    int first, int n, int num_rest, const float *__restrict__ opacity, const uint8_t *__restrict__ visible,
+    int n, int num_rest, const float *__restrict__ opacity, const uint8_t *__restrict__ visible,
     const float *__restrict__ cfg_alpha_threshold, const float *__restrict__ cfg_exp_power,
     const uint8_t *__restrict__ cfg_enable_sh, const int32_t *__restrict__ current_sh_degree, int max_sh_degree,
     const float *__restrict__ mean, const float *__restrict__ cam_origin, const SHT *__restrict__ sh_dc,
     const SHT *__restrict__ sh_rest, float *__restrict__ channels, float2 *__restrict__ live,
     uint8_t *__restrict__ was_visible, uint32_t *__restrict__ total_num_calls, uint32_t *__restrict__ hit_counter,
-    uint8_t *__restrict__ grads_enabled, int grads, int reset_frame, int count_call) {
+    uint8_t *__restrict__ grads_enabled, int grads, int reset_frame) {
     extern __shared__ __align__(16) unsigned char prep_smem[];
     SHT *stage = reinterpret_cast<SHT *>(prep_smem);  // kPrepThreads * num_rest * 3 coefficients
-    const int i0 = first + blockIdx.x * kPrepThreads;
+    const int i0 = blockIdx.x * kPrepThreads;
     const int i = i0 + threadIdx.x;
-    if (count_call && blockIdx.x == 0 && threadIdx.x == 0) {
+    if (reset_frame && blockIdx.x == 0 && threadIdx.x == 0) {
         *total_num_calls += 1u;
         *hit_counter = 0u;
         if (grads >= 0) *grads_enabled = (uint8_t)grads;
@@ -453,7 +464,7 @@ __device__ __forceinline__ void prep_issue_loads(unsigned char *stg, uint64_t *b
 
 template <typename SHT>
 __global__ void __launch_bounds__(kPrepTile) forward_prep_bulk_kernel(
-    int tiles, int num_rest, const float *__restrict__ opacity, const uint8_t *__restrict__ visible,
+    int n, int tiles, int num_rest, const float *__restrict__ opacity, const uint8_t *__restrict__ visible,
     const float *__restrict__ cfg_alpha_threshold, const float *__restrict__ cfg_exp_power,
     const uint8_t *__restrict__ cfg_enable_sh, const int32_t *__restrict__ current_sh_degree, int max_sh_degree,
     const float *__restrict__ mean, const float *__restrict__ cam_origin, const SHT *__restrict__ sh_dc,
@@ -491,6 +502,20 @@ __global__ void __launch_bounds__(kPrepTile) forward_prep_bulk_kernel(
     int tile = blockIdx.x;
     if (t == 0 && tile < tiles)
         prep_issue_loads<SHT>(stages, &bar[0], tile, per, enable_sh, nb > 0, opacity, mean, visible, sh_dc, sh_rest);
+    if (blockIdx.x == gridDim.x - 1 && tiles * (int)T + t < n) {
+        // the Gaussians past the last full tile, while the block's first tile loads
+        const size_t i = (size_t)tiles * T + t;
+        const float o = sigmoid_act(opacity[i]);
+        live[i] = make_float2(visible[i] ? o : __int_as_float(0xff800000), scaling_factor(o, athr, pw));
+        if (enable_sh) {
+            const float mu[3] = {mean[3 * i], mean[3 * i + 1], mean[3 * i + 2]};
+            float col[3];
+            sh_colour<SHT>(mu, cam, sh_dc + 3 * i, sh_rest + (size_t)per * i, nb, col);
+#pragma unroll
+            for (int c = 0; c < 3; c++) channels[3 * i + c] = col[c];
+        }
+        if (reset_frame) was_visible[i] = 0;
+    }
     int it = 0;
     bool timed_out = false;
     for (; tile < tiles; it++, tile += gridDim.x) {
@@ -568,21 +593,17 @@ static cudaError_t forward_prep_typed(const gray_params &p, bool reset_frame, in
         // on another stream, and its blocks need shared memory too
         const int want = sms * min(per_sm, kPrepBlocksPerSm);
         forward_prep_bulk_kernel<SHT><<<tiles < want ? tiles : want, kPrepTile, smem, s>>>(
-            tiles, num_rest, g.opacity, p.scene.visible, p.config.alpha_threshold, p.config.exp_power,
+            n, tiles, num_rest, g.opacity, p.scene.visible, p.config.alpha_threshold, p.config.exp_power,
             p.config.enable_sh, g.current_sh_degree, g.max_sh_degree, g.mean, p.camera.origin, dc, rest, g.channels,
             live, g.was_visible, p.metadata.total_num_calls, p.hitlist.total_words, p.metadata.grads_enabled, grads,
             reset_frame ? 1 : 0, p.status);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        return cudaGetLastError();
     }
-    const int first = tiles * kPrepTile;
-    if (first < n) {
-        const size_t tail_smem = (size_t)kPrepThreads * (size_t)(num_rest > 0 ? num_rest : 1) * 3 * sizeof(SHT);
-        forward_prep_kernel<SHT><<<blocks_for(n - first, kPrepThreads), kPrepThreads, tail_smem, s>>>(
-            first, n, num_rest, g.opacity, p.scene.visible, p.config.alpha_threshold, p.config.exp_power,
-            p.config.enable_sh, g.current_sh_degree, g.max_sh_degree, g.mean, p.camera.origin, dc, rest, g.channels,
-            live, g.was_visible, p.metadata.total_num_calls, p.hitlist.total_words, p.metadata.grads_enabled, grads,
-            reset_frame ? 1 : 0, reset_frame && tiles == 0 ? 1 : 0);
-    }
+    const size_t staged = (size_t)kPrepThreads * (size_t)(num_rest > 0 ? num_rest : 1) * 3 * sizeof(SHT);
+    forward_prep_kernel<SHT><<<blocks_for(n, kPrepThreads), kPrepThreads, staged, s>>>(
+        n, num_rest, g.opacity, p.scene.visible, p.config.alpha_threshold, p.config.exp_power, p.config.enable_sh,
+        g.current_sh_degree, g.max_sh_degree, g.mean, p.camera.origin, dc, rest, g.channels, live, g.was_visible,
+        p.metadata.total_num_calls, p.hitlist.total_words, p.metadata.grads_enabled, grads, reset_frame ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -2580,24 +2580,31 @@ __device__ __forceinline__ void bwd_record_one(float2 lv, const float log_s[3], 
     r[5] = make_float4(q.x / qlen, q.y / qlen, q.z / qlen, q.w / qlen);
 }
 
-// One thread per Gaussian of [first, n): the tail of the bulk-pipelined kernel, and the whole pass
-// when a pointer is not 16-byte aligned.
-__global__ void __launch_bounds__(256) bwd_record_kernel(int first, int n, const float2 *__restrict__ live,
+// Gaussian i's record, straight from and to memory.
+__device__ __forceinline__ void bwd_record_row(int i, const float2 *__restrict__ live, const float *__restrict__ scale,
+                                               const float4 *__restrict__ rotation,
+                                               const float *__restrict__ channels, const float4 *__restrict__ l2w,
+                                               float eps, float4 *__restrict__ rec) {
+    const float ls[3] = {scale[3 * i], scale[3 * i + 1], scale[3 * i + 2]};
+    const float ch[3] = {channels[3 * i], channels[3 * i + 1], channels[3 * i + 2]};
+    float4 r[kRecVec];
+    bwd_record_one(live[i], ls, rotation[i], ch, l2w[3 * i], l2w[3 * i + 1], l2w[3 * i + 2], eps, r);
+    float4 *o = rec + kRecVec * (size_t)i;
+#pragma unroll
+    for (int k = 0; k < kRecVec; k++) o[k] = r[k];
+}
+
+// One thread per Gaussian: the whole pass when there are fewer than a tile or a pointer is not 16-byte
+// aligned.
+__global__ void __launch_bounds__(256) bwd_record_kernel(int n, const float2 *__restrict__ live,
                                                          const float *__restrict__ scale,
                                                          const float4 *__restrict__ rotation,
                                                          const float *__restrict__ channels,
                                                          const float4 *__restrict__ l2w,
                                                          const float *__restrict__ eps_scale_grad,
                                                          float4 *__restrict__ rec) {
-    const int i = first + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float ls[3] = {scale[3 * i], scale[3 * i + 1], scale[3 * i + 2]};
-    const float ch[3] = {channels[3 * i], channels[3 * i + 1], channels[3 * i + 2]};
-    float4 r[kRecVec];
-    bwd_record_one(live[i], ls, rotation[i], ch, l2w[3 * i], l2w[3 * i + 1], l2w[3 * i + 2], *eps_scale_grad, r);
-    float4 *o = rec + kRecVec * (size_t)i;
-#pragma unroll
-    for (int k = 0; k < kRecVec; k++) o[k] = r[k];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) bwd_record_row(i, live, scale, rotation, channels, l2w, *eps_scale_grad, rec);
 }
 
 // Bulk-pipelined record pass: persistent blocks take tiles of kRecTile Gaussians; one thread loads
@@ -2631,7 +2638,7 @@ __device__ __forceinline__ void rec_issue_loads(RecIn &in, uint64_t *bar, int ti
 }
 
 __global__ void __launch_bounds__(kRecTile) bwd_record_bulk_kernel(
-    int tiles, const float2 *__restrict__ live, const float *__restrict__ scale, const float4 *__restrict__ rotation,
+    int n, int tiles, const float2 *__restrict__ live, const float *__restrict__ scale, const float4 *__restrict__ rotation,
     const float *__restrict__ channels, const float4 *__restrict__ l2w, const float *__restrict__ eps_scale_grad,
     float4 *__restrict__ rec, int32_t *__restrict__ status) {
     __shared__ __align__(16) RecIn in[2];
@@ -2647,6 +2654,9 @@ __global__ void __launch_bounds__(kRecTile) bwd_record_bulk_kernel(
     const float eps = *eps_scale_grad;
     int tile = blockIdx.x;
     if (t == 0 && tile < tiles) rec_issue_loads(in[0], &bar[0], tile, live, scale, rotation, channels, l2w);
+    // the Gaussians past the last full tile are the last block's, while its first tile loads
+    if (blockIdx.x == gridDim.x - 1 && tiles * kRecTile + t < n)
+        bwd_record_row(tiles * kRecTile + t, live, scale, rotation, channels, l2w, eps, rec);
     int it = 0;
     bool timed_out = false;
     for (; tile < tiles; it++, tile += gridDim.x) {
@@ -2871,22 +2881,18 @@ cudaError_t launch_trace_backward(const gray_params &p, cudaStream_t s) {
         const int tiles = bulk ? n / kRecTile : 0;
         cudaError_t e;
         if (tiles > 0) {
-            int dev = 0, sms = 0, per_sm = 0;
-            if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-            if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bwd_record_bulk_kernel, kRecTile, 0)) !=
-                cudaSuccess)
+            int sms = 0, per_sm = 0;
+            if ((e = resident_blocks(reinterpret_cast<const void *>(&bwd_record_bulk_kernel), kRecTile, 0, &sms,
+                                     &per_sm)) != cudaSuccess)
                 return e;
-            const int want = sms * (per_sm > 0 ? per_sm : 1);
+            const int want = sms * per_sm;
             bwd_record_bulk_kernel<<<tiles < want ? tiles : want, kRecTile, 0, s>>>(
-                tiles, live, p.gaussians.scale, rot, p.gaussians.channels, l2w, p.config.eps_scale_grad, rec,
+                n, tiles, live, p.gaussians.scale, rot, p.gaussians.channels, l2w, p.config.eps_scale_grad, rec,
                 p.status);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        } else {
+            bwd_record_kernel<<<(unsigned int)((n + 255) / 256), 256, 0, s>>>(
+                n, live, p.gaussians.scale, rot, p.gaussians.channels, l2w, p.config.eps_scale_grad, rec);
         }
-        const int first = tiles * kRecTile;
-        if (first < n)
-            bwd_record_kernel<<<(unsigned int)((n - first + 255) / 256), 256, 0, s>>>(
-                first, n, live, p.gaussians.scale, rot, p.gaussians.channels, l2w, p.config.eps_scale_grad, rec);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     BwdArgs a;
