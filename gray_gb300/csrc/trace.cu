@@ -42,6 +42,8 @@ constexpr int kMaxTraversals = 4 * kMaxPasses * 2;  // bound on re-traversals of
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kBatch = 128;       // leaves fetched and tested together by a block (one per thread)
 constexpr int kTileStack = 448;   // per-block traversal stack
+constexpr int kSplitStack = 1536;  // of a block that traces a split tile's packet
+constexpr int kStackReserve = 72;  // entries left to a depth-first descent (deeper than any tree)
 constexpr int kTileQueue = kBatch + 2 * kFwdThreads;  // queued leaves: < kBatch before a step, + up to 2 per thread
 static_assert(kBatch == kFwdThreads, "one leaf per thread");
 constexpr int kSchedHeader = 64;  // schedule words before the per-tile estimates
@@ -461,9 +463,10 @@ __device__ __forceinline__ float conic_coefficients(const ConicBasis &cb, const 
     return -__fdividef(fdot3(lo, l0), ll0);
 }
 
-// Shared memory of a block that traces one pixel tile (one ray per thread).
-template <int KB>
+// Shared memory of a block that traces one pixel tile (one ray per thread), or, SPLIT, a packet of one.
+template <int KB, bool SPLIT>
 struct TileShared {
+    static constexpr int kStack = SPLIT ? kSplitStack : kTileStack;
     unsigned long long kbuf[KB][kFwdThreads];
     // the batch's candidates, filled once per batch by the block (one candidate per thread):
     float4 g[kBatch][3];       // snapshot rows with the tile's object-space origin: (M | M (o - mu))
@@ -471,7 +474,7 @@ struct TileShared {
     float4 conic[kBatch / 2][3];  // coefficients of candidates 2i, 2i+1: (F F' D D') (E E' A A') (B B' C C')
     float sf[kBatch];          // live scaling factor
     uint32_t gid[kBatch];
-    uint32_t stk[kTileStack];
+    uint32_t stk[kStack];
     alignas(16) uint32_t queue[kTileQueue];
     Frustum fr;
     ConicBasis cb;
@@ -496,7 +499,7 @@ struct TileShared {
 template <int KB, bool SPLIT>
 __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px,
                                                    float py, bool want, bool first, LaneState &st,
-                                                   TileShared<KB> &sh, int take, int nc) {
+                                                   TileShared<KB, SPLIT> &sh, int take, int nc) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     {
         uint32_t gid = 0;
@@ -624,11 +627,11 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
 // kFrontierMax or a null pointer: none) the traversal starts there instead of at the root: the frontier
 // goes onto the stack with its first entry on top, and a frontier leaf is queued when it is popped.
 // px, py: the ray's offset from the tile's centre in the conics' basis.  Returns false if the stack
-// filled up (the caller then repeats the traversal per ray).
+// filled up (a malformed tree; the caller then repeats the traversal per ray).
 template <int KB, bool SPLIT>
 __device__ __forceinline__ bool traverse_tile(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px,
                                               float py, bool want, bool first, LaneState &st,
-                                              TileShared<KB> &sh, const uint32_t *front, int32_t *status) {
+                                              TileShared<KB, SPLIT> &sh, const uint32_t *front, int32_t *status) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
     const int n = sc.n;
@@ -656,9 +659,11 @@ __device__ __forceinline__ bool traverse_tile(const TraceScene &sc, const TraceK
                 sp = 0;
                 break;
             }
-            // a popped node frees its entry and pushes at most two
-            const int take = min(min(sp, kFwdThreads), kTileStack - sp);
-            if (take <= 0) return false;
+            // a popped node frees its entry and pushes at most two: as many at once as fit below the reserve, and
+            // in it one by one (a descent adds one entry per level, fewer than the reserve holds)
+            const int room = TileShared<KB, SPLIT>::kStack - kStackReserve - sp;
+            const int take = min(min(sp, kFwdThreads), max(room, 1));
+            if (room + kStackReserve <= 1) return false;
             const uint32_t node = t < take ? sh.stk[sp - 1 - t] : GRAY_NULL;
             // children as (a, b) = (nearer, farther) along the tile's mean direction
             bool pa = false, pb = false;
@@ -738,13 +743,13 @@ struct SplitView {
     uint32_t *gids;  // [kSplitKeys][32]
     uint8_t *src;    // [kSplitKeys][32]
     int *bound;      // [kWarps][32]
-    __device__ __forceinline__ explicit SplitView(TileShared<KB> &sh)
+    __device__ __forceinline__ explicit SplitView(TileShared<KB, true> &sh)
         : gids(reinterpret_cast<uint32_t *>(sh.g)), src(reinterpret_cast<uint8_t *>(sh.conic)),
           bound(reinterpret_cast<int *>(sh.sf)) {}
 };
 
 template <int KB>
-__device__ __forceinline__ void merge_split(LaneState &st, TileShared<KB> &sh, bool first) {
+__device__ __forceinline__ void merge_split(LaneState &st, TileShared<KB, true> &sh, bool first) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     long long *sums = reinterpret_cast<long long *>(sh.g);          // [5][128]
     int *counts = reinterpret_cast<int *>(sums + 5 * kFwdThreads);  // [3][128]
@@ -820,7 +825,7 @@ __device__ __forceinline__ void merge_split(LaneState &st, TileShared<KB> &sh, b
 template <int KB, bool SPLIT>
 __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px, float py,
                                            bool alive, bool tile, bool grads, const HitSink &hs,
-                                           int32_t *status, TileShared<KB> &sh, const uint32_t *front,
+                                           int32_t *status, TileShared<KB, SPLIT> &sh, const uint32_t *front,
                                            RayResult &res) {
     unsigned long long(*kbuf)[kFwdThreads] = sh.kbuf;
     const int lane = threadIdx.x & 31;
@@ -1265,7 +1270,7 @@ __device__ __noinline__ bool ray_cone_warp(const float *__restrict__ ray_o, cons
 // ANY: rays from the caller too (they cost the camera rays' kernels registers: 1.8% of the forward); else
 // rays_from_python is off.
 template <int KB, bool SPLIT, bool ANY>
-__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, int sub, TileShared<KB> &sh) {
+__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, int sub, TileShared<KB, SPLIT> &sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rw = SPLIT ? a.tile_w : a.tile_w * kBlockWarpsX, rh = SPLIT ? a.tile_h : a.tile_h * kBlockWarpsY;
     const int pk = SPLIT ? sub : warp;  // the warp's packet
@@ -1399,7 +1404,7 @@ __device__ __forceinline__ void grid_wait_before() {
 // Grid launch: block (x, y) renders tile (x, y).
 template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_kernel(const FwdArgs a) {
-    __shared__ TileShared<KB> sh;
+    __shared__ TileShared<KB, false> sh;
     if (*a.render_ellipsoids) return;  // the ellipsoid view (ellipsoid_kernel) renders this frame
     forward_tile<KB, false, true>(a, blockIdx.x, blockIdx.y, 0, sh);
 }
@@ -1411,7 +1416,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_kernel(const 
 // reads them).
 template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(const FwdArgs a) {
-    __shared__ TileShared<KB> sh;
+    __shared__ TileShared<KB, false> sh;
     __shared__ uint32_t s_next, s_packets, s_retraced;
     grid_launch_next();
     // automatic choice: both kernels are launched, the one the order kernel did not choose leaves
@@ -1453,7 +1458,9 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
 // switch, 2.44 ms with two inlined bodies, 2.40 ms with a call).
 template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(const FwdArgs a) {
-    __shared__ TileShared<KB> sh;
+    __shared__ TileShared<KB, true> sh;
+    auto &whole_sh = reinterpret_cast<TileShared<KB, false> &>(sh);
+    static_assert(sizeof(TileShared<KB, false>) <= sizeof(sh), "whole tiles use the same memory");
     __shared__ uint32_t s_next, s_packets, s_retraced;
     grid_launch_next();
     if (*a.render_ellipsoids) return;
@@ -1477,7 +1484,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(
         } else {
             const uint32_t tile = a.schedule[kSchedHeader + a.ntiles + t - items];
             again = forward_tile<KB, false, true>(a, (int)(tile % (uint32_t)a.tiles_x),
-                                                  (int)(tile / (uint32_t)a.tiles_x), 0, sh);
+                                                  (int)(tile / (uint32_t)a.tiles_x), 0, whole_sh);
         }
         if ((threadIdx.x & 31) == 0 && (threadIdx.x == 0 || t >= items)) {
             atomicAdd(&s_packets, 1u);
@@ -1511,7 +1518,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(
 // kSuperWords words per super-tile.
 // ---------------------------------------------------------------------------------------------
 constexpr int kCostCut = 512;
-constexpr int kCostStack = 256;
+constexpr int kCostStack = 512;  // (a super-tile's entries and what their walk pushes)
 constexpr int kSuperTiles = 4;
 constexpr uint32_t kSuperCut = 1024;
 constexpr int kSuperMax = 255;          // entries of a super-tile frontier (fits the walk's buffer)
@@ -1594,8 +1601,11 @@ __device__ __forceinline__ void frontier_sort_out(const FrontierScratch &fs, int
 // One warp walks the top of the BVH for a pixel rectangle whose frustum is in fs.fr: returns (on
 // every lane) the number of leaves under the frontier, the nodes of at most `cut` leaves (and the
 // leaves) it reaches; with `out`, writes the frontier there sorted front to back (count + entries),
-// or a count of kFrontierNone when the walk was cut short, the frontier does not fit or the tree is
-// malformed.  n > 1.  seed (may be null; a count above kSuperMax means none): a super-tile frontier
+// or a count of kFrontierNone when the frontier does not fit or the tree is malformed.  The walk ends
+// there (or when its stack is full), and the leaves under the nodes it has not opened count in full: the
+// densest tiles, whose frontiers do not fit, must not seem light (stopped with what had been reached, one
+// tile of 6M Gaussians at 1280x720 was the last to start, 9.1 ms for a view that takes 2.2).  n > 1.
+// seed (may be null; a count above kSuperMax means none): a super-tile frontier
 // to start from instead of the root -- each entry whose box meets this frustum is walked further
 // (more than `cut` leaves) or is a frontier entry.  SUPER: the walk of a super-tile; with `out` it
 // writes its entries unsorted with their leaf counts and boxes (kSuperWords words), or
@@ -1608,6 +1618,7 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
     const Frustum &fr = fs.fr;
     const float4 cdir = fr.pn[4];  // the near plane's normal: the rectangle's mean direction
     uint32_t est = 0;
+    uint32_t pending = 0;  // leaves under the nodes on the stack (this lane's pushes less its pops, modulo 2^32)
     int nf = 0, sp = 0;
     bool complete = true, stop = false;
     const uint32_t nseed = seed ? seed[0] : kFrontierNone;
@@ -1635,16 +1646,12 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
                     } else {
                         bad = true;
                     }
+                    if (push) pending += lv;
                     key = fmaf(bmin[2] + bmax[2], cdir.z, fmaf(bmin[1] + bmax[1], cdir.y, (bmin[0] + bmax[0]) * cdir.x));
                 }
             }
             if (__any_sync(kFull, bad)) complete = false;
             const uint32_t mp = __ballot_sync(kFull, push);
-            if (sp + __popc(mp) > kCostStack) {
-                complete = false;  // an estimate from what was reached is enough
-                stop = true;
-                break;
-            }
             if (push) fs.stk[sp + __popc(mp & lanemask_lt)] = link;
             sp += __popc(mp);
             const uint32_t mr = __ballot_sync(kFull, rec);
@@ -1656,16 +1663,21 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
             nf += __popc(mr);
         }
     } else {
-        if (lane == 0) fs.stk[0] = 0u;
+        if (lane == 0) {
+            fs.stk[0] = 0u;
+            pending = (uint32_t)n;
+        }
         sp = 1;
     }
     __syncwarp();
-    for (int guard = 0; sp > 0 && !stop; guard++) {
-        if (guard >= 4096) {
+    for (int guard = 0; sp > 0; guard++) {
+        // a popped node frees its entry and pushes at most two
+        const int take = min(min(sp, 32), kCostStack - sp);
+        if (guard >= 4096 || nf > (SUPER ? kSuperMax : kFrontierMax) || take <= 0) {
             complete = false;
+            stop = true;
             break;
         }
-        const int take = sp < 32 ? sp : 32;
         uint32_t node = GRAY_NULL;
         if (lane < take) node = fs.stk[sp - 1 - lane];
         __syncwarp();
@@ -1685,6 +1697,7 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
                 const float b1min[3] = {q1.z, q1.w, q2.x}, b1max[3] = {q2.y, q2.z, q2.w};
                 const uint32_t c0 = __float_as_uint(q3.x), c1 = __float_as_uint(q3.y);
                 const uint32_t l0 = __float_as_uint(q3.w), l1 = __float_as_uint(q3.z) - l0;
+                pending -= l0 + l1;
                 const bool p0 = frustum_box(fr, b0min, b0max), p1 = frustum_box(fr, b1min, b1max);
                 const float s0 = fmaf(q0.z + q1.y, cdir.z, fmaf(q0.y + q1.x, cdir.y, (q0.x + q0.w) * cdir.x));
                 const float s1 = fmaf(q2.x + q2.w, cdir.z, fmaf(q1.w + q2.z, cdir.y, (q1.z + q2.y) * cdir.x));
@@ -1739,12 +1752,10 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
         }
         // a malformed tree: leave it to the forward's own checks (root start)
         if (__any_sync(kFull, bad)) complete = false;
+        if (ia) pending += la;
+        if (ib) pending += lb;
         const uint32_t ma = __ballot_sync(kFull, ia), mb = __ballot_sync(kFull, ib);
         const int ni = __popc(ma) + __popc(mb);
-        if (sp + ni > kCostStack) {
-            complete = false;  // an estimate from what was reached is enough
-            break;
-        }
         const int above = __popc(ma & lanemask_lt) + __popc(mb & lanemask_lt);
         if (ia) fs.stk[sp + ni - 1 - above] = ca;
         if (ib) fs.stk[sp + ni - 1 - above - (ia ? 1 : 0)] = cb;
@@ -1773,6 +1784,7 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
         nf += __popc(qa) + __popc(qb);
         __syncwarp();
     }
+    if (stop) est += pending;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) est += __shfl_xor_sync(kFull, est, off);
     if (!out) return est;
@@ -2176,7 +2188,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB)
                        int nviews, uint32_t total_packets, float *__restrict__ out, uint32_t *__restrict__ counter,
                        int tile_w, const uint32_t *__restrict__ frontier, uint32_t total_groups,
                        int32_t *status) {
-    __shared__ TileShared<KB> sh;
+    __shared__ TileShared<KB, false> sh;
     // the group's scene and view parameters live in shared memory (read where used), which keeps
     // them out of the registers the traversal needs
     __shared__ TraceScene s_sc;
