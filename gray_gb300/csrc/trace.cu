@@ -2345,6 +2345,13 @@ struct FwdPlan {
     int nsuper;  // super-tiles whose coarse frontiers seed the tile walks (0: tiles walk from the root)
 };
 
+// The automatic choice's frontier cut.  Finer frontiers shorten the tiles' traversals and sharpen their
+// estimates, and lengthen the tile walks, which take as long as the preparation beside them from about
+// 2M Gaussians on.  Measured, display at cuts 16, 32 and 64 (us): 30k / 1280x720 228, 241, 248; 300k /
+// 1920x1080 653, 670, 690; 500k / 640x480 326, 340, 384; 1M / 1920x1080 1030, 1042, 1066, 1M / 640x480 547,
+// 476, 513; 2M / 1920x1080 1583, 1528, 1526; 3M / 1920x1080 2078, 1997, 1965; 6M / 4K 9233, 9107, 9008.
+static uint32_t automatic_cut(int n) { return n <= 600000 ? 16u : n <= 1500000 ? 32u : (uint32_t)kFrontierCutDefault; }
+
 static FwdPlan plan_forward(const gray_params &p, bool display) {
     FwdPlan q;
     q.nsuper = 0;
@@ -2387,7 +2394,11 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
             q.kern = reinterpret_cast<const void *>(&trace_forward_sched_kernel<16, 6>);
             q.kern_wide = reinterpret_cast<const void *>(&trace_forward_sched_kernel<32, 4>);
         }
-        a.frontier_cut = fcut == 0 ? kFrontierCutDefault : fcut == 1 ? 32u : fcut == 2 ? 128u : 0u;
+        a.frontier_cut = automatic   ? automatic_cut(a.n)
+                         : fcut == 0 ? kFrontierCutDefault
+                         : fcut == 1 ? 32u
+                         : fcut == 2 ? 128u
+                                     : 0u;
         if (a.frontier_cut > 0 && (size_t)a.ntiles <= (words - kSchedHeader) / (1 + kOrderPerTile + kFrontierWords))
             a.frontier = a.schedule + kSchedHeader + (1 + kOrderPerTile) * (size_t)a.ntiles;
         if (a.frontier) {

@@ -174,10 +174,11 @@ typedef struct gray_params {
      * cap, bit 2 = 8x4 or 4x8 pixel packets, bits 3-4 = where a pixel tile's traversals start (BVH
      * nodes of at most 64, 32 or 128 leaves that the tile's frustum reaches, or the root), bit 5 is
      * accepted and has no effect.
-     * 0 (default): 4x8 packets from 64-leaf frontiers, with the 16-key buffer (six blocks per SM)
-     * or the 32-key one (four blocks per SM) chosen on the device from the previous scheduled
-     * forward of the same schedule buffer (the 32-key one when more than 6/128 of its packets needed
-     * a second traversal with 16 keys, 1/128 in a small frame); both kernels are launched and the one not chosen returns at once.
+     * 0 (default): 4x8 packets from frontiers of 16, 32 or 64 leaves (by the Gaussian count), with the
+     * 16-key buffer (six blocks per SM) or the 32-key one (four blocks per SM) chosen on the device
+     * from the previous scheduled forward of the same schedule buffer (the 32-key one when more than
+     * 6/128 of its packets needed a second traversal with 16 keys, 1/128 in a small frame); both
+     * kernels are launched and the one not chosen returns at once.
      * Results are identical for every variant; only speed differs. */
     int32_t trace_variant;
 } gray_params;
