@@ -106,3 +106,39 @@ def test_jittered_tiles_match_the_oracle(oracle, size):
         ro, rd = _camera_rays_gpu(rt, cam)
         fwd = oracle.trace_forward(ro, rd, geom, live, chan, vis, oracle.TraceConfig(t_threshold=1e-3))
         _compare_forward(rt, fwd)
+
+
+@pytest.mark.parametrize("offsets", ["numbered", "gap", "none"])
+def test_ordered_batch_equals_plain_views(offsets):
+    """A batch with more than four groups per block renders its densest groups first; views whose group
+    offsets do not number the groups one after another, or no frontier at all, keep the views' order.  The
+    pixels are the plain forward's in every case."""
+    import ctypes
+
+    from gray_gb300.batch import BatchRenderer, BatchViewC
+
+    sc = synthetic.clustered_scene(20_000, seed=3)
+    rt = G.make_tracer(640, 480, sc.mean, sc.rotation, sc.scale, sc.opacity,
+                       channels=np.random.default_rng(1).uniform(0, 1, (sc.n, 3)).astype(np.float32))
+    cams = [synthetic.orbit_camera(0.9 * k, w, h) for k, (w, h) in enumerate(((640, 480), (633, 471), (640, 480)))]
+    br = BatchRenderer([rt], use_graph=False, autotune=False, variant=5, blocks_per_sm=1)
+    reqs = [(0, c) for c in cams]
+    br.render(reqs)
+    plan = next(iter(br.plans.values()))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert plan.total_groups > 4 * sms
+    if offsets == "gap":
+        views = (BatchViewC * 3).from_buffer(plan.views_host.numpy())
+        views[2].group_offset += 1
+    if offsets == "none":
+        plan.total_groups = 0
+    plan.out.zero_()
+    br._launch(plan)
+    br.check_status()
+    for i, c in enumerate(cams):
+        rt.set_render_resolution(c.image_width, c.image_height)
+        rt.set_view(c.origin_cuda(), c.rotation_c2w_blender_cuda(), c.fov_y, 0.0, 99999.9)
+        rt.forward_pass_display()
+        plain = rt.get_framebuffer().output_channels[:c.image_height, :c.image_width]
+        got = plan.out[plan.offsets[i]:plan.offsets[i] + plain.numel()].view(plain.shape)
+        assert torch.equal(got, plain), i
