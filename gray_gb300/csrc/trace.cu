@@ -65,11 +65,11 @@ constexpr uint32_t kChoiceNarrow = 1u, kChoiceWide = 2u;
 // so the choice does not depend on which one ran), the narrow one (16 slots, six blocks per SM)
 // otherwise; with at most kWideTiles tiles per resident block, more than kWideSmall / 128.  A second
 // traversal is repeated by the packet's whole tile, and in a small frame it is the launch's tail.  Measured,
-// narrow against wide: 3M / 1080p with 4% of the packets 2.88 and 3.12 ms, with 31-38% 2.7-3.7 and 2.0-2.4;
+// narrow against wide: 3M / 1080p with 5% of the packets 2.88 and 3.12 ms, with 31-38% 2.7-3.7 and 2.0-2.4;
 // 1M / 1600x1040, 17-20%, 1.15-1.25 and 0.98-1.07; 500k / 1280x720 (7 tiles per block), 5.5-8.5%, 0.52-0.76
 // and 0.46-0.53; 300k / 800x600, 1.5-3%, 0.36-0.50 and 0.28-0.32; equal within 3% where none or almost
 // none do (100k / 320x240, 64 Gaussians / 256x256).
-constexpr uint32_t kWideLarge = 6u, kWideSmall = 1u;
+constexpr uint32_t kWideLarge = 10u, kWideSmall = 1u;
 constexpr int kWideTiles = 8;
 // Per pixel tile, the BVH frontier its frustum reaches (kFrontierWords words: count, then up to
 // kFrontierMax node or leaf entries); a count of kFrontierNone means "start at the root".  A frontier
