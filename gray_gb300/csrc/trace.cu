@@ -62,7 +62,7 @@ constexpr int kStatChoice = 50;    // kernel of the automatic choice: kChoiceNar
 constexpr uint32_t kChoiceNarrow = 1u, kChoiceWide = 2u;
 // The wide kernel (32 hit slots, four blocks per SM) is chosen when more than kWideLarge / 128 of the last
 // forward's packets need more than one traversal with 16 slots (counted the same way by both kernels,
-// so the choice does not depend on which one ran), the narrow one (16 slots, six blocks per SM)
+// so the choice does not depend on which one ran), the narrow one (16 slots, five blocks per SM)
 // otherwise; with at most kWideTiles tiles per resident block, more than kWideSmall / 128.  A second
 // traversal is repeated by the packet's whole tile, and in a small frame it is the launch's tail.  Measured,
 // narrow against wide: 3M / 1080p with 5% of the packets 2.88 and 3.12 ms, with 31-38% 2.7-3.7 and 2.0-2.4;
@@ -2439,7 +2439,8 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     // tile frontier's cut (64 leaves, 32, 128, no frontier); bit 5 is accepted and has no effect
     // variant 0 (the default) chooses between the narrow and the wide kernel of kDefaultTraceVariant's
     // packet shape and cut from the last scheduled forward's re-traversals: the 16-slot hit buffer with
-    // six blocks per SM is faster where few rays composite more than 16 hits, the 32-slot one with
+    // five blocks per SM (4, 5, 6: 3.08, 2.83, 2.91 ms on the benchmark's training view at 3M / 1080p; six leave
+    // 80 registers, with twice the spills) is faster where few rays composite more than 16 hits, the 32-slot one with
     // four blocks where many do (a re-traversal repeats the packet's whole traversal)
     const bool automatic = p.trace_variant <= 0;
     const int v = p.trace_variant > 0 ? p.trace_variant : kDefaultTraceVariant;
@@ -2463,13 +2464,13 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
         case 0: q.kern = GRAY_FWD_KERNEL(32, 1); break;
         case 1: q.kern = GRAY_FWD_KERNEL(32, 4); break;
         case 2: q.kern = GRAY_FWD_KERNEL(16, 1); break;
-        default: q.kern = GRAY_FWD_KERNEL(16, 6); break;
+        default: q.kern = GRAY_FWD_KERNEL(16, 5); break;
     }
 #undef GRAY_FWD_KERNEL
     if (q.sched) {
         a.schedule = p.hitlist.schedule;
         if (automatic) {
-            q.kern = reinterpret_cast<const void *>(&trace_forward_sched_kernel<16, 6>);
+            q.kern = reinterpret_cast<const void *>(&trace_forward_sched_kernel<16, 5>);
             q.kern_wide = reinterpret_cast<const void *>(&trace_forward_sched_kernel<32, 4>);
         }
         a.frontier_cut = automatic   ? automatic_cut(a.n)

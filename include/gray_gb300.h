@@ -175,7 +175,7 @@ typedef struct gray_params {
      * nodes of at most 64, 32 or 128 leaves that the tile's frustum reaches, or the root), bit 5 is
      * accepted and has no effect.
      * 0 (default): 4x8 packets from frontiers of 16, 32 or 64 leaves (by the Gaussian count), with the
-     * 16-key buffer (six blocks per SM) or the 32-key one (four blocks per SM) chosen on the device
+     * 16-key buffer (five blocks per SM) or the 32-key one (four blocks per SM) chosen on the device
      * from the previous scheduled forward of the same schedule buffer (the 32-key one when more than
      * 10/128 of its packets needed a second traversal with 16 keys, 1/128 in a small frame); both
      * kernels are launched and the one not chosen returns at once.
