@@ -427,9 +427,10 @@ def gpu_arm(a, rank, world, local_rank):
         "trace_backward": 120.0 * A + 72.0 * R,
         "forward_prep": 228.0 * n,
         # every accumulator row is read (64 B); rows of Gaussians the replay touched are cleared (64 B),
-        # folded into the gradients (read + write of 60 B), flagged visible (1 B), and run through the
-        # SH backward (mean 12, coefficients 180 + colour 12 read; grad_dc 12 + grad_rest 180 written)
-        "fold_sh_backward": 64.0 * n + (64.0 + 120.0 + 1.0 + 12.0 + 180.0 + 12.0 + 12.0 + 180.0) * V,
+        # carried to the parameters (snapshot rows 96, live 8, scale 12, rotation 16), folded into the
+        # gradients (read + write of 60 B), flagged visible (1 B), and run through the SH backward
+        # (mean 12, coefficients 180 + colour 12 read; grad_dc 12 + grad_rest 180 written)
+        "fold_sh_backward": 64.0 * n + (64.0 + 132.0 + 120.0 + 1.0 + 12.0 + 180.0 + 12.0 + 12.0 + 180.0) * V,
         "adam": (59 * 32.0 + 12.0) * n,  # 59 Adam floats x (p, m, v, g) read + written; channel grads zeroed
         "snapshot": (44.0 + 48 + 48 + 32) * n,
         "refit": 44.0 * n + 24.0 * (2 * n - 1),
@@ -439,20 +440,14 @@ def gpu_arm(a, rank, world, local_rank):
     dom_ms = res[dominant][0] / res[dominant][1]
     peak, peak_kind = measured_peak_gbs()
     achieved = algo.get(dominant, 0.0) / (dom_ms / 1000.0) / 1e9
-    # kernels behind one profiled scope: adam = step count + update; trace_backward = backward
-    # record + replay; tile_schedule = super-tile walk + tile walk + bucket scan + scatter (on the
-    # library's side stream, beside forward_prep), then trace_forward = the trace: with the default
-    # variant the narrow and the wide kernel, one of which returns at once (all in trace_forward
-    # when no side stream could be had); refit = block-local climb + upper tree.  The snapshot, the
-    # forward preparation and the backward record run a bulk-copy kernel over whole tiles (128, 64
-    # and 128 Gaussians) and a plain one over the rest.
-    def tiled(tile):
-        return int(n >= tile) + int(n % tile != 0)
-
-    traces = 2 if not a.trace_variant else 1
-    kernels_per_group = {"adam": 2, "trace_backward": 1 + tiled(128), "refit": 2, "tile_schedule": 4,
-                         "trace_forward": traces if "tile_schedule" in res else 4 + traces, "snapshot": tiled(128),
-                         "forward_prep": tiled(64)}
+    # kernels behind one profiled scope: adam = step count + update; tile_schedule = super-tile walk +
+    # tile walk + work order (on the library's side stream, beside forward_prep), then trace_forward =
+    # the split tiles' kernel and the whole tiles': with the default variant the narrow and the wide
+    # one, one of which returns at once (the schedule is in trace_forward too when no side stream
+    # could be had); refit = block-local climb + upper tree.  Every other scope is one kernel.
+    traces = 3 if not a.trace_variant else 2
+    kernels_per_group = {"adam": 2, "refit": 2, "tile_schedule": 3,
+                         "trace_forward": traces if "tile_schedule" in res else 3 + traces}
     launches = sum(cnt * kernels_per_group.get(name, 1) for name, (_, cnt) in res.items())
     roofline = {"bound": "hbm", "kernel": dominant, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "peak_source": peak_kind,

@@ -295,7 +295,7 @@ class _SceneWorkspace:
         self.sort_tmp = torch.zeros(max(words, 1), **i32)
         self.root_box = torch.zeros(8, **f)
         self.bounds = torch.zeros(8, **i32)
-        self.bwd_rec = torch.zeros(nn if training else 1, 24, **f)
+        self.bwd_rec = torch.zeros(1, 24, **f)
         self.bvh_valid = False
 
     def struct(self) -> _lib.SceneC:

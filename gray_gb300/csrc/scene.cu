@@ -730,10 +730,10 @@ cudaError_t launch_batch_prep(const gray_params &p, const float *origins, int nv
 
 // ---------------------------------------------------------------------------------------------
 // Gradient fold + SH backward.  The trace backward accumulates per-Gaussian gradients with
-// 16-byte vector reductions into grad_acc ([n,16]: rot4 | mean3 opacity | scale3 pruning |
-// channels3 count); this kernel adds them to the reference-layout gradient arrays, sets
-// was_visible, clears grad_acc and runs the SH backward for visible Gaussians (reference:
-// sh_backward_kernel, cuda/utils/sh.cu:249-287).
+// 16-byte vector reductions into grad_acc ([n,16]: sums of q and q x^T, opacity, pruning weight, channels,
+// count; replay_hit, trace.cu); this kernel carries them to mean, scale, rotation and opacity
+// (fold_geometry), adds them to the reference-layout gradient arrays, sets was_visible, clears grad_acc and
+// runs the SH backward for visible Gaussians (reference: sh_backward_kernel, cuda/utils/sh.cu:249-287).
 //
 // A view composites a part of the Gaussians only (11% at 3M / 1080p, 28% at 1M / 1600x1040), scattered over
 // the rows.  A block reads the counts of kFoldScan rows, lists the visible ones and then folds those with
@@ -747,13 +747,65 @@ constexpr int kFoldScan = 512;  // rows per block (1024: 1M 91 instead of 79 us;
 constexpr int kFoldRow = 45;     // words of a coefficient row at degree 3 (an odd stride: no bank conflicts)
 constexpr int kFoldRows = 8;     // coefficient rows a warp loads at a time
 
+// The geometric gradients of one Gaussian from its sums: with M (rows g0..g2) the world-to-object matrix, L
+// the rows of the object-to-world one, x = sf u and s = exp(scale),
+//   d/d mean = sf M^T sum(q),  d/d L = G = sf M^T sum(q x^T),
+//   d/d scale_k = sum_r G_rk L_rk s_k / (s_k sf + eps)  (cuda/backward_pass.cu:101-111),
+// and the rotation's is that of R = (G_rk s_k) pulled back to the quaternion through its normalisation
+// (cuda/utils/activations.cu:68-70: (g - (g . qn) qn) / |q|).
+struct FoldGeometry {
+    float4 rot;
+    float mean[3], scale[3];
+};
+
+__device__ __forceinline__ FoldGeometry fold_geometry(float4 a0, float4 a1, float4 a2, const float4 *__restrict__ g,
+                                                      const float4 *__restrict__ l, float sf, const float ls[3],
+                                                      float4 rotation, float eps) {
+    const float M[3][3] = {{g[0].x, g[0].y, g[0].z}, {g[1].x, g[1].y, g[1].z}, {g[2].x, g[2].y, g[2].z}};
+    const float L[3][3] = {{l[0].x, l[0].y, l[0].z}, {l[1].x, l[1].y, l[1].z}, {l[2].x, l[2].y, l[2].z}};
+    const float q[3] = {a0.x, a0.y, a0.z};
+    const float S[3][3] = {{a1.x, a1.y, a1.z}, {a1.y, a1.w, a2.x}, {a1.z, a2.x, a2.y}};
+    FoldGeometry o;
+    float R[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; r++) o.mean[r] = (M[0][r] * q[0] + M[1][r] * q[1] + M[2][r] * q[2]) * sf;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float s = gexp(ls[k]), d = s * sf + eps;
+        float acc = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            const float G = (M[0][r] * S[0][k] + M[1][r] * S[1][k] + M[2][r] * S[2][k]) * sf;
+            acc = acc + G * (L[r][k] / d * s);
+            R[r][k] = G * s;
+        }
+        o.scale[k] = acc;
+    }
+    const float qlen = sqrtf(rotation.x * rotation.x + rotation.y * rotation.y + rotation.z * rotation.z +
+                             rotation.w * rotation.w);
+    const float iq = 1.0f / qlen;
+    const float qw = rotation.x / qlen, qx = rotation.y / qlen, qy = rotation.z / qlen, qz = rotation.w / qlen;
+    const float g_r = 2.0f * qx * (R[2][1] - R[1][2]) + 2.0f * qy * (R[0][2] - R[2][0]) + 2.0f * qz * (R[1][0] - R[0][1]);
+    const float g_x = -4.0f * qx * (R[1][1] + R[2][2]) + 2.0f * qy * (R[0][1] + R[1][0]) +
+                      2.0f * qz * (R[0][2] + R[2][0]) + 2.0f * qw * (R[2][1] - R[1][2]);
+    const float g_y = 2.0f * qx * (R[0][1] + R[1][0]) - 4.0f * qy * (R[0][0] + R[2][2]) +
+                      2.0f * qz * (R[1][2] + R[2][1]) + 2.0f * qw * (R[0][2] - R[2][0]);
+    const float g_z = 2.0f * qx * (R[0][2] + R[2][0]) + 2.0f * qy * (R[1][2] + R[2][1]) -
+                      4.0f * qz * (R[0][0] + R[1][1]) + 2.0f * qw * (R[1][0] - R[0][1]);
+    const float dq = g_r * qw + g_x * qx + g_y * qy + g_z * qz;
+    o.rot = make_float4((g_r - dq * qw) * iq, (g_x - dq * qx) * iq, (g_y - dq * qy) * iq, (g_z - dq * qz) * iq);
+    return o;
+}
+
 __global__ void __launch_bounds__(kFoldThreads) fold_sh_backward_kernel(
     int n, int num_rest, float4 *__restrict__ grad_acc, float4 *__restrict__ grad_rotation,
     float *__restrict__ grad_mean, float *__restrict__ grad_opacity, float *__restrict__ grad_scale,
     float *__restrict__ pruning_weight, float *__restrict__ grad_channels, uint8_t *__restrict__ was_visible,
     const uint8_t *__restrict__ cfg_enable_sh, const int32_t *__restrict__ current_sh_degree, int max_sh_degree,
     const float *__restrict__ mean, const float *__restrict__ cam_origin, const float *__restrict__ sh_rest,
-    const float *__restrict__ channels, float *__restrict__ grad_sh_dc, float *__restrict__ grad_sh_rest) {
+    const float *__restrict__ channels, float *__restrict__ grad_sh_dc, float *__restrict__ grad_sh_rest,
+    const float4 *__restrict__ geom, const float4 *__restrict__ l2w, const float2 *__restrict__ live,
+    const float *__restrict__ scale, const float4 *__restrict__ rotation, const float *__restrict__ eps_scale_grad) {
     __shared__ float s_rows[kFoldThreads * kFoldRow];
     __shared__ uint16_t s_list[kFoldScan];
     __shared__ int s_count;
@@ -785,8 +837,9 @@ __global__ void __launch_bounds__(kFoldThreads) fold_sh_backward_kernel(
     for (int c0 = t & ~31; c0 < count; c0 += kFoldThreads) {
         const bool on = c0 + lane < count;
         const int i = base + (on ? (int)s_list[c0 + lane] : 0);
-        float4 a0, a1, a2, a3, gr;
-        float gm[3], gs[3], gc[3], m[3], col[3], go = 0.0f, gp = 0.0f;
+        float4 a0, a1, a2, a3, gr, mr[3], lr[3], rot;
+        float2 lv;
+        float gm[3], gs[3], gc[3], m[3], col[3], ls[3], go = 0.0f, gp = 0.0f;
         if (on) {
             a0 = grad_acc[4 * (size_t)i];
             a1 = grad_acc[4 * (size_t)i + 1];
@@ -802,7 +855,12 @@ __global__ void __launch_bounds__(kFoldThreads) fold_sh_backward_kernel(
                 gc[k] = grad_channels[3 * (size_t)i + k];
                 m[k] = sh ? mean[3 * (size_t)i + k] : 0.0f;
                 col[k] = sh ? channels[3 * (size_t)i + k] : 0.0f;
+                mr[k] = geom[3 * (size_t)i + k];
+                lr[k] = l2w[3 * (size_t)i + k];
+                ls[k] = scale[3 * (size_t)i + k];
             }
+            rot = rotation[i];
+            lv = live[i];
         }
         if (nb > 0) {
             for (int r0 = 0; r0 < 32 && c0 + r0 < count; r0 += kFoldRows) {
@@ -828,18 +886,18 @@ __global__ void __launch_bounds__(kFoldThreads) fold_sh_backward_kernel(
             grad_acc[4 * (size_t)i + 2] = z;
             grad_acc[4 * (size_t)i + 3] = z;
             was_visible[i] = 1;
-            grad_rotation[i] = make_float4(gr.x + a0.x, gr.y + a0.y, gr.z + a0.z, gr.w + a0.w);
-            grad_opacity[i] = go + a1.w;
-            pruning_weight[i] = gp + a2.w;
-            gm[0] = gm[0] + a1.x;
-            gm[1] = gm[1] + a1.y;
-            gm[2] = gm[2] + a1.z;
+            const FoldGeometry f = fold_geometry(a0, a1, a2, mr, lr, lv.y, ls, rot, *eps_scale_grad);
+            grad_rotation[i] = make_float4(gr.x + f.rot.x, gr.y + f.rot.y, gr.z + f.rot.z, gr.w + f.rot.w);
+            grad_opacity[i] = go + a0.w * lv.x * (1.0f - lv.x);
+            pruning_weight[i] = gp + a2.z;
             gc[0] = gc[0] + a3.x;
             gc[1] = gc[1] + a3.y;
             gc[2] = gc[2] + a3.z;
-            grad_scale[3 * (size_t)i] = gs[0] + a2.x;
-            grad_scale[3 * (size_t)i + 1] = gs[1] + a2.y;
-            grad_scale[3 * (size_t)i + 2] = gs[2] + a2.z;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                gm[k] = gm[k] + f.mean[k];
+                grad_scale[3 * (size_t)i + k] = gs[k] + f.scale[k];
+            }
 #pragma unroll
             for (int c = 0; c < 3; c++) grad_channels[3 * (size_t)i + c] = gc[c];
             if (sh) {
@@ -904,7 +962,9 @@ cudaError_t launch_fold_and_sh_backward(const gray_params &p, cudaStream_t s) {
         reinterpret_cast<float4 *>(g.grad_rotation), g.grad_mean, g.grad_opacity, g.grad_scale, g.pruning_weight,
         g.grad_channels, g.was_visible, p.config.enable_sh, g.current_sh_degree, g.max_sh_degree, g.mean,
         p.camera.origin, reinterpret_cast<const float *>(g.sh_coeffs_rest), g.channels, g.grad_sh_coeffs_dc,
-        g.grad_sh_coeffs_rest);
+        g.grad_sh_coeffs_rest, reinterpret_cast<const float4 *>(p.scene.geom),
+        reinterpret_cast<const float4 *>(p.scene.l2w), reinterpret_cast<const float2 *>(p.scene.live), g.scale,
+        reinterpret_cast<const float4 *>(g.rotation), p.config.eps_scale_grad);
     return cudaGetLastError();
 }
 

@@ -3,7 +3,7 @@
 // Forward (replaces the OptiX launch of cuda/shaders.cu:69-106 with cuda/forward_pass.cu):
 //   A block renders an 8x16-pixel tile of rays that share one origin, each warp a 4x8 (or 8x4)
 //   pixel packet of it.  A per-tile kernel first walks the top of the BVH with the tile's frustum and
-//   records the tile's frontier (the nodes of at most 64 leaves it reaches, sorted front to back);
+//   records the tile's frontier (the nodes of at most 16 to 64 leaves it reaches, sorted front to back);
 //   the block's traversal starts there.  The block traverses as one frustum: each step pops up to
 //   128 nodes (one per thread) from a shared-memory stack, tests both child boxes against the
 //   frustum, pushes the nearer child last and queues leaves.  Queued leaves are taken in batches of
@@ -25,7 +25,6 @@
 //   recomputes alpha in fp32 and reduces the 16 per-hit gradient values into the per-Gaussian
 //   accumulator: lanes holding the same Gaussian combine in a tree, and the lowest issues four
 //   16-byte vector reductions.
-#include "gray_bulk.cuh"
 #include "gray_device.cuh"
 #include "gray_internal.h"
 
@@ -627,7 +626,7 @@ __device__ __forceinline__ void trace_batch_leaves(const TraceScene &sc, const T
 // instead of 4 x 970 and 4 x 268 at 3M Gaussians; with the conics, the forward of 3M / 1080p went from
 // 3.11 to 2.75 ms, 500k / 640x480 from 0.83 to 0.58 ms, 6M / 4K from 18.3 to 15.6 ms, the image and its
 // colours included; the kernel is bound by instruction issue and the latency of each ray's own
-// hit chain, at six or four blocks per SM).  With a frontier (count, entries; a count above
+// hit chain, at five or four blocks per SM).  With a frontier (count, entries; a count above
 // kFrontierMax or a null pointer: none) the traversal starts there instead of at the root: the frontier
 // goes onto the stack with its first entry on top, and a frontier leaf is queued when it is popped.
 // px, py: the ray's offset from the tile's centre in the conics' basis.  Returns false if the stack
@@ -2610,8 +2609,10 @@ cudaError_t launch_trace_batch(const gray_batch_scene *scenes, const gray_batch_
 struct BwdArgs {
     uint32_t alloc_w, render_w, render_h;
     int n;
-    const float *exp_power, *alpha_threshold, *eps_scale_grad, *bg;
-    const float4 *geom, *rec;
+    const float *exp_power, *bg;
+    const float4 *geom;
+    const float2 *live;
+    const float *channels;
     const float *pix_T, *pix_fullT, *pix_rem, *ray_o, *ray_d, *grad_out;
     const uint32_t *head, *pool;
     uint32_t pool_size;
@@ -2623,7 +2624,7 @@ __device__ __forceinline__ void red_add4(float *addr, float x, float y, float z,
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(x), "f"(y), "f"(z), "f"(w));
 }
 
-// Adds one hit's 16 gradient values to the Gaussian's accumulator row.  Neighbouring pixels
+// Adds one hit's 14 gradient sums, and its count, to the Gaussian's accumulator row.  Neighbouring pixels
 // composite the same Gaussians at the same replay step (on the benchmark scene a warp's lanes form
 // groups of 16 on average, often the whole warp), and vector reductions on one row serialise in L2,
 // so the lanes that hold the same Gaussian first combine their values and the lowest of them issues
@@ -2631,8 +2632,10 @@ __device__ __forceinline__ void red_add4(float *addr, float x, float y, float z,
 // member of its group (`nxt`, the member `s` ranks further after the round of stride s, found by
 // pointer jumping), and in the round of stride s the members whose rank is a multiple of 2s add
 // the partial sum of the member s ranks further; after ceil(log2(largest group)) rounds the lowest
-// member holds the group's sum (16 shuffles per round instead of 16 per member).
-__device__ __forceinline__ void reduce_hit(float *row, uint32_t gid, float (&v)[16]) {
+// member holds the group's sum (14 shuffles per round; the count is the group's size).
+constexpr int kHitSums = 14;
+
+__device__ __forceinline__ void reduce_hit(float *row, uint32_t gid, float (&v)[kHitSums]) {
     const unsigned active = __activemask();
     const unsigned grp = __match_any_sync(active, gid);
     const int lane = threadIdx.x & 31;
@@ -2645,7 +2648,7 @@ __device__ __forceinline__ void reduce_hit(float *row, uint32_t gid, float (&v)[
         const int src = nxt >= 0 ? nxt : lane;
         const bool take = nxt >= 0 && (rank & (2 * s - 1)) == 0;
 #pragma unroll
-        for (int k = 0; k < 16; k++) {
+        for (int k = 0; k < kHitSums; k++) {
             const float t = __shfl_sync(active, v[k], src);
             if (take) v[k] += t;
         }
@@ -2655,175 +2658,28 @@ __device__ __forceinline__ void reduce_hit(float *row, uint32_t gid, float (&v)[
     if (rank == 0) {
         red_add4(row, v[0], v[1], v[2], v[3]);
         red_add4(row + 4, v[4], v[5], v[6], v[7]);
-        red_add4(row + 8, v[8], v[9], v[10], v[11]);
-        red_add4(row + 12, v[12], v[13], v[14], v[15]);
+        red_add4(row + 8, v[8], v[9], v[10], 0.0f);
+        red_add4(row + 12, v[11], v[12], v[13], (float)__popc(grp));
     }
 }
 
-// Per-Gaussian backward record: what the reverse replay needs of one Gaussian besides its snapshot
-// rows (M | mu), precomputed once per backward pass instead of once per composited hit.  Written
-// from the state the forward used: live opacity o and scaling factor sf, colour c, current log-scale
-// and rotation q, snapshot L2W rows L.  24 floats (6 x float4):
-//   [o, sf, 1/|q|, s0] [s1, s2, c0, c1] [c2, K00, K01, K02] [K10, K11, K12, K20] [K21, K22, 0, 0]
-//   [qn0, qn1, qn2, qn3]
-// with s = exp(scale), K_rk = L_rk / (s_k sf + eps_scale_grad) * s_k (the scale gradient's factor,
-// cuda/backward_pass.cu:101-111) and qn = q / |q|.
-constexpr int kRecVec = 6;
-
-__device__ __forceinline__ void bwd_record_one(float2 lv, const float log_s[3], float4 q, const float ch[3], float4 L0,
-                                               float4 L1, float4 L2, float eps, float4 r[kRecVec]) {
-    const float sf = lv.y;
-    float s[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) s[k] = gexp(log_s[k]);
-    const float qlen = sqrtf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
-    const float d0 = s[0] * sf + eps, d1 = s[1] * sf + eps, d2 = s[2] * sf + eps;
-    r[0] = make_float4(lv.x, sf, 1.0f / qlen, s[0]);
-    r[1] = make_float4(s[1], s[2], ch[0], ch[1]);
-    r[2] = make_float4(ch[2], L0.x / d0 * s[0], L0.y / d1 * s[1], L0.z / d2 * s[2]);
-    r[3] = make_float4(L1.x / d0 * s[0], L1.y / d1 * s[1], L1.z / d2 * s[2], L2.x / d0 * s[0]);
-    r[4] = make_float4(L2.y / d1 * s[1], L2.z / d2 * s[2], 0.0f, 0.0f);
-    r[5] = make_float4(q.x / qlen, q.y / qlen, q.z / qlen, q.w / qlen);
-}
-
-// Gaussian i's record, straight from and to memory.
-__device__ __forceinline__ void bwd_record_row(int i, const float2 *__restrict__ live, const float *__restrict__ scale,
-                                               const float4 *__restrict__ rotation,
-                                               const float *__restrict__ channels, const float4 *__restrict__ l2w,
-                                               float eps, float4 *__restrict__ rec) {
-    const float ls[3] = {scale[3 * i], scale[3 * i + 1], scale[3 * i + 2]};
-    const float ch[3] = {channels[3 * i], channels[3 * i + 1], channels[3 * i + 2]};
-    float4 r[kRecVec];
-    bwd_record_one(live[i], ls, rotation[i], ch, l2w[3 * i], l2w[3 * i + 1], l2w[3 * i + 2], eps, r);
-    float4 *o = rec + kRecVec * (size_t)i;
-#pragma unroll
-    for (int k = 0; k < kRecVec; k++) o[k] = r[k];
-}
-
-// One thread per Gaussian: the whole pass when there are fewer than a tile or a pointer is not 16-byte
-// aligned.
-__global__ void __launch_bounds__(256) bwd_record_kernel(int n, const float2 *__restrict__ live,
-                                                         const float *__restrict__ scale,
-                                                         const float4 *__restrict__ rotation,
-                                                         const float *__restrict__ channels,
-                                                         const float4 *__restrict__ l2w,
-                                                         const float *__restrict__ eps_scale_grad,
-                                                         float4 *__restrict__ rec) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) bwd_record_row(i, live, scale, rotation, channels, l2w, *eps_scale_grad, rec);
-}
-
-// Bulk-pipelined record pass: persistent blocks take tiles of kRecTile Gaussians; one thread loads
-// a tile's inputs (live, scale, rotation, channels, l2w rows: 96 B per Gaussian, five contiguous
-// ranges) into one of two shared-memory stages with bulk copies completing on an mbarrier, so the
-// next tile's loads are in flight while this one is computed, and stores the tile's records (96 B
-// per Gaussian) from a shared-memory copy with one bulk copy.  Every copy starts on a 16-byte
-// boundary and spans a multiple of 16 bytes (the launcher checks the pointers).
-constexpr int kRecTile = 128;
-static_assert(kRecTile % 16 == 0, "every per-tile range must span a multiple of 16 bytes");
-
-struct RecIn {
-    float4 l2w[3 * kRecTile];
-    float4 rotation[kRecTile];
-    float2 live[kRecTile];
-    float scale[3 * kRecTile];
-    float channels[3 * kRecTile];
-};
-constexpr uint32_t kRecInBytes = 96u * kRecTile;
-
-__device__ __forceinline__ void rec_issue_loads(RecIn &in, uint64_t *bar, int tile, const float2 *live,
-                                                const float *scale, const float4 *rotation, const float *channels,
-                                                const float4 *l2w) {
-    const size_t g0 = (size_t)tile * kRecTile;
-    mbar_expect_tx(bar, kRecInBytes);
-    bulk_load(in.l2w, l2w + 3 * g0, 48u * kRecTile, bar);
-    bulk_load(in.rotation, rotation + g0, 16u * kRecTile, bar);
-    bulk_load(in.live, live + g0, 8u * kRecTile, bar);
-    bulk_load(in.scale, scale + 3 * g0, 12u * kRecTile, bar);
-    bulk_load(in.channels, channels + 3 * g0, 12u * kRecTile, bar);
-}
-
-__global__ void __launch_bounds__(kRecTile) bwd_record_bulk_kernel(
-    int n, int tiles, const float2 *__restrict__ live, const float *__restrict__ scale, const float4 *__restrict__ rotation,
-    const float *__restrict__ channels, const float4 *__restrict__ l2w, const float *__restrict__ eps_scale_grad,
-    float4 *__restrict__ rec, int32_t *__restrict__ status) {
-    __shared__ __align__(16) RecIn in[2];
-    __shared__ __align__(16) float4 out[kRecVec * kRecTile];
-    __shared__ __align__(8) uint64_t bar[2];
-    const int t = threadIdx.x;
-    if (t == 0) {
-        mbar_init(&bar[0], 1);
-        mbar_init(&bar[1], 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    const float eps = *eps_scale_grad;
-    int tile = blockIdx.x;
-    if (t == 0 && tile < tiles) rec_issue_loads(in[0], &bar[0], tile, live, scale, rotation, channels, l2w);
-    // the Gaussians past the last full tile are the last block's, while its first tile loads
-    if (blockIdx.x == gridDim.x - 1 && tiles * kRecTile + t < n)
-        bwd_record_row(tiles * kRecTile + t, live, scale, rotation, channels, l2w, eps, rec);
-    int it = 0;
-    bool timed_out = false;
-    for (; tile < tiles; it++, tile += gridDim.x) {
-        const int st = it & 1;
-        const int next = tile + gridDim.x;
-        if (t == 0 && next < tiles) {
-            fence_proxy_async();  // in[st ^ 1] was last read in the previous tile, before its barriers
-            rec_issue_loads(in[st ^ 1], &bar[st ^ 1], next, live, scale, rotation, channels, l2w);
-        }
-        const bool ok = __syncthreads_and(mbar_wait(&bar[st], (uint32_t)(it >> 1) & 1u, kBulkWaitNs));
-        if (!ok) {
-            if (t == 0) atomicOr(status, GRAY_STATUS_COPY_TIMEOUT);
-            timed_out = true;
-            break;
-        }
-        float4 r[kRecVec];
-        {
-            const RecIn &x = in[st];
-            const float ls[3] = {x.scale[3 * t], x.scale[3 * t + 1], x.scale[3 * t + 2]};
-            const float ch[3] = {x.channels[3 * t], x.channels[3 * t + 1], x.channels[3 * t + 2]};
-            bwd_record_one(x.live[t], ls, x.rotation[t], ch, x.l2w[3 * t], x.l2w[3 * t + 1], x.l2w[3 * t + 2], eps,
-                           r);
-        }
-        if (t == 0) bulk_wait_read();  // the previous tile's store has read the output copy
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kRecVec; k++) out[kRecVec * t + k] = r[k];
-        fence_proxy_async();
-        __syncthreads();
-        if (t == 0) {
-            bulk_store(rec + kRecVec * (size_t)tile * kRecTile, out, 16u * kRecVec * kRecTile);
-            bulk_commit();
-        }
-    }
-    if (t == 0) {
-        bulk_wait_all();
-        if (timed_out) {
-            // bounded waits for the loads still in flight before the block's shared memory goes
-            mbar_wait(&bar[it & 1], (uint32_t)(it >> 1) & 1u, kBulkWaitNs);
-            if (tile + (int)gridDim.x < tiles)
-                mbar_wait(&bar[(it + 1) & 1], (uint32_t)((it + 1) >> 1) & 1u, kBulkWaitNs);
-        }
-    }
-}
-
-// What one composited hit reads: the snapshot rows and the backward record (9 x 16 B).
+// What one composited hit reads: the snapshot rows, the live opacity and scaling factor, the colour.
 struct BwdHit {
-    float4 g0, g1, g2, r0, r1, r2, r3, r4, r5;
+    float4 g0, g1, g2;
+    float2 live;
+    float c0, c1, c2;
 };
 
 __device__ __forceinline__ void load_hit(const BwdArgs &a, uint32_t gid, BwdHit &h) {
-    const float4 *gp = a.geom + 3 * (size_t)gid, *rp = a.rec + kRecVec * (size_t)gid;
+    const float4 *gp = a.geom + 3 * (size_t)gid;
+    const float *cp = a.channels + 3 * (size_t)gid;
     h.g0 = __ldg(gp);
     h.g1 = __ldg(gp + 1);
     h.g2 = __ldg(gp + 2);
-    h.r0 = __ldg(rp);
-    h.r1 = __ldg(rp + 1);
-    h.r2 = __ldg(rp + 2);
-    h.r3 = __ldg(rp + 3);
-    h.r4 = __ldg(rp + 4);
-    h.r5 = __ldg(rp + 5);
+    h.live = __ldg(a.live + gid);
+    h.c0 = __ldg(cp);
+    h.c1 = __ldg(cp + 1);
+    h.c2 = __ldg(cp + 2);
 }
 
 // Reverse-order walk of a pixel's segment chain (newest segment first, each segment back to front).
@@ -2864,11 +2720,19 @@ struct BwdPixel {
 
 // One step of the reverse replay (cuda/backward_pass.cu:17-137) for hit h; T and gT are the
 // running transmittance and colour-gradient tail.
+//
+// With x the hit's scaled object-space point and q = d loss / d x (up to sign), the gradients of mean,
+// scale and rotation are linear in q and in q x^T, with coefficients of the Gaussian alone, and q is
+// parallel to x.  So a hit adds q (3 sums) and the symmetric q x^T (6), and the pass over the Gaussians that
+// follows applies the coefficients once per Gaussian instead of once per hit.  A hit that carried them
+// to the parameters itself needed a record of 24 floats per Gaussian, written by a pass of its own over all
+// Gaussians.  Accumulator row: [q | opacity] [xx xy xz yy] [yz zz, pruning weight, 0] [channels | count].
+// Train step at 3M / 1080p 4.15 -> 3.98 ms, at 1M / 1600x1040 1.99 -> 1.89 ms, 301k / 799x533 0.66 -> 0.64 ms.
+// 54 registers instead of 72; bound by instruction issue and the reductions; fetching the next hit's id ahead changed nothing.
 __device__ __forceinline__ void replay_hit(const BwdArgs &a, const BwdPixel &px, uint32_t gid, const BwdHit &h,
                                            float &T, float &gT) {
-    const float o = h.r0.x, sf = h.r0.y, iq = h.r0.z;
-    const f3 s = mk3(h.r0.w, h.r1.x, h.r1.y);
-    const f3 c = mk3(h.r1.z, h.r1.w, h.r2.x);
+    const float o = h.live.x, sf = h.live.y;
+    const f3 c = mk3(h.c0, h.c1, h.c2);
     LocalHit lh;
     local_ray(h.g0, h.g1, h.g2, px.ro, px.rd, lh);
     closest_point(lh);
@@ -2888,42 +2752,16 @@ __device__ __forceinline__ void replay_hit(const BwdArgs &a, const BwdPixel &px,
     ga = ga + -(px.fT * rom) * px.dbg;
     ga = ga + -((px.Tfin - px.fT) * rom) * px.drem;
     gT = gT + (dgc - gT) * alpha;
-    float go = maxalpha_mul(ga, gv);
-    go = go * o * (1.0f - o);
     const float ggv = maxalpha_mul(ga, o);
     float gsq;
     if (px.pw == 1.0f) gsq = gv;
     else if (px.pw == 2.0f) gsq = gv * sq;
     else if (px.pw == 3.0f) gsq = gv * sq * sq;
     else gsq = gv * gpow(sq, px.pw - 1.0f);
-    const f3 gxl = mk3(-x.x * gsq * ggv, -x.y * gsq * ggv, -x.z * gsq * ggv);
-    const f3 gxw = mk3((h.g0.x * gxl.x + h.g1.x * gxl.y + h.g2.x * gxl.z) * sf,
-                       (h.g0.y * gxl.x + h.g1.y * gxl.y + h.g2.y * gxl.z) * sf,
-                       (h.g0.z * gxl.x + h.g1.z * gxl.y + h.g2.z * gxl.z) * sf);
-    // d loss / d L2W rows: -gxw_r * x
-    const f3 gl0 = mk3(-gxw.x * x.x, -gxw.x * x.y, -gxw.x * x.z);
-    const f3 gl1 = mk3(-gxw.y * x.x, -gxw.y * x.y, -gxw.y * x.z);
-    const f3 gl2 = mk3(-gxw.z * x.x, -gxw.z * x.y, -gxw.z * x.z);
-    const f3 gs = mk3(gl0.x * h.r2.y + gl1.x * h.r3.x + gl2.x * h.r3.w,
-                      gl0.y * h.r2.z + gl1.y * h.r3.y + gl2.y * h.r4.x,
-                      gl0.z * h.r2.w + gl1.z * h.r3.z + gl2.z * h.r4.y);
-    // rotation-matrix gradient and its pull-back to the quaternion through the normalisation
-    const float r00 = gl0.x * s.x, r01 = gl0.y * s.y, r02 = gl0.z * s.z;
-    const float r10 = gl1.x * s.x, r11 = gl1.y * s.y, r12 = gl1.z * s.z;
-    const float r20 = gl2.x * s.x, r21 = gl2.y * s.y, r22 = gl2.z * s.z;
-    const float qw = h.r5.x, qx = h.r5.y, qy = h.r5.z, qz = h.r5.w;
-    const float g_r = 2.0f * qx * (r21 - r12) + 2.0f * qy * (r02 - r20) + 2.0f * qz * (r10 - r01);
-    const float g_x = -4.0f * qx * (r11 + r22) + 2.0f * qy * (r01 + r10) + 2.0f * qz * (r02 + r20) +
-                      2.0f * qw * (r21 - r12);
-    const float g_y = 2.0f * qx * (r01 + r10) - 4.0f * qy * (r00 + r22) + 2.0f * qz * (r12 + r21) +
-                      2.0f * qw * (r02 - r20);
-    const float g_z = 2.0f * qx * (r02 + r20) + 2.0f * qy * (r12 + r21) - 4.0f * qz * (r00 + r11) +
-                      2.0f * qw * (r10 - r01);
-    // (g - (g . qn) qn) / |q| == g / |q| - (g . q) q / |q|^3 (cuda/utils/activations.cu:68-70)
-    const float dq = g_r * qw + g_x * qx + g_y * qy + g_z * qz;
-    float v[16] = {(g_r - dq * qw) * iq, (g_x - dq * qx) * iq, (g_y - dq * qy) * iq, (g_z - dq * qz) * iq,
-                   -gxw.x, -gxw.y, -gxw.z, go, gs.x, gs.y, gs.z, w * px.inv_npix,
-                   px.gout.x * w, px.gout.y * w, px.gout.z * w, 1.0f};
+    const f3 q = mk3(x.x * gsq * ggv, x.y * gsq * ggv, x.z * gsq * ggv);
+    float v[kHitSums] = {q.x,       q.y,       q.z,       maxalpha_mul(ga, gv), q.x * x.x,       q.x * x.y,
+                         q.x * x.z, q.y * x.y, q.y * x.z, q.z * x.z,            w * px.inv_npix, px.gout.x * w,
+                         px.gout.y * w, px.gout.z * w};
     reduce_hit(a.grad_acc + 16 * (size_t)gid, gid, v);
     T = Tr;
 }
@@ -2977,41 +2815,16 @@ __global__ void __launch_bounds__(128) trace_backward_kernel(const BwdArgs a) {
 
 cudaError_t launch_trace_backward(const gray_params &p, cudaStream_t s) {
     const int n = p.gaussians.count;
-    if (n > 0) {
-        const float2 *live = reinterpret_cast<const float2 *>(p.scene.live);
-        const float4 *rot = reinterpret_cast<const float4 *>(p.gaussians.rotation);
-        const float4 *l2w = reinterpret_cast<const float4 *>(p.scene.l2w);
-        float4 *rec = reinterpret_cast<float4 *>(p.scene.bwd_rec);
-        const bool bulk = p.status && aligned16(live) && aligned16(p.gaussians.scale) && aligned16(rot) &&
-                          aligned16(p.gaussians.channels) && aligned16(l2w) && aligned16(rec);
-        const int tiles = bulk ? n / kRecTile : 0;
-        cudaError_t e;
-        if (tiles > 0) {
-            int sms = 0, per_sm = 0;
-            if ((e = resident_blocks(reinterpret_cast<const void *>(&bwd_record_bulk_kernel), kRecTile, 0, &sms,
-                                     &per_sm)) != cudaSuccess)
-                return e;
-            const int want = sms * per_sm;
-            bwd_record_bulk_kernel<<<tiles < want ? tiles : want, kRecTile, 0, s>>>(
-                n, tiles, live, p.gaussians.scale, rot, p.gaussians.channels, l2w, p.config.eps_scale_grad, rec,
-                p.status);
-        } else {
-            bwd_record_kernel<<<(unsigned int)((n + 255) / 256), 256, 0, s>>>(
-                n, live, p.gaussians.scale, rot, p.gaussians.channels, l2w, p.config.eps_scale_grad, rec);
-        }
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
     BwdArgs a;
     a.alloc_w = p.image_width;
     a.render_w = p.render_width;
     a.render_h = p.render_height;
     a.n = n;
     a.exp_power = p.config.exp_power;
-    a.alpha_threshold = p.config.alpha_threshold;
-    a.eps_scale_grad = p.config.eps_scale_grad;
     a.bg = p.config.background_channels;
     a.geom = reinterpret_cast<const float4 *>(p.scene.geom);
-    a.rec = reinterpret_cast<const float4 *>(p.scene.bwd_rec);
+    a.live = reinterpret_cast<const float2 *>(p.scene.live);
+    a.channels = p.gaussians.channels;
     a.pix_T = p.framebuffer.transmittance;
     a.pix_fullT = p.framebuffer.full_transmittance;
     a.pix_rem = p.framebuffer.remaining_channels_estimate;

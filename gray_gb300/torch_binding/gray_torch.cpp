@@ -338,7 +338,7 @@ struct Raytracer : torch::CustomClassHolder {
         sort_tmp = at::zeros({std::max<int64_t>((int64_t)gray_sort_tmp_words((int32_t)n), 1)}, i32());
         root_box = at::zeros({8}, f32());
         bounds = at::zeros({8}, i32());
-        bwd_rec = at::zeros({inference_only ? 1 : nn, 24}, f32());
+        bwd_rec = at::zeros({1, 24}, f32());
         bvh_valid = false;
     }
 

@@ -153,8 +153,8 @@ typedef struct gray_scene {
                              refit then climbs the whole tree with global counters, slower) */
     float *root_box;      /* [8] */
     uint32_t *bounds;     /* [8] order-preserving encoded scene bounds (scratch) */
-    float *bwd_rec;       /* [N,24] per-Gaussian backward record, written at the start of each
-                             backward pass (training tracers; may be NULL for inference) */
+    float *bwd_rec;       /* not read or written; a NULL marks a scene without a backward pass, which
+                             gray_backward_pass refuses */
     int32_t bvh_valid;    /* host flag: a rebuild has been done for this count */
 } gray_scene;
 
