@@ -740,7 +740,8 @@ cudaError_t launch_batch_prep(const gray_params &p, const float *origins, int nv
 // every lane at work: a warp takes 32 of them, loads all it needs of them at once and moves their
 // coefficient rows through shared memory, a row's words by consecutive lanes.  A thread per row had 3.5 of a
 // warp's lanes follow the same chain of dependent loads (64 stall cycles per instruction) and wrote
-// rows of 180 bytes word by word: 3M / 1080p 289 -> 140 us, 1M / 1600x1040 118 -> 79 us.
+// rows of 180 bytes word by word: 3M / 1080p 289 -> 140 us, 1M / 1600x1040 118 -> 79 us (176 and 93 since the
+// geometric gradients are made here, which took 94 and 33 us of records and more from the replay).
 // ---------------------------------------------------------------------------------------------
 constexpr int kFoldThreads = 128;
 constexpr int kFoldScan = 512;  // rows per block (1024: 1M 91 instead of 79 us; 256: 3M 165 instead of 140)
