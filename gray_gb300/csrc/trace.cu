@@ -162,7 +162,8 @@ struct LaneState {
     int kcount, ncand;
     unsigned long long kmax;
     float dfar;  // +inf, or once the buffer is full the fp16 distance after its last key's: a hit beyond it
-                 // rounds to a larger distance than every kept key's
+                 // rounds to a larger distance than every kept key's (+inf too where the last key's distance
+                 // is -0, which a negative znear keeps: keys order it after every other)
     // resume key for the next traversal
     unsigned long long resume;
     bool has_resume;
@@ -250,7 +251,7 @@ __device__ __forceinline__ void on_leaf_data(uint32_t gid, const float4 g0, cons
     kbuf[pos][t] = key;
     if (st.kcount == KB) {
         st.kmax = kbuf[KB - 1][t];
-        st.dfar = h2f_bits((uint16_t)(st.kmax >> 48) + 1u);
+        st.dfar = (long long)st.kmax < 0 ? __int_as_float(0x7f800000) : h2f_bits((uint16_t)(st.kmax >> 48) + 1u);
     }
 }
 
