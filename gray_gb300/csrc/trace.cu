@@ -1159,8 +1159,11 @@ __device__ __forceinline__ void make_conic_basis(ConicBasis &cb, const float *w,
     }
     cb.hx = hx;
     cb.hy = hy;
-    // |x0 + x dx| <= ax over the image's pixels, and twice that over a tile that reaches past it
-    cb.mag = 2.0f * (sqrtf(n0) * fabsf(ax) + sqrtf(n1) * fabsf(vs)) + sqrtf(n2);
+    // V's terms: the pixel's (2 (x + 0.5) / width is below 2) and the basis' own, which are larger where a tile
+    // reaches past a small image (one pixel wide, x0 is 7 or 15 ax)
+    const float mx = fmaxf(2.0f * fabsf(ax), fabsf(x0) + hx * fabsf(dx));
+    const float my = fmaxf(2.0f * fabsf(vs), fabsf(y0) + hy * fabsf(dy));
+    cb.mag = sqrtf(n0) * mx + sqrtf(n1) * my + sqrtf(n2);
 }
 
 // Rays that the caller supplied for the pixels [x0, x1] x [y0, y1]: when those that are alive share
