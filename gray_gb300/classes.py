@@ -12,12 +12,15 @@ selected during traversal), and the backward hit list stores gaussian ids only.
 """
 from __future__ import annotations
 
+import math
+
 import torch
 
 from . import _lib
 
 CHANNELS = 3
 MAX_ALPHA = 0.9999
+FLOAT32_MAX = 3.4028234663852886e38
 NULL_PTR = 0xFFFFFFFF
 
 
@@ -29,6 +32,16 @@ def _dev():
 
 def _p(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
+
+
+def _as_float32(v) -> bool:
+    """A Python number whose magnitude a float32 holds (infinities and NaN among them)."""
+    return isinstance(v, (int, float)) and (v != v or abs(v) <= FLOAT32_MAX or abs(v) == math.inf)
+
+
+def _is_plain(t: torch.Tensor, shape: tuple, device) -> bool:
+    return (tuple(t.shape) == shape and t.dtype == torch.float32 and t.device == device and t.is_contiguous()
+            and not t.is_neg())
 
 
 class CameraDataHolder:
@@ -435,14 +448,16 @@ class Raytracer:
         """A camera for the next forwards: what filling vertical_fov_radians, znear, zfar and
         rays_from_python (False) and camera_data.set_pose do, in one launch."""
         c = self.camera_data
-        for t, shape in ((c2w_origin, (3,)), (c2w_rotation, (3, 3))):
-            if tuple(t.shape) != shape or t.dtype != torch.float32 or t.device != self.device or not t.is_contiguous():
-                c.vertical_fov_radians.fill_(vertical_fov_radians)
-                c.znear.fill_(znear)
-                c.zfar.fill_(zfar)
-                self.config_data.rays_from_python.fill_(False)
-                c.set_pose(c2w_origin, c2w_rotation)
-                return
+        # the launch takes numbers that a float32 holds (a tensor's would have to be waited for) and the pose's
+        # own float32 memory; fill_ and copy_ take or refuse the rest
+        if not (all(_as_float32(v) for v in (vertical_fov_radians, znear, zfar))
+                and _is_plain(c2w_origin, (3,), self.device) and _is_plain(c2w_rotation, (3, 3), self.device)):
+            c.vertical_fov_radians.fill_(vertical_fov_radians)
+            c.znear.fill_(znear)
+            c.zfar.fill_(zfar)
+            self.config_data.rays_from_python.fill_(False)
+            c.set_pose(c2w_origin, c2w_rotation)
+            return
         self._call("gray_set_view", c2w_origin.data_ptr(), c2w_rotation.data_ptr(), float(vertical_fov_radians),
                    float(znear), float(zfar), 0)
 
