@@ -251,7 +251,7 @@ __device__ __forceinline__ void on_leaf_data(uint32_t gid, const float4 g0, cons
     kbuf[pos][t] = key;
     if (st.kcount == KB) {
         st.kmax = kbuf[KB - 1][t];
-        st.dfar = (long long)st.kmax < 0 ? __int_as_float(0x7f800000) : h2f_bits((uint16_t)(st.kmax >> 48) + 1u);
+        st.dfar = h2f_bits((uint16_t)min((uint32_t)(st.kmax >> 48) + 1u, 0x7c00u));
     }
 }
 
@@ -1160,10 +1160,11 @@ __device__ __forceinline__ void make_conic_basis(ConicBasis &cb, const float *w,
     cb.hx = hx;
     cb.hy = hy;
     // V's terms: the pixel's (2 (x + 0.5) / width is below 2) and the basis' own, which are larger where a tile
-    // reaches past a small image (one pixel wide, x0 is 7 or 15 ax)
+    // reaches past a small image (one pixel wide, x0 is 7 or 15 ax).  The block waits for this chain: with
+    // square roots rounded to nearest a light frame's tiles took 1% longer (20k Gaussians, 1920x1080).
     const float mx = fmaxf(2.0f * fabsf(ax), fabsf(x0) + hx * fabsf(dx));
     const float my = fmaxf(2.0f * fabsf(vs), fabsf(y0) + hy * fabsf(dy));
-    cb.mag = sqrtf(n0) * mx + sqrtf(n1) * my + sqrtf(n2);
+    cb.mag = sqrt_approx(n0) * mx + sqrt_approx(n1) * my + sqrt_approx(n2);
 }
 
 // Rays that the caller supplied for the pixels [x0, x1] x [y0, y1]: when those that are alive share
