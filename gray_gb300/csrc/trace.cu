@@ -19,7 +19,7 @@
 //   32-slot multi-pass selection exactly (pass boundaries, the strict `distance > tmin` drop of
 //   equal distances, the 99-pass cap, zfar, t_threshold).  Composited ids are appended to the
 //   backward hit list in warp-aggregated segments.  Jittered rays, and rays from the caller that share
-//   their tile's origin within a cone (ray_cone_warp), go the same way; other rays from the caller, and
+//   their tile's origin within a cone (ray_cone), go the same way; other rays from the caller, and
 //   tiles whose traversal overflows the shared stack, take a per-ray slab traversal instead.
 // Backward (cuda/backward_pass.cu:2-142): one thread per pixel walks its segments back to front,
 //   recomputes alpha in fp32 and reduces the 16 per-hit gradient values into the per-Gaussian
@@ -410,9 +410,8 @@ struct ConicBasis {
     float v0[3], du[3], dv[3];
     float hx, hy;  // largest |x| and |y| of the tile
     float mag;     // V
-    // rays from the caller (ray_cone_warp): their common origin, and the axis and centre of their cone
+    // rays from the caller (ray_cone): their common origin, and the axis and centre of their cone
     float origin[3], axis[3], ca, cb;
-    int cone;
 };
 
 // (a.x * b.x + c.x, a.y * b.y + c.y), each rounded once: one issue slot for two FMAs.
@@ -1168,55 +1167,94 @@ __device__ __forceinline__ void make_conic_basis(ConicBasis &cb, const float *w,
 }
 
 // Rays that the caller supplied for the pixels [x0, x1] x [y0, y1]: when those that are alive share
-// their origin and lie within about 53 degrees of their mean direction, a warp builds their frustum and the
-// conics' basis (may be null) and returns true (on every lane; the warp calls this together).  With the
-// axis m and unit vectors u, v across it, a ray is the direction m + a u + b v up to its length; the
-// frustum spans the rectangle of the rays' (a, b), widened by 4e-6 (some 60 roundings of what they are
-// computed from), and the conics' plane is that of (a, b) about its centre.  Lengths outside [2^-10, 2^10]
-// (whose object-space squares could leave the normal range) and NaNs are left to the per-ray traversal,
-// in which a warp pops one node at a time for all of its rays: 401x301 rays over 100k Gaussians took
-// 0.66 ms that way and take 0.25 ms as tiles (the latency of their own hit chains; 950 tiles).
+// their origin and lie within about 53 degrees of their mean direction, the T threads of a block (they call
+// this together, and wait for one another afterwards; part: scratch of a row per warp) build their frustum
+// and the conics' basis and return true.  With the axis m and unit vectors u, v across it, a ray is the direction m + a u + b v up to its
+// length; the frustum spans the rectangle of the rays' (a, b), widened by 4e-6 (some 60 roundings of what
+// they are computed from), and the conics' plane is that of (a, b) about its centre.  Lengths outside
+// [2^-10, 2^10] (whose object-space squares could leave the normal range) and NaNs are left to the
+// per-ray traversal.
 // Not inlined: its registers would cost the camera rays' kernels 2%.
-__device__ __noinline__ bool ray_cone_warp(const float *__restrict__ ray_o, const float *__restrict__ ray_d,
-                                           uint32_t alloc_w, const float *__restrict__ root_box, int x0, int y0,
-                                           int x1, int y1, Frustum &fr, ConicBasis *cb) {
-    const int lane = threadIdx.x & 31;
+constexpr int kConePart = 16;
+
+template <int T>
+__device__ __noinline__ bool ray_cone(const float *__restrict__ ray_o, const float *__restrict__ ray_d,
+                                      uint32_t alloc_w, const float *__restrict__ root_box, int x0, int y0,
+                                      int x1, int y1, Frustum &fr, ConicBasis &cb, float (*part)[kConePart]) {
+    constexpr int W = T / 32;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int w = x1 - x0 + 1, count = w * (y1 - y0 + 1);
     if (w <= 0 || y1 < y0) return false;  // a split tile's packet beyond the image
     bool have = false, bad = false;
-    f3 o = mk3(0.0f, 0.0f, 0.0f), m = mk3(0.0f, 0.0f, 0.0f);
-    for (int i = lane; i < count; i += 32) {
+    int rays = 0;
+    f3 ref = mk3(0.0f, 0.0f, 0.0f), m = mk3(0.0f, 0.0f, 0.0f);
+    for (int i0 = 0; i0 < count; i0 += T) {
+        const int i = i0 + t;
         const size_t px = 3 * ((size_t)(y0 + i / w) * alloc_w + (size_t)(x0 + i % w));
-        const f3 d = mk3(ray_d[px], ray_d[px + 1], ray_d[px + 2]);
+        f3 d = mk3(0.0f, 0.0f, 0.0f), o = d;
+        if (i < count) {
+            d = mk3(ray_d[px], ray_d[px + 1], ray_d[px + 2]);
+            o = mk3(ray_o[px], ray_o[px + 1], ray_o[px + 2]);
+        }
         const float len2 = dot3(d, d);
-        if (sqrtf(len2) == 0.0f) continue;
-        if (!(len2 >= 0x1.0p-20f && len2 <= 0x1.0p20f)) bad = true;
-        const f3 ro = mk3(ray_o[px], ray_o[px + 1], ray_o[px + 2]);
-        if (!have) o = ro;
-        have = true;
-        if (!(ro.x == o.x && ro.y == o.y && ro.z == o.z)) bad = true;
-        const float inv = 1.0f / sqrtf(len2);
-        m = mk3(fmaf(d.x, inv, m.x), fmaf(d.y, inv, m.y), fmaf(d.z, inv, m.z));
+        const bool on = !(sqrtf(len2) == 0.0f);
+        const uint32_t who = __ballot_sync(kFull, on);
+        rays += __popc(who);
+        if (!have && who != 0u) {
+            const int lead = __ffs((int)who) - 1;
+            ref = mk3(__shfl_sync(kFull, o.x, lead), __shfl_sync(kFull, o.y, lead), __shfl_sync(kFull, o.z, lead));
+            have = true;
+        }
+        if (on) {
+            if (!(len2 >= 0x1.0p-20f && len2 <= 0x1.0p20f)) bad = true;
+            if (!(o.x == ref.x && o.y == ref.y && o.z == ref.z)) bad = true;
+            const float inv = 1.0f / sqrtf(len2);
+            m = mk3(fmaf(d.x, inv, m.x), fmaf(d.y, inv, m.y), fmaf(d.z, inv, m.z));
+        }
+        if (__any_sync(kFull, bad)) break;  // (origins of their own: the first round tells)
     }
-    const uint32_t who = __ballot_sync(kFull, have);
-    if (who == 0u) return false;
-    const int lead = __ffs((int)who) - 1;
-    const f3 ref = mk3(__shfl_sync(kFull, o.x, lead), __shfl_sync(kFull, o.y, lead), __shfl_sync(kFull, o.z, lead));
-    if (have && !(o.x == ref.x && o.y == ref.y && o.z == ref.z)) bad = true;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1)
         m = mk3(m.x + __shfl_xor_sync(kFull, m.x, off), m.y + __shfl_xor_sync(kFull, m.y, off),
                 m.z + __shfl_xor_sync(kFull, m.z, off));
+    bad = __any_sync(kFull, bad);
+    if constexpr (W > 1) {
+        if (lane == 0) {
+            float *p = part[warp];
+            p[0] = m.x;
+            p[1] = m.y;
+            p[2] = m.z;
+            p[3] = ref.x;
+            p[4] = ref.y;
+            p[5] = ref.z;
+            p[6] = bad ? -1.0f : (float)rays;
+        }
+        __syncthreads();
+        m = mk3(0.0f, 0.0f, 0.0f);
+        have = bad = false;
+        rays = 0;
+        for (int q = 0; q < W; q++) {
+            const float *p = part[q];
+            if (p[6] < 0.0f) bad = true;
+            if (!(p[6] > 0.0f)) continue;  // no ray of this warp
+            if (!have) ref = mk3(p[3], p[4], p[5]);
+            have = true;
+            if (!(p[3] == ref.x && p[4] == ref.y && p[5] == ref.z)) bad = true;
+            m = mk3(m.x + p[0], m.y + p[1], m.z + p[2]);
+            rays += (int)p[6];
+        }
+    }
+    if (bad || rays == 0) return false;
     const float inv = 1.0f / sqrtf(dot3(m, m));
     m = mk3(m.x * inv, m.y * inv, m.z * inv);
-    if (!(dot3(m, m) > 0.99f)) bad = true;  // (directions that cancel, NaN)
+    if (!(dot3(m, m) > 0.99f)) return false;  // (directions that cancel, NaN)
     f3 u = fabsf(m.x) < 0.7f ? mk3(0.0f, m.z, -m.y) : mk3(-m.z, 0.0f, m.x);
     const float ul = 1.0f / sqrtf(dot3(u, u));
     u = mk3(u.x * ul, u.y * ul, u.z * ul);
     const f3 v = cross3(m, u);
     const float big = __int_as_float(0x7f800000);
     float a0 = big, a1 = -big, b0 = big, b1 = -big;
-    for (int i = lane; i < count; i += 32) {
+    for (int i = t; i < count; i += T) {
         const size_t px = 3 * ((size_t)(y0 + i / w) * alloc_w + (size_t)(x0 + i % w));
         const f3 d = mk3(ray_d[px], ray_d[px + 1], ray_d[px + 2]);
         const float len = sqrtf(dot3(d, d));
@@ -1229,7 +1267,6 @@ __device__ __noinline__ bool ray_cone_warp(const float *__restrict__ ray_o, cons
         b0 = fminf(b0, rb);
         b1 = fmaxf(b1, rb);
     }
-    if (__any_sync(kFull, bad)) return false;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         a0 = fminf(a0, __shfl_xor_sync(kFull, a0, off));
@@ -1237,36 +1274,59 @@ __device__ __noinline__ bool ray_cone_warp(const float *__restrict__ ray_o, cons
         b0 = fminf(b0, __shfl_xor_sync(kFull, b0, off));
         b1 = fmaxf(b1, __shfl_xor_sync(kFull, b1, off));
     }
+    bad = __any_sync(kFull, bad);
+    if constexpr (W > 1) {
+        if (lane == 0) {
+            float *p = part[warp];
+            p[8] = a0;
+            p[9] = a1;
+            p[10] = b0;
+            p[11] = b1;
+            p[12] = bad ? 1.0f : 0.0f;
+        }
+        __syncthreads();
+        for (int q = 0; q < W; q++) {
+            const float *p = part[q];
+            a0 = fminf(a0, p[8]);
+            a1 = fmaxf(a1, p[9]);
+            b0 = fminf(b0, p[10]);
+            b1 = fmaxf(b1, p[11]);
+            if (p[12] != 0.0f) bad = true;
+        }
+    }
+    if (bad) return false;
     const float wide = 4e-6f * (1.0f + fmaxf(fabsf(a0), fabsf(a1)) + fmaxf(fabsf(b0), fabsf(b1)));
     a0 -= wide;
     a1 += wide;
     b0 -= wide;
     b1 += wide;
-    f3 d[4];
+    if (t < 5) {
+        f3 d[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        const float ea = e == 1 || e == 2 ? a1 : a0, eb = e >= 2 ? b1 : b0;
-        d[e] = mk3(fmaf(eb, v.x, fmaf(ea, u.x, m.x)), fmaf(eb, v.y, fmaf(ea, u.y, m.y)),
-                   fmaf(eb, v.z, fmaf(ea, u.z, m.z)));
+        for (int e = 0; e < 4; e++) {
+            const float ea = e == 1 || e == 2 ? a1 : a0, eb = e >= 2 ? b1 : b0;
+            d[e] = mk3(fmaf(eb, v.x, fmaf(ea, u.x, m.x)), fmaf(eb, v.y, fmaf(ea, u.y, m.y)),
+                       fmaf(eb, v.z, fmaf(ea, u.z, m.z)));
+        }
+        frustum_plane(t, ref, d, root_box, fr.pn[t], fr.pa[t]);
     }
-    if (lane < 5) frustum_plane(lane, ref, d, root_box, fr.pn[lane], fr.pa[lane]);
-    if (cb && lane == 0) {
+    if (t == 0) {
         const float ca = 0.5f * (a0 + a1), cc = 0.5f * (b0 + b1);
         const float mm[3] = {m.x, m.y, m.z}, uu[3] = {u.x, u.y, u.z}, vv[3] = {v.x, v.y, v.z};
         const float oo[3] = {ref.x, ref.y, ref.z};
 #pragma unroll
         for (int e = 0; e < 3; e++) {
-            cb->v0[e] = fmaf(cc, vv[e], fmaf(ca, uu[e], mm[e]));
-            cb->du[e] = uu[e];
-            cb->dv[e] = vv[e];
-            cb->origin[e] = oo[e];
-            cb->axis[e] = mm[e];
+            cb.v0[e] = fmaf(cc, vv[e], fmaf(ca, uu[e], mm[e]));
+            cb.du[e] = uu[e];
+            cb.dv[e] = vv[e];
+            cb.origin[e] = oo[e];
+            cb.axis[e] = mm[e];
         }
-        cb->ca = ca;
-        cb->cb = cc;
-        cb->hx = 0.5f * (a1 - a0);
-        cb->hy = 0.5f * (b1 - b0);
-        cb->mag = 2.0f * (1.0f + fmaxf(fabsf(a0), fabsf(a1)) + fmaxf(fabsf(b0), fabsf(b1)));
+        cb.ca = ca;
+        cb.cb = cc;
+        cb.hx = 0.5f * (a1 - a0);
+        cb.hy = 0.5f * (b1 - b0);
+        cb.mag = 2.0f * (1.0f + fmaxf(fabsf(a0), fabsf(a1)) + fmaxf(fabsf(b0), fabsf(b1)));
     }
     __syncwarp();
     return true;
@@ -1327,21 +1387,20 @@ __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, i
 
     // rays that share their origin: the block traverses its tile together
     bool tile = true;
-    float x, y;  // the ray's place in the conics' plane
+    float x = 0.0f, y = 0.0f;  // the ray's place in the conics' plane
     if (given) {
-        if (warp == 0) {
-            const bool cone = ray_cone_warp(a.ray_o, a.ray_d, a.alloc_w, a.root_box, tx0, ty0,
-                                            min(tx0 + rw, (int)a.render_w) - 1, min(ty0 + rh, (int)a.render_h) - 1,
-                                            sh.fr, &sh.cb);
-            if (lane == 0) sh.cb.cone = cone ? 1 : 0;
-        }
+        static_assert(sizeof(sh.kbuf) >= sizeof(float) * kWarps * kConePart, "the cone's scratch does not fit");
+        tile = ray_cone<kFwdThreads>(a.ray_o, a.ray_d, a.alloc_w, a.root_box, tx0, ty0,
+                                     min(tx0 + rw, (int)a.render_w) - 1, min(ty0 + rh, (int)a.render_h) - 1, sh.fr,
+                                     sh.cb, reinterpret_cast<float(*)[kConePart]>(sh.kbuf));
         __syncthreads();
-        tile = sh.cb.cone != 0;
-        const f3 m = mk3(sh.cb.axis[0], sh.cb.axis[1], sh.cb.axis[2]);
-        const float c = fdot3(rd, m);
-        x = fdot3(rd, mk3(sh.cb.du[0], sh.cb.du[1], sh.cb.du[2])) / c - sh.cb.ca;
-        y = fdot3(rd, mk3(sh.cb.dv[0], sh.cb.dv[1], sh.cb.dv[2])) / c - sh.cb.cb;
-        if (tile && !alive) ro = mk3(sh.cb.origin[0], sh.cb.origin[1], sh.cb.origin[2]);
+        if (tile) {
+            const f3 m = mk3(sh.cb.axis[0], sh.cb.axis[1], sh.cb.axis[2]);
+            const float c = fdot3(rd, m);
+            x = fdot3(rd, mk3(sh.cb.du[0], sh.cb.du[1], sh.cb.du[2])) / c - sh.cb.ca;
+            y = fdot3(rd, mk3(sh.cb.dv[0], sh.cb.dv[1], sh.cb.dv[2])) / c - sh.cb.cb;
+            if (!alive) ro = mk3(sh.cb.origin[0], sh.cb.origin[1], sh.cb.origin[2]);
+        }
     } else {
         const float wide = *a.jitter ? 0.5f : 0.0f;
         const float hx = (float)(rw - 1) * 0.5f, hy = (float)(rh - 1) * 0.5f;
@@ -1823,17 +1882,14 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
     return est;
 }
 
-// The frustum of this forward's rays through a pixel rectangle (a warp together); false for rays from the
-// caller that do not share an origin and a cone.
-__device__ __forceinline__ bool make_tile_frustum(const FwdArgs &a, int x0, int y0, int x1, int y1, Frustum &fr) {
-    if (*a.rays_from_python) 
-        return ray_cone_warp(a.ray_o, a.ray_d, a.alloc_w, a.root_box, x0, y0, x1, y1, fr, nullptr);
+// The frustum of the camera's rays through a pixel rectangle (a warp together).
+__device__ __forceinline__ void make_tile_frustum(const FwdArgs &a, int x0, int y0, int x1, int y1, Frustum &fr) {
     make_frustum_warp(fr, mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]), a.w2c, *a.fov, x0, y0, x1, y1,
                       a.render_w, a.render_h, a.root_box, *a.jitter ? 0.5f : 0.0f);
-    return true;
 }
 
-// Coarse frontiers of the super-tiles (kSuperTiles x kSuperTiles block tiles each), one warp each.
+// Coarse frontiers of the super-tiles (kSuperTiles x kSuperTiles block tiles each), one warp each.  Not for the
+// caller's rays: a warp would read 2048 of them first (60 us), more than the walks that start at the root take.
 __global__ void __launch_bounds__(32) super_cost_kernel(const FwdArgs a, int bw, int bh, int nsuper) {
     __shared__ FrontierScratch fs;
     __shared__ SuperScratch ss;
@@ -1841,36 +1897,40 @@ __global__ void __launch_bounds__(32) super_cost_kernel(const FwdArgs a, int bw,
     if (st >= nsuper) return;
     uint32_t *out = a.super_frontier + (size_t)st * kSuperWords;
     const int n = a.n;
-    bool walk = !*a.render_ellipsoids && n > 1;
-    if (walk) {
-        const int x0 = (st % a.super_x) * kSuperTiles * bw, y0 = (st / a.super_x) * kSuperTiles * bh;
-        const int x1 = min(x0 + kSuperTiles * bw, (int)a.render_w) - 1;
-        const int y1 = min(y0 + kSuperTiles * bh, (int)a.render_h) - 1;
-        walk = make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
-        if (walk) frontier_walk<true>(a.nodes, n, kSuperCut, fs, &ss, out, nullptr);
+    if (*a.render_ellipsoids || *a.rays_from_python || n <= 1) {
+        if (lane == 0) out[0] = kFrontierNone;
+        return;
     }
-    if (!walk && lane == 0) out[0] = kFrontierNone;
+    const int x0 = (st % a.super_x) * kSuperTiles * bw, y0 = (st / a.super_x) * kSuperTiles * bh;
+    const int x1 = min(x0 + kSuperTiles * bw, (int)a.render_w) - 1;
+    const int y1 = min(y0 + kSuperTiles * bh, (int)a.render_h) - 1;
+    make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
+    frontier_walk<true>(a.nodes, n, kSuperCut, fs, &ss, out, nullptr);
 }
 
-__global__ void __launch_bounds__(32) tile_cost_kernel(const FwdArgs a, int bw, int bh) {
+__global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int bw, int bh) {
     __shared__ FrontierScratch fs;
+    __shared__ ConicBasis cb;
     const int tile = blockIdx.x, lane = threadIdx.x;
     uint32_t *out = a.frontier ? a.frontier + (size_t)tile * kFrontierWords : nullptr;
     uint32_t est = 0;
     const int n = a.n;
+    const int x0 = (tile % a.tiles_x) * bw, y0 = (tile / a.tiles_x) * bh;
+    const int x1 = min(x0 + bw, (int)a.render_w) - 1, y1 = min(y0 + bh, (int)a.render_h) - 1;
     bool walk = !*a.render_ellipsoids && n > 1;
+    if (walk && *a.rays_from_python) {
+        walk = ray_cone<32>(a.ray_o, a.ray_d, a.alloc_w, a.root_box, x0, y0, x1, y1, fs.fr, cb, nullptr);
+    } else if (walk) {
+        make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
+    }
     if (walk) {
-        const int x0 = (tile % a.tiles_x) * bw, y0 = (tile / a.tiles_x) * bh;
-        const int x1 = min(x0 + bw, (int)a.render_w) - 1, y1 = min(y0 + bh, (int)a.render_h) - 1;
-        walk = make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
         const uint32_t *seed = nullptr;
         if (a.super_frontier) {
             const int sx = (tile % a.tiles_x) / kSuperTiles, sy = (tile / a.tiles_x) / kSuperTiles;
             seed = a.super_frontier + (size_t)(sy * a.super_x + sx) * kSuperWords;
         }
-        if (walk)
-            est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut, fs,
-                                       nullptr, out, seed);
+        est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut, fs, nullptr,
+                                   out, seed);
     }
     if (!walk && out && lane == 0) out[0] = kFrontierNone;
     if (lane == 0) a.schedule[kSchedHeader + tile] = est;
