@@ -49,6 +49,9 @@ constexpr int kSchedHeader = 64;  // schedule words before the per-tile estimate
 constexpr int kSchedItems = 1;       // header word: tiles of the work order
 constexpr int kSchedSplitNext = 2;   // work counter of the split tiles' packets
 constexpr int kSchedSplitItems = 3;  // packets of split tiles
+constexpr int kSchedRays = 4;        // tiles whose rays are traversed one by one (see kRayTile)
+constexpr int kSchedRayNext = 5;     // work counter of their packets
+constexpr uint32_t kRayTile = 0xffffffffu;  // estimate of such a tile
 constexpr int kItemShift = 29;       // a split tile's packet: its tile, and the packet from this bit on
 constexpr uint32_t kItemTile = (1u << kItemShift) - 1u;
 constexpr int kOrderPerTile = 5;     // words of the work order per tile: itself, or its four packets
@@ -96,7 +99,7 @@ struct FwdArgs {
     int auto_role;  // 0, or kChoiceNarrow / kChoiceWide: the launch of the automatic choice this is
     uint32_t *schedule;  // work order of the pixel tiles (null: tiles in launch order)
     int tiles_x, ntiles;
-    int slots_narrow, slots_wide;  // blocks resident at once in the narrow and in the wide kernel
+    int slots_split;  // blocks of the split kernel resident at once
     uint32_t *frontier;  // per-tile BVH frontiers (null: packets start at the root)
     uint32_t frontier_cut;
     uint32_t *super_frontier;  // per super-tile coarse frontiers seeding the tile walks (null: root)
@@ -469,6 +472,7 @@ __device__ __forceinline__ float conic_coefficients(const ConicBasis &cb, const 
 // Shared memory of a block that traces one pixel tile (one ray per thread), or, SPLIT, a packet of one.
 template <int KB, bool SPLIT>
 struct TileShared {
+    static constexpr bool kTiles = true;
     static constexpr int kStack = SPLIT ? kSplitStack : kTileStack;
     unsigned long long kbuf[KB][kFwdThreads];
     // the batch's candidates, filled once per batch by the block (one candidate per thread):
@@ -482,6 +486,13 @@ struct TileShared {
     Frustum fr;
     ConicBasis cb;
     uint32_t cnt[kWarps];      // per-warp counts of a step
+};
+
+// Shared memory of a block whose warps trace packets of rays one ray per lane, each lane by itself.
+template <int KB>
+struct RayShared {
+    static constexpr bool kTiles = false;
+    unsigned long long kbuf[KB][kFwdThreads];
 };
 
 // A batch: the block's queued leaves queue[0, take) (take <= kBatch, every thread calls this together;
@@ -824,12 +835,13 @@ __device__ __forceinline__ void merge_split(LaneState &st, TileShared<KB, true> 
 // and lie inside sh.fr, and are traversed together from the frontier `front` (see traverse_tile, px,
 // py); else every warp traverses its own rays.  SPLIT: the four warps hold the same 32 rays and share
 // their candidates (see merge_split); each ends with the same result, and warp 0 alone writes hit
-// lists.  Every thread of the block calls this together.
-template <int KB, bool SPLIT>
+// lists.  Every thread of the block calls this together; with RayShared (no tiles) the warps are on their own.
+template <int KB, bool SPLIT, class Shared>
 __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnobs &k, f3 ro, f3 rd, float px, float py,
                                            bool alive, bool tile, bool grads, const HitSink &hs,
-                                           int32_t *status, TileShared<KB, SPLIT> &sh, const uint32_t *front,
+                                           int32_t *status, Shared &sh, const uint32_t *front,
                                            RayResult &res) {
+    if constexpr (!Shared::kTiles) tile = false;
     unsigned long long(*kbuf)[kFwdThreads] = sh.kbuf;
     const int lane = threadIdx.x & 31;
     LaneState &st = res.st;
@@ -861,22 +873,24 @@ __device__ __forceinline__ void trace_rays(const TraceScene &sc, const TraceKnob
         // ---------------- traversal ----------------
         bool per_ray = !tile;
         bool ranked = false;  // the keys are those of the four warps, in merge_split's order
-        if (tile && traverse_tile<KB, SPLIT>(sc, k, ro, rd, px, py, want, first, st, sh, front, status)) {
-            if constexpr (SPLIT) {
-                merge_split<KB>(st, sh, first);
-                ranked = true;
+        if constexpr (Shared::kTiles) {
+            if (tile && traverse_tile<KB, SPLIT>(sc, k, ro, rd, px, py, want, first, st, sh, front, status)) {
+                if constexpr (SPLIT) {
+                    merge_split<KB>(st, sh, first);
+                    ranked = true;
+                }
+            } else if (tile) {
+                // the tile's stack filled up: discard what was gathered, trace per ray
+                st.kcount = 0;
+                st.ncand = 0;
+                st.dfar = __int_as_float(0x7f800000);
+                if (first) {
+                    st.lfx = 0;
+                    st.afx = st.cfx0 = st.cfx1 = st.cfx2 = 0;
+                    st.nhit = 0;
+                }
+                per_ray = true;
             }
-        } else if (tile) {
-            // the tile's stack filled up: discard what was gathered, trace per ray
-            st.kcount = 0;
-            st.ncand = 0;
-            st.dfar = __int_as_float(0x7f800000);
-            if (first) {
-                st.lfx = 0;
-                st.afx = st.cfx0 = st.cfx1 = st.cfx2 = 0;
-                st.nhit = 0;
-            }
-            per_ray = true;
         }
         if (!per_ray) {
         } else if (n == 1) {
@@ -1332,24 +1346,7 @@ __device__ __noinline__ bool ray_cone(const float *__restrict__ ray_o, const flo
     return true;
 }
 
-// The block's pixel tile (bx, by): 2x2 packets of tile_w x tile_h pixels, one packet per warp; or, SPLIT:
-// packet sub of it alone, its candidates shared by the four warps.  Returns whether the calling
-// warp's packet needs more than one traversal with 16 hit slots (RayResult::retraced).
-// ANY: rays from the caller too (they cost the camera rays' kernels registers: 1.8% of the forward); else
-// rays_from_python is off.
-template <int KB, bool SPLIT, bool ANY>
-__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, int sub, TileShared<KB, SPLIT> &sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int rw = SPLIT ? a.tile_w : a.tile_w * kBlockWarpsX, rh = SPLIT ? a.tile_h : a.tile_h * kBlockWarpsY;
-    const int pk = SPLIT ? sub : warp;  // the warp's packet
-    const int px0 = bx * (a.tile_w * kBlockWarpsX) + (pk % kBlockWarpsX) * a.tile_w;
-    const int py0 = by * (a.tile_h * kBlockWarpsY) + (pk / kBlockWarpsX) * a.tile_h;
-    // the pixels the block traces start at (tx0, ty0)
-    const int tx0 = SPLIT ? px0 : bx * (a.tile_w * kBlockWarpsX), ty0 = SPLIT ? py0 : by * (a.tile_h * kBlockWarpsY);
-    const int px = px0 + (lane % a.tile_w), py = py0 + (lane / a.tile_w);
-    const bool inside = px < (int)a.render_w && py < (int)a.render_h;
-    const uint32_t pixel = (uint32_t)py * a.alloc_w + (uint32_t)px;
-
+__device__ __forceinline__ TraceKnobs trace_knobs(const FwdArgs &a) {
     TraceKnobs k;
     k.znear = *a.znear;
     k.zfar = *a.zfar;
@@ -1357,74 +1354,12 @@ __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, i
     k.pw = *a.exp_power;
     k.tthr = *a.t_threshold;
     k.render_depth = *a.render_depth != 0;
-    const bool grads = !a.display && *a.grads_enabled != 0;
-    const TraceScene sc{a.geom, a.l2w, a.live, a.channels, a.nodes, a.root_box, a.n};
-    const HitSink hs{a.counter, a.pool, a.pool_size};
+    return k;
+}
 
-    // ---- ray generation (cuda/shaders.cu:76-88) ----
-    f3 ro = mk3(0.0f, 0.0f, 0.0f), rd = mk3(0.0f, 0.0f, 0.0f);
-    float jx = 0.0f, jy = 0.0f;
-    bool alive = false;
-    // every thread holds the camera origin, inactive ones too (a tile's candidates get their
-    // object-space origin from whichever thread fetches them)
-    const bool given = ANY && *a.rays_from_python;
-    if (!given) ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
-    if (inside) {
-        if (given) {
-            ro = mk3(a.ray_o[3 * pixel], a.ray_o[3 * pixel + 1], a.ray_o[3 * pixel + 2]);
-            rd = mk3(a.ray_d[3 * pixel], a.ray_d[3 * pixel + 1], a.ray_d[3 * pixel + 2]);
-        } else {
-            ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
-            if (*a.jitter) {
-                uint32_t h = pcg_hash(pixel ^ pcg_hash(*a.total_num_calls));
-                jx = (float)(h & 0xFFFFu) * 0x1.0p-16f - 0.5f;
-                jy = (float)(h >> 16) * 0x1.0p-16f - 0.5f;
-            }
-            rd = camera_ray(a.w2c, *a.fov, px, py, a.render_w, a.render_h, jx, jy);
-        }
-        alive = !(sqrtf(dot3(rd, rd)) == 0.0f);
-    }
-
-    // rays that share their origin: the block traverses its tile together
-    bool tile = true;
-    float x = 0.0f, y = 0.0f;  // the ray's place in the conics' plane
-    if (given) {
-        static_assert(sizeof(sh.kbuf) >= sizeof(float) * kWarps * kConePart, "the cone's scratch does not fit");
-        tile = ray_cone<kFwdThreads>(a.ray_o, a.ray_d, a.alloc_w, a.root_box, tx0, ty0,
-                                     min(tx0 + rw, (int)a.render_w) - 1, min(ty0 + rh, (int)a.render_h) - 1, sh.fr,
-                                     sh.cb, reinterpret_cast<float(*)[kConePart]>(sh.kbuf));
-        __syncthreads();
-        if (tile) {
-            const f3 m = mk3(sh.cb.axis[0], sh.cb.axis[1], sh.cb.axis[2]);
-            const float c = fdot3(rd, m);
-            x = fdot3(rd, mk3(sh.cb.du[0], sh.cb.du[1], sh.cb.du[2])) / c - sh.cb.ca;
-            y = fdot3(rd, mk3(sh.cb.dv[0], sh.cb.dv[1], sh.cb.dv[2])) / c - sh.cb.cb;
-            if (!alive) ro = mk3(sh.cb.origin[0], sh.cb.origin[1], sh.cb.origin[2]);
-        }
-    } else {
-        const float wide = *a.jitter ? 0.5f : 0.0f;
-        const float hx = (float)(rw - 1) * 0.5f, hy = (float)(rh - 1) * 0.5f;
-        // (the loop of trace_rays starts with a block barrier)
-        if (warp == 0)
-            make_frustum_warp(sh.fr, ro, a.w2c, *a.fov, tx0, ty0, tx0 + rw - 1, ty0 + rh - 1, a.render_w, a.render_h,
-                              a.root_box, wide);
-        if (threadIdx.x == kFwdThreads - 1)
-            make_conic_basis(sh.cb, a.w2c, *a.fov, (float)tx0 + hx, (float)ty0 + hy, hx + wide, hy + wide, a.render_w,
-                             a.render_h);
-        // (pixel plus jitter as camera_ray rounds it; the differences are exact)
-        x = ((float)px + jx) - ((float)tx0 + hx);
-        y = ((float)py + jy) - ((float)ty0 + hy);
-    }
-    const uint32_t *front =
-        tile && a.frontier ? a.frontier + (size_t)(by * a.tiles_x + bx) * kFrontierWords : nullptr;
-    RayResult r;
-    trace_rays<KB, SPLIT>(sc, k, ro, rd, x, y, alive, tile, grads, hs, a.status, sh, front, r);
-    if (SPLIT && warp != 0) return false;
-    if (!inside) return r.retraced;
-    if (!alive) {
-        a.head[pixel] = GRAY_NULL;  // inactive pixel: empty list, nothing else written
-        return r.retraced;
-    }
+// What a traced ray leaves behind (cuda/forward_pass.cu:131-151).
+__device__ __forceinline__ void store_ray(const FwdArgs &a, const TraceKnobs &k, bool grads, uint32_t pixel, f3 ro,
+                                          f3 rd, RayResult &r) {
     float r0, r1, r2;
     finish_ray(r, a.bg, *a.eps_fwd, k.render_depth, r0, r1, r2);
     a.out_rgb[3 * pixel] = r.C0;
@@ -1456,6 +1391,127 @@ __device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, i
         }
         a.head[pixel] = GRAY_NULL;
     }
+}
+
+// Where a tile's rays come from: the camera; whatever rays_from_python says, supplied rays of a tile that
+// share a cone being traversed together; or the same, supplied rays being traversed one by one.
+constexpr int kCamera = 0, kCones = 1, kSingles = 2;
+
+// The block's pixel tile (bx, by): 2x2 packets of tile_w x tile_h pixels, one packet per warp; or, SPLIT:
+// packet sub of it alone, its candidates shared by the four warps.  Returns whether the calling
+// warp's packet needs more than one traversal with 16 hit slots (RayResult::retraced).
+// RAYS: other rays than the camera's cost its kernels registers (1.8% of the forward).
+template <int KB, bool SPLIT, int RAYS>
+__device__ __forceinline__ bool forward_tile(const FwdArgs &a, int bx, int by, int sub, TileShared<KB, SPLIT> &sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rw = SPLIT ? a.tile_w : a.tile_w * kBlockWarpsX, rh = SPLIT ? a.tile_h : a.tile_h * kBlockWarpsY;
+    const int pk = SPLIT ? sub : warp;  // the warp's packet
+    const int px0 = bx * (a.tile_w * kBlockWarpsX) + (pk % kBlockWarpsX) * a.tile_w;
+    const int py0 = by * (a.tile_h * kBlockWarpsY) + (pk / kBlockWarpsX) * a.tile_h;
+    // the pixels the block traces start at (tx0, ty0)
+    const int tx0 = SPLIT ? px0 : bx * (a.tile_w * kBlockWarpsX), ty0 = SPLIT ? py0 : by * (a.tile_h * kBlockWarpsY);
+    const int px = px0 + (lane % a.tile_w), py = py0 + (lane / a.tile_w);
+    const bool inside = px < (int)a.render_w && py < (int)a.render_h;
+    const uint32_t pixel = (uint32_t)py * a.alloc_w + (uint32_t)px;
+
+    const TraceKnobs k = trace_knobs(a);
+    const bool grads = !a.display && *a.grads_enabled != 0;
+    const TraceScene sc{a.geom, a.l2w, a.live, a.channels, a.nodes, a.root_box, a.n};
+    const HitSink hs{a.counter, a.pool, a.pool_size};
+
+    // ---- ray generation (cuda/shaders.cu:76-88) ----
+    f3 ro = mk3(0.0f, 0.0f, 0.0f), rd = mk3(0.0f, 0.0f, 0.0f);
+    float jx = 0.0f, jy = 0.0f;
+    bool alive = false;
+    // every thread holds the camera origin, inactive ones too (a tile's candidates get their
+    // object-space origin from whichever thread fetches them)
+    const bool given = RAYS != kCamera && *a.rays_from_python;
+    if (!given) ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
+    if (inside) {
+        if (given) {
+            ro = mk3(a.ray_o[3 * pixel], a.ray_o[3 * pixel + 1], a.ray_o[3 * pixel + 2]);
+            rd = mk3(a.ray_d[3 * pixel], a.ray_d[3 * pixel + 1], a.ray_d[3 * pixel + 2]);
+        } else {
+            ro = mk3(a.cam_origin[0], a.cam_origin[1], a.cam_origin[2]);
+            if (*a.jitter) {
+                uint32_t h = pcg_hash(pixel ^ pcg_hash(*a.total_num_calls));
+                jx = (float)(h & 0xFFFFu) * 0x1.0p-16f - 0.5f;
+                jy = (float)(h >> 16) * 0x1.0p-16f - 0.5f;
+            }
+            rd = camera_ray(a.w2c, *a.fov, px, py, a.render_w, a.render_h, jx, jy);
+        }
+        alive = !(sqrtf(dot3(rd, rd)) == 0.0f);
+    }
+
+    // rays that share their origin: the block traverses its tile together
+    bool tile = true;
+    float x = 0.0f, y = 0.0f;  // the ray's place in the conics' plane
+    if (given) {
+        tile = false;
+        if constexpr (RAYS == kCones) {
+            static_assert(sizeof(sh.kbuf) >= sizeof(float) * kWarps * kConePart, "the cone's scratch does not fit");
+            tile = ray_cone<kFwdThreads>(a.ray_o, a.ray_d, a.alloc_w, a.root_box, tx0, ty0,
+                                         min(tx0 + rw, (int)a.render_w) - 1, min(ty0 + rh, (int)a.render_h) - 1, sh.fr,
+                                         sh.cb, reinterpret_cast<float(*)[kConePart]>(sh.kbuf));
+            __syncthreads();
+            if (tile) {
+                const f3 m = mk3(sh.cb.axis[0], sh.cb.axis[1], sh.cb.axis[2]);
+                const float c = fdot3(rd, m);
+                x = fdot3(rd, mk3(sh.cb.du[0], sh.cb.du[1], sh.cb.du[2])) / c - sh.cb.ca;
+                y = fdot3(rd, mk3(sh.cb.dv[0], sh.cb.dv[1], sh.cb.dv[2])) / c - sh.cb.cb;
+                if (!alive) ro = mk3(sh.cb.origin[0], sh.cb.origin[1], sh.cb.origin[2]);
+            }
+        }
+    } else {
+        const float wide = *a.jitter ? 0.5f : 0.0f;
+        const float hx = (float)(rw - 1) * 0.5f, hy = (float)(rh - 1) * 0.5f;
+        // (the loop of trace_rays starts with a block barrier)
+        if (warp == 0)
+            make_frustum_warp(sh.fr, ro, a.w2c, *a.fov, tx0, ty0, tx0 + rw - 1, ty0 + rh - 1, a.render_w, a.render_h,
+                              a.root_box, wide);
+        if (threadIdx.x == kFwdThreads - 1)
+            make_conic_basis(sh.cb, a.w2c, *a.fov, (float)tx0 + hx, (float)ty0 + hy, hx + wide, hy + wide, a.render_w,
+                             a.render_h);
+        // (pixel plus jitter as camera_ray rounds it; the differences are exact)
+        x = ((float)px + jx) - ((float)tx0 + hx);
+        y = ((float)py + jy) - ((float)ty0 + hy);
+    }
+    const uint32_t *front =
+        tile && a.frontier ? a.frontier + (size_t)(by * a.tiles_x + bx) * kFrontierWords : nullptr;
+    RayResult r;
+    trace_rays<KB, SPLIT>(sc, k, ro, rd, x, y, alive, tile, grads, hs, a.status, sh, front, r);
+    if (SPLIT && warp != 0) return false;
+    if (!inside) return r.retraced;
+    if (!alive) {
+        a.head[pixel] = GRAY_NULL;  // inactive pixel: empty list, nothing else written
+        return r.retraced;
+    }
+    store_ray(a, k, grads, pixel, ro, rd, r);
+    return r.retraced;
+}
+
+// Packet sub of the pixel tile (bx, by) on the caller's rays, traced by one warp ray by ray.
+template <int KB>
+__device__ __forceinline__ bool forward_ray_packet(const FwdArgs &a, int bx, int by, int sub, RayShared<KB> &sh) {
+    const int lane = threadIdx.x & 31;
+    const int px = (bx * kBlockWarpsX + sub % kBlockWarpsX) * a.tile_w + lane % a.tile_w;
+    const int py = (by * kBlockWarpsY + sub / kBlockWarpsX) * a.tile_h + lane / a.tile_w;
+    const bool inside = px < (int)a.render_w && py < (int)a.render_h;
+    const uint32_t pixel = (uint32_t)py * a.alloc_w + (uint32_t)px;
+    const TraceKnobs k = trace_knobs(a);
+    const bool grads = !a.display && *a.grads_enabled != 0;
+    const TraceScene sc{a.geom, a.l2w, a.live, a.channels, a.nodes, a.root_box, a.n};
+    const HitSink hs{a.counter, a.pool, a.pool_size};
+    f3 ro = mk3(0.0f, 0.0f, 0.0f), rd = ro;
+    if (inside) {
+        ro = mk3(a.ray_o[3 * pixel], a.ray_o[3 * pixel + 1], a.ray_o[3 * pixel + 2]);
+        rd = mk3(a.ray_d[3 * pixel], a.ray_d[3 * pixel + 1], a.ray_d[3 * pixel + 2]);
+    }
+    const bool alive = inside && !(sqrtf(dot3(rd, rd)) == 0.0f);
+    RayResult r;
+    trace_rays<KB, false>(sc, k, ro, rd, 0.0f, 0.0f, alive, false, grads, hs, a.status, sh, nullptr, r);
+    if (alive) store_ray(a, k, grads, pixel, ro, rd, r);
+    else if (inside) a.head[pixel] = GRAY_NULL;
     return r.retraced;
 }
 
@@ -1473,7 +1529,7 @@ template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_kernel(const FwdArgs a) {
     __shared__ TileShared<KB, false> sh;
     if (*a.render_ellipsoids) return;  // the ellipsoid view (ellipsoid_kernel) renders this frame
-    forward_tile<KB, false, true>(a, blockIdx.x, blockIdx.y, 0, sh);
+    forward_tile<KB, false, kSingles>(a, blockIdx.x, blockIdx.y, 0, sh);
 }
 
 // Persistent launch: the blocks take tiles from the schedule's order, densest first, until none is
@@ -1506,7 +1562,7 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
         if (t >= items) break;
         const uint32_t tile = a.schedule[kSchedHeader + a.ntiles + t];
         const bool again =
-            forward_tile<KB, false, false>(a, (int)(tile % (uint32_t)a.tiles_x), (int)(tile / (uint32_t)a.tiles_x), 0, sh);
+            forward_tile<KB, false, kCamera>(a, (int)(tile % (uint32_t)a.tiles_x), (int)(tile / (uint32_t)a.tiles_x), 0, sh);
         if ((threadIdx.x & 31) == 0) {
             atomicAdd(&s_packets, 1u);
             if (again) atomicAdd(&s_retraced, 1u);
@@ -1519,10 +1575,48 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_sched_kernel(
     grid_wait_before();
 }
 
-// The split tiles' packets (see sched_order_kernel), and every tile of a forward on the caller's rays; launched before the kernel of the whole tiles, which
-// starts as soon as this one's blocks have and fills what they leave free.  A kernel of its own: with
-// both bodies in one, the whole tiles' loop lost registers (3M / 1080p 2.28 to 2.33 ms with a run-time
-// switch, 2.44 ms with two inlined bodies, 2.40 ms with a call).
+// The tiles whose rays, the caller's, are traversed one by one (kRayTile): a warp traces a packet.  The last of a
+// forward's kernels: without such tiles its blocks leave at once, which costs the camera's frames nothing
+// there (as the first, 500k / 640x480 336 to 344 us).  A block begins with the four packets of one tile (so that a few tiles spread over all SMs), and its
+// warps then take the next packets each by itself, so that none waits for its tile's slowest.  The packets
+// have 32 hit slots at four blocks per SM, whatever trace_variant says: origins of their own, with 16 or 32
+// slots as for the camera's rays at six or four blocks and these, 19 000 Gaussians in a box / 256x200 752 and
+// 661 us, 100k / 160x120 433 and 361, 100k / 1280x720 606 and 599, shuffled 9.25 and 9.36 ms (five blocks:
+// 707, 391, 588 us, 8.9 ms, but 16x16 rays over 1M 3.36 to 3.53 ms).
+constexpr int kRaySlots = 32, kRayBlocks = 4;
+
+template <int KB, int MINB>
+__global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_rays_kernel(const FwdArgs a) {
+    __shared__ RayShared<KB> sh;
+    grid_launch_next();
+    if (*a.render_ellipsoids || !*a.rays_from_python || a.schedule[kSchedRays] == 0u) {
+        grid_wait_before();
+        return;
+    }
+    const uint32_t packets = kWarps * a.schedule[kSchedRays];
+    const int lane = threadIdx.x & 31;
+    uint32_t traced = 0u, retraced = 0u;
+    for (uint32_t q = blockIdx.x * kWarps + (threadIdx.x >> 5); q < packets;) {
+        const uint32_t tile = a.schedule[kSchedHeader + 2 * a.ntiles - 1 - q / kWarps];
+        const bool again = forward_ray_packet<KB>(a, (int)(tile % (uint32_t)a.tiles_x),
+                                                  (int)(tile / (uint32_t)a.tiles_x), (int)(q % kWarps), sh);
+        traced++;
+        retraced += again ? 1u : 0u;
+        if (lane == 0) q = gridDim.x * kWarps + atomicAdd(a.schedule + kSchedRayNext, 1u);
+        q = __shfl_sync(kFull, q, 0);
+    }
+    if (lane == 0 && traced > 0u) {
+        atomicAdd(&a.schedule[kStatPackets], traced);
+        atomicAdd(&a.schedule[kStatRetraced], retraced);
+    }
+    grid_wait_before();
+}
+
+// The split tiles' packets (see sched_order_kernel), and the tiles of the caller's rays that are traversed
+// together; launched before the kernel of the whole tiles, which starts as soon as this one's blocks have
+// and fills what they leave free.  A kernel of its own: with both bodies in one, the whole tiles' loop lost
+// registers (3M / 1080p 2.28 to 2.33 ms with a run-time switch, 2.44 ms with two inlined bodies, 2.40 ms
+// with a call).
 template <int KB, int MINB>
 __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(const FwdArgs a) {
     __shared__ TileShared<KB, true> sh;
@@ -1546,12 +1640,12 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(
         bool again;
         if (t < items) {
             const uint32_t item = a.schedule[kSchedHeader + 2 * a.ntiles + t], tile = item & kItemTile;
-            again = forward_tile<KB, true, true>(a, (int)(tile % (uint32_t)a.tiles_x),
-                                                 (int)(tile / (uint32_t)a.tiles_x), (int)(item >> kItemShift), sh);
+            again = forward_tile<KB, true, kCones>(a, (int)(tile % (uint32_t)a.tiles_x),
+                                                   (int)(tile / (uint32_t)a.tiles_x), (int)(item >> kItemShift), sh);
         } else {
             const uint32_t tile = a.schedule[kSchedHeader + a.ntiles + t - items];
-            again = forward_tile<KB, false, true>(a, (int)(tile % (uint32_t)a.tiles_x),
-                                                  (int)(tile / (uint32_t)a.tiles_x), 0, whole_sh);
+            again = forward_tile<KB, false, kCones>(a, (int)(tile % (uint32_t)a.tiles_x),
+                                                    (int)(tile / (uint32_t)a.tiles_x), 0, whole_sh);
         }
         if ((threadIdx.x & 31) == 0 && (threadIdx.x == 0 || t >= items)) {
             atomicAdd(&s_packets, 1u);
@@ -1580,9 +1674,10 @@ __global__ void __launch_bounds__(kFwdThreads, MINB) trace_forward_split_kernel(
 // super-tile's entries, testing each entry's own box against the tile's frustum, instead of from the
 // root.  Every leaf a ray of the tile can hit lies under an entry of the super-tile (its ancestors
 // meet the tile's frustum, hence the super-tile's), so the tile still reaches it.  Schedule words:
-// [0..3] work counters and lengths, [kSchedHeader, +ntiles) estimates, [kSchedHeader + ntiles, +ntiles)
-// order of the whole tiles, [kSchedHeader + 2 ntiles, +4 ntiles) of the split tiles' packets, then (when frontiers are on) kFrontierWords words per tile, then
-// kSuperWords words per super-tile.
+// [0..5] work counters and lengths, [kSchedHeader, +ntiles) estimates, [kSchedHeader + ntiles, +ntiles) order of
+// the whole tiles and, from its end backwards, the tiles of single rays, [kSchedHeader + 2 ntiles, +4 ntiles) the
+// split tiles' packets, then (when frontiers are on) kFrontierWords words per tile, then kSuperWords words per
+// super-tile.
 // ---------------------------------------------------------------------------------------------
 constexpr int kCostCut = 512;
 constexpr int kCostStack = 512;  // (a super-tile's entries and what their walk pushes)
@@ -1908,31 +2003,45 @@ __global__ void __launch_bounds__(32) super_cost_kernel(const FwdArgs a, int bw,
     frontier_walk<true>(a.nodes, n, kSuperCut, fs, &ss, out, nullptr);
 }
 
+// The tiles of the caller's rays are traversed together when their rays share a cone (ray_cone), over more than
+// a few Gaussians; the others' estimate is kRayTile.  Without candidates to speak of, one by one is faster: 64
+// Gaussians / 64x64 40 us and 49 (105 when every tile was walked), 200 / 1280x720 126 us and 161, 400 / 1280x720
+// 1.00 to 1.07 times.
+constexpr int kTogetherIdle = 128, kTogetherLoaded = 512;
+
 __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int bw, int bh) {
     __shared__ FrontierScratch fs;
     __shared__ ConicBasis cb;
     const int tile = blockIdx.x, lane = threadIdx.x;
     uint32_t *out = a.frontier ? a.frontier + (size_t)tile * kFrontierWords : nullptr;
-    uint32_t est = 0;
     const int n = a.n;
-    const int x0 = (tile % a.tiles_x) * bw, y0 = (tile / a.tiles_x) * bh;
-    const int x1 = min(x0 + bw, (int)a.render_w) - 1, y1 = min(y0 + bh, (int)a.render_h) - 1;
-    bool walk = !*a.render_ellipsoids && n > 1;
-    if (walk && *a.rays_from_python) {
-        walk = ray_cone<32>(a.ray_o, a.ray_d, a.alloc_w, a.root_box, x0, y0, x1, y1, fs.fr, cb, nullptr);
-    } else if (walk) {
-        make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
-    }
+    bool walk = !*a.render_ellipsoids && n > 1, single = false;
     if (walk) {
-        const uint32_t *seed = nullptr;
-        if (a.super_frontier) {
-            const int sx = (tile % a.tiles_x) / kSuperTiles, sy = (tile / a.tiles_x) / kSuperTiles;
-            seed = a.super_frontier + (size_t)(sy * a.super_x + sx) * kSuperWords;
+        const int x0 = (tile % a.tiles_x) * bw, y0 = (tile / a.tiles_x) * bh;
+        const int x1 = min(x0 + bw, (int)a.render_w) - 1, y1 = min(y0 + bh, (int)a.render_h) - 1;
+        if (*a.rays_from_python) {
+            const bool loaded = 2 * a.ntiles > a.slots_split;
+            walk = n > (loaded ? kTogetherLoaded : kTogetherIdle) &&
+                   ray_cone<32>(a.ray_o, a.ray_d, a.alloc_w, a.root_box, x0, y0, x1, y1, fs.fr, cb, nullptr);
+            single = !walk;
+        } else {
+            make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
         }
-        est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut, fs, nullptr,
-                                   out, seed);
     }
-    if (!walk && out && lane == 0) out[0] = kFrontierNone;
+    if (!walk) {
+        if (lane == 0) {
+            if (out) out[0] = kFrontierNone;
+            a.schedule[kSchedHeader + tile] = single ? kRayTile : 0u;
+        }
+        return;
+    }
+    const uint32_t *seed = nullptr;
+    if (a.super_frontier) {
+        const int sx = (tile % a.tiles_x) / kSuperTiles, sy = (tile / a.tiles_x) / kSuperTiles;
+        seed = a.super_frontier + (size_t)(sy * a.super_x + sx) * kSuperWords;
+    }
+    const uint32_t est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut,
+                                              fs, nullptr, out, seed);
     if (lane == 0) a.schedule[kSchedHeader + tile] = est;
 }
 
@@ -1956,19 +2065,21 @@ constexpr uint32_t kSplitLeast = 96;
 constexpr int kSplitBlocks = 4;  // blocks per SM of the split kernel
 
 __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sched, int ntiles, int slots_narrow,
-                                                                    int slots_wide) {
+                                                                    int slots_wide, int slots_split,
+                                                                    const uint8_t *rays_from_python) {
     __shared__ unsigned long long s_sum[32];
-    __shared__ uint32_t s_bucket[2 * kOrderBuckets];  // whole tiles, then split ones
+    __shared__ uint32_t s_bucket[2 * kOrderBuckets + 1];  // whole tiles, then split ones; tiles of single rays
     __shared__ uint32_t s_split;
     const int t = threadIdx.x, lane = t & 31;
     const uint32_t *est = sched + kSchedHeader;
+    const bool given = *rays_from_python;
     unsigned long long sum = 0ull;
 #pragma unroll 8
-    for (int i = t; i < ntiles; i += kOrderThreads) sum += est[i];
+    for (int i = t; i < ntiles; i += kOrderThreads) sum += est[i] != kRayTile ? est[i] : 0u;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
     if (lane == 0) s_sum[t >> 5] = sum;
-    if (t < 2 * kOrderBuckets) s_bucket[t] = 0u;
+    if (t <= 2 * kOrderBuckets) s_bucket[t] = 0u;
     __syncthreads();
     if (t == 0) {
         const uint32_t packets = sched[kStatPackets], retraced = sched[kStatRetraced];
@@ -1984,9 +2095,13 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
         sched[kStatRetraced] = 0u;
         sched[0] = 0u;
         sched[kSchedSplitNext] = 0u;
+        sched[kSchedRayNext] = 0u;
         unsigned long long total = 0ull;
         for (int w = 0; w < kOrderThreads / 32; w++) total += s_sum[w];
-        const unsigned long long slots = (unsigned long long)(choice == kChoiceWide ? slots_wide : slots_narrow);
+        // (the split kernel has all tiles of the caller's rays)
+        const unsigned long long slots = (unsigned long long)(given                   ? slots_split
+                                                              : choice == kChoiceWide ? slots_wide
+                                                                                      : slots_narrow);
         const unsigned long long thr = total * kSplitEighths / (8ull * (slots > 0ull ? slots : 1ull));
         s_split = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
     }
@@ -2006,9 +2121,10 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
             const uint32_t e = ahead[0];
 #pragma unroll
             for (int j = 0; j + 1 < kOrderAhead; j++) ahead[j] = ahead[j + 1];
-            const bool four = e > split;
-            const uint32_t key = i < ntiles ? (uint32_t)__clz((int)e) + (four ? (uint32_t)kOrderBuckets : 0u)
-                                            : 2u * kOrderBuckets;  // dense first
+            const bool single = e == kRayTile, four = e > split && !single;
+            const uint32_t key = i >= ntiles ? 2u * kOrderBuckets + 1u
+                                 : single    ? 2u * kOrderBuckets
+                                             : (uint32_t)__clz((int)e) + (four ? (uint32_t)kOrderBuckets : 0u);  // dense first
             const uint32_t peers = __match_any_sync(kFull, key);
             const int lead = __ffs((int)peers) - 1;
             uint32_t base = 0u;
@@ -2016,7 +2132,9 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
             base = __shfl_sync(kFull, base, lead) + __popc(peers & ((1u << lane) - 1u));
             if (pass == 1 && i < ntiles) {
                 uint32_t *out = sched + kSchedHeader + ntiles;
-                if (four) {
+                if (single) {
+                    out[ntiles - 1 - (int)base] = (uint32_t)i;  // (the whole tiles' order fills from the front)
+                } else if (four) {
                     out += ntiles + 4u * base;
                     for (uint32_t s = 0; s < 4u; s++) out[s] = (uint32_t)i | s << kItemShift;
                 } else {
@@ -2033,6 +2151,10 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
                 acc += c;
             }
             sched[t == 0 ? kSchedItems : kSchedSplitItems] = t == 0 ? acc : 4u * acc;
+        }
+        if (pass == 0 && t == 2) {
+            sched[kSchedRays] = s_bucket[2 * kOrderBuckets];
+            s_bucket[2 * kOrderBuckets] = 0u;
         }
         __syncthreads();
     }
@@ -2212,9 +2334,10 @@ __device__ __forceinline__ void ellipsoid_pixel(const FwdArgs &a, int px, int py
 // Grid-stride over 16x8-pixel tiles (a few blocks per SM): the launch made on every forward costs
 // little when the view is off.
 __global__ void __launch_bounds__(kEllTileX * kEllTileY) ellipsoid_kernel(const FwdArgs a, int tiles_x, int ntiles) {
-    if (!*a.render_ellipsoids) return;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
-        ellipsoid_pixel(a, (t % tiles_x) * kEllTileX + threadIdx.x, (t / tiles_x) * kEllTileY + threadIdx.y);
+    if (*a.render_ellipsoids)
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x)
+            ellipsoid_pixel(a, (t % tiles_x) * kEllTileX + threadIdx.x, (t / tiles_x) * kEllTileY + threadIdx.y);
+    grid_wait_before();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -2450,7 +2573,7 @@ static FwdArgs forward_args(const gray_params &p, bool display) {
     a.status = p.status;
     a.render_ellipsoids = p.config.render_ellipsoids;
     a.ellipsoid_min_opacity = p.config.ellipsoid_min_opacity;
-    a.slots_narrow = a.slots_wide = 1;
+    a.slots_split = 1;
     a.tile_w = 8;
     a.tile_h = 4;
     a.schedule = nullptr;
@@ -2466,13 +2589,25 @@ cudaError_t launch_ellipsoids(const gray_params &p, bool display, cudaStream_t s
     const int tiles_x = (int)((p.render_width + kEllTileX - 1) / kEllTileX);
     const int ntiles = tiles_x * (int)((p.render_height + kEllTileY - 1) / kEllTileY);
     if (ntiles <= 0) return cudaSuccess;
-    int dev = 0, sms = 0;
+    int sms = 0, per_sm = 0;
     cudaError_t e;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    const int grid = ntiles < 8 * sms ? ntiles : 8 * sms;
-    ellipsoid_kernel<<<grid, dim3(kEllTileX, kEllTileY), 0, s>>>(a, tiles_x, ntiles);
-    return cudaGetLastError();
+    if ((e = resident_blocks(reinterpret_cast<const void *>(&ellipsoid_kernel), kEllTileX * kEllTileY, 0, &sms,
+                             &per_sm)) != cudaSuccess)
+        return e;
+    // the last of the forward's programmatic launches: what it reads was there before the chain's first
+    int tx = tiles_x, nt = ntiles;
+    FwdArgs args_a = a;
+    void *args[] = {&args_a, &tx, &nt};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ntiles < 8 * sms ? ntiles : 8 * sms);
+    cfg.blockDim = dim3(kEllTileX, kEllTileY);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void *>(&ellipsoid_kernel), args);
 }
 
 // Launch shape of one forward: the kernel arguments, the trace kernel and its grid, and whether the
@@ -2550,7 +2685,8 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
             const int sy = ((int)q.grid.y + kSuperTiles - 1) / kSuperTiles;
             const size_t used =
                 (size_t)kSchedHeader + (size_t)(1 + kOrderPerTile + kFrontierWords) * (size_t)a.ntiles;
-            if (used + (size_t)sx * (size_t)sy * kSuperWords <= words) {
+            // (in a small tree they leave the tiles' walks two levels to save, and are a launch more)
+            if (a.n > (int)(4 * kSuperCut) && used + (size_t)sx * (size_t)sy * kSuperWords <= words) {
                 a.super_frontier = a.frontier + (size_t)a.ntiles * kFrontierWords;
                 a.super_x = sx;
                 q.nsuper = sx * sy;
@@ -2567,19 +2703,20 @@ cudaError_t launch_trace_schedule(const gray_params &p, bool display, cudaStream
     if (!q.sched) return cudaSuccess;
     // densest tiles first: per-tile estimate and frontier, then the work order
     FwdArgs a = q.a;
-    const void *kerns[2] = {q.kern, q.kern_wide ? q.kern_wide : q.kern};
-    int slots[2] = {0, 0};
-    for (int i = 0; i < 2; i++) {
+    const void *kerns[3] = {q.kern, q.kern_wide ? q.kern_wide : q.kern,
+                            reinterpret_cast<const void *>(&trace_forward_split_kernel<16, kSplitBlocks>)};
+    int slots[3] = {0, 0, 0};
+    for (int i = 0; i < 3; i++) {
         int sms = 0, per_sm = 0;
         const cudaError_t e = resident_blocks(kerns[i], kFwdThreads, 0, &sms, &per_sm);
         if (e != cudaSuccess) return e;
         slots[i] = sms * per_sm;
     }
-    a.slots_narrow = slots[0];
-    a.slots_wide = slots[1];
+    a.slots_split = slots[2];
     if (q.nsuper > 0) super_cost_kernel<<<q.nsuper, 32, 0, s>>>(a, q.bw, q.bh, q.nsuper);
     tile_cost_kernel<<<a.ntiles, 32, 0, s>>>(a, q.bw, q.bh);
-    sched_order_kernel<<<1, kOrderThreads, 0, s>>>(a.schedule, a.ntiles, a.slots_narrow, a.slots_wide);
+    sched_order_kernel<<<1, kOrderThreads, 0, s>>>(a.schedule, a.ntiles, slots[0], slots[1], slots[2],
+                                                   a.rays_from_python);
     return cudaGetLastError();
 }
 
@@ -2592,13 +2729,15 @@ cudaError_t launch_trace_forward(const gray_params &p, bool display, bool schedu
         return cudaGetLastError();
     }
     if (!schedule_ready && (e = launch_trace_schedule(p, display, s)) != cudaSuccess) return e;
-    // persistent grids that take the split tiles' packets and the whole tiles in the schedule's order; with
-    // the automatic choice both kernels of the whole tiles are launched and the one not chosen returns
-    // at once.  The chain's second and third launch are programmatic: they run beside the one before.
-    const void *kerns[3] = {reinterpret_cast<const void *>(&trace_forward_split_kernel<16, kSplitBlocks>), q.kern,
-                            q.kern_wide};
-    const int roles[3] = {0, q.kern_wide ? (int)kChoiceNarrow : 0, (int)kChoiceWide};
-    for (int i = 0; i < 3 && kerns[i]; i++) {
+    // persistent grids that take the split tiles' packets, the whole tiles in the schedule's order and the single
+    // rays' packets; with the automatic choice both kernels of the whole tiles are launched and the one not
+    // chosen returns at once.  All but the chain's first are programmatic: they run beside the one before.
+    const void *kerns[4] = {reinterpret_cast<const void *>(&trace_forward_split_kernel<16, kSplitBlocks>), q.kern,
+                            q.kern_wide,
+                            reinterpret_cast<const void *>(&trace_forward_rays_kernel<kRaySlots, kRayBlocks>)};
+    const int roles[4] = {0, q.kern_wide ? (int)kChoiceNarrow : 0, (int)kChoiceWide, 0};
+    for (int i = 0; i < 4; i++) {
+        if (!kerns[i]) continue;
         int sms = 0, per_sm = 0;
         if ((e = resident_blocks(kerns[i], kFwdThreads, 0, &sms, &per_sm)) != cudaSuccess) return e;
         const unsigned int want = (unsigned int)(sms * per_sm);

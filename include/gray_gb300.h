@@ -179,6 +179,8 @@ typedef struct gray_params {
      * from the previous scheduled forward of the same schedule buffer (the 32-key one when more than
      * 10/128 of its packets needed a second traversal with 16 keys, 1/128 in a small frame); both
      * kernels are launched and the one not chosen returns at once.
+     * On the caller's rays (rays_from_python) only the packet shape and the frontier apply: tiles whose rays
+     * share an origin and a cone have 16 keys, the other tiles' rays, traversed one by one, 32.
      * Results are identical for every variant; only speed differs. */
     int32_t trace_variant;
 } gray_params;
