@@ -413,8 +413,9 @@ struct ConicBasis {
     float v0[3], du[3], dv[3];
     float hx, hy;  // largest |x| and |y| of the tile
     float mag;     // V
-    // rays from the caller (ray_cone): their common origin, and the axis and centre of their cone
-    float origin[3], axis[3], ca, cb;
+    // rays from the caller (ray_cone): their common origin, the axis and centre of their cone, and how many of
+    // the tile's pixels have one
+    float origin[3], axis[3], ca, cb, share;
 };
 
 // (a.x * b.x + c.x, a.y * b.y + c.y), each rounded once: one issue slot for two FMAs.
@@ -1341,6 +1342,7 @@ __device__ __noinline__ bool ray_cone(const float *__restrict__ ray_o, const flo
         cb.hx = 0.5f * (a1 - a0);
         cb.hy = 0.5f * (b1 - b0);
         cb.mag = 2.0f * (1.0f + fmaxf(fabsf(a0), fabsf(a1)) + fmaxf(fabsf(b0), fabsf(b1)));
+        cb.share = (float)rays / (float)count;
     }
     __syncwarp();
     return true;
@@ -1692,6 +1694,7 @@ struct FrontierScratch {
     uint32_t stk[kCostStack];
     float key[kFrontierSort];
     uint32_t val[kFrontierSort];
+    int entries;  // of val that the last walk filled
 };
 
 // What the super-tile walk also keeps of each frontier entry.
@@ -1947,6 +1950,7 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
         __syncwarp();
     }
     if (stop) est += pending;
+    if (lane == 0) fs.entries = min(nf, kFrontierSort);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) est += __shfl_xor_sync(kFull, est, off);
     if (!out) return est;
@@ -2003,15 +2007,73 @@ __global__ void __launch_bounds__(32) super_cost_kernel(const FwdArgs a, int bw,
     frontier_walk<true>(a.nodes, n, kSuperCut, fs, &ss, out, nullptr);
 }
 
-// The tiles of the caller's rays are traversed together when their rays share a cone (ray_cone), over more than
-// a few Gaussians; the others' estimate is kRayTile.  Without candidates to speak of, one by one is faster: 64
-// Gaussians / 64x64 40 us and 49 (105 when every tile was walked), 200 / 1280x720 126 us and 161, 400 / 1280x720
+// Whether the Gaussians that the rays in cb's cone may hit are met by fewer than `least` of them on average:
+// each lane follows one of the walk's frontier entries down to a Gaussian and compares its extent, seen
+// from the rays' origin, with the cone's; up to three times more while the answer is within a factor of two.
+// Not inlined: its registers would cost the walks of the camera's tiles (1M Gaussians, 64x64 537 to 543 us).
+__device__ __noinline__ bool sparse_tile(const float4 *__restrict__ nodes, const float4 *__restrict__ l2w, int n,
+                                         const FrontierScratch &fs, const ConicBasis &cb, float least) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    const int entries = fs.entries, take = min(entries, 32);
+    float sum = 0.0f, found = 0.0f;
+    for (int round = 0; round < 4; round++) {
+        uint32_t link = lane < take ? fs.val[(4 * lane + round) * entries / (4 * take)] : GRAY_NULL;
+        for (int guard = 0; guard < 64 && !(link & GRAY_LEAF_BIT); guard++) {
+            if (link >= (uint32_t)(n - 1)) {
+                link = GRAY_NULL;
+                break;
+            }
+            const float4 q0 = nodes[4 * (size_t)link], q1 = nodes[4 * (size_t)link + 1],
+                         q2 = nodes[4 * (size_t)link + 2], q3 = nodes[4 * (size_t)link + 3];
+            const float b0min[3] = {q0.x, q0.y, q0.z}, b0max[3] = {q0.w, q1.x, q1.y};
+            const float b1min[3] = {q1.z, q1.w, q2.x}, b1max[3] = {q2.y, q2.z, q2.w};
+            const bool p0 = frustum_box(fs.fr, b0min, b0max), p1 = frustum_box(fs.fr, b1min, b1max);
+            const bool second = p0 && p1 ? (((lane ^ (7 * round)) >> (guard % 5)) & 1) != 0 : p1;
+            link = !(p0 || p1) ? GRAY_NULL : __float_as_uint(second ? q3.y : q3.x);
+        }
+        const uint32_t gid = link & ~GRAY_LEAF_BIT;
+        const bool on = link != GRAY_NULL && (link & GRAY_LEAF_BIT) && gid < (uint32_t)n;
+        float met = 0.0f;
+        if (on) {
+            const float4 r0 = l2w[3 * (size_t)gid], r1 = l2w[3 * (size_t)gid + 1], r2 = l2w[3 * (size_t)gid + 2];
+            const float size = (2.0f / 3.0f) * (norm_approx(mk3(r0.x, r0.y, r0.z)) + norm_approx(mk3(r1.x, r1.y, r1.z)) +
+                                                norm_approx(mk3(r2.x, r2.y, r2.z)));
+            const float z = (r0.w - cb.origin[0]) * cb.axis[0] + (r1.w - cb.origin[1]) * cb.axis[1] +
+                            (r2.w - cb.origin[2]) * cb.axis[2];
+            const float seen = z > size ? size / z : 1.0f;
+            met = cb.share * (float)kFwdThreads * fminf(1.0f, seen / (2.0f * cb.hx)) * fminf(1.0f, seen / (2.0f * cb.hy));
+            met = fminf(met, 4.0f * least);  // (a few near or large ones say little of the rest)
+        }
+        found += (float)__popc(__ballot_sync(kFull, on));
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) met += __shfl_xor_sync(kFull, met, off);
+        sum += met;
+        if (!(sum > 0.5f * least * found && sum < 2.0f * least * found)) break;
+    }
+    return sum < least * found;
+}
+
+// Which tiles of the caller's rays are traversed together: those whose rays share a cone (ray_cone), over more than a
+// few Gaussians, unless the candidates are many and met by few of the rays (rays all over the view in any
+// order, thumbnails, 16x16 rays for a whole scene).  The others' estimate is kRayTile.  A tile's time grows with its
+// candidates, est; that of its rays one by one with the hits and more slowly.  Measured, rays met per
+// candidate, est, together against one by one:
+//   tiles that fill the SMs: 0.02, 7e3: 3.1 and 2.3 ms; 0.37, 2e4: 58 and 43; 0.05, 3.5e4: 15.0 and 6.9;
+//     0.08, 3.5e5: 364 and 35; 0.7 (0.2 to 17), 2e3: 0.17 and 0.57
+//   few tiles: 0.014, 7e3: 0.14 and 0.29; 0.05, 3.5e4: 0.30 and 0.73; 0.015, 6.5e4: 1.3 and 0.76; 0.08,
+//     3.5e5: 2.8 and 4.8; 0.03, 6.5e5: 15 and 4.1; 0.11, 1e6: 8.3 and 10.9
+// so the line is at 2.7e-3 and 1.1e-4 sqrt(est) rays.  Without candidates to speak of, one by one is faster:
+// 64 Gaussians / 64x64 40 us and 49 (105 when every tile was walked), 200 / 1280x720 126 us and 161, 400 / 1280x720
 // 1.00 to 1.07 times.
 constexpr int kTogetherIdle = 128, kTogetherLoaded = 512;
+constexpr uint32_t kSparseFrom = 512;
+constexpr float kSparseIdle = 1.2e-8f, kSparseLoaded = 7.2e-6f;  // squares of the factors
 
 __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int bw, int bh) {
     __shared__ FrontierScratch fs;
     __shared__ ConicBasis cb;
+    __shared__ float s_sparse;  // factor of the caller's rays, 0 for the camera's (in no register over the walk)
     const int tile = blockIdx.x, lane = threadIdx.x;
     uint32_t *out = a.frontier ? a.frontier + (size_t)tile * kFrontierWords : nullptr;
     const int n = a.n;
@@ -2021,10 +2083,12 @@ __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int 
         const int x1 = min(x0 + bw, (int)a.render_w) - 1, y1 = min(y0 + bh, (int)a.render_h) - 1;
         if (*a.rays_from_python) {
             const bool loaded = 2 * a.ntiles > a.slots_split;
+            if (lane == 0) s_sparse = loaded ? kSparseLoaded : kSparseIdle;
             walk = n > (loaded ? kTogetherLoaded : kTogetherIdle) &&
                    ray_cone<32>(a.ray_o, a.ray_d, a.alloc_w, a.root_box, x0, y0, x1, y1, fs.fr, cb, nullptr);
             single = !walk;
         } else {
+            if (lane == 0) s_sparse = 0.0f;
             make_tile_frustum(a, x0, y0, x1, y1, fs.fr);
         }
     }
@@ -2040,8 +2104,11 @@ __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int 
         const int sx = (tile % a.tiles_x) / kSuperTiles, sy = (tile / a.tiles_x) / kSuperTiles;
         seed = a.super_frontier + (size_t)(sy * a.super_x + sx) * kSuperWords;
     }
-    const uint32_t est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut,
-                                              fs, nullptr, out, seed);
+    uint32_t est = frontier_walk<false>(a.nodes, n, a.frontier_cut > 0 ? a.frontier_cut : (uint32_t)kCostCut, fs,
+                                        nullptr, out, seed);
+    const float factor = *(volatile float *)&s_sparse;
+    if (factor > 0.0f && est > kSparseFrom && sparse_tile(a.nodes, a.l2w, n, fs, cb, sqrt_approx((float)est * factor)))
+        est = kRayTile;
     if (lane == 0) a.schedule[kSchedHeader + tile] = est;
 }
 

@@ -22,7 +22,10 @@ def _cuda(gray_lib):
 def _rays(kind, W, H, distance, rng):
     i, j = np.meshgrid(np.arange(W), np.arange(H))
     o = np.tile(np.array([0.1, -distance, 0.2], np.float32), (W * H, 1))
-    x, y = 0.5 * W / H * (2 * (i + 0.5) / W - 1), 0.5 * (2 * (j + 0.5) / H - 1)
+    if kind == "mosaic":  # thumbnails of 16x16 rays, each of the whole view
+        x, y = 0.5 * (2 * (i % 16 + 0.5) / 16 - 1), 0.5 * (2 * (j % 16 + 0.5) / 16 - 1)
+    else:
+        x, y = 0.5 * W / H * (2 * (i + 0.5) / W - 1), 0.5 * (2 * (j + 0.5) / H - 1)
     d = np.stack([x, np.ones_like(x), -y], -1).reshape(-1, 3)
     d /= np.linalg.norm(d, axis=-1, keepdims=True)
     if kind == "shuffled":  # every tile's rays all over the view
@@ -52,9 +55,12 @@ def _scene(kind, n):
     ("small", 1500, (45, 39), "shuffled", "none"),
     ("clustered", 60_000, (64, 48), "pinhole", "none"),
     ("clustered", 60_000, (64, 48), "origins", "all"),
+    ("clustered", 60_000, (64, 48), "shuffled", "all"),
+    ("clustered", 60_000, (192, 256), "mosaic", "all"),
 ])
 def test_routes_of_supplied_rays(oracle, scene, n, size, kind, single):
-    """Tiny scenes and rays with origins of their own go one by one."""
+    """Tiny scenes, origins of their own and tiles that few of their rays' candidates are met in (rays of a
+    clustered scene shuffled over the view, or thumbnails) go one by one."""
     W, H = size
     sc, distance = _scene(scene, n)
     chan = np.random.default_rng(n).uniform(0, 1, (n, 3)).astype(np.float32)
