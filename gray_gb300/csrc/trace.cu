@@ -2132,7 +2132,7 @@ constexpr uint32_t kSplitLeast = 96;
 constexpr int kSplitBlocks = 4;  // blocks per SM of the split kernel
 
 __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sched, int ntiles, int slots_narrow,
-                                                                    int slots_wide, int slots_split,
+                                                                    int slots_wide, int slots_split, int never_split,
                                                                     const uint8_t *rays_from_python) {
     __shared__ unsigned long long s_sum[32];
     __shared__ uint32_t s_bucket[2 * kOrderBuckets + 1];  // whole tiles, then split ones; tiles of single rays
@@ -2171,6 +2171,7 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
                                                                                       : slots_narrow);
         const unsigned long long thr = total * kSplitEighths / (8ull * (slots > 0ull ? slots : 1ull));
         s_split = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
+        if (never_split) s_split = 0xffffffffu;
     }
     __syncthreads();
     const uint32_t split = s_split;
@@ -2685,7 +2686,7 @@ struct FwdPlan {
     const void *kern_wide;  // automatic choice: the wide kernel, launched after `kern` (else null)
     dim3 grid;
     int bw, bh;
-    bool sched;
+    bool sched, split;  // split: dense tiles may be traced as their four packets
     int nsuper;  // super-tiles whose coarse frontiers seed the tile walks (0: tiles walk from the root)
 };
 
@@ -2702,7 +2703,7 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     FwdArgs &a = q.a;
     a = forward_args(p, display);
     // variant: bits 0-1 select (buffer size, register cap), bit 2 the packet shape, bits 3-4 the
-    // tile frontier's cut (64 leaves, 32, 128, no frontier); bit 5 is accepted and has no effect
+    // tile frontier's cut (64 leaves, 32, 128, no frontier), bit 5 leaves dense tiles whole
     // variant 0 (the default) chooses between the narrow and the wide kernel of kDefaultTraceVariant's
     // packet shape and cut from the last scheduled forward's re-traversals: the 16-slot hit buffer with
     // five blocks per SM (4, 5, 6: 3.08, 2.83, 2.91 ms on the benchmark's training view at 3M / 1080p; six leave
@@ -2711,6 +2712,7 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     const bool automatic = p.trace_variant <= 0;
     const int v = p.trace_variant > 0 ? p.trace_variant : kDefaultTraceVariant;
     const int fcut = (v >> 3) & 3;
+    q.split = (v & 32) == 0;
     q.kern_wide = nullptr;
     a.tile_w = (v & 4) ? 4 : 8;
     a.tile_h = 32 / a.tile_w;
@@ -2783,7 +2785,7 @@ cudaError_t launch_trace_schedule(const gray_params &p, bool display, cudaStream
     if (q.nsuper > 0) super_cost_kernel<<<q.nsuper, 32, 0, s>>>(a, q.bw, q.bh, q.nsuper);
     tile_cost_kernel<<<a.ntiles, 32, 0, s>>>(a, q.bw, q.bh);
     sched_order_kernel<<<1, kOrderThreads, 0, s>>>(a.schedule, a.ntiles, slots[0], slots[1], slots[2],
-                                                   a.rays_from_python);
+                                                   q.split ? 0 : 1, a.rays_from_python);
     return cudaGetLastError();
 }
 

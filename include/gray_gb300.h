@@ -172,8 +172,8 @@ typedef struct gray_params {
     int32_t *status; /* device int32, GRAY_STATUS_* bits */
     /* forward-trace kernel variant: bits 0-1 = physical hit buffer of 32 or 16 keys and register
      * cap, bit 2 = 8x4 or 4x8 pixel packets, bits 3-4 = where a pixel tile's traversals start (BVH
-     * nodes of at most 64, 32 or 128 leaves that the tile's frustum reaches, or the root), bit 5 is
-     * accepted and has no effect.
+     * nodes of at most 64, 32 or 128 leaves that the tile's frustum reaches, or the root), bit 5
+     * leaves dense tiles whole (else they are traced as their four packets, with 16 keys).
      * 0 (default): 4x8 packets from frontiers of 16, 32 or 64 leaves (by the Gaussian count), with the
      * 16-key buffer (five blocks per SM) or the 32-key one (four blocks per SM) chosen on the device
      * from the previous scheduled forward of the same schedule buffer (the 32-key one when more than
