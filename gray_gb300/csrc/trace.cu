@@ -73,17 +73,16 @@ constexpr uint32_t kChoiceNarrow = 1u, kChoiceWide = 2u;
 // none do (100k / 320x240, 64 Gaussians / 256x256).
 constexpr uint32_t kWideLarge = 10u, kWideSmall = 1u;
 constexpr int kWideTiles = 8;
-// Per pixel tile, the BVH frontier its frustum reaches (kFrontierWords words: count, then up to
-// kFrontierMax node or leaf entries); a count of kFrontierNone means "start at the root".  A frontier
-// goes onto the traversal stack, so it leaves room there for the traversal's own pushes.
+// Per pixel tile, or group of a batch, kFrontierWords words: the BVH frontier its frustum reaches (a count, then
+// up to kFrontierMax node or leaf entries), and three that a batch uses: the group's estimate and, in slot
+// i, entry i of the batch's work order (in slot 0 also whether there is one).  A count of kFrontierNone
+// means "start at the root".  A frontier goes onto the traversal stack, so it leaves room there for the
+// traversal's own pushes.
 constexpr int kFrontierWords = GRAY_FRONTIER_WORDS;
-constexpr int kFrontierMax = kFrontierWords - 1;
-// A batch's groups keep a few words less: the last ones of a slot hold the group's estimate and, in slot i,
-// entry i of the batch's work order (slot 0 also whether there is one).
-constexpr int kBatchFrontierMax = kFrontierMax - 3;
+constexpr int kFrontierMax = kFrontierWords - 4;
+constexpr uint32_t kFrontierNone = 0xFFFFFFFFu;
 constexpr int kBatchOrdered = kFrontierWords - 3, kBatchEst = kFrontierWords - 2, kBatchOrder = kFrontierWords - 1;
 constexpr int kFrontierSort = 256;  // sort buffer of the frontier walk (a power of two > kFrontierMax)
-constexpr uint32_t kFrontierNone = 0xFFFFFFFFu;
 constexpr int kFrontierCutDefault = 64;  // frontier nodes hold at most this many leaves
 
 struct FwdArgs {
@@ -1777,7 +1776,7 @@ __device__ __forceinline__ void frontier_sort_out(const FrontierScratch &fs, int
 // kFrontierNone when they do not fit.
 template <bool SUPER>
 __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, uint32_t cut, FrontierScratch &fs,
-                                               SuperScratch *ss, uint32_t *out, const uint32_t *seed, int most = kFrontierMax) {
+                                               SuperScratch *ss, uint32_t *out, const uint32_t *seed) {
     const int lane = threadIdx.x & 31;
     const uint32_t lanemask_lt = (1u << lane) - 1u;
     const Frustum &fr = fs.fr;
@@ -1838,7 +1837,7 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
     for (int guard = 0; sp > 0; guard++) {
         // a popped node frees its entry and pushes at most two
         const int take = min(min(sp, 32), kCostStack - sp);
-        if (guard >= 4096 || nf > (SUPER ? kSuperMax : most) || take <= 0) {
+        if (guard >= 4096 || nf > (SUPER ? kSuperMax : kFrontierMax) || take <= 0) {
             complete = false;
             stop = true;
             break;
@@ -1969,7 +1968,7 @@ __device__ __forceinline__ uint32_t frontier_walk(const float4 *nodes, int n, ui
         }
         return est;
     }
-    if (complete && nf <= most) {
+    if (complete && nf <= kFrontierMax) {
         if (nf <= 32) frontier_sort_out<1>(fs, nf, out);
         else if (nf <= 64) frontier_sort_out<2>(fs, nf, out);
         else if (nf <= 128) frontier_sort_out<4>(fs, nf, out);
@@ -2443,7 +2442,7 @@ __global__ void __launch_bounds__(32) batch_frontier_kernel(const gray_batch_sce
     make_frustum_warp(fs.fr, mk3(vw.origin[0], vw.origin[1], vw.origin[2]), vw.w2c, vw.fov_y, x0, y0, x1, y1, vw.width,
                       vw.height, bs.root_box);
     const uint32_t est = frontier_walk<false>(reinterpret_cast<const float4 *>(bs.nodes), bs.n, cut, fs, nullptr, out,
-                                              nullptr, kBatchFrontierMax);
+                                              nullptr);
     if (lane == 0) out[kBatchEst] = est;
 }
 

@@ -216,9 +216,10 @@ typedef struct gray_batch_view {
 uint32_t gray_batch_packets(uint32_t width, uint32_t height, int32_t variant);
 
 /* Frontier groups (2x2 packets) of a width x height view for a kernel variant; a batch's frontier
- * buffer holds GRAY_FRONTIER_WORDS words per group of all its views. */
+ * buffer holds GRAY_FRONTIER_WORDS words per group of all its views (a count, up to 160 BVH nodes, and
+ * three words of the batch's work order). */
 uint32_t gray_batch_groups(uint32_t width, uint32_t height, int32_t variant);
-#define GRAY_FRONTIER_WORDS 161
+#define GRAY_FRONTIER_WORDS 164
 uint32_t gray_frontier_words(void);
 
 /* Per-view colours of one scene: live values (as forward_pass_display) and, when enable_sh, the SH
