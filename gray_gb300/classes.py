@@ -34,16 +34,6 @@ def _p(t: torch.Tensor | None) -> int | None:
     return None if t is None else t.data_ptr()
 
 
-def _as_float32(v) -> bool:
-    """A Python number whose magnitude a float32 holds (infinities and NaN among them)."""
-    return isinstance(v, (int, float)) and (v != v or abs(v) <= FLOAT32_MAX or abs(v) == math.inf)
-
-
-def _is_plain(t: torch.Tensor, shape: tuple, device) -> bool:
-    return (tuple(t.shape) == shape and t.dtype == torch.float32 and t.device == device and t.is_contiguous()
-            and not t.is_neg())
-
-
 class CameraDataHolder:
     """cuda/core/camera.h:39-77"""
 
@@ -450,8 +440,15 @@ class Raytracer:
         c = self.camera_data
         # the launch takes numbers that a float32 holds (a tensor's would have to be waited for) and the pose's
         # own float32 memory; fill_ and copy_ take or refuse the rest
-        if not (all(_as_float32(v) for v in (vertical_fov_radians, znear, zfar))
-                and _is_plain(c2w_origin, (3,), self.device) and _is_plain(c2w_rotation, (3, 3), self.device)):
+        plain = True
+        for v in (vertical_fov_radians, znear, zfar):
+            if not (isinstance(v, (float, int)) and (abs(v) <= FLOAT32_MAX or v != v or abs(v) == math.inf)):
+                plain = False
+        for t, shape in ((c2w_origin, (3,)), (c2w_rotation, (3, 3))):
+            if (t.shape != shape or t.dtype != torch.float32 or t.device != self.device or not t.is_contiguous()
+                    or t.is_neg()):
+                plain = False
+        if not plain:
             c.vertical_fov_radians.fill_(vertical_fov_radians)
             c.znear.fill_(znear)
             c.zfar.fill_(zfar)
