@@ -22,7 +22,7 @@
 //   their tile's origin within a cone (ray_cone), go the same way; other rays from the caller, and
 //   tiles whose traversal overflows the shared stack, take a per-ray slab traversal instead.
 // Backward (cuda/backward_pass.cu:2-142): one thread per pixel walks its segments back to front,
-//   recomputes alpha in fp32 and reduces the 16 per-hit gradient values into the per-Gaussian
+//   recomputes alpha in fp32 and adds the hit's 14 gradient sums and its count to the per-Gaussian
 //   accumulator: lanes holding the same Gaussian combine in a tree, and the lowest issues four
 //   16-byte vector reductions.
 #include "gray_device.cuh"
@@ -2116,35 +2116,88 @@ __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int 
 // forward from the last scheduled forward's packet counts (the narrow kernel when there are none yet).
 //
 // Dense tiles are split.  A tile whose estimate exceeds kSplitEighths / 8 of what the resident blocks
-// have to do on average (the sum of the estimates over the blocks resident at once) would still run when
+// have to do on average (the sum of the estimates over the blocks resident at once) may still run when
 // the others are done: it is entered as its four packets, each traced by a block whose four warps share
-// its candidates (merge_split).  Below kSplitLeast leaves a tile is too short for that to pay.
-// Measured (render 500k / 640x480 and train step 301k / 799x533, us; unsplit 662 and 842, the longest
-// tile taking 2.7 times what the blocks had to do on average): 2/8 512 and 903, 3/8 490 and 840, 5/8 497
-// and 818, 8/8 560 and 818.  Split, a tile costs more (all of them split: 3M / 1080p 2.27 -> 5.09 ms), so
-// large frames, whose average is far above any tile, split none.
+// its candidates (merge_split).  Below kSplitLeast leaves a tile is too short for that to pay.  Split, a
+// tile costs more (all of them split: 3M / 1080p 2.27 -> 5.09 ms), so of many such tiles only the densest
+// are: with up to slots / 4 tiles (a tile or so per SM) all; with up to slots, all if they are at most slots / 3,
+// else about slots / 12 (split_limit); with more, about slots / 8.  "About": a quarter octave of estimates
+// is split or left together, so that a frame of tiles alike is left whole.  Measured over 144 frames (10 scenes
+// of 1000 to 3M Gaussians, 160x120 to 1920x1080, seen from outside and within), each with 2 to 13 thresholds:
+// this rule is 2.7% (geometric mean) and at most 15% above the best threshold, splitting all candidates 11%
+// and 91%, none 15% and 144%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243, 420 (all
+// candidates) 322; 500k / 640x480 none 394, 32 379, 64 286, 169 324, all 559; 3M / 480x360 none 2061, 32
+// 1040, 64 907, 218 915.
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderAhead = 8;
 constexpr int kOrderBuckets = 33;  // leading zeros of an estimate
 constexpr unsigned long long kSplitEighths = 5;
 constexpr uint32_t kSplitLeast = 96;
+constexpr int kSplitBuckets = 128;  // four per octave of an estimate
+
+__device__ __forceinline__ int split_bucket(uint32_t e) {  // e >= kSplitLeast
+    const int octave = 31 - __clz((int)e);
+    return 4 * octave + (int)((e >> (octave - 2)) & 3u);
+}
+
+// Of `candidates` tiles above the threshold, how many may be split.
+__device__ __forceinline__ uint32_t split_limit(uint32_t candidates, uint32_t ntiles, uint32_t slots) {
+    if (ntiles <= slots / 4u) return candidates;
+    if (ntiles <= slots) return candidates <= slots / 3u ? candidates : slots / 12u;
+    return slots / 8u;
+}
+
+// The lowest bucket edge with at most `limit` candidates from it on (counts: candidates per bucket), less one;
+// 0xffffffff if the densest bucket holds more.  One warp.
+__device__ __forceinline__ uint32_t split_above(const uint32_t *counts, uint32_t limit) {
+    const int lane = threadIdx.x & 31, first = kSplitBuckets - 4 - 4 * lane;  // the densest in lane 0
+    const uint32_t own = counts[first] + counts[first + 1] + counts[first + 2] + counts[first + 3];
+    uint32_t from = own;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t v = __shfl_up_sync(kFull, from, off);
+        if (lane >= off) from += v;
+    }
+    from -= own;  // candidates of the denser lanes
+    uint32_t edge = 0xffffffffu;
+#pragma unroll
+    for (int j = 3; j >= 0; j--) {
+        const int b = first + j;
+        from += counts[b];
+        if (counts[b] > 0u && from <= limit) edge = ((uint32_t)(4 + (b & 3)) << (b / 4 - 2)) - 1u;
+    }
+    return __reduce_min_sync(kFull, edge);
+}
+
 constexpr int kSplitBlocks = 4;  // blocks per SM of the split kernel
 
 __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sched, int ntiles, int slots_narrow,
                                                                     int slots_wide, int slots_split, int never_split,
                                                                     const uint8_t *rays_from_python) {
     __shared__ unsigned long long s_sum[32];
+    __shared__ uint32_t s_max[32], s_dense[kSplitBuckets], s_candidates, s_slots;
     __shared__ uint32_t s_bucket[2 * kOrderBuckets + 1];  // whole tiles, then split ones; tiles of single rays
     __shared__ uint32_t s_split;
     const int t = threadIdx.x, lane = t & 31;
     const uint32_t *est = sched + kSchedHeader;
     const bool given = *rays_from_python;
     unsigned long long sum = 0ull;
+    uint32_t most = 0u;
 #pragma unroll 8
-    for (int i = t; i < ntiles; i += kOrderThreads) sum += est[i] != kRayTile ? est[i] : 0u;
+    for (int i = t; i < ntiles; i += kOrderThreads) {
+        const uint32_t e = est[i] != kRayTile ? est[i] : 0u;
+        sum += e;
+        most = max(most, e);
+    }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(kFull, sum, off);
-    if (lane == 0) s_sum[t >> 5] = sum;
+    most = __reduce_max_sync(kFull, most);
+    if (lane == 0) {
+        s_sum[t >> 5] = sum;
+        s_max[t >> 5] = most;
+    }
+    if (t < kSplitBuckets) s_dense[t] = 0u;
+    if (t == 0) s_candidates = 0u;
     if (t <= 2 * kOrderBuckets) s_bucket[t] = 0u;
     __syncthreads();
     if (t == 0) {
@@ -2169,11 +2222,31 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
                                                               : choice == kChoiceWide ? slots_wide
                                                                                       : slots_narrow);
         const unsigned long long thr = total * kSplitEighths / (8ull * (slots > 0ull ? slots : 1ull));
-        s_split = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
-        if (never_split) s_split = 0xffffffffu;
+        uint32_t densest = 0u;
+        for (int w = 0; w < kOrderThreads / 32; w++) densest = max(densest, s_max[w]);
+        const uint32_t above = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
+        s_split = never_split || densest <= above ? 0xffffffffu : above;
+        s_slots = (uint32_t)slots;
     }
     __syncthreads();
-    const uint32_t split = s_split;
+    uint32_t split = s_split;
+    if (split != 0xffffffffu) {
+        for (int i0 = 0; i0 < ntiles; i0 += kOrderThreads) {
+            const uint32_t e = i0 + t < ntiles ? est[i0 + t] : 0u;
+            const bool dense = e > split && e != kRayTile;
+            if (dense) atomicAdd(&s_dense[split_bucket(e)], 1u);
+            const uint32_t c = (uint32_t)__popc(__ballot_sync(kFull, dense));
+            if (lane == 0 && c > 0u) atomicAdd(&s_candidates, c);
+        }
+        __syncthreads();
+        if (t < 32) {
+            const uint32_t limit = split_limit(s_candidates, (uint32_t)ntiles, s_slots);
+            if (s_candidates > limit) split = split_above(s_dense, limit);
+            if (t == 0) s_split = split;
+        }
+        __syncthreads();
+        split = s_split;
+    }
     for (int pass = 0; pass < 2; pass++) {
         // pass 0 counts the buckets' tiles, pass 1 writes them; the lanes of a warp that fall in one
         // bucket share an atomic
@@ -2704,7 +2777,7 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     // variant: bits 0-1 select (buffer size, register cap), bit 2 the packet shape, bits 3-4 the
     // tile frontier's cut (64 leaves, 32, 128, no frontier), bit 5 leaves dense tiles whole
     // variant 0 (the default) chooses between the narrow and the wide kernel of kDefaultTraceVariant's
-    // packet shape and cut from the last scheduled forward's re-traversals: the 16-slot hit buffer with
+    // packet shape, with automatic_cut's frontiers, from the last scheduled forward's re-traversals: the 16-slot hit buffer with
     // five blocks per SM (4, 5, 6: 3.08, 2.83, 2.91 ms on the benchmark's training view at 3M / 1080p; six leave
     // 80 registers, with twice the spills) is faster where few rays composite more than 16 hits, the 32-slot one with
     // four blocks where many do (a re-traversal repeats the packet's whole traversal)

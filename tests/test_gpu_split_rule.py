@@ -1,0 +1,58 @@
+"""Which tiles a forward enters as split packets: the schedule's counts against the rule computed from its own
+estimates.  Needs a GB300."""
+import numpy as np
+import pytest
+import torch
+
+from gray_gb300 import synthetic
+from tests import gpu_util as G
+
+pytestmark = pytest.mark.gpu
+
+HEADER, WHOLE, SPLIT, CHOICE = 64, 1, 3, 50
+
+
+def expected_split(est, slots):
+    """The number of tiles that are split."""
+    est = np.asarray(est, np.int64)
+    above = max(96, int(est.sum()) * 5 // (8 * slots))
+    dense = np.sort(est[est > above])[::-1]
+    limit = slots // 8
+    if est.size <= slots // 4:
+        limit = dense.size
+    elif est.size <= slots:
+        limit = dense.size if dense.size <= slots // 3 else slots // 12
+    if dense.size <= limit:
+        return dense.size
+    octave = np.floor(np.log2(dense)).astype(np.int64)
+    edge = (dense >> (octave - 2)) << (octave - 2)  # the lower edge of each one's quarter octave
+    return max((int((dense >= e).sum()) for e in edge if (dense >= e).sum() <= limit), default=0)
+
+
+@pytest.mark.parametrize("scene,n,size,distance", [
+    ("small", 1000, (160, 120), 2.2), ("small", 10_000, (160, 120), 4.0), ("small", 10_000, (320, 240), 2.2),
+    ("small", 10_000, (320, 240), 4.0), ("small", 10_000, (640, 480), 4.0), ("small", 3000, (480, 360), 2.2),
+    ("clustered", 200_000, (160, 120), 8.0), ("clustered", 200_000, (320, 240), 8.0),
+    ("clustered", 200_000, (640, 480), 8.0), ("clustered", 500_000, (480, 360), 8.0),
+    ("clustered", 500_000, (1280, 720), 8.0)])
+def test_split_tiles_follow_the_rule(gray_lib, scene, n, size, distance):
+    """Few tiles, as many as resident blocks, more; tiles alike (none split) and a few dense ones."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    W, H = size
+    sc = synthetic.clustered_scene(n, seed=3) if scene == "clustered" else synthetic.small_scene(seed=n, n=n)
+    rt = G.make_tracer(W, H, sc.mean, sc.rotation, sc.scale, sc.opacity, inference_only=True,
+                       channels=np.zeros((sc.n, 3), np.float32))
+    cam = synthetic.look_at((0.6 * distance, -0.8 * distance, 0.2), (0, 0, 0), (0, 0, 1), 0.9, W, H)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tiles = -(-W // 8) * -(-H // 16)
+    for variant, slots in ((0, None), (7, 5 * sms), (5, 4 * sms), (32 + 7, 0)):
+        rt.set_trace_variant(variant)
+        rt.set_view(cam.origin_cuda(), cam.rotation_c2w_blender_cuda(), cam.fov_y, 0.0, 99999.9)
+        for _ in range(2):
+            rt.forward_pass_display()
+        words = rt.schedule[:HEADER + tiles].cpu().tolist()
+        if slots is None:
+            slots = (4 if words[CHOICE] == 2 else 5) * sms
+        want = expected_split(words[HEADER:], slots) if slots else 0
+        assert words[SPLIT] == 4 * want and words[WHOLE] == tiles - want, (variant, want, words[SPLIT] // 4)
