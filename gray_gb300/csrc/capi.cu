@@ -166,7 +166,7 @@ bool side_stream(SideStream *out) {
 }
 
 // forward_prep (live values, colours) and the tile schedule (per-tile BVH frontier and work order,
-// from the BVH and the camera only) read and write disjoint state: the schedule runs on the side
+// from the BVH and the camera or the caller's rays only) read and write disjoint state: the schedule runs on the side
 // stream between a fork and a join event while forward_prep runs on s, and the trace follows both.
 int forward(const gray_params *p, bool display, int grads, cudaStream_t s) {
     SideStream side;

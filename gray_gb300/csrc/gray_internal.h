@@ -47,7 +47,7 @@ constexpr size_t sort_tmp_words(int n) {
 // trace.cu
 // display: forward_pass_display (colour only; no hit lists or saved state, whatever grads_enabled holds)
 // the forward's tile schedule (per-tile work estimate and BVH frontier, densest-first order); it
-// reads only the BVH and the camera, so it may run on another stream than forward_prep
+// reads only the BVH and the camera or the caller's rays, so it may run on another stream than forward_prep
 bool trace_forward_has_schedule(const gray_params &p);
 cudaError_t launch_trace_schedule(const gray_params &p, bool display, cudaStream_t s);
 // schedule_ready: launch_trace_schedule has been issued for this forward (and ordered before s)
