@@ -2119,15 +2119,16 @@ __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int 
 // have to do on average (the sum of the estimates over the blocks resident at once) may still run when
 // the others are done: it is entered as its four packets, each traced by a block whose four warps share
 // its candidates (merge_split).  Below kSplitLeast leaves a tile is too short for that to pay.  Split, a
-// tile costs more (all of them split: 3M / 1080p 2.27 -> 5.09 ms), so of many such tiles only the densest
-// are: with up to slots / 4 tiles (a tile or so per SM) all; with up to slots, all if they are at most slots / 3,
-// else about slots / 12 (split_limit); with more, about slots / 8.  "About": a quarter octave of estimates
-// is split or left together, so that a frame of tiles alike is left whole.  Measured over 144 frames (10 scenes
-// of 1000 to 3M Gaussians, 160x120 to 1920x1080, seen from outside and within), each with 2 to 13 thresholds:
-// this rule is 2.7% (geometric mean) and at most 15% above the best threshold, splitting all candidates 11%
-// and 91%, none 15% and 144%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243, 420 (all
-// candidates) 322; 500k / 640x480 none 394, 32 379, 64 286, 169 324, all 559; 3M / 480x360 none 2061, 32
-// 1040, 64 907, 218 915.
+// tile costs more (all of them split: 3M / 1080p 2.27 -> 5.09 ms), so all such tiles are only in frames of up
+// to slots / 4 tiles (a tile or so per SM) and where the densest has kSplitSteep times the average: the
+// others are done long before it.  Else the densest are, about slots / 12 in a frame of up to slots tiles
+// and slots / 8 in a larger one.  "About": a quarter octave of estimates is split or left together, so that a
+// frame of tiles alike is left whole.  Measured over 173 frames (scenes of 1000 to 3M Gaussians, 89x69 to
+// 3840x2160, seen from outside and within), each with 2 to 13 thresholds: this rule is 2.7% (geometric mean)
+// and at most 15% above the best threshold and never above splitting all candidates, which is 10% and 91%
+// above it; none split is 15% and 144%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243, all
+// 420 candidates 322; 500k / 640x480 none 394, 32 379, 64 286, 169 324, all tiles 559; 1.9M / 260x349 (the
+// densest 5.4 times the average) none 2154, 64 1179, 304 656.
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderAhead = 8;
 constexpr int kOrderBuckets = 33;  // leading zeros of an estimate
@@ -2140,12 +2141,7 @@ __device__ __forceinline__ int split_bucket(uint32_t e) {  // e >= kSplitLeast
     return 4 * octave + (int)((e >> (octave - 2)) & 3u);
 }
 
-// Of `candidates` tiles above the threshold, how many may be split.
-__device__ __forceinline__ uint32_t split_limit(uint32_t candidates, uint32_t ntiles, uint32_t slots) {
-    if (ntiles <= slots / 4u) return candidates;
-    if (ntiles <= slots) return candidates <= slots / 3u ? candidates : slots / 12u;
-    return slots / 8u;
-}
+constexpr unsigned long long kSplitSteep = 5;
 
 // The lowest bucket edge with at most `limit` candidates from it on (counts: candidates per bucket), less one;
 // 0xffffffff if the densest bucket holds more.  One warp.
@@ -2175,7 +2171,7 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
                                                                     int slots_wide, int slots_split, int never_split,
                                                                     const uint8_t *rays_from_python) {
     __shared__ unsigned long long s_sum[32];
-    __shared__ uint32_t s_max[32], s_dense[kSplitBuckets], s_candidates, s_slots;
+    __shared__ uint32_t s_max[32], s_dense[kSplitBuckets], s_candidates, s_limit;
     __shared__ uint32_t s_bucket[2 * kOrderBuckets + 1];  // whole tiles, then split ones; tiles of single rays
     __shared__ uint32_t s_split;
     const int t = threadIdx.x, lane = t & 31;
@@ -2226,7 +2222,9 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
         for (int w = 0; w < kOrderThreads / 32; w++) densest = max(densest, s_max[w]);
         const uint32_t above = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
         s_split = never_split || densest <= above ? 0xffffffffu : above;
-        s_slots = (uint32_t)slots;
+        const uint32_t n = (uint32_t)ntiles, places = (uint32_t)slots;
+        s_limit = n <= places / 4u || densest * slots >= kSplitSteep * total ? 0xffffffffu
+                                                                             : places / (n <= places ? 12u : 8u);
     }
     __syncthreads();
     uint32_t split = s_split;
@@ -2240,8 +2238,7 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
         }
         __syncthreads();
         if (t < 32) {
-            const uint32_t limit = split_limit(s_candidates, (uint32_t)ntiles, s_slots);
-            if (s_candidates > limit) split = split_above(s_dense, limit);
+            if (s_candidates > s_limit) split = split_above(s_dense, s_limit);
             if (t == 0) s_split = split;
         }
         __syncthreads();
@@ -2801,9 +2798,9 @@ static FwdPlan plan_forward(const gray_params &p, bool display) {
     (!q.sched ? reinterpret_cast<const void *>(&trace_forward_kernel<KB, MINB>)                     \
               : reinterpret_cast<const void *>(&trace_forward_sched_kernel<KB, MINB>))
     switch (v & 3) {
-        case 0: q.kern = GRAY_FWD_KERNEL(32, 1); break;
+        case 0: q.kern = GRAY_FWD_KERNEL(32, 3); break;
         case 1: q.kern = GRAY_FWD_KERNEL(32, 4); break;
-        case 2: q.kern = GRAY_FWD_KERNEL(16, 1); break;
+        case 2: q.kern = GRAY_FWD_KERNEL(16, 3); break;
         default: q.kern = GRAY_FWD_KERNEL(16, 5); break;
     }
 #undef GRAY_FWD_KERNEL

@@ -17,11 +17,9 @@ def expected_split(est, slots):
     est = np.asarray(est, np.int64)
     above = max(96, int(est.sum()) * 5 // (8 * slots))
     dense = np.sort(est[est > above])[::-1]
-    limit = slots // 8
-    if est.size <= slots // 4:
+    limit = slots // 12 if est.size <= slots else slots // 8
+    if est.size <= slots // 4 or int(est.max()) * slots >= 5 * int(est.sum()):
         limit = dense.size
-    elif est.size <= slots:
-        limit = dense.size if dense.size <= slots // 3 else slots // 12
     if dense.size <= limit:
         return dense.size
     octave = np.floor(np.log2(dense)).astype(np.int64)
@@ -34,9 +32,10 @@ def expected_split(est, slots):
     ("small", 10_000, (320, 240), 4.0), ("small", 10_000, (640, 480), 4.0), ("small", 3000, (480, 360), 2.2),
     ("clustered", 200_000, (160, 120), 8.0), ("clustered", 200_000, (320, 240), 8.0),
     ("clustered", 200_000, (640, 480), 8.0), ("clustered", 500_000, (480, 360), 8.0),
-    ("clustered", 500_000, (1280, 720), 8.0)])
+    ("clustered", 500_000, (1280, 720), 8.0), ("clustered", 1_000_000, (320, 240), 12.0)])
 def test_split_tiles_follow_the_rule(gray_lib, scene, n, size, distance):
-    """Few tiles, as many as resident blocks, more; tiles alike (none split) and a few dense ones."""
+    """Few tiles, as many as resident blocks, more; tiles alike (none split), a few dense ones, one far denser
+    than the average."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     W, H = size
