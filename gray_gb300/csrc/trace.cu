@@ -2122,13 +2122,13 @@ __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int 
 // tile costs more (all of them split: 3M / 1080p 2.27 -> 5.09 ms), so all such tiles are only in frames of up
 // to slots / 4 tiles (a tile or so per SM) and where the densest has kSplitSteep times the average: the
 // others are done long before it.  Else the densest are, about slots / 12 in a frame of up to slots tiles
-// and slots / 8 in a larger one.  "About": a quarter octave of estimates is split or left together, so that a
-// frame of tiles alike is left whole.  Measured over 173 frames (scenes of 1000 to 3M Gaussians, 89x69 to
-// 3840x2160, seen from outside and within), each with 2 to 13 thresholds: this rule is 2.7% (geometric mean)
-// and at most 15% above the best threshold and never above splitting all candidates, which is 10% and 91%
-// above it; none split is 15% and 144%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243, all
-// 420 candidates 322; 500k / 640x480 none 394, 32 379, 64 286, 169 324, all tiles 559; 1.9M / 260x349 (the
-// densest 5.4 times the average) none 2154, 64 1179, 304 656.
+// and slots / 6 in a larger one.  "About": a quarter octave of estimates is split or left together, so that a
+// frame of tiles alike is left whole.  Measured over 197 frames (scenes of 1000 to 3M Gaussians, 89x69 to
+// 3840x2160, seen from outside and within), each with 2 to 16 thresholds: this rule is 3.6% (geometric mean)
+// and at most 20% above the best threshold and at most 1% above splitting all candidates, which is 10% and
+// 91% above it; none split is 15% and 144%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243,
+// all 420 candidates 322; 500k / 640x480 none 394, 32 379, 64 286, 169 324, all tiles 559; 1.9M / 260x349
+// (the densest 5.4 times the average) none 2154, 64 1179, 304 656.
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderAhead = 8;
 constexpr int kOrderBuckets = 33;  // leading zeros of an estimate
@@ -2224,7 +2224,7 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
         s_split = never_split || densest <= above ? 0xffffffffu : above;
         const uint32_t n = (uint32_t)ntiles, places = (uint32_t)slots;
         s_limit = n <= places / 4u || densest * slots >= kSplitSteep * total ? 0xffffffffu
-                                                                             : places / (n <= places ? 12u : 8u);
+                                                                             : places / (n <= places ? 12u : 6u);
     }
     __syncthreads();
     uint32_t split = s_split;

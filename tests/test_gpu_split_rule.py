@@ -17,7 +17,7 @@ def expected_split(est, slots):
     est = np.asarray(est, np.int64)
     above = max(96, int(est.sum()) * 5 // (8 * slots))
     dense = np.sort(est[est > above])[::-1]
-    limit = slots // 12 if est.size <= slots else slots // 8
+    limit = slots // 12 if est.size <= slots else slots // 6
     if est.size <= slots // 4 or int(est.max()) * slots >= 5 * int(est.sum()):
         limit = dense.size
     if dense.size <= limit:
