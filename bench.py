@@ -440,14 +440,16 @@ def gpu_arm(a, rank, world, local_rank):
     dom_ms = res[dominant][0] / res[dominant][1]
     peak, peak_kind = measured_peak_gbs()
     achieved = algo.get(dominant, 0.0) / (dom_ms / 1000.0) / 1e9
-    # kernels behind one profiled scope: adam = step count + update; tile_schedule = super-tile walk +
-    # tile walk + work order (on the library's side stream, beside forward_prep), then trace_forward =
-    # the split tiles' kernel and the whole tiles': with the default variant the narrow and the wide
-    # one, one of which returns at once (the schedule is in trace_forward too when no side stream
-    # could be had); refit = block-local climb + upper tree.  Every other scope is one kernel.
-    traces = 3 if not a.trace_variant else 2
-    kernels_per_group = {"adam": 2, "refit": 2, "tile_schedule": 3,
-                         "trace_forward": traces if "tile_schedule" in res else 3 + traces}
+    # kernels behind one profiled scope: adam = step count + update; tile_schedule = super-tile walk (above
+    # 4096 Gaussians) + tile walk + work order (on the library's side stream, beside forward_prep), then
+    # trace_forward = the split tiles' kernel, the whole tiles' (with the default variant the narrow and
+    # the wide one, one of which returns at once) and the single rays' (the schedule is in trace_forward
+    # too when no side stream could be had); refit = block-local climb + upper tree.  Every other scope
+    # is one kernel.
+    traces = 4 if not a.trace_variant else 3
+    schedule = 3 if a.n_gaussians > 4096 else 2
+    kernels_per_group = {"adam": 2, "refit": 2, "tile_schedule": schedule,
+                         "trace_forward": traces if "tile_schedule" in res else schedule + traces}
     launches = sum(cnt * kernels_per_group.get(name, 1) for name, (_, cnt) in res.items())
     roofline = {"bound": "hbm", "kernel": dominant, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "peak_source": peak_kind,
