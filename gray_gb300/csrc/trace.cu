@@ -2062,12 +2062,12 @@ __device__ __noinline__ bool sparse_tile(const float4 *__restrict__ nodes, const
 //     0.08, 3.5e5: 364 and 35; 0.7 (0.2 to 17), 2e3: 0.17 and 0.57
 //   few tiles: 0.014, 7e3: 0.14 and 0.29; 0.05, 3.5e4: 0.30 and 0.73; 0.015, 6.5e4: 1.3 and 0.76; 0.08,
 //     3.5e5: 2.8 and 4.8; 0.03, 6.5e5: 15 and 4.1; 0.11, 1e6: 8.3 and 10.9
-// so the line is at 2.7e-3 and 1.1e-4 sqrt(est) rays.  Without candidates to speak of, one by one is faster:
+// so the line is at 3.2e-3 and 1.1e-4 sqrt(est) rays.  Without candidates to speak of, one by one is faster:
 // 64 Gaussians / 64x64 40 us and 49 (105 when every tile was walked), 200 / 1280x720 126 us and 161, 400 / 1280x720
 // 1.00 to 1.07 times.
 constexpr int kTogetherIdle = 128, kTogetherLoaded = 512;
 constexpr uint32_t kSparseFrom = 512;
-constexpr float kSparseIdle = 1.2e-8f, kSparseLoaded = 7.2e-6f;  // squares of the factors
+constexpr float kSparseIdle = 1.2e-8f, kSparseLoaded = 1.0e-5f;  // squares of the factors
 
 __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int bw, int bh) {
     __shared__ FrontierScratch fs;
@@ -2128,7 +2128,8 @@ __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int 
 // and at most 20% above the best threshold and at most 1% above splitting all candidates, which is 10% and
 // 91% above it; none split is 15% and 144%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243,
 // all 420 candidates 322; 500k / 640x480 none 394, 32 379, 64 286, 169 324, all tiles 559; 1.9M / 260x349
-// (the densest 5.4 times the average) none 2154, 64 1179, 304 656.
+// (the densest 5.4 times the average) none 2154, 64 1179, 304 656.  On the caller's rays up to slots / 2: whole,
+// their tiles have 16 hit slots, split 64 (160 thumbnail tiles over 1M: whole 30 ms, split 3).
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderAhead = 8;
 constexpr int kOrderBuckets = 33;  // leading zeros of an estimate
@@ -2223,7 +2224,7 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
         const uint32_t above = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
         s_split = never_split || densest <= above ? 0xffffffffu : above;
         const uint32_t n = (uint32_t)ntiles, places = (uint32_t)slots;
-        s_limit = n <= places / 4u || densest * slots >= kSplitSteep * total ? 0xffffffffu
+        s_limit = n <= places / (given ? 2u : 4u) || densest * slots >= kSplitSteep * total ? 0xffffffffu
                                                                              : places / (n <= places ? 12u : 6u);
     }
     __syncthreads();

@@ -55,3 +55,25 @@ def test_split_tiles_follow_the_rule(gray_lib, scene, n, size, distance):
             slots = (4 if words[CHOICE] == 2 else 5) * sms
         want = expected_split(words[HEADER:], slots) if slots else 0
         assert words[SPLIT] == 4 * want and words[WHOLE] == tiles - want, (variant, want, words[SPLIT] // 4)
+
+
+@pytest.mark.parametrize("size", [(160, 120), (320, 240)])
+def test_split_tiles_of_supplied_rays(gray_lib, size):
+    """Thumbnails, every tile alike: all split in a frame of up to two tiles per SM, none in a larger one."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    W, H = size
+    n = 10_000
+    sc = synthetic.small_scene(seed=n, n=n)
+    rt = G.make_tracer(W, H, sc.mean, sc.rotation, sc.scale, sc.opacity, inference_only=True,
+                       channels=np.zeros((n, 3), np.float32))
+    i, j = np.meshgrid(np.arange(W), np.arange(H))
+    x, y = 0.2 * (2 * (i % 16 + 0.5) / 16 - 1), 0.2 * (2 * (j % 16 + 0.5) / 16 - 1)
+    d = np.stack([x, np.ones_like(x), -y], -1).reshape(-1, 3)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    G.trace_rays(rt, np.tile(np.array([0.1, -3.5, 0.2]), (W * H, 1)), d, grads=False)
+    tiles = -(-W // 8) * -(-H // 16)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    words = rt.schedule[:HEADER + tiles].cpu().tolist()
+    assert words[4] == 0  # none one by one
+    assert words[SPLIT] == (4 * tiles if tiles <= 2 * sms else 0), (words[:6], min(words[HEADER:]), max(words[HEADER:]))
