@@ -2121,12 +2121,15 @@ __global__ void __launch_bounds__(32, 32) tile_cost_kernel(const FwdArgs a, int 
 // its candidates (merge_split).  Below kSplitLeast leaves a tile is too short for that to pay.  Split, a
 // tile costs more (all of them split: 3M / 1080p 2.27 -> 5.09 ms), so all such tiles are only in frames of up
 // to slots / 4 tiles (a tile or so per SM) and where the densest has kSplitSteep times the average: the
-// others are done long before it.  Else the densest are, about slots / 12 in a frame of up to slots tiles
+// others are done long before it.  Half that will do from kSplitLong leaves on, where the densest tile takes
+// about as long as such a frame and a block's share is some long tiles (5.5M / 357x204: at most 50 split 2439
+// us, all 1763; 200 000 in a box / 480x360, all alike and as dense: 17 split 3500, 450 4460).  Else the
+// densest are, about slots / 12 in a frame of up to slots tiles
 // and slots / 6 in a larger one.  "About": a quarter octave of estimates is split or left together, so that a
-// frame of tiles alike is left whole.  Measured over 197 frames (scenes of 1000 to 3M Gaussians, 89x69 to
-// 3840x2160, seen from outside and within), each with 2 to 16 thresholds: this rule is 3.6% (geometric mean)
-// and at most 20% above the best threshold and at most 1% above splitting all candidates, which is 10% and
-// 91% above it; none split is 15% and 144%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243,
+// frame of tiles alike is left whole.  Measured over 215 frames (scenes of 1000 to 5.5M Gaussians, 89x69 to
+// 3840x2160, seen from outside and within), each with 2 to 16 thresholds: this rule is 4.0% (geometric mean)
+// and at most 26% above the best threshold and at most 1% above splitting all candidates, which is 10% and
+// 91% above it; none split is 27% and 347%.  10 000 in a box / 640x480 from afar: none 191 us, 64 tiles 243,
 // all 420 candidates 322; 500k / 640x480 none 394, 32 379, 64 286, 169 324, all tiles 559; 1.9M / 260x349
 // (the densest 5.4 times the average) none 2154, 64 1179, 304 656.  On the caller's rays up to slots / 2: whole,
 // their tiles have 16 hit slots, split 64 (160 thumbnail tiles over 1M: whole 30 ms, split 3).
@@ -2143,6 +2146,7 @@ __device__ __forceinline__ int split_bucket(uint32_t e) {  // e >= kSplitLeast
 }
 
 constexpr unsigned long long kSplitSteep = 5;
+constexpr uint32_t kSplitLong = 16384;
 
 // The lowest bucket edge with at most `limit` candidates from it on (counts: candidates per bucket), less one;
 // 0xffffffff if the densest bucket holds more.  One warp.
@@ -2224,8 +2228,8 @@ __global__ void __launch_bounds__(kOrderThreads) sched_order_kernel(uint32_t *sc
         const uint32_t above = thr < kSplitLeast ? kSplitLeast : thr < 0xffffffffull ? (uint32_t)thr : 0xffffffffu;
         s_split = never_split || densest <= above ? 0xffffffffu : above;
         const uint32_t n = (uint32_t)ntiles, places = (uint32_t)slots;
-        s_limit = n <= places / (given ? 2u : 4u) || densest * slots >= kSplitSteep * total ? 0xffffffffu
-                                                                             : places / (n <= places ? 12u : 6u);
+        const bool steep = 2ull * densest * slots >= (densest >= kSplitLong ? kSplitSteep : 2ull * kSplitSteep) * total;
+        s_limit = n <= places / (given ? 2u : 4u) || steep ? 0xffffffffu : places / (n <= places ? 12u : 6u);
     }
     __syncthreads();
     uint32_t split = s_split;

@@ -18,7 +18,8 @@ def expected_split(est, slots):
     above = max(96, int(est.sum()) * 5 // (8 * slots))
     dense = np.sort(est[est > above])[::-1]
     limit = slots // 12 if est.size <= slots else slots // 6
-    if est.size <= slots // 4 or int(est.max()) * slots >= 5 * int(est.sum()):
+    steep = 5 if int(est.max()) >= 16384 else 10
+    if est.size <= slots // 4 or 2 * int(est.max()) * slots >= steep * int(est.sum()):
         limit = dense.size
     if dense.size <= limit:
         return dense.size
@@ -32,7 +33,8 @@ def expected_split(est, slots):
     ("small", 10_000, (320, 240), 4.0), ("small", 10_000, (640, 480), 4.0), ("small", 3000, (480, 360), 2.2),
     ("clustered", 200_000, (160, 120), 8.0), ("clustered", 200_000, (320, 240), 8.0),
     ("clustered", 200_000, (640, 480), 8.0), ("clustered", 500_000, (480, 360), 8.0),
-    ("clustered", 500_000, (1280, 720), 8.0), ("clustered", 1_000_000, (320, 240), 12.0)])
+    ("clustered", 500_000, (1280, 720), 8.0), ("clustered", 1_000_000, (320, 240), 12.0),
+    ("clustered", 3_000_000, (480, 360), 8.0)])
 def test_split_tiles_follow_the_rule(gray_lib, scene, n, size, distance):
     """Few tiles, as many as resident blocks, more; tiles alike (none split), a few dense ones, one far denser
     than the average."""
